@@ -822,15 +822,30 @@ constexpr int CO_THREADS = 256;
 constexpr uint32_t CO_CHUNK = 2048;  // centroids per step of the exact fallback
 
 // mu: the mean of up to 1,024 evenly spaced centroids (any shift is exact
-// for L2; the mean keeps the fp16 values small)
-__global__ void __launch_bounds__(CO_THREADS) coarse_mu_kernel(const float* __restrict__ cent, uint32_t nlist,
-                                                               uint32_t dim, float* __restrict__ mu) {
-  const uint32_t d = blockIdx.x * CO_THREADS + threadIdx.x;
-  if (d >= dim) return;
+// for L2; the mean keeps the fp16 values small). A block owns 32 dimensions
+// and 32 strided row groups, so a thread's chain is 32 additions with
+// independent loads: one thread per dimension over all 1,024 rows was a
+// single block bound by that serial chain (4,096 x 128: 525 us of a 2,085 us
+// search of 2,000 queries, now 1,584 us).
+constexpr int MU_ROWS = 32;
+__global__ void __launch_bounds__(32 * MU_ROWS) coarse_mu_kernel(const float* __restrict__ cent, uint32_t nlist,
+                                                                 uint32_t dim, float* __restrict__ mu) {
+  __shared__ float part[MU_ROWS][33];
+  const uint32_t lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const uint32_t d = blockIdx.x * 32 + lane;
   const uint32_t s = min(nlist, 1024u);
   float acc = 0.f;
-  for (uint32_t i = 0; i < s; ++i) acc += __ldg(cent + (size_t)((uint64_t)i * nlist / s) * dim + d);
-  mu[d] = acc / (float)s;
+  if (d < dim) {
+#pragma unroll 8
+    for (uint32_t i = g; i < s; i += MU_ROWS) acc += __ldg(cent + (size_t)((uint64_t)i * nlist / s) * dim + d);
+  }
+  part[g][lane] = acc;
+  __syncthreads();
+  if (g == 0 && d < dim) {
+    float sum = 0.f;
+    for (int r = 0; r < MU_ROWS; ++r) sum += part[r][lane];
+    mu[d] = sum / (float)s;
+  }
 }
 
 // One block per row: rows [0, nlist) are centroids -> fp16 (c - mu) padded to
@@ -1138,7 +1153,7 @@ static int launch_coarse_tc(const IvfPlan& Q, const IvfLaunch& L, uint8_t* scrat
   cudaError_t e = cudaMemsetAsync(flags, 0, (size_t)L.nq * 4, stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(cmax, 0, 4, stream);
   if (e != cudaSuccess) return (int)e;
-  coarse_mu_kernel<<<(L.dim + CO_THREADS - 1) / CO_THREADS, CO_THREADS, 0, stream>>>(L.centroids, L.nlist, L.dim, mu);
+  coarse_mu_kernel<<<(L.dim + 31) / 32, 32 * MU_ROWS, 0, stream>>>(L.centroids, L.nlist, L.dim, mu);
   coarse_prep_kernel<<<L.nlist + L.nq, 128, 0, stream>>>(L.centroids, L.nlist, L.queries, L.nq, L.dim, pd16, mu, c16,
                                                          cnorm, cmax, qc);
   note_launch(2);
