@@ -47,23 +47,110 @@ __device__ __forceinline__ uint16_t f32_to_f16_halfup(float x) {
   return (uint16_t)(sign | (uint16_t)(e << 10) | (uint16_t)(r >> 13));
 }
 
-__global__ void __launch_bounds__(256) encode_fp16_kernel(const float* __restrict__ x, uint32_t n, uint32_t dim,
-                                                          uint32_t pd, uint16_t* __restrict__ out,
-                                                          float* __restrict__ norms) {
-  const uint64_t row = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  const float* src = x + row * dim;
-  uint16_t* dst = out + row * pd;
-  for (uint32_t d = lane; d < pd; d += 32) dst[d] = d < dim ? f32_to_f16_halfup(__ldg(src + d)) : (uint16_t)0;
-  if (lane == 0 && norms) {
-    float s = 0.f;
-    for (uint32_t d = 0; d < dim; ++d) {
-      const float v = __ldg(src + d);
-      s = __fadd_rn(s, __fmul_rn(v, v));
-    }
-    norms[row] = s;
+// Four values at once: magnitudes in [2^-14, 65504 + rounding) share one
+// exponent shift, and a mantissa that rounds over carries into the exponent
+// (up to infinity) by itself; anything else takes the general conversion.
+__device__ __forceinline__ uint2 f32_to_f16_halfup4(float4 v) {
+  const uint32_t b[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
+  uint32_t h[4];
+  bool normal = true;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t a = (b[i] & 0x7fffffffu) - 0x38800000u;  // 113 << 23: the exponent of 2^-14
+    normal = normal && a < 0x0f000000u;                     // below 143 << 23: the exponent of 2^16
+    h[i] = ((a + 0x00801000u) >> 13) | ((b[i] >> 16) & 0x8000u);
   }
+  if (!normal) {
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+      const float f = i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
+      const uint32_t c = f32_to_f16_halfup(f);
+      h[0] = i == 0 ? c : h[0];
+      h[1] = i == 1 ? c : h[1];
+      h[2] = i == 2 ? c : h[2];
+      h[3] = i == 3 ? c : h[3];
+    }
+  }
+  return make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+}
+
+// A warp encodes 32 rows, 32 dimensions at a time: the chunk is read with
+// whole-row segments (128 bytes a row; 16-byte loads where VEC), converted
+// and stored, and its squares are transposed through shared memory so that
+// lane r adds row r's squares in dimension order. The next chunk's loads are
+// in flight meanwhile. ||x||^2 is a sequential fp32 sum, so the transposition
+// is what lets 32 rows advance together: with one lane per row reading its
+// row alone, 500,000 x 768 took 2,221 us (15% of the copy bandwidth).
+constexpr int E16_WARPS = 8;
+template <bool VEC>
+__global__ void __launch_bounds__(32 * E16_WARPS, 3) encode_fp16_kernel(const float* __restrict__ x, uint32_t n,
+                                                                     uint32_t dim, uint32_t pd,
+                                                                     uint16_t* __restrict__ out,
+                                                                     float* __restrict__ norms) {
+  __shared__ float sq[E16_WARPS][32][33];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint64_t row0 = ((uint64_t)blockIdx.x * E16_WARPS + warp) * 32;
+  if (row0 >= n) return;
+  const uint32_t rows = (uint32_t)min((uint64_t)32, n - row0);
+  float(*t)[33] = sq[warp];
+  float sum = 0.f;
+  if constexpr (VEC) {
+    const uint32_t r4 = lane >> 3, c4 = (lane & 7) * 4;  // load i: row 4 i + r4, columns c4..c4+3 of the chunk
+    float4 cur[8];
+    auto load = [&](uint32_t d0, float4 (&v)[8]) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t r = 4 * i + r4;
+        v[i] = (r < rows && d0 + c4 < dim)
+                   ? __ldg(reinterpret_cast<const float4*>(x + (row0 + r) * dim + d0 + c4))
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
+    load(0, cur);
+    for (uint32_t d0 = 0; d0 < pd; d0 += 32) {
+      float4 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = cur[i];
+      if (d0 + 32 < dim) load(d0 + 32, cur);
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t r = 4 * i + r4;
+        t[r][c4] = __fmul_rn(v[i].x, v[i].x);
+        t[r][c4 + 1] = __fmul_rn(v[i].y, v[i].y);
+        t[r][c4 + 2] = __fmul_rn(v[i].z, v[i].z);
+        t[r][c4 + 3] = __fmul_rn(v[i].w, v[i].w);
+        if (r < rows && d0 + c4 < pd) {
+          // dim is a multiple of 4: four columns in or out together
+          *reinterpret_cast<uint2*>(out + (row0 + r) * pd + d0 + c4) =
+              d0 + c4 < dim ? f32_to_f16_halfup4(v[i]) : make_uint2(0u, 0u);
+        }
+      }
+      __syncwarp();
+      const int m = d0 < dim ? (int)min(32u, dim - d0) : 0;
+      if (m == 32) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sum = __fadd_rn(sum, t[lane][j]);
+      } else {
+        for (int j = 0; j < m; ++j) sum = __fadd_rn(sum, t[lane][j]);
+      }
+    }
+  } else {
+    for (uint32_t d0 = 0; d0 < pd; d0 += 32) {
+      const uint32_t d = d0 + lane;
+      __syncwarp();
+#pragma unroll 8
+      for (uint32_t r = 0; r < rows; ++r) {
+        const float v = d < dim ? __ldg(x + (row0 + r) * dim + d) : 0.f;
+        t[r][lane] = __fmul_rn(v, v);
+        if (d < pd) out[(row0 + r) * pd + d] = d < dim ? f32_to_f16_halfup(v) : (uint16_t)0;
+      }
+      __syncwarp();
+      const int m = d0 < dim ? (int)min(32u, dim - d0) : 0;
+      for (int j = 0; j < m; ++j) sum = __fadd_rn(sum, t[lane][j]);
+    }
+  }
+  if (norms && lane < (int)rows) norms[row0 + lane] = sum;
 }
 
 // Neumaier accumulation of one term.
@@ -193,8 +280,13 @@ __global__ void __launch_bounds__(256) encode_fp8_per_vector_kernel(const float*
 int launch_encode_fp16(const float* x, uint32_t n, uint32_t dim, uint32_t pd, uint16_t* out, float* norms,
                        cudaStream_t stream) {
   if (n == 0) return 0;
-  const uint64_t blocks = ((uint64_t)n * 32 + 255) / 256;
-  encode_fp16_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, n, dim, pd, out, norms);
+  const uint64_t blocks = ((uint64_t)n + 32 * E16_WARPS - 1) / (32 * E16_WARPS);
+  // 16-byte loads and 8-byte stores where every row starts on such a boundary
+  const bool vec = dim % 4 == 0 && pd % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)out % 8 == 0;
+  if (vec)
+    encode_fp16_kernel<true><<<(unsigned)blocks, 32 * E16_WARPS, 0, stream>>>(x, n, dim, pd, out, norms);
+  else
+    encode_fp16_kernel<false><<<(unsigned)blocks, 32 * E16_WARPS, 0, stream>>>(x, n, dim, pd, out, norms);
   note_launch();
   return (int)cudaGetLastError();
 }
