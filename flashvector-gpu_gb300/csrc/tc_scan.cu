@@ -277,26 +277,61 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
     s.out[(size_t)q * s.k + r] = key_to_result(r < kp ? keys[r] : kSentinelKey, nullptr);
 }
 
-// Pre-pass result: per query, the distance of the r-th best key among the
-// sample's per-range heaps -- the query's admission bound for the full scan
-// (1e30, i.e. no bound, when the sample holds fewer than r admissible rows).
-__global__ void __launch_bounds__(128) tc_tau_kernel(const uint64_t* __restrict__ partial, uint32_t total,
-                                                     uint32_t pow2, uint32_t r, float* __restrict__ tau) {
-  extern __shared__ uint64_t keys[];
-  __shared__ uint32_t n_live;
-  const uint32_t q = blockIdx.x;
-  const uint64_t* src = partial + (size_t)q * total;
-  const uint32_t live = block_compact_keys(src, total, keys, &n_live);
-  if (live < r) {
-    // fewer than r sampled keys: no bound
-    if (threadIdx.x == 0) tau[q] = kSentinelDist;
-    return;
+// The admission bound of each query: the r-th smallest of its `cnt` minima
+// (no bound, 1e30, when fewer than r of them are distances), raised by a few
+// ulps so that the scan admits every row behind it. One block per
+// query, NV values per thread in registers (the rest re-read from L2), the
+// answer built bit by bit from the top of the ordered representation by
+// counting values: 32 rounds of NV compares and one barrier. Also clears the
+// query's re-scan flag.
+constexpr int TAU_THREADS = 128;
+template <int NV>
+__global__ void __launch_bounds__(TAU_THREADS) tc_tau_kernel(const float* __restrict__ pmin, uint32_t cnt,
+                                                             uint32_t stride, uint32_t r, float* __restrict__ tau,
+                                                             uint32_t* __restrict__ redo) {
+  __shared__ uint32_t part[2][TAU_THREADS / 32];
+  const uint32_t q = blockIdx.x, tid = threadIdx.x;
+  const float* src = pmin + (size_t)q * stride;
+  uint32_t u[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const uint32_t at = (uint32_t)i * TAU_THREADS + tid;
+    u[i] = at < cnt ? float_order(__ldcg(src + at)) : 0xFFFFFFFFu;
   }
-  const uint32_t sp2 = next_pow2_dev(max(live, 2u));
-  for (uint32_t i = live + threadIdx.x; i < sp2; i += blockDim.x) keys[i] = kSentinelKey;
-  __syncthreads();
-  block_bitonic_sort(keys, sp2);
-  if (threadIdx.x == 0) tau[q] = key_dist(keys[r - 1]);
+  uint32_t ans = 0;
+#pragma unroll 1
+  for (int bit = 31; bit >= 0; --bit) {
+    const uint32_t test = ans | ((1u << bit) - 1u);
+    uint32_t c = 0;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) c += u[i] <= test;
+    for (uint32_t at = NV * TAU_THREADS + tid; at < cnt; at += TAU_THREADS) c += float_order(__ldcg(src + at)) <= test;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((tid & 31) == 0) part[bit & 1][tid >> 5] = c;
+    __syncthreads();
+    uint32_t total = 0;
+#pragma unroll
+    for (int w = 0; w < TAU_THREADS / 32; ++w) total += part[bit & 1][w];
+    if (total < r) ans |= 1u << bit;
+  }
+  if (tid == 0) {
+    const float t = order_float(ans);
+    tau[q] = t < kSentinelDist ? t + 1e-6f * fabsf(t) : kSentinelDist;
+    redo[q] = 0u;
+  }
+}
+
+void launch_tau(const float* pmin, uint32_t nq, uint32_t cnt, uint32_t stride, uint32_t r, float* tau, uint32_t* redo,
+                cudaStream_t stream) {
+  auto go = [&](auto kern) { kern<<<nq, TAU_THREADS, 0, stream>>>(pmin, cnt, stride, r, tau, redo); };
+  if (cnt <= 4 * TAU_THREADS)
+    go(tc_tau_kernel<4>);
+  else if (cnt <= 8 * TAU_THREADS)
+    go(tc_tau_kernel<8>);
+  else if (cnt <= 16 * TAU_THREADS)
+    go(tc_tau_kernel<16>);
+  else
+    go(tc_tau_kernel<32>);
 }
 
 // cuTensorMapEncodeTiled resolved through the runtime, so the library does
@@ -391,7 +426,7 @@ uint32_t fill_waves(uint32_t s_min, uint32_t nqb, uint32_t ntiles, uint32_t sms,
   uint32_t best = s_min;
   double best_f = fullness(s_min);
   for (uint32_t s = s_min + 1; s <= std::max(2 * s_min, 32u) && s <= ntiles; ++s) {
-    if (next_pow2(s * keys_per_split) > 16384u) break;
+    if ((uint64_t)s * keys_per_split > 16384u) break;
     const double f = fullness(s);
     if (f > best_f + 0.01) {
       best = s;
@@ -409,11 +444,12 @@ uint32_t fill_waves(uint32_t s_min, uint32_t nqb, uint32_t ntiles, uint32_t sms,
 struct TcPlan {
   bool fp8 = false, pair = false, prepass = false;
   uint32_t elem = 0, kblocks = 0, shortlist = 0, kl = 0, kl_tmpl = 0;
-  int groups = 1, pgroups = 1;  // epilogue groups of the main scan and of the pre-pass
+  int groups = 1;  // epilogue groups of the main scan (the minima pass runs at most 2)
   uint32_t nqb = 0, nqb_grid = 0, splits = 0, tps = 0;
-  uint32_t pstride = 0, pr = 0, pkl_tmpl = 0, psplits = 0, ptps = 0;
+  uint32_t pstride = 0, pr = 0, psplits = 0, ptps = 0;  // minima pass: tile stride, rank of the bound, splits
+  uint32_t pgran = 0, pcount = 0;                        // columns per minimum, minima per query
   uint32_t nq_rows = 0, slot_stride = 0;
-  size_t q_bytes = 0, qn_bytes = 0, part_bytes = 0, slot_bytes = 0, ppart_bytes = 0, tau_bytes = 0;
+  size_t q_bytes = 0, qn_bytes = 0, part_bytes = 0, slot_bytes = 0, tau_bytes = 0;
   size_t scratch_bytes = 0;
 };
 
@@ -461,58 +497,73 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   uint32_t tps = (ntiles + splits - 1) / splits;
   splits = (ntiles + tps - 1) / tps;
 
-  // Sampled pre-pass: the CTAs of a query cannot share a bound when the
-  // shortlist exceeds the per-range heap, so each range would insert
-  // ~kl (1 + ln(rows / kl)) keys per query. A scan of every stride-th tile
-  // gives each query its r-th best sampled distance (r from the Poisson tail
-  // below, or ceil(margin * shortlist / stride) when the margin knob is
-  // set), an upper bound on its shortlist-th distance unless the sample is
-  // unlucky (probability < 1e-7 per query); the full scan then admits only
-  // rows within it. Queries whose bounded scan comes up short are scanned
-  // again without the bound (device-side, no host round trip).
+  // Pre-pass: each query's admission bound for the scan, from the minima pass
+  // over every pstride-th tile. A sample of stride s holds each of the
+  // query's top (shortlist - 1) rows with probability 1 / s; the bound is the
+  // r-th smallest minimum, r from the Poisson tail below (or ceil(margin *
+  // shortlist / stride) when the margin knob is set), and the sampled r-th
+  // distance is an upper bound on the shortlist-th distance unless the sample
+  // is unlucky (probability < 1e-7 per query); with s = 1 it always is, at
+  // r = shortlist (the same accumulators, hence the same distances, are
+  // behind the bound and the scan). The scan then admits only rows within it.
+  // After a sample (s > 1), queries whose bounded scan comes up short are
+  // scanned again without the bound (device-side, no host round trip).
+  //
+  // Automatic stride. Long rows are bound by the MMA, whose pass costs 1 / s
+  // of the scan again: 64 sampled tiles. Short rows (at most two K blocks)
+  // are bound by the candidate path, which a tighter bound shortens: 256
+  // tiles. At most 32 either way (the share of the scan is then 3% and the
+  // bound admits rows of rank ~8 shortlists), more only to keep a query's
+  // minima within 4,096.
   int64_t pp_knob = tune_value("tc.prepass", -1);
   if (pp_knob < 0 && te && te->prepass >= 0) pp_knob = te->prepass;
   int64_t stride_knob = tune_value("tc.prepass_stride", 0);
-  if (stride_knob <= 0) stride_knob = (te && te->stride > 0) ? te->stride : 32;
-  const uint32_t pstride = (uint32_t)std::max<int64_t>(2, stride_knob);
+  if (stride_knob <= 0 && te && te->stride > 0) stride_knob = te->stride;
+  const uint32_t auto_stride = std::max(std::min(32u, std::max(1u, ntiles / (kblocks > 2 ? 64u : 256u))),
+                                        (ntiles + 2047u) / 2048u);
+  const uint32_t pstride =
+      stride_knob > 0 ? (uint32_t)std::min<int64_t>(std::max<int64_t>(2, stride_knob), 1 << 20) : auto_stride;
   const int64_t pmargin = tune_value("tc.prepass_margin", 0);
-  const uint32_t pr = std::max<uint32_t>(
-      1u, std::min<uint32_t>(kl_cap, pmargin > 0 ? (uint32_t)((pmargin * shortlist + pstride - 1) / pstride)
-                                                 : poisson_rank((double)shortlist / pstride, 1e-7)));
   const uint32_t psampled = (ntiles + pstride - 1) / pstride;
-  // automatic: bases of >= 64 sampled tiles (the main scan then uses the
-  // pre-pass bound instead of the cross-CTA shared one); forced on (knob 1):
-  // any base
-  const bool prepass = psampled > 0 && (pp_knob == 1 || (pp_knob != 0 && psampled >= 64u));
-  // the pre-pass keeps two groups where the main scan runs four: its tiles
-  // are far apart, and two groups alternating them (each its own
-  // accumulator buffer) beat four splitting every tile's columns
-  const int pgroups = groups == 4 ? 2 : groups;
-  const uint32_t pkl_tmpl = std::min<uint32_t>(pgroups == 2 ? 48u : 64u, (pr + 15) / 16 * 16);
+  const uint32_t pr =
+      std::max<uint32_t>(1u, pmargin > 0 ? (uint32_t)((pmargin * shortlist + pstride - 1) / pstride)
+                                         : (pstride == 1 ? shortlist : poisson_rank((double)shortlist / pstride, 1e-7)));
+  const size_t part_bytes = align_up((size_t)nq * splits * groups * kl * 8, 256);
+  // The coarsest minima (fewest to store and to select from) that still number
+  // 8 r, so that two of a query's r best rows seldom share one. They live in
+  // the space of the range heaps, which are written after the bound is
+  // known: a call takes no more scratch than its unbounded scan.
+  uint32_t pgran = 0, pcount = 0;
+  for (uint32_t g = 128; g >= 8 && !pgran; g >>= 1) {
+    const uint32_t c = psampled * (TC_N / g);
+    if ((c >= 8 * pr || g == 8) && (size_t)nq * c * 4 <= part_bytes) {
+      pgran = g;
+      pcount = c;
+    }
+  }
+  // off where the base is so small that the minima cannot bound (the heaps
+  // then hold about every row anyway); the knob turns it off anywhere
+  const bool prepass = pp_knob != 0 && pgran && pcount >= 2 * pr;
   uint32_t psplits = std::max<uint32_t>(1u, std::min<uint32_t>((uint32_t)sms / nqb_grid, psampled));
-  psplits = fill_waves(psplits, nqb_grid, psampled, (uint32_t)sms, pgroups * pr);
-  while (psplits > 1 && next_pow2(psplits * pgroups * pr) > 16384u) --psplits;
+  psplits = fill_waves(psplits, nqb_grid, psampled, (uint32_t)sms, 0);
   const uint32_t ptps = (psampled + psplits - 1) / psplits;
   psplits = (psampled + ptps - 1) / ptps;
 
-  // scratch: prepared queries | ||q||^2 | q scales | partial heaps | slots
-  //          [| pre-pass heaps | tau | redo flags]
+  // scratch: prepared queries | ||q||^2 | q scales | minima, then range heaps |
+  //          bounds and re-scan flags (pre-pass), or shared-bound slots
   // prepared queries padded with zero rows to whole query blocks (of the
   // CTA pairs' grid when pairs run)
   const uint32_t nq_rows = nqb_grid * TC_M;
   const size_t q_bytes = align_up((size_t)nq_rows * t.padded_dim * elem, 1024);
   const size_t qn_bytes = align_up((size_t)nq * 4, 256);
-  const size_t part_bytes = align_up((size_t)nq * splits * groups * kl * 8, 256);
-  const uint32_t slot_stride = ((prepass ? std::max(kl, pr) : kl) + 3) / 4 * 4;
+  const uint32_t slot_stride = prepass ? 0u : (kl + 3) / 4 * 4;
   const size_t slot_bytes = align_up((size_t)nq * slot_stride * 4, 256);
-  const size_t ppart_bytes = prepass ? align_up((size_t)nq * psplits * pgroups * pr * 8, 256) : 0;
-  const size_t tau_bytes = prepass ? 2 * qn_bytes : 0;
+  const size_t tau_bytes = prepass ? align_up((size_t)nq * 8, 256) : 0;
   P.fp8 = fp8;
   P.elem = elem;
   P.kblocks = kblocks;
   P.shortlist = shortlist;
   P.groups = groups;
-  P.pgroups = pgroups;
   P.kl = kl;
   P.kl_tmpl = kl_tmpl;
   P.nqb = nqb;
@@ -523,7 +574,8 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   P.prepass = prepass;
   P.pstride = pstride;
   P.pr = pr;
-  P.pkl_tmpl = pkl_tmpl;
+  P.pgran = pgran;
+  P.pcount = pcount;
   P.psplits = psplits;
   P.ptps = ptps;
   P.nq_rows = nq_rows;
@@ -532,9 +584,8 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   P.part_bytes = part_bytes;
   P.slot_stride = slot_stride;
   P.slot_bytes = slot_bytes;
-  P.ppart_bytes = ppart_bytes;
   P.tau_bytes = tau_bytes;
-  P.scratch_bytes = q_bytes + 2 * qn_bytes + part_bytes + slot_bytes + ppart_bytes + tau_bytes;
+  P.scratch_bytes = q_bytes + 2 * qn_bytes + part_bytes + slot_bytes + tau_bytes;
   return P;
 }
 
@@ -555,13 +606,11 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
   const TcPlan P = plan_tc_scan(t, nq, k, metric, opt);
   const bool fp8 = P.fp8;
   const uint32_t elem = P.elem, kblocks = P.kblocks, shortlist = P.shortlist, kl = P.kl, kl_tmpl = P.kl_tmpl;
-  const int groups = P.groups, pgroups = P.pgroups;
+  const int groups = P.groups;
   const uint32_t nqb = P.nqb, nqb_grid = P.nqb_grid, splits = P.splits, tps = P.tps;
   const bool pair = P.pair, prepass = P.prepass;
-  const uint32_t pstride = P.pstride, pr = P.pr, pkl_tmpl = P.pkl_tmpl, psplits = P.psplits, ptps = P.ptps;
   const uint32_t nq_rows = P.nq_rows, slot_stride = P.slot_stride;
-  const size_t q_bytes = P.q_bytes, qn_bytes = P.qn_bytes, part_bytes = P.part_bytes, slot_bytes = P.slot_bytes;
-  const size_t ppart_bytes = P.ppart_bytes;
+  const size_t q_bytes = P.q_bytes, qn_bytes = P.qn_bytes, part_bytes = P.part_bytes;
   uint8_t* scratch = static_cast<uint8_t*>(ext_scratch ? ext_scratch : scratch_get(stream, P.scratch_bytes));
   if (!scratch) return (int)cudaErrorMemoryAllocation;
   void* qprep = scratch;
@@ -569,17 +618,15 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
   float* qscale = reinterpret_cast<float*>(scratch + q_bytes + qn_bytes);
   uint64_t* partial = reinterpret_cast<uint64_t*>(scratch + q_bytes + 2 * qn_bytes);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(scratch + q_bytes + 2 * qn_bytes + part_bytes);
-  uint8_t* extra = scratch + q_bytes + 2 * qn_bytes + part_bytes + slot_bytes;
-  uint64_t* ppartial = prepass ? reinterpret_cast<uint64_t*>(extra) : nullptr;
-  float* tau = prepass ? reinterpret_cast<float*>(extra + ppart_bytes) : nullptr;
-  uint32_t* redo = prepass ? reinterpret_cast<uint32_t*>(extra + ppart_bytes + qn_bytes) : nullptr;
+  float* tau = prepass ? reinterpret_cast<float*>(tslot) : nullptr;
+  uint32_t* redo = prepass ? tslot + nq : nullptr;
 
   {
     ProfScope ps(fp8 ? "tc_prep_queries_fp8" : "tc_prep_queries_fp16", stream);
     const uint32_t blocks = (nq_rows * 32 + 255) / 256;
-    // the shared-bound slots serve the scan that shares a bound: the main
-    // scan when its heap holds the whole shortlist, else the pre-pass
-    const uint32_t slot_kl = prepass ? pr : kl;
+    // the shared-bound slots serve a scan without the pre-pass (none with it:
+    // slot_stride is 0)
+    const uint32_t slot_kl = kl;
     if (fp8)
       tc_prep_queries_kernel<true><<<blocks, 256, 0, stream>>>(queries, nq, t.dim, t.padded_dim, qprep, qnorm, qscale,
                                                                tslot, slot_kl, slot_stride, t.scales, (int)metric,
@@ -630,24 +677,19 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
   cudaError_t e;
   if (prepass) {
     TcScanArgs p = a;
-    p.splits = psplits;
-    p.tiles_per_split = ptps;
-    p.partial = ppartial;
-    p.kl = pr;
-    p.share = 1;  // the pre-pass heap holds its whole "shortlist" (pr keys)
-    p.tile_stride = pstride;
-    e = scan(p, (int)pkl_tmpl, psplits, fp8 ? "tc_prepass_fp8" : "tc_prepass_fp16", pair, pgroups);
-    if (e != cudaSuccess) return (int)e;
-    const uint32_t total = psplits * pgroups * pr, pow2 = next_pow2(total);
-    e = cudaFuncSetAttribute(tc_tau_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(pow2 * 8));
+    p.splits = P.psplits;
+    p.tiles_per_split = P.ptps;
+    p.tile_stride = P.pstride;
+    p.pmin = reinterpret_cast<float*>(partial);
+    p.pm_stride = P.pcount;
+    p.gran = P.pgran;
+    e = scan(p, 0, P.psplits, fp8 ? "tc_prepass_fp8" : "tc_prepass_fp16", pair, groups > 2 ? 2 : groups);
     if (e != cudaSuccess) return (int)e;
     {
       ProfScope ps("tc_tau", stream);
-      tc_tau_kernel<<<nq, 128, pow2 * 8, stream>>>(ppartial, total, pow2, pr, tau);
+      launch_tau(p.pmin, nq, P.pcount, P.pcount, P.pr, tau, redo, stream);
       note_launch();
     }
-    e = cudaMemsetAsync(redo, 0, (size_t)nq * 4, stream);
-    if (e != cudaSuccess) return (int)e;
   }
   a.splits = splits;
   a.tiles_per_split = tps;
@@ -670,7 +712,7 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
     tc_select_kernel<<<nq, SEL_THREADS, sel_smem, stream>>>(s);
     note_launch();
   }
-  if (prepass) {
+  if (prepass && P.pstride > 1) {
     // queries whose bound was too tight: scanned again without it (blocks
     // holding none of them exit at once), then selected again
     TcScanArgs f = a;

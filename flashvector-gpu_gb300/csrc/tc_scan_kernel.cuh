@@ -64,6 +64,10 @@ struct TcScanArgs {
   const uint32_t* active;      // per-query flags: only flagged queries are scanned (null: all)
   uint32_t tile_stride;        // scan every tile_stride-th 256-row tile (a sample when > 1)
   uint64_t wait_ns;            // limit of the pipeline's waits (the drains keep their own)
+  // minima pass only: the smallest distance of every `gran` consecutive
+  // scanned columns (8, 16, 32, 64 or 128), [nq][pm_stride], column order
+  float* pmin;
+  uint32_t pm_stride, gran;
 };
 
 // PAIR: a CTA of a cta_group::2 pair holds half of each 256-row base tile.
@@ -152,21 +156,15 @@ static __device__ __forceinline__ float select32(const float* v, int j) {
 }
 
 // G epilogue groups, each with its own heaps, dumped as separate lists
-// (partial row split * G + g). With G = 2 a full scan splits columns: both
-// groups drain every tile, group g the columns [128 g, 128 g + 128) of it,
-// so the MMA of tile i + 1 (the other accumulator buffer) runs while tile i
-// is drained. A sampled scan (tile stride > 1, whose tile loads are further
-// apart) alternates tiles instead: group g drains tiles g, g + 2, .. (each
-// group owns one buffer), so each group's wait for its next tile overlaps
-// the other group's work.
+// (partial row split * G + g). With G = 2 both groups drain every tile, group
+// g the columns [128 g, 128 g + 128) of it, so the MMA of tile i + 1 (the
+// other accumulator buffer) runs while tile i is drained.
 //
-// G = 4 (fused fp8 with one K block per tile, shortlists above 48 keys; the
-// host runs that call's sampled pre-pass with G = 2): 16 epilogue warps,
-// group g draining the 32-column chunks g and g + 4 of every tile, in any
-// scan (alternating tiles would put two groups on one accumulator buffer,
-// and a parity wait cannot tell its phase from the phase two uses later).
-// Heaps of at most 32 keys fit four groups' heaps in shared memory;
-// interleaved chunks spread runs of consecutive slots over the groups.
+// G = 4 (fused fp8 with one K block per tile, shortlists above 48 keys; that
+// call's minima pass runs G = 2): 16 epilogue warps, group g draining the
+// 32-column chunks g and g + 4 of every tile. Heaps of at most 32 keys fit
+// four groups' heaps in shared memory; interleaved chunks spread runs of
+// consecutive slots over the groups.
 //
 // PAIR: the CTA is one of a cluster of two (a cta_group::2 pair) sharing the
 // same base range: CTA r holds query block 2p + r and rows [128 r, 128 r +
@@ -176,7 +174,16 @@ static __device__ __forceinline__ float select32(const float* v, int j) {
 // TMA loads count on the even CTA's full barriers; the even CTA's commits
 // are multicast to both CTAs' barriers; the odd CTA's epilogue arrives on
 // the even CTA's accumulator barriers.
-template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR, bool TS>
+//
+// MINP: the pass that finds every query's admission bound. No heaps: the
+// epilogue reduces each tile's accumulators to the smallest distance of every
+// `gran` columns and stores those, so its cost per tile is the minimum tree
+// alone and the freed shared memory holds a deeper ring. The r-th smallest
+// of a query's minima is >= the r-th smallest distance scanned (minima of
+// disjoint columns are distances of distinct rows), so it bounds from above.
+// Keeping the sample's best r keys in heaps instead spent the pass filling
+// them: 123 us for 1/32 of a 1M x 768 scan of 1,024 queries.
+template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR, bool TS, bool MINP>
 __global__ void __launch_bounds__(scan_threads(G), 1)
     tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TcScanArgs a) {
   using L = ScanLayout<FP8, KL, STAGES, METRIC, G, PAIR, TS>;
@@ -219,7 +226,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     if (!__syncthreads_or(any)) return;
   }
   const uint32_t tstride = a.tile_stride ? a.tile_stride : 1u;
-  const bool col_split = G == 4 || (G == 2 && tstride == 1);
+  constexpr bool col_split = G >= 2;
   const uint32_t ntiles = ((a.n + TC_N - 1) / TC_N + tstride - 1) / tstride;
   const uint32_t t_begin = split * a.tiles_per_split;
   const uint32_t t_end = min(t_begin + a.tiles_per_split, ntiles);
@@ -364,7 +371,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     const uint32_t q = qb * TC_M + row;
     const bool qvalid = q < a.nq && (a.active == nullptr || a.active[q] != 0u);
     uint64_t* h = heap + (size_t)grp * KL * TC_M + row;
-    const int kl = (int)a.kl;
+    const int kl = MINP ? 0 : (int)a.kl;
     for (int i = 0; i < kl; ++i) h[i * TC_M] = kSentinelKey;
     const float qn = qvalid ? __ldg(a.qnorm + q) : 0.f;
     const QueryFilter qf = (a.filters && qvalid) ? load_filter(a.filters, q) : QueryFilter{nullptr, 0u, 0u};
@@ -381,7 +388,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     float worst = kSentinelDist;  // this CTA's kl-th best distance (1e30 until the heap is full)
     // admission bound: the query's pre-pass bound, lowered by the shared slots
     float bound = (a.qbound && qvalid) ? __ldg(a.qbound + q) : kSentinelDist;
-    uint32_t* slots = (a.share && qvalid) ? a.tslot + (size_t)q * a.tslot_stride : nullptr;
+    uint32_t* slots = (!MINP && a.share && qvalid) ? a.tslot + (size_t)q * a.tslot_stride : nullptr;
 
     // Until kl keys are held the heap is an unordered list (appends cost
     // one store); on the kl-th key it is heapified once and from then on a
@@ -419,13 +426,12 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
 
     // per-warp copy of the current tile's column data (norms, fp8 factors,
     // mask words): staged by the warp itself, so the epilogue warps never
-    // wait on one another. The global loads for tile i + G are issued into
+    // wait on one another. The global loads for tile i + 1 are issued into
     // registers while tile i is processed (lane l holds columns l + 32 r).
     float* cb = colbuf + (warp - 2) * 2 * TC_N;
     uint32_t* cm = colmask + (warp - 2) * 8;
-    // this group's tiles (first, step) and columns [c_lo, c_hi) of each;
-    // only its own columns' data is staged
-    const uint32_t t_first = col_split ? 0u : (uint32_t)grp, t_step = col_split ? 1u : (uint32_t)G;
+    // this group's columns [c_lo, c_hi) of each tile; only its own columns'
+    // data is staged
     const int c_lo = col_split ? grp * (TC_N / G) : 0, c_hi = col_split ? c_lo + TC_N / G : TC_N;
     float pre_n[TC_N / 32], pre_s[TC_N / 32];
     uint32_t pre_m = 0;
@@ -451,8 +457,8 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
         }
       }
     };
-    if (t_first < my_tiles) prefetch(t_first);
-    for (uint32_t i = t_first; i < my_tiles; i += t_step) {
+    if (my_tiles) prefetch(0);
+    for (uint32_t i = 0; i < my_tiles; ++i) {
       const uint32_t buf = i & 1, use = i >> 1;
       const uint32_t v0 = (t_begin + i) * tstride * TC_N;
       __syncwarp();
@@ -464,7 +470,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
       }
       if (lane < 8) cm[lane] = pre_m;
       __syncwarp();
-      if (i + t_step < my_tiles) prefetch(i + t_step);
+      if (i + 1 < my_tiles) prefetch(i + 1);
       // the shared bound, loaded before the accumulator wait hides its latency
       uint32_t smax = 0;
       if (slots)
@@ -527,6 +533,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
           chunk32(ra, col, m32);
         }
       } else {
+        [[maybe_unused]] float best128 = 0.f;
 #pragma unroll 1
         for (int c0 = c_lo; c0 < c_hi; c0 += 64) {
           uint32_t ra[32], rb[32];
@@ -540,7 +547,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
           }
           tc::tmem_wait_ld(ra);
           tc::reg_fence(rb);
-          if (mw == 0ull) continue;
+          if (!MINP && mw == 0ull) continue;
           // the chunk's admission test and insertions; FU: the accumulator is
           // the ranking value (fp8 table-scale tables)
           auto chunk = [&](auto fu_tag) {
@@ -601,6 +608,47 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
                 asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(x), "f"(y), "f"(z));
               return d;
             };
+            if constexpr (MINP) {
+              // the smallest distance of every 8 columns (none where the mask
+              // admits none), then of every `gran`
+              const float none = FU ? -INFINITY : INFINITY;
+              if (mw != ~0ull) {
+#pragma unroll
+                for (int j = 0; j < 64; ++j) v[j] = ((mw >> j) & 1ull) ? v[j] : none;
+              }
+              float m[8];
+#pragma unroll
+              for (int b = 0; b < 8; ++b) {
+                const float* w = v + 8 * b;
+                m[b] = best3(best3(w[0], w[1], w[2]), best3(w[3], w[4], w[5]), better(w[6], w[7]));
+              }
+              if (!qvalid) return;
+              float* dst = a.pmin + (size_t)q * a.pm_stride;
+              const uint32_t at = (t_begin + i) * TC_N + (uint32_t)c0;  // scanned column
+              if (a.gran == 8) {
+                float4* o = reinterpret_cast<float4*>(dst + at / 8);
+                o[0] = make_float4(D(m[0]), D(m[1]), D(m[2]), D(m[3]));
+                o[1] = make_float4(D(m[4]), D(m[5]), D(m[6]), D(m[7]));
+                return;
+              }
+              const float p0 = better(m[0], m[1]), p1 = better(m[2], m[3]), p2 = better(m[4], m[5]),
+                          p3 = better(m[6], m[7]);
+              if (a.gran == 16) {
+                *reinterpret_cast<float4*>(dst + at / 16) = make_float4(D(p0), D(p1), D(p2), D(p3));
+                return;
+              }
+              const float h0 = better(p0, p1), h1 = better(p2, p3), all = better(h0, h1);
+              if (a.gran == 32) {
+                *reinterpret_cast<float2*>(dst + at / 32) = make_float2(D(h0), D(h1));
+              } else if (a.gran == 64) {
+                dst[at / 64] = D(all);
+              } else if ((c0 & 64) == 0) {
+                best128 = all;
+              } else {
+                dst[at / 128] = D(better(best128, all));
+              }
+              return;
+            } else {
             float r[22], s8[8];
 #pragma unroll
             for (int i = 0; i < 21; ++i) r[i] = best3(v[3 * i], v[3 * i + 1], v[3 * i + 2]);
@@ -632,6 +680,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
                 refresh();
               }
             }
+            }
           };
           chunk(std::integral_constant<bool, fused>{});
         }
@@ -647,7 +696,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
           tc::mbar_arrive_relaxed(&acc_empty[buf]);
       }
     }
-    if (qvalid) {
+    if (!MINP && qvalid) {
       // entry 0 of a dumped list is its largest key (the select kernel tests
       // it for overflow): a full heap has it there already; a list that never
       // filled gets one of its sentinels moved there
@@ -679,12 +728,12 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
 }
 
 
-template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR = false, bool TS = true>
+template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR = false, bool TS = true, bool MINP = false>
 cudaError_t launch_scan_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const TcScanArgs& a, uint32_t grid,
                                cudaStream_t stream) {
   using L = ScanLayout<FP8, KL, STAGES, METRIC, G, PAIR, TS>;
   static_assert(L::bytes <= 227 * 1024, "scan shared memory above the 227 KB per-CTA limit");
-  auto kern = tc_scan_kernel<FP8, KL, STAGES, METRIC, G, PAIR, TS>;
+  auto kern = tc_scan_kernel<FP8, KL, STAGES, METRIC, G, PAIR, TS, MINP>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes);
   if (e != cudaSuccess) return e;
   if constexpr (PAIR) {
@@ -718,6 +767,12 @@ cudaError_t launch_scan_kernel(const CUtensorMap& ta, const CUtensorMap& tb, con
 template <bool FP8, int METRIC, bool TS>
 cudaError_t dispatch_scan_kl(int kl, int groups, const CUtensorMap& ta, const CUtensorMap& tb, const TcScanArgs& a,
                              uint32_t grid, cudaStream_t stream) {
+  if (kl == 0) {
+    // the minima pass: no heaps, so the ring takes their shared memory
+    if (groups == -1) return launch_scan_kernel<FP8, 0, 6, METRIC, 1, true, TS, true>(ta, tb, a, grid, stream);
+    if (groups == 1) return launch_scan_kernel<FP8, 0, 4, METRIC, 1, false, TS, true>(ta, tb, a, grid, stream);
+    return launch_scan_kernel<FP8, 0, 4, METRIC, 2, false, TS, true>(ta, tb, a, grid, stream);
+  }
   if (groups == -1) {
     // cta_group::2 pairs (one epilogue group): 16 KB of base per stage frees
     // room for 4-6 stages

@@ -330,11 +330,12 @@ int fv_profile_enable(int on);
 int fv_profile_summary(char* buf, size_t len);
 /* Process-wide tuning knobs (no reference counterpart). Keys:
  *   "tc.prepass"        -1 automatic (default), 0 off, 1 on where it applies:
- *                       tensor-core scans whose shortlist exceeds the 64-entry
- *                       per-range heap first scan a strided sample of the
- *                       base for a per-query admission bound
+ *                       tensor-core scans first find a per-query admission
+ *                       bound from the minima of a strided sample of the
+ *                       base (all of it where it is small); bases too small
+ *                       to bound are scanned without
  *   "tc.prepass_stride" sample stride in 256-row tiles (0 automatic: the
- *                       tuned value, else 32)
+ *                       tuned value, else 1 to 32 growing with the base)
  *   "tc.prepass_margin" 0 (default): the sampled rank r is the smallest
  *                       with P(Poisson(shortlist / stride) >= r) < 1e-7;
  *                       m > 0: r = ceil(m * shortlist / stride)

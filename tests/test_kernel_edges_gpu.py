@@ -28,3 +28,33 @@ def test_encode_fp16_row_and_column_remainders(cuda, oracle_mod, n, dim, pd, off
     assert np.array_equal(got[:, :dim], ref_codes[:, :dim])
     assert not got[:, dim:].any()
     assert np.array_equal(norms.cpu().numpy().view(np.uint32), ref_norms.view(np.uint32))
+
+
+@pytest.mark.parametrize("metric", ["l2", "ip", "cosine"])
+@pytest.mark.parametrize(
+    "n,dim,nq,k",
+    [(200, 96, 3, 100), (256, 64, 129, 1), (1000, 100, 33, 10), (4097, 128, 300, 12), (20_001, 70, 5, 100),
+     (33_000, 200, 257, 25), (140_003, 48, 64, 60), (140_003, 264, 1, 10)],
+)
+@pytest.mark.parametrize("fp8,masked", [(False, False), (False, True), (True, True)])
+def test_bounded_scan_equals_unbounded(cuda, metric, n, dim, nq, k, fp8, masked):
+    """The scan bounded by the minima pass (every width of a minimum, sampled
+    and whole bases, one and several query blocks, partial last tiles, bases
+    too small for it) returns what the scan without a bound returns."""
+    from fvgb300 import datasets, scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(n + dim + k)
+    x = torch.randn((n, dim), generator=g, device="cuda")
+    q = torch.randn((nq, dim), generator=g, device="cuda")
+    t = scan.Fp8Table(x) if fp8 else scan.Fp16Table(x)
+    search = scan.fp8_search if fp8 else scan.fp16_search
+    mask = torch.from_numpy(datasets.bernoulli_mask_words(n, 0.3, 7).view(np.int32)).cuda() if masked else None
+    with scan.tuned(tc_prepass=0):
+        ref = search(t, q, k, metric, mask=mask)
+    # (one tile and a 400-row shortlist: its range heaps report an overflow)
+    status = scan.device_status()
+    got = search(t, q, k, metric, mask=mask)
+    torch.cuda.synchronize()
+    assert scan.device_status() == status
+    assert torch.equal(got, ref)
