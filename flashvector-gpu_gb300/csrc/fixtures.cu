@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(256) distance_matrix_kernel(const float* __res
 __global__ void __launch_bounds__(256) bitonic_test_kernel(const float* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                            float* __restrict__ kout, uint32_t* __restrict__ vout,
                                                            uint32_t n, uint32_t pow2) {
-  extern __shared__ uint64_t keys[];
+  extern __shared__ __align__(16) uint64_t keys[];
   for (uint32_t i = threadIdx.x; i < pow2; i += blockDim.x)
     keys[i] = i < n ? ((uint64_t)float_order(kin[i]) << 32) | vin[i] : kSentinelKey;
   __syncthreads();

@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(NT) flat_f32_scan_kernel(FlatArgs a) {
 __global__ void __launch_bounds__(256) merge_partial_topk_kernel(const uint64_t* __restrict__ partial, uint32_t lists,
                                                                  uint32_t k, uint32_t pow2, const uint32_t* vec_ids,
                                                                  GpuSearchResult* __restrict__ out, uint32_t out_k) {
-  extern __shared__ uint64_t keys[];
+  extern __shared__ __align__(16) uint64_t keys[];
   const uint32_t q = blockIdx.x;
   const uint32_t total = lists * k;
   const uint64_t* src = partial + (size_t)q * total;

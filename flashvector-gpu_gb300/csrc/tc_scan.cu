@@ -154,7 +154,7 @@ __device__ double warp_distance_f64(const float* __restrict__ q, const float* __
 
 struct SelectArgs {
   const uint64_t* partial;   // [nq][lists][KL]
-  uint32_t lists, kl, pow2, shortlist, k;
+  uint32_t lists, kl, cap, shortlist, k;  // cap: keys that fit the block's shared memory (power of two)
   const float* queries;      // fp32 queries (rescore)
   const float* vectors;      // fp32 rows (null: no rescore)
   uint32_t dim;
@@ -176,7 +176,7 @@ constexpr int BAND_MAX = 64;
 // keys, rescore them in fp32 (the reference's warp-order distance), sort,
 // re-rank the band |d - d_k| <= eps * scale in fp64, write the top k.
 __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
-  extern __shared__ uint64_t keys[];
+  extern __shared__ __align__(16) uint64_t keys[];
   __shared__ double band_d[BAND_MAX];
   __shared__ int band_lo, band_hi;
   __shared__ int incomplete;
@@ -190,7 +190,13 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
   // only the kept keys are sorted (lists that stayed partly empty hold
   // sentinels); sorted they are the same sequence as the whole table sorted
   const uint32_t kp = min(s.shortlist, total);
-  const uint32_t live = block_compact_keys(src, total, keys, &n_live);
+  uint32_t live = block_compact_keys(src, total, keys, &n_live, s.cap);
+  if (live > s.cap) {
+    // more keys than the launch foresaw (an unlucky sample, rows in an order
+    // that fills one range): keep the best kp by their kp-th key
+    const uint64_t limit = block_kth_key(src, total, kp);
+    live = block_compact_keys(src, total, keys, &n_live, s.cap, limit);
+  }
   const uint32_t sp2 = next_pow2_dev(max(max(live, kp), 2u));
   for (uint32_t i = live + threadIdx.x; i < sp2; i += SEL_THREADS) keys[i] = kSentinelKey;
   __syncthreads();
@@ -215,12 +221,30 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
 
   const float* qv = s.queries + (size_t)q * s.dim;
   if (s.vectors) {
-    for (uint32_t c = warp; c < kp; c += SEL_THREADS / 32) {
-      const uint64_t key = keys[c];
-      if (key == kSentinelKey) continue;
-      const uint32_t slot = key_slot(key);
-      const float d = warp_metric_distance(qv, s.vectors + (size_t)slot * s.dim, s.dim, lane, (MetricType)s.metric);
-      if (lane == 0) keys[c] = d < kSentinelDist ? make_key(d, slot) : kSentinelKey;
+    // four candidates per warp pass, so that four rows' gathers are in flight
+    constexpr uint32_t NW = SEL_THREADS / 32, R = 4;
+    for (uint32_t c0 = warp; c0 < kp; c0 += R * NW) {
+      if (keys[c0] == kSentinelKey) break;  // sorted: the rest are sentinels too
+      const float* rows[R];
+      uint32_t slot[R];
+#pragma unroll
+      for (uint32_t r = 0; r < R; ++r) {
+        // a missing candidate re-reads the first one and is not stored
+        const uint32_t c = c0 + r * NW;
+        const uint64_t key = c < kp ? keys[c] : kSentinelKey;
+        slot[r] = key_slot(key != kSentinelKey ? key : keys[c0]);
+        rows[r] = s.vectors + (size_t)slot[r] * s.dim;
+      }
+      float d[R];
+      warp_metric_distances<R, 4>(qv, rows, s.dim, lane, (MetricType)s.metric, d);
+      __syncwarp();
+      if (lane == 0) {
+#pragma unroll
+        for (uint32_t r = 0; r < R; ++r) {
+          const uint32_t c = c0 + r * NW;
+          if (c < kp && keys[c] != kSentinelKey) keys[c] = d[r] < kSentinelDist ? make_key(d[r], slot[r]) : kSentinelKey;
+        }
+      }
     }
     const uint32_t p2 = next_pow2_dev(kp);
     for (uint32_t i = kp + threadIdx.x; i < p2; i += SEL_THREADS) keys[i] = kSentinelKey;
@@ -700,11 +724,19 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
   e = scan(a, (int)kl_tmpl, splits, fp8 ? "tc_scan_fp8" : "tc_scan_fp16", pair, groups);
   if (e != cudaSuccess) return (int)e;
 
-  SelectArgs s{partial, splits * groups, kl, next_pow2(splits * groups * kl), shortlist, k, queries, t.vectors, t.dim,
+  // The keys that a block sorts: all of them without a bound; with one, about
+  // r s rows pass it, within 5 standard deviations of the sampled rank (a
+  // query beyond that selects by its kp-th key). Room for every list instead
+  // (up to 128 KB) left one block per SM.
+  const uint32_t all_keys = next_pow2(splits * groups * kl);
+  const double foreseen = (double)P.pstride * (P.pr + (P.pstride > 1 ? 5.0 * std::sqrt((double)P.pr) : 0.125 * P.pr));
+  const uint32_t foreseen_keys = next_pow2((uint32_t)std::min(foreseen, 16384.0) + 64u);
+  const uint32_t sel_keys = std::max(std::max(2u, next_pow2(shortlist)), prepass ? std::min(all_keys, foreseen_keys) : all_keys);
+  SelectArgs s{partial, splits * groups, kl, sel_keys, shortlist, k, queries, t.vectors, t.dim,
                (int)metric,
                opt.boundary_fp64 ? 1u : 0u, 0.f, out, status_word(), tau, redo, nullptr, incomplete_q};
   s.eps = opt.boundary_eps > 0.f ? opt.boundary_eps : (float)((t.dim + 31) / 32 + 5) * 2.0f * 5.960464477539063e-08f;
-  const size_t sel_smem = (size_t)std::max(s.pow2, next_pow2(shortlist)) * 8;
+  size_t sel_smem = (size_t)sel_keys * 8;
   e = cudaFuncSetAttribute(tc_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem);
   if (e != cudaSuccess) return (int)e;
   {
@@ -722,6 +754,10 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
     e = scan(f, (int)kl_tmpl, splits, fp8 ? "tc_rescan_fp8" : "tc_rescan_fp16", false, groups);
     if (e != cudaSuccess) return (int)e;
     SelectArgs r = s;
+    r.cap = std::max(sel_keys, all_keys);
+    sel_smem = (size_t)r.cap * 8;
+    e = cudaFuncSetAttribute(tc_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem);
+    if (e != cudaSuccess) return (int)e;
     r.tau = nullptr;
     r.redo = nullptr;
     r.only = redo;

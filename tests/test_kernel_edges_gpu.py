@@ -58,3 +58,41 @@ def test_bounded_scan_equals_unbounded(cuda, metric, n, dim, nq, k, fp8, masked)
     torch.cuda.synchronize()
     assert scan.device_status() == status
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("nq,k", [(1, 10), (130, 10)])
+def test_select_with_more_keys_than_foreseen(cuda, nq, k):
+    """The sampled tiles (every 32nd) hold only far rows, so the bound admits
+    nearly every row and the selection meets full range heaps, more keys than
+    its block holds: it falls back to their k-th key, same answer."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(3)
+    n = 64 * 32 * 256 + 77
+    x = torch.randn((n, 32), generator=g, device="cuda")
+    x[(torch.arange(n, device="cuda") // 256) % 32 == 0] *= 100.0
+    q = torch.randn((nq, 32), generator=g, device="cuda")
+    t = scan.Fp16Table(x)
+    with scan.tuned(tc_prepass=0):
+        ref = scan.fp16_search(t, q, k, "l2")
+    with scan.tuned(tc_prepass_stride=32):
+        got = scan.fp16_search(t, q, k, "l2")
+    torch.cuda.synchronize()
+    assert scan.device_status() == 0
+    assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 33, 64, 100, 127, 128, 129, 255, 256, 257, 1000, 1024, 2048, 2049, 4096])
+def test_block_sort_sizes(cuda, n):
+    """The block sort around its warp (128 keys) and barrier strides."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(n)
+    keys = torch.randint(-50, 50, (n,), generator=g, device="cuda").float()
+    vals = torch.randperm(n, generator=g, device="cuda").to(torch.int32)
+    ko, vo = scan.bitonic_sort(keys, vals)
+    order = np.lexsort((vals.cpu().numpy(), keys.cpu().numpy()))
+    assert np.array_equal(ko.cpu().numpy(), keys.cpu().numpy()[order])
+    assert np.array_equal(vo.cpu().numpy(), vals.cpu().numpy()[order])
