@@ -87,7 +87,8 @@ int launch_fill_sentinel(GpuSearchResult* out, size_t count, cudaStream_t stream
 // exact fp32 flat scan (flat_fp32.cu)
 struct FlatPlan {
   uint32_t splits = 1, tiles_per_split = 0;
-  size_t scratch_bytes = 0;  // per-split heaps (0 when one split)
+  uint32_t query_tile = 64;  // queries per CTA
+  size_t scratch_bytes = 0;  // per-split lists (0 when one split)
 };
 FlatPlan plan_flat_f32(uint32_t n, uint32_t nq, uint32_t k, uint32_t forced_splits);
 // fused = true accumulates fmaf(diff, diff, acc) (L2 only): the coarse quantizer

@@ -96,3 +96,26 @@ def test_block_sort_sizes(cuda, n):
     order = np.lexsort((vals.cpu().numpy(), keys.cpu().numpy()))
     assert np.array_equal(ko.cpu().numpy(), keys.cpu().numpy()[order])
     assert np.array_equal(vo.cpu().numpy(), vals.cpu().numpy()[order])
+
+
+@pytest.mark.parametrize("metric", ["l2", "ip", "cosine"])
+@pytest.mark.parametrize("nq", [1, 8, 9, 16, 17, 33, 64, 77, 129])
+@pytest.mark.parametrize("n,dim,k", [(1, 1, 1), (127, 31, 32), (129, 32, 33), (700, 36, 128), (1500, 101, 129),
+                                     (5000, 64, 256)])
+def test_flat_query_tiles_and_list_lengths(cuda, oracle_mod, metric, nq, n, dim, k):
+    """Every query-tile width with its remainder, row and dimension
+    remainders, list lengths around the 32 and 128 keys of a merge; integer
+    rows give many equal distances (ties -> lower slot)."""
+    from fvgb300 import datasets, scan
+
+    torch = cuda
+    rng = np.random.default_rng(n * 7 + nq)
+    base = np.rint(rng.uniform(-3, 3, (n, dim))).astype(np.float32)
+    queries = rng.standard_normal((nq, dim), dtype=np.float32) if nq % 2 else base[rng.integers(0, n, nq)]
+    mask = datasets.bernoulli_mask_words(n, 0.6, 3) if nq > 8 else None
+    md = None if mask is None else torch.from_numpy(mask.view(np.int32)).cuda()
+    res = scan.flat_scan(torch.from_numpy(base).cuda(), torch.from_numpy(queries).cuda(), k, metric, mask=md)
+    r = res.cpu().numpy()
+    ref = oracle_mod.exact_knn(base, queries, k, metric, mask=mask)
+    assert np.array_equal(r[..., 0].view(np.uint32), ref["id"])
+    assert np.array_equal(r[..., 1].view(np.uint32), ref["distance"].view(np.uint32))
