@@ -49,6 +49,7 @@ struct FlatArgs {
   uint64_t* partial;      // [nq][splits][k] sorted lists when splits > 1
   uint32_t splits, tiles_per_split;
   const QueryFilter* filters;  // per-query filters over logical ids (vec_ids[slot], or slot), or null
+  const uint32_t* active;      // only the flagged queries (blocks without one leave at once), or null
 };
 
 // Merges the m (<= 128) candidates of one query's tile into its sorted list
@@ -204,6 +205,7 @@ __global__ void __launch_bounds__(NT, QT >= 32 ? 2 : 3) flat_f32_scan_kernel(Fla
   const int tq = QT >= 16 ? ty * QPT : (ty & 7);     // first query of this thread
   const int xh = QT >= 16 ? 0 : (ty >> 3) * 16;      // QT = 8: row group offset of this thread's half
   const uint32_t q0 = blockIdx.x * QT;
+  if (a.active && !__syncthreads_or(tid < QT && q0 + tid < a.nq && a.active[q0 + tid] != 0u)) return;
   const uint32_t k = a.k;
   const uint32_t ntiles = (a.n + VT - 1) / VT;
   const uint32_t t_begin = blockIdx.y * a.tiles_per_split;
@@ -429,6 +431,7 @@ __global__ void __launch_bounds__(NT, QT >= 32 ? 2 : 3) flat_f32_scan_kernel(Fla
   for (uint32_t i = tid; i < QT * k; i += NT) {
     const uint32_t q = q0 + i / k, r = i % k;
     if (q >= a.nq) break;
+    if (a.active && a.active[q] == 0u) continue;
     if (a.splits == 1)
       a.out[(size_t)q * k + r] = key_to_result(list[i], a.vec_ids);
     else
@@ -442,9 +445,11 @@ __global__ void __launch_bounds__(NT, QT >= 32 ? 2 : 3) flat_f32_scan_kernel(Fla
 // ascending top-k; one CTA per query, bitonic sort in shared memory.
 __global__ void __launch_bounds__(256) merge_partial_topk_kernel(const uint64_t* __restrict__ partial, uint32_t lists,
                                                                  uint32_t k, uint32_t pow2, const uint32_t* vec_ids,
-                                                                 GpuSearchResult* __restrict__ out, uint32_t out_k) {
+                                                                 GpuSearchResult* __restrict__ out, uint32_t out_k,
+                                                                 const uint32_t* __restrict__ active) {
   extern __shared__ __align__(16) uint64_t keys[];
   const uint32_t q = blockIdx.x;
+  if (active && active[q] == 0u) return;
   const uint32_t total = lists * k;
   const uint64_t* src = partial + (size_t)q * total;
   for (uint32_t i = threadIdx.x; i < pow2; i += blockDim.x) keys[i] = i < total ? src[i] : kSentinelKey;
@@ -513,8 +518,14 @@ FlatPlan plan_flat_f32(uint32_t n, uint32_t nq, uint32_t k, uint32_t forced_spli
 int launch_flat_f32(const float* vectors, const uint32_t* vec_ids, uint32_t n, uint32_t dim, const float* queries,
                     uint32_t nq, uint32_t k, MetricType metric, const uint32_t* mask, GpuSearchResult* out,
                     uint32_t forced_splits, cudaStream_t stream, const QueryFilter* filters) {
-  const FlatPlan p = plan_flat_f32(n, nq, k, forced_splits);
   void* scratch = nullptr;
+  if (!filters && !forced_splits) {
+    const size_t bytes = flat_tc_bytes(n, dim, nq, k, metric);
+    // (a caller's arena that only fits the plain scan keeps it)
+    if (bytes && (scratch = scratch_get(stream, bytes)) != nullptr)
+      return launch_flat_tc(vectors, vec_ids, n, dim, queries, nq, k, metric, mask, out, scratch, stream);
+  }
+  const FlatPlan p = plan_flat_f32(n, nq, k, forced_splits);
   if (p.scratch_bytes) {
     scratch = scratch_get(stream, p.scratch_bytes);
     if (!scratch) return (int)cudaErrorMemoryAllocation;
@@ -526,11 +537,11 @@ int launch_flat_f32(const float* vectors, const uint32_t* vec_ids, uint32_t n, u
 int launch_flat_f32_planned(const FlatPlan& p, const float* vectors, const uint32_t* vec_ids, uint32_t n,
                             uint32_t dim, const float* queries, uint32_t nq, uint32_t k, MetricType metric,
                             const uint32_t* mask, GpuSearchResult* out, bool fused, void* scratch,
-                            cudaStream_t stream, const QueryFilter* filters) {
+                            cudaStream_t stream, const QueryFilter* filters, const uint32_t* active) {
   const uint32_t qt = p.query_tile, nqb = (nq + qt - 1) / qt;
   const uint32_t splits = p.splits, tps = p.tiles_per_split;
   FlatArgs a{vectors, vec_ids, n, dim, queries, nq, k, mask, out, static_cast<uint64_t*>(scratch), splits, tps,
-             filters};
+             filters, active};
   if (splits > 1 && !a.partial) return (int)cudaErrorMemoryAllocation;
 
   const bool vec4 = (dim % 4 == 0) && ((uintptr_t)vectors % 16 == 0) && ((uintptr_t)queries % 16 == 0);
@@ -568,7 +579,7 @@ int launch_flat_f32_planned(const FlatPlan& p, const float* vectors, const uint3
     const uint32_t pow2 = next_pow2(splits * k);
     const size_t msmem = (size_t)pow2 * 8;
     cudaFuncSetAttribute(merge_partial_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem);
-    merge_partial_topk_kernel<<<nq, 256, msmem, stream>>>(a.partial, splits, k, pow2, vec_ids, out, k);
+    merge_partial_topk_kernel<<<nq, 256, msmem, stream>>>(a.partial, splits, k, pow2, vec_ids, out, k, active);
     note_launch();
   }
   return (int)cudaGetLastError();

@@ -91,11 +91,13 @@ struct FlatPlan {
   size_t scratch_bytes = 0;  // per-split lists (0 when one split)
 };
 FlatPlan plan_flat_f32(uint32_t n, uint32_t nq, uint32_t k, uint32_t forced_splits);
-// fused = true accumulates fmaf(diff, diff, acc) (L2 only): the coarse quantizer
+// fused = true accumulates fmaf(diff, diff, acc) (L2 only): the coarse quantizer;
+// active: only the flagged queries are scanned and written
 int launch_flat_f32_planned(const FlatPlan& p, const float* vectors, const uint32_t* vec_ids, uint32_t n,
                             uint32_t dim, const float* queries, uint32_t nq, uint32_t k, MetricType metric,
                             const uint32_t* mask, GpuSearchResult* out, bool fused, void* scratch,
-                            cudaStream_t stream, const QueryFilter* filters = nullptr);
+                            cudaStream_t stream, const QueryFilter* filters = nullptr,
+                            const uint32_t* active = nullptr);
 int launch_flat_f32(const float* vectors, const uint32_t* vec_ids, uint32_t n, uint32_t dim, const float* queries,
                     uint32_t nq, uint32_t k, MetricType metric, const uint32_t* mask, GpuSearchResult* out,
                     uint32_t forced_splits, cudaStream_t stream, const QueryFilter* filters = nullptr);
@@ -128,6 +130,39 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
 // The scratch bytes launch_tc_scan takes from the stream's arena for the
 // same arguments (same plan, same tuning knobs).
 size_t tc_scan_scratch_bytes(const TcTables& t, uint32_t nq, uint32_t k, MetricType metric, const FvScanOptions& opt);
+
+// The collecting pass behind the exact flat scan's tensor-core filter
+// (tc_scan.cu): every row whose ranking value max(floor, qnorm + row_norm -
+// 2 <q16, row16>) is at most the query's bound, which is a bound on the
+// rank-th smallest value, raised by margin_rel |b| + margin_norm |qnorm| +
+// margin_abs. Rows that did not fit a list are those at or above the largest
+// key of a full list (a list's entry 0, the sentinel when it is not full).
+struct TcCollect {
+  const void* rows16;      // [n][padded_dim] fp16
+  const float* row_norms;  // [n]
+  uint32_t n, dim, padded_dim, nq;
+  uint32_t rank, room;     // bound rank; rows per query that the lists should hold
+  const void* q16;         // [query_rows][padded_dim] fp16, zero past nq
+  const float* qnorm;      // [nq]
+  float floor, margin_rel, margin_norm, margin_abs;
+  const uint32_t* mask;
+  // set by launch_tc_collect, inside its scratch
+  uint64_t* partial;       // [nq][lists][kl]
+  uint32_t lists, kl;
+  float* bound;            // [nq]
+  uint32_t* flags;         // [nq], zero
+};
+// scratch of the pass and the rows its query table must have; 0: no bound can
+// be found for this shape
+size_t tc_collect_bytes(const TcCollect& c, uint32_t* query_rows);
+int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream);
+
+// exact flat scan behind a tensor-core filter (flat_tc.cu): the scratch it
+// takes, 0 where the plain scan is the better (or only) way
+size_t flat_tc_bytes(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, MetricType metric);
+int launch_flat_tc(const float* vectors, const uint32_t* vec_ids, uint32_t n, uint32_t dim, const float* queries,
+                   uint32_t nq, uint32_t k, MetricType metric, const uint32_t* mask, GpuSearchResult* out,
+                   void* scratch, cudaStream_t stream);
 
 // IVF-PQ / IVF-SQ8 search (ivf.cu)
 struct IvfLaunch {

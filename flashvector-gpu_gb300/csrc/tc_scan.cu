@@ -307,12 +307,17 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
 // query, NV values per thread in registers (the rest re-read from L2), the
 // answer built bit by bit from the top of the ordered representation by
 // counting values: 32 rounds of NV compares and one barrier. Also clears the
-// query's re-scan flag.
+// query's re-scan flag. A scan whose distances carry an error raises the
+// bound b to b + m.rel |b| + m.per_norm qnorm[q] + m.abs.
+struct TauMargin {
+  float rel = 1e-6f, per_norm = 0.f, abs = 0.f;
+  const float* qnorm = nullptr;
+};
 constexpr int TAU_THREADS = 128;
 template <int NV>
 __global__ void __launch_bounds__(TAU_THREADS) tc_tau_kernel(const float* __restrict__ pmin, uint32_t cnt,
-                                                             uint32_t stride, uint32_t r, float* __restrict__ tau,
-                                                             uint32_t* __restrict__ redo) {
+                                                             uint32_t stride, uint32_t r, TauMargin m,
+                                                             float* __restrict__ tau, uint32_t* __restrict__ redo) {
   __shared__ uint32_t part[2][TAU_THREADS / 32];
   const uint32_t q = blockIdx.x, tid = threadIdx.x;
   const float* src = pmin + (size_t)q * stride;
@@ -340,14 +345,15 @@ __global__ void __launch_bounds__(TAU_THREADS) tc_tau_kernel(const float* __rest
   }
   if (tid == 0) {
     const float t = order_float(ans);
-    tau[q] = t < kSentinelDist ? t + 1e-6f * fabsf(t) : kSentinelDist;
+    const float up = m.rel * fabsf(t) + m.abs + (m.qnorm ? m.per_norm * fabsf(m.qnorm[q]) : 0.f);
+    tau[q] = t < kSentinelDist ? t + up : kSentinelDist;
     redo[q] = 0u;
   }
 }
 
-void launch_tau(const float* pmin, uint32_t nq, uint32_t cnt, uint32_t stride, uint32_t r, float* tau, uint32_t* redo,
-                cudaStream_t stream) {
-  auto go = [&](auto kern) { kern<<<nq, TAU_THREADS, 0, stream>>>(pmin, cnt, stride, r, tau, redo); };
+void launch_tau(const float* pmin, uint32_t nq, uint32_t cnt, uint32_t stride, uint32_t r, const TauMargin& m,
+                float* tau, uint32_t* redo, cudaStream_t stream) {
+  auto go = [&](auto kern) { kern<<<nq, TAU_THREADS, 0, stream>>>(pmin, cnt, stride, r, m, tau, redo); };
   if (cnt <= 4 * TAU_THREADS)
     go(tc_tau_kernel<4>);
   else if (cnt <= 8 * TAU_THREADS)
@@ -477,13 +483,16 @@ struct TcPlan {
   size_t scratch_bytes = 0;
 };
 
-TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metric, const FvScanOptions& opt) {
+// rank > 0: a collecting pass (launch_tc_collect): the bound is for the rank
+// best rows, and the heaps have room for k.
+TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metric, const FvScanOptions& opt,
+                    uint32_t rank = 0) {
   TcPlan P{};
   const bool fp8 = t.fp8;
   const uint32_t elem = fp8 ? 1 : 2;
   const uint32_t kb_elems = fp8 ? 128 : 64;
   const uint32_t kblocks = (t.padded_dim + kb_elems - 1) / kb_elems;
-  const TuneEntry* te = tune_lookup(fp8, (int)metric, t.dim, t.n, nq, k);
+  const TuneEntry* te = rank ? nullptr : tune_lookup(fp8, (int)metric, t.dim, t.n, nq, k);
   const uint32_t overfetch = opt.overfetch ? opt.overfetch : (te && te->overfetch > 0 ? (uint32_t)te->overfetch : 4u);
   const uint32_t shortlist = t.vectors ? std::min<uint32_t>(std::max(k, overfetch * k), 4096u) : k;
   // short K (at most two 64-element fp16 / 128-element fp8 blocks per tile):
@@ -547,11 +556,12 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
                                         (ntiles + 2047u) / 2048u);
   const uint32_t pstride =
       stride_knob > 0 ? (uint32_t)std::min<int64_t>(std::max<int64_t>(2, stride_knob), 1 << 20) : auto_stride;
-  const int64_t pmargin = tune_value("tc.prepass_margin", 0);
+  const int64_t pmargin = rank ? 0 : tune_value("tc.prepass_margin", 0);
+  const uint32_t ranked = rank ? rank : shortlist;  // rows that the bound is for
   const uint32_t psampled = (ntiles + pstride - 1) / pstride;
   const uint32_t pr =
-      std::max<uint32_t>(1u, pmargin > 0 ? (uint32_t)((pmargin * shortlist + pstride - 1) / pstride)
-                                         : (pstride == 1 ? shortlist : poisson_rank((double)shortlist / pstride, 1e-7)));
+      std::max<uint32_t>(1u, pmargin > 0 ? (uint32_t)((pmargin * ranked + pstride - 1) / pstride)
+                                         : (pstride == 1 ? ranked : poisson_rank((double)ranked / pstride, 1e-7)));
   const size_t part_bytes = align_up((size_t)nq * splits * groups * kl * 8, 256);
   // The coarsest minima (fewest to store and to select from) that still number
   // 8 r, so that two of a query's r best rows seldom share one. They live in
@@ -711,7 +721,7 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
     if (e != cudaSuccess) return (int)e;
     {
       ProfScope ps("tc_tau", stream);
-      launch_tau(p.pmin, nq, P.pcount, P.pcount, P.pr, tau, redo, stream);
+      launch_tau(p.pmin, nq, P.pcount, P.pcount, P.pr, TauMargin{}, tau, redo, stream);
       note_launch();
     }
   }
@@ -766,6 +776,78 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
     note_launch();
   }
   return (int)cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// Collecting pass (flat_tc.cu): the minima pass and the bounded scan over
+// prepared fp16 rows and queries, ranking by max(floor, qnorm + norm -
+// 2 dot). Leaves the range lists and the bounds for the caller to finish.
+// ---------------------------------------------------------------------------
+static TcPlan plan_collect(const TcCollect& c) {
+  const TcTables t{false, c.rows16, c.row_norms, nullptr, nullptr, c.n, c.dim, c.padded_dim};
+  return plan_tc_scan(t, c.nq, c.room, METRIC_L2, FvScanOptions{0, 0, 0.f, 0}, c.rank);
+}
+
+size_t tc_collect_bytes(const TcCollect& c, uint32_t* query_rows) {
+  const TcPlan P = plan_collect(c);
+  if (!P.prepass) return 0;
+  *query_rows = P.nq_rows;
+  return P.part_bytes + P.tau_bytes;
+}
+
+int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream) {
+  const TcPlan P = plan_collect(c);
+  if (!P.prepass) return FV_ERR_ARG;
+  c.partial = static_cast<uint64_t*>(scratch);
+  c.bound = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + P.part_bytes);
+  c.flags = reinterpret_cast<uint32_t*>(c.bound + c.nq);
+  c.lists = P.splits * P.groups;
+  c.kl = P.kl;
+  const uint64_t row_bytes = (uint64_t)c.padded_dim * 2;
+  CUtensorMap ta, tb, tb_half;
+  if (!encode_tmap(&ta, c.q16, false, c.padded_dim, P.nq_rows, row_bytes, TC_M) ||
+      !encode_tmap(&tb, c.rows16, false, c.padded_dim, c.n, row_bytes, TC_N) ||
+      (P.pair && !encode_tmap(&tb_half, c.rows16, false, c.padded_dim, c.n, row_bytes, TC_N / 2)))
+    return FV_ERR_ARG;
+  TcScanArgs a{};
+  a.n = c.n;
+  a.nq = c.nq;
+  a.kblocks = P.kblocks;
+  a.nqb = P.nqb;
+  a.xnorm = c.row_norms;
+  a.qnorm = c.qnorm;
+  a.mask = c.mask;
+  a.floor = c.floor;
+  a.status = status_word();
+  const int64_t wl = tune_value("tc.wait_limit_ns", 0);
+  a.wait_ns = wl > 0 ? (uint64_t)wl : 2000000000ull;
+  auto scan = [&](const TcScanArgs& args, int kl_t, uint32_t splits_n, const char* name) -> cudaError_t {
+    ProfScope ps(name, stream);
+    return dispatch_tc_scan_fp16(kl_t, P.pair ? -1 : P.groups, METRIC_L2, true, ta, P.pair ? tb_half : tb, args,
+                                 (P.pair ? P.nqb_grid : P.nqb) * splits_n, stream);
+  };
+  TcScanArgs p = a;
+  p.splits = P.psplits;
+  p.tiles_per_split = P.ptps;
+  p.tile_stride = P.pstride;
+  p.pmin = reinterpret_cast<float*>(c.partial);
+  p.pm_stride = P.pcount;
+  p.gran = P.pgran;
+  cudaError_t e = scan(p, 0, P.psplits, "tc_prepass_fp16");
+  if (e != cudaSuccess) return (int)e;
+  {
+    ProfScope ps("tc_tau", stream);
+    const TauMargin m{c.margin_rel, c.margin_norm, c.margin_abs, c.qnorm};
+    launch_tau(p.pmin, c.nq, P.pcount, P.pcount, P.pr, m, c.bound, c.flags, stream);
+    note_launch();
+  }
+  a.splits = P.splits;
+  a.tiles_per_split = P.tps;
+  a.tile_stride = 1;
+  a.partial = c.partial;
+  a.kl = P.kl;
+  a.qbound = c.bound;
+  return (int)scan(a, (int)P.kl_tmpl, P.splits, "tc_scan_fp16");
 }
 
 }  // namespace fv

@@ -62,6 +62,7 @@ struct TcScanArgs {
   const QueryFilter* filters;  // per-query filters over slots (== logical ids), or null
   const float* qbound;         // per-query admission bound (distance), or null
   const uint32_t* active;      // per-query flags: only flagged queries are scanned (null: all)
+  float floor;                 // L2: lower limit of a distance (0, or -inf for a ranking value that may be negative)
   uint32_t tile_stride;        // scan every tile_stride-th 256-row tile (a sample when > 1)
   uint64_t wait_ns;            // limit of the pipeline's waits (the drains keep their own)
   // minima pass only: the smallest distance of every `gran` consecutive
@@ -257,9 +258,12 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
   if constexpr (PAIR) tc::cluster_sync();  // both CTAs' barriers exist before either signals the other's
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  // one K block per tile: the query tile is loaded once (with the first base
-  // tile, into stage 0) and stays resident; only base tiles stream after it
-  const bool a_resident = !PAIR && a.kblocks == 1;
+  // K blocks that fit the query-tile buffers: the query tile is loaded once
+  // (block kb with the first base tile's, into buffer kb) and stays resident;
+  // only base tiles stream after it (with two K blocks and the query tile
+  // reloaded, a third of the L2 traffic was query tiles)
+  constexpr uint32_t A_BUFS = G == 4 ? 1 : STAGES;
+  const bool a_resident = !PAIR && a.kblocks <= A_BUFS;
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
             const bool load_a = !a_resident || i == 0;
             tc::mbar_arrive_expect_tx(&full[stage], (load_a ? A_STAGE : 0) + B_STAGE);
             if (load_a)
-              tc::tma_load_2d(sA + stage * A_STAGE, &tmA, &full[stage], (int32_t)(kb * kb_elems),
+              tc::tma_load_2d(sA + (a_resident ? kb : stage) * A_STAGE, &tmA, &full[stage], (int32_t)(kb * kb_elems),
                               (int32_t)(qb * TC_M), pol_a);
             tc::tma_load_2d(sB + stage * B_STAGE, &tmB, &full[stage], (int32_t)(kb * kb_elems), row_b, pol_b);
           }
@@ -331,7 +335,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
             break;
           }
           tc::tc_fence_after();
-          const uint32_t a_base = tc::smem_addr(sA + (a_resident ? 0u : stage * A_STAGE));
+          const uint32_t a_base = tc::smem_addr(sA + (a_resident ? kb : stage) * A_STAGE);
           const uint32_t b_base = tc::smem_addr(sB + stage * b_stage);
 #pragma unroll
           for (uint32_t kk = 0; kk < 4; ++kk) {
@@ -553,7 +557,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
           auto chunk = [&](auto fu_tag) {
             constexpr bool FU = decltype(fu_tag)::value;
             // per-column values v, v[0..32) columns c0.., v[32..64) columns
-            // c0+32..; the distance is D(v): L2  D(v) = max(0, ||q||^2 + v) with
+            // c0+32..; the distance is D(v): L2  D(v) = max(floor, ||q||^2 + v) with
             // v = ||x||^2 - 2 <q, x> (the query's norm is added after the
             // minimum, D being monotone), IP  D(v) = v = -<q, x>, cosine the
             // full expression. FP8 cosine dots carry the query and table scales.
@@ -591,7 +595,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
             // D: distance from v (fused fp8: from the accumulator, v = sc * acc)
             auto D = [&](float x) {
               if (FU) x *= sc;
-              return METRIC == METRIC_L2 ? fmaxf(0.f, qn + x) : x;
+              return METRIC == METRIC_L2 ? fmaxf(a.floor, qn + x) : x;
             };
             // better(x, y): the smaller v, i.e. the larger accumulator when fused
             auto better = [](float x, float y) { return FU ? fmaxf(x, y) : fminf(x, y); };

@@ -350,6 +350,10 @@ int fv_profile_summary(char* buf, size_t len);
  *                       other short-row scans with two (heaps of <= 48);
  *                       2 or 4: that many wherever the four-group form
  *                       applies. Same answers
+ *   "flat.tc"           -1 (default): large exact scans find the rows worth
+ *                       an exact distance with a tensor-core pass over fp16
+ *                       copies made per call (same answer bit for bit); 0:
+ *                       never; 1: for every shape that the pass takes
  *   "tc.wait_limit_ns"  0 (default): the tensor-core scan's pipeline waits give
  *                       up after 2 s; n > 0: after n ns. A wait that runs
  *                       out ends the scan early (its answer is not valid)

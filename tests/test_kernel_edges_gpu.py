@@ -119,3 +119,46 @@ def test_flat_query_tiles_and_list_lengths(cuda, oracle_mod, metric, nq, n, dim,
     ref = oracle_mod.exact_knn(base, queries, k, metric, mask=mask)
     assert np.array_equal(r[..., 0].view(np.uint32), ref["id"])
     assert np.array_equal(r[..., 1].view(np.uint32), ref["distance"].view(np.uint32))
+
+
+@pytest.mark.parametrize("metric", ["l2", "ip", "cosine"])
+@pytest.mark.parametrize("data", ["normal", "integers", "shifted", "outliers", "tiny", "huge", "duplicates", "broken",
+                                  "sorted"])
+@pytest.mark.parametrize("n,dim,nq,k,masked", [(2048, 8, 32, 1, False), (2305, 33, 130, 10, True),
+                                               (9001, 100, 65, 256, False), (40_003, 256, 48, 100, True)])
+def test_filtered_flat_scan_equals_plain(cuda, metric, data, n, dim, nq, k, masked):
+    """The exact scan behind the tensor-core filter returns the plain scan's
+    answer bit for bit: ordinary rows, ties, a common offset, rows far outside
+    the others' scale, values near the ends of fp32, equal rows, zero and
+    non-finite rows and queries, rows in order of distance."""
+    from fvgb300 import datasets, scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(n + dim)
+    x = torch.randn((n, dim), generator=g, device="cuda")
+    q = torch.randn((nq, dim), generator=g, device="cuda")
+    if data == "integers":
+        x, q = (x * 3).round(), (q * 3).round()
+    elif data == "shifted":
+        x, q = x + 300.0, q + 300.0
+    elif data == "outliers":
+        x[::97] *= 5000.0
+        q[::7] *= 5000.0
+    elif data == "tiny":
+        x, q = x * 1e-21, q * 1e-21
+    elif data == "huge":
+        x, q = x * 1e17, q * 1e17
+    elif data == "duplicates":
+        x = x[torch.randint(0, 40, (n,), generator=g, device="cuda")]
+    elif data == "broken":
+        x[5], x[n - 1, 0], x[7], q[3], q[4, 0], q[5, -1] = 0.0, float("nan"), float("inf"), 0.0, float("nan"), -float("inf")
+    elif data == "sorted":
+        x = x[torch.argsort((x - q[0]).square().sum(1))]
+    mask = torch.from_numpy(datasets.bernoulli_mask_words(n, 0.5, 9).view(np.int32)).cuda() if masked else None
+    ids = torch.randperm(4 * n, generator=g, device="cuda")[:n].to(torch.int32) if masked else None
+    with scan.tuned(flat_tc=0):
+        ref = scan.flat_scan(x, q, k, metric, mask=mask, vec_ids=ids)
+    with scan.tuned(flat_tc=1):
+        got = scan.flat_scan(x, q, k, metric, mask=mask, vec_ids=ids)
+    torch.cuda.synchronize()
+    assert torch.equal(got, ref)
