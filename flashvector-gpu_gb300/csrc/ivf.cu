@@ -28,15 +28,19 @@
 // the results are bit-identical to the oracle's restatement.
 //
 // Machine mapping. The coarse probe is the exact flat scan kernel in its
-// fused-FMA mode (a Q x nlist tiled scan with a fused top-nprobe). The list
-// scan is one persistent launch: CTAs pull queries from a device work
-// counter and drain that query's (query, list) pairs: per pair the LUT (or
-// the query residual) is built in shared memory, the posting list is
-// streamed with 16-byte code loads (contiguous rows when the codes are laid
-// out list-major, gathered by id in the reference's layout), and a running
-// shortlist is kept in shared memory: rows whose key cannot beat the
-// current shortlist's worst key are dropped, the rest are appended to a
-// buffer that is bitonic-merged into the shortlist when it fills.
+// fused-FMA mode (a Q x nlist tiled scan with a fused top-nprobe), or the
+// tensor-core candidates below. The list scan is one persistent launch: CTAs
+// pull queries from a device work counter. The query's probed lists are taken
+// up to 32 at a time; their postings form one sequence that the CTA's threads
+// walk together, so a list costs no barriers of its own and short lists share
+// a round (most lists of a Zipf base hold a fraction of one). What a list
+// needs first is made for all of them at once: RaBitQ query codes one warp per
+// list; SQ8 subtracts the centroid on the fly. PQ builds the 256-entry tables
+// only for lists with enough postings to use them (they read the whole
+// codebook, 128 KB at m = 32) and evaluates the few table entries that a short
+// list needs in place, in the same operations. A running shortlist is kept in
+// shared memory: rows whose key cannot beat its worst key are dropped, the
+// rest are appended to a buffer that is sorted into it when it fills.
 #include <cuda_fp16.h>
 
 #include "../../include/fv_bridge.h"
@@ -87,9 +91,11 @@ struct IvfArgs {
   const QueryFilter* filters;     // per-query filters over ids, or null
   const GpuSearchResult* probes;  // [nq][nprobe] coarse result (id = list)
   uint32_t* work;                 // work counter (zeroed before the launch)
+  const uint32_t* order;          // queries in the order they are pulled, or null (as given)
   GpuSearchResult* out;
   uint32_t* status;
   uint32_t keys_pow2;             // pow2(largest shortlist + IVF_BUF)
+  uint32_t list_chunk;            // probed lists walked as one sequence (<= 32)
   uint32_t items_per_q;           // G: a query's probed postings are cut into G ranges
   uint64_t* partial;              // G > 1: [nq * G][part_stride] sorted shortlists of the ranges
   uint32_t part_stride;           // >= every query's shortlist
@@ -127,27 +133,38 @@ __device__ __forceinline__ ListSpan list_span(const IvfArgs& a, uint32_t l) {
 // Rerank of a query's shortlist keys[0, S) (sorted, sentinels last) with the
 // reference's warp-order fp32 distance, sort, and the query's top k into
 // out[q][0, top_k) (sentinels past k). Block-collective.
+template <uint32_t R, int B>
 __device__ void ivf_finish_query(const IvfArgs& a, uint64_t* keys, uint32_t q, uint32_t S, uint32_t kq,
                                  bool do_rerank, const float* qv) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (do_rerank) {
-    // Two candidates per warp pass (c and c + NW, both owned by warp c % NW
-    // as with one at a time), so two rows' gathers are in flight per warp.
+    // R candidates per warp pass (c, c + NW, .., all owned by warp c % NW as
+    // with one at a time), so R rows' gathers, B loads ahead each, are in
+    // flight per warp.
     constexpr uint32_t NW = IVF_THREADS / 32;
-    for (uint32_t c0 = warp; c0 < S; c0 += 2 * NW) {
-      const uint32_t c1 = c0 + NW;
-      const uint64_t k0 = keys[c0], k1 = c1 < S ? keys[c1] : kSentinelKey;
-      const bool v0 = k0 != kSentinelKey && key_slot(k0) < a.num_vectors;
-      const bool v1 = k1 != kSentinelKey && key_slot(k1) < a.num_vectors;
-      if (!v0 && !v1) continue;
-      // an unused slot re-reads the other (valid) row and its result is dropped
-      const uint32_t s0 = key_slot(v0 ? k0 : k1), s1 = key_slot(v1 ? k1 : k0);
-      const float* const rows[2] = {a.vectors + (size_t)s0 * a.dim, a.vectors + (size_t)s1 * a.dim};
-      float d[2];
-      warp_metric_distances<2, 4>(qv, rows, a.dim, lane, (MetricType)a.metric, d);
+    for (uint32_t c0 = warp; c0 < S; c0 += R * NW) {
+      if (keys[c0] == kSentinelKey) break;  // sorted: the rest are sentinels too
+      const float* rows[R];
+      uint32_t slot[R];
+      bool any = false;
+#pragma unroll
+      for (uint32_t r = 0; r < R; ++r) {
+        const uint32_t c = c0 + r * NW;
+        const uint64_t key = c < S ? keys[c] : kSentinelKey;
+        const bool ok = key != kSentinelKey && key_slot(key) < a.num_vectors;
+        // an unused slot reads row 0 and its result is dropped
+        slot[r] = ok ? key_slot(key) : kInvalidId;
+        rows[r] = a.vectors + (size_t)(ok ? slot[r] : 0u) * a.dim;
+        any = any || ok;
+      }
+      if (!any) continue;
+      float d[R];
+      warp_metric_distances<R, B>(qv, rows, a.dim, lane, (MetricType)a.metric, d);
+      __syncwarp();
       if (lane == 0) {
-        if (v0) keys[c0] = make_key(d[0], s0);
-        if (v1) keys[c1] = make_key(d[1], s1);
+#pragma unroll
+        for (uint32_t r = 0; r < R; ++r)
+          if (slot[r] != kInvalidId) keys[c0 + r * NW] = make_key(d[r], slot[r]);
       }
     }
     const uint32_t p2 = next_pow2_dev(S);
@@ -171,19 +188,29 @@ __host__ __device__ __forceinline__ uint32_t ivf_clamps(uint32_t& top_k, uint32_
   return s < MAX_SHORTLIST ? s : MAX_SHORTLIST;
 }
 
+constexpr uint32_t LIST_CHUNK = 32;
+
 struct IvfSmem {
-  // [keys_pow2] u64 keys | table | query (dim f32) | PQ: query residual to the probed centroid (dim f32)
-  // table: PQ LUT (m*256 f32); SQ8 residual+mins+scales (3*dim f32);
-  //        RaBitQ rotated query (P f32) + rotated residual (P f32) + bit-planes (4*W u32)
-  __host__ __device__ static size_t table_floats(int mode, uint32_t dim, uint32_t m_pq, uint32_t P) {
-    return mode == IVF_PQ ? (size_t)m_pq * 256 : mode == IVF_SQ8 ? (size_t)3 * dim : (size_t)2 * P + P / 8;
+  // [keys_pow2] u64 keys | table | query (dim f32) | PQ: query residual to the
+  // probed centroid (dim f32) | the lists of a chunk: first posting, list,
+  // postings before it (3 LC + 1 u32)
+  // table: PQ LUT (m*256 f32); SQ8 mins+scales (2*dim f32); RaBitQ rotated
+  //        query (P f32) + per list of a chunk its query code (4*W u32
+  //        bit-planes, min, delta, sum u, centroid distance)
+  __host__ __device__ static size_t table_floats(int mode, uint32_t dim, uint32_t m_pq, uint32_t P, uint32_t lc) {
+    return mode == IVF_PQ ? (size_t)m_pq * 256
+                          : mode == IVF_SQ8 ? ((size_t)2 * dim + 3) / 4 * 4 : (size_t)P + (size_t)lc * (P / 8 + 4);
   }
-  static size_t bytes(int mode, uint32_t keys_pow2, uint32_t dim, uint32_t m_pq, uint32_t P) {
+  static size_t bytes(int mode, uint32_t keys_pow2, uint32_t dim, uint32_t m_pq, uint32_t P, uint32_t lc) {
     size_t b = (size_t)keys_pow2 * 8;
-    b += table_floats(mode, dim, m_pq, P) * 4;
-    b += (size_t)dim * 4;
+    b += table_floats(mode, dim, m_pq, P, lc) * 4;
+    b += ((size_t)dim + 3) / 4 * 16;
     if (mode == IVF_PQ) b += (size_t)dim * 4;
-    return b + 64;
+    return b + (3 * lc + 1) * 4;
+  }
+  // SQ8 with staged rows: the warps' staging areas follow, 16-byte aligned
+  static size_t staged_bytes(uint32_t keys_pow2, uint32_t dim, uint32_t lc) {
+    return (bytes(IVF_SQ8, keys_pow2, dim, 0, 0, lc) + 15) / 16 * 16 + (size_t)(IVF_THREADS / 32) * (2 * 32 * 80);
   }
 };
 
@@ -219,18 +246,14 @@ __device__ void rabitq_rotate_query(float* rq, const float* qs, const IvfArgs& a
 // (ivf_quant_lookup.cu:381-460): diff = rq - rot_centroid over all P
 // coordinates, u = clamp(rint((diff - min) * (15 / range)), 0, 15) (all 0
 // when range <= 1e-12), bit-plane j word w bit l = bit j of u[32 w + l].
-// Writes planes[4][W]; returns (min, delta = range / 15, sum u) in s_par.
-// Block-collective.
-__device__ void rabitq_query_code(const float* rq, float* rdiff, uint32_t* planes, const IvfArgs& a, uint32_t l,
-                                  float* s_par) {
-  __shared__ float s_lo[IVF_THREADS / 32], s_hi[IVF_THREADS / 32];
-  __shared__ uint32_t s_sum;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+// Writes planes[4][W], then min, delta = range / 15, sum u (exact: at most
+// 15 * 4096) and the query's distance to the centroid. Warp-collective.
+__device__ void rabitq_query_code(const float* rq, uint32_t* code, const IvfArgs& a, uint32_t l, float qc) {
+  const int lane = threadIdx.x & 31;
   const float* rc = a.rot_centroids + (size_t)l * a.P;
   float lo = 1e30f, hi = -1e30f;
-  for (uint32_t d = tid; d < a.P; d += IVF_THREADS) {
+  for (uint32_t d = lane; d < a.P; d += 32) {
     const float v = __fsub_rn(rq[d], __ldg(rc + d));
-    rdiff[d] = v;
     lo = fminf(lo, v);
     hi = fmaxf(hi, v);
   }
@@ -239,44 +262,33 @@ __device__ void rabitq_query_code(const float* rq, float* rdiff, uint32_t* plane
     lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
-  if (lane == 0) {
-    s_lo[warp] = lo;
-    s_hi[warp] = hi;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    for (int w = 1; w < IVF_THREADS / 32; ++w) {
-      lo = fminf(lo, s_lo[w]);
-      hi = fmaxf(hi, s_hi[w]);
-    }
-    const float range = __fsub_rn(hi, lo);
-    const bool live = range > 1e-12f;
-    s_par[0] = lo;
-    s_par[1] = live ? __fdiv_rn(range, 15.0f) : 0.f;
-    s_par[2] = live ? __fdiv_rn(15.0f, range) : 0.f;
-    s_sum = 0;
-  }
-  __syncthreads();
-  const float qmin = s_par[0], delta = s_par[1], inv = s_par[2];
+  const float range = __fsub_rn(hi, lo);
+  const bool live = range > 1e-12f;
+  const float delta = live ? __fdiv_rn(range, 15.0f) : 0.f;
+  const float inv = live ? __fdiv_rn(15.0f, range) : 0.f;
   uint32_t su = 0;
-  for (uint32_t w = warp; w < a.W; w += IVF_THREADS / 32) {
+  for (uint32_t w = 0; w < a.W; ++w) {
     uint32_t u = 0;
     if (delta > 0.f) {
-      const int qi = __float2int_rn(__fmul_rn(__fsub_rn(rdiff[w * 32 + lane], qmin), inv));
+      const float v = __fsub_rn(rq[w * 32 + lane], __ldg(rc + w * 32 + lane));
+      const int qi = __float2int_rn(__fmul_rn(__fsub_rn(v, lo), inv));
       u = (uint32_t)min(max(qi, 0), 15);
     }
     su += u;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t pj = __ballot_sync(0xffffffffu, (u >> j) & 1u);
-      if (lane == 0) planes[j * a.W + w] = pj;
+      if (lane == 0) code[j * a.W + w] = pj;
     }
   }
   su = __reduce_add_sync(0xffffffffu, su);
-  if (lane == 0 && su) atomicAdd(&s_sum, su);
-  __syncthreads();
-  if (tid == 0) s_par[3] = (float)s_sum;  // exact: sum u <= 15 * 4096
-  __syncthreads();
+  if (lane == 0) {
+    float* par = reinterpret_cast<float*>(code + 4 * a.W);
+    par[0] = lo;
+    par[1] = delta;
+    par[2] = (float)su;
+    par[3] = qc;
+  }
 }
 
 // RaBitQ estimate of one posting from s_bu = sum_j 2^j popc(bits & plane_j)
@@ -363,68 +375,220 @@ __device__ __forceinline__ float adc_words(const float* __restrict__ lut, const 
   return s;
 }
 
-// SQ8: squared L2 between the query residual and the decoded row.
-__device__ __forceinline__ float sq8_row(const float* __restrict__ qres, const float* __restrict__ mins,
-                                         const float* __restrict__ scales, const uint8_t* __restrict__ row,
-                                         uint32_t dim, bool vec16) {
+// PQ: ADC of one row without tables: the entry of each sub-space evaluated in
+// place with the table's operations (the residual to the list's centroid
+// rounded once per dimension, fmaf in sub-dimension order), added in sub-space
+// order. Eight sub-spaces' codewords are in flight at a time where rows of
+// four dimensions load as float4 (v4).
+template <typename CodeAt>
+__device__ __forceinline__ float adc_direct(const IvfArgs& a, const float* qs, const float* __restrict__ cent,
+                                            CodeAt code, bool v4) {
   float s = 0.f;
-  uint32_t d = 0;
-  if (vec16) {
-    for (; d + 16 <= dim; d += 16) {
-      const uint4 w = __ldg(reinterpret_cast<const uint4*>(row + d));
-      const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+  if (v4) {
+    const float4* cb = reinterpret_cast<const float4*>(a.codebooks);
+    const float4* cc = reinterpret_cast<const float4*>(cent);
+    constexpr uint32_t B = 4;
+    for (uint32_t m0 = 0; m0 < a.m_pq; m0 += B) {
+      float4 w[B], c[B];
 #pragma unroll
-      for (int b = 0; b < 16; ++b) {
-        const float c = (float)((ws[b >> 2] >> ((b & 3) * 8)) & 0xFFu);
-        const float rec = fmaf(c, scales[d + b], mins[d + b]);
-        const float t = qres[d + b] - rec;
-        s = fmaf(t, t, s);
+      for (uint32_t b = 0; b < B; ++b) {
+        const uint32_t m = min(m0 + b, a.m_pq - 1);
+        w[b] = __ldg(cb + (size_t)m * 256 + code(m));
+        c[b] = __ldg(cc + m);
+      }
+#pragma unroll
+      for (uint32_t b = 0; b < B; ++b) {
+        if (m0 + b >= a.m_pq) break;
+        const float4 q = *reinterpret_cast<const float4*>(qs + (m0 + b) * 4);
+        const float t0 = __fsub_rn(__fsub_rn(q.x, c[b].x), w[b].x), t1 = __fsub_rn(__fsub_rn(q.y, c[b].y), w[b].y);
+        const float t2 = __fsub_rn(__fsub_rn(q.z, c[b].z), w[b].z), t3 = __fsub_rn(__fsub_rn(q.w, c[b].w), w[b].w);
+        s = __fadd_rn(s, fmaf(t3, t3, fmaf(t2, t2, fmaf(t1, t1, fmaf(t0, t0, 0.f)))));
       }
     }
+    return s;
   }
-  for (; d < dim; ++d) {
+  for (uint32_t m = 0; m < a.m_pq; ++m) {
+    const float* cb = a.codebooks + ((size_t)m * 256 + code(m)) * a.sub_dim;
+    float e = 0.f;
+    for (uint32_t sd = 0; sd < a.sub_dim; ++sd) {
+      const uint32_t d = m * a.sub_dim + sd;
+      const float t = __fsub_rn(__fsub_rn(qs[d], __ldg(cent + d)), __ldg(cb + sd));
+      e = fmaf(t, t, e);
+    }
+    s = __fadd_rn(s, e);
+  }
+  return s;
+}
+
+// SQ8: squared L2 between the query's residual to the list's centroid and the
+// decoded row, in dimension order; one row per thread (where the staging below
+// does not fit).
+__device__ __forceinline__ float sq8_row(const float* qs, const float* __restrict__ cent, const float* mins,
+                                         const float* scales, const uint8_t* __restrict__ row, uint32_t dim) {
+  float s = 0.f;
+  for (uint32_t d = 0; d < dim; ++d) {
     const float rec = fmaf((float)__ldg(row + d), scales[d], mins[d]);
-    const float t = qres[d] - rec;
+    const float t = __fsub_rn(__fsub_rn(qs[d], __ldg(cent + d)), rec);
     s = fmaf(t, t, s);
   }
   return s;
 }
 
-// MODE: PQ, SQ8 or RaBitQ. MW > 0: code rows of 16 * MW bytes at 16-byte-
-// aligned rows (PQ m_pq = 16, 32, 64; RaBitQ P = 128 MW with 16-byte-aligned
-// meta rows), scanned by the register-prefetching loop with R postings per
-// thread per round, software-pipelined across rounds (PIPE).
+// SQ8, staged: a warp scores 2 x 32 rows, each lane two of them, 64 dimensions
+// at a time. The rows' codes come in through shared memory by whole segments
+// (a lane reading its own row touches one line per 16 bytes: 32 L1 wavefronts
+// where the segment takes 8), and one read of the query, centroid and decoding
+// parameters serves both rows. Rows may start at any byte: words are loaded
+// aligned and shifted into place. A byte becomes a float by taking the
+// mantissa's place in 2^23. row[i]: the lane's rows (null: none).
+// Warp-collective.
+constexpr uint32_t SQ_CHUNK = 64;   // dimensions per staged chunk
+constexpr uint32_t SQ_STRIDE = 80;  // bytes per staged row: 17 words, 16-byte steps off the same bank
+constexpr uint32_t SQ_WARP_BYTES = 2 * 32 * SQ_STRIDE;
+__device__ __forceinline__ void sq8_rows(const float* qs, const float* const (&cent)[2], const float* mins,
+                                         const float* scales, const uint8_t* const (&row)[2], uint32_t dim,
+                                         bool aligned, bool cent16, uint8_t* stage, float (&out)[2]) {
+  const uint32_t lane = threadIdx.x & 31u;
+  out[0] = out[1] = 0.f;
+  for (uint32_t d0 = 0; d0 < dim; d0 += SQ_CHUNK) {
+    const uint32_t nd = min(SQ_CHUNK, dim - d0);
+    __syncwarp();  // the previous chunk is consumed
+    if (aligned) {
+      // four lanes a row, 16 bytes each
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint4 w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t r = 8 * j + (lane >> 2), c = (lane & 3u) * 16;
+          const uint64_t p = __shfl_sync(0xffffffffu, (uint64_t)(uintptr_t)row[i], r);
+          w[j] = p && c < nd ? __ldg(reinterpret_cast<const uint4*>(p + d0 + c)) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t r = 8 * j + (lane >> 2), c = (lane & 3u) * 16;
+          *reinterpret_cast<uint4*>(stage + (i * 32 + r) * SQ_STRIDE + c) = w[j];
+        }
+      }
+    } else {
+      // a half-warp a row, one aligned word each, and a 17th word where the
+      // row's chunk reaches into it
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+#pragma unroll 4
+        for (int j = 0; j < 16; ++j) {
+          const uint32_t r = 2 * j + (lane >> 4), c = (lane & 15u) * 4;
+          const uint64_t p = __shfl_sync(0xffffffffu, (uint64_t)(uintptr_t)row[i], r);
+          const uint64_t at = (p + d0) & ~(uint64_t)3, end = p + d0 + nd;
+          if (p && at + c < end)
+            *reinterpret_cast<uint32_t*>(stage + (i * 32 + r) * SQ_STRIDE + c) =
+                __ldg(reinterpret_cast<const uint32_t*>(at + c));
+        }
+        const uint64_t p = (uint64_t)(uintptr_t)row[i];
+        const uint64_t at = ((p + d0) & ~(uint64_t)3) + 64;
+        if (p && at < p + d0 + nd)
+          *reinterpret_cast<uint32_t*>(stage + (i * 32 + lane) * SQ_STRIDE + 64) =
+              __ldg(reinterpret_cast<const uint32_t*>(at));
+      }
+    }
+    __syncwarp();
+    const uint32_t sh0 = 8 * ((uint32_t)((uintptr_t)row[0] + d0) & 3u), sh1 = 8 * ((uint32_t)((uintptr_t)row[1] + d0) & 3u);
+    const uint8_t* st0 = stage + lane * SQ_STRIDE;
+    const uint8_t* st1 = st0 + 32 * SQ_STRIDE;
+    auto term = [&](float& s, uint32_t w, int b, float qd, float cd, float m, float k) {
+      const float code = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + b)) - 8388608.0f;  // exact
+      const float t = __fsub_rn(__fsub_rn(qd, cd), fmaf(code, k, m));
+      s = fmaf(t, t, s);
+    };
+    if (aligned && cent16) {
+      for (uint32_t d = 0; d < nd; d += 16) {
+        const uint4 wa = *reinterpret_cast<const uint4*>(st0 + d), wb = *reinterpret_cast<const uint4*>(st1 + d);
+        const uint32_t a4[4] = {wa.x, wa.y, wa.z, wa.w}, b4[4] = {wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t at = d0 + d + 4 * j;
+          const float4 q = *reinterpret_cast<const float4*>(qs + at);
+          const float4 mn = *reinterpret_cast<const float4*>(mins + at);
+          const float4 sc = *reinterpret_cast<const float4*>(scales + at);
+          const float4 ca = __ldg(reinterpret_cast<const float4*>(cent[0] + at));
+          const float4 cb = cent[1] == cent[0] ? ca : __ldg(reinterpret_cast<const float4*>(cent[1] + at));
+          term(out[0], a4[j], 0, q.x, ca.x, mn.x, sc.x);
+          term(out[1], b4[j], 0, q.x, cb.x, mn.x, sc.x);
+          term(out[0], a4[j], 1, q.y, ca.y, mn.y, sc.y);
+          term(out[1], b4[j], 1, q.y, cb.y, mn.y, sc.y);
+          term(out[0], a4[j], 2, q.z, ca.z, mn.z, sc.z);
+          term(out[1], b4[j], 2, q.z, cb.z, mn.z, sc.z);
+          term(out[0], a4[j], 3, q.w, ca.w, mn.w, sc.w);
+          term(out[1], b4[j], 3, q.w, cb.w, mn.w, sc.w);
+        }
+      }
+    } else {
+      for (uint32_t d = 0; d < nd; d += 4) {
+        const uint32_t* pa = reinterpret_cast<const uint32_t*>(st0 + d);
+        const uint32_t* pb = reinterpret_cast<const uint32_t*>(st1 + d);
+        const uint32_t wa = __funnelshift_r(pa[0], pa[1], sh0), wb = __funnelshift_r(pb[0], pb[1], sh1);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const uint32_t at = d0 + d + b;
+          if (at >= dim) break;
+          const float q = qs[at], mn = mins[at], sc = scales[at];
+          const float ca = __ldg(cent[0] + at), cb = cent[1] == cent[0] ? ca : __ldg(cent[1] + at);
+          term(out[0], wa, b, q, ca, mn, sc);
+          term(out[1], wb, b, q, cb, mn, sc);
+        }
+      }
+    }
+  }
+}
+
+// A PQ list of at least this many postings gets its tables: building them
+// reads the whole codebook and costs about as much as evaluating 128 rows in
+// place (32 of the 8,192 entries each).
+constexpr uint32_t PQ_TABLE_MIN = 128;
+
 // Resident CTAs per SM each variant is compiled for (its register budget:
 // 4 -> 64, 3 -> 85, 2 -> 128 registers per thread): the list scans are
 // load-latency bound, so occupancy is worth more than registers.
-template <int MODE, int MW, bool PIPE>
+template <int MODE, int MW>
 constexpr int ivf_min_blocks() {
-  return (MODE == IVF_PQ && (MW == 4 || (PIPE && MW == 2))) ? 2 : (PIPE || (MODE == IVF_RABITQ && MW >= 4)) ? 3 : 4;
+  return MODE == IVF_PQ ? (MW == 4 ? 2 : 3) : MODE == IVF_RABITQ && MW >= 4 ? 3 : 4;
 }
 
-template <int MODE, int MW, int R = 4, bool PIPE = false>
-__global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW, PIPE>()) ivf_scan_kernel(IvfArgs a) {
+// MODE: PQ, SQ8 or RaBitQ. MW > 0: code rows of 16 * MW bytes at 16-byte-
+// aligned rows (PQ m_pq = 16, 32, 64; RaBitQ P = 128 MW with 16-byte-aligned
+// meta rows; SQ8 with staged rows, MW = 1, R = 2), R postings per thread per
+// round, all their loads before any is scored.
+template <int MODE, int MW, int R>
+__global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_scan_kernel(IvfArgs a) {
   // a round offers at most IVF_THREADS * R candidates, appended after the
   // shortlist; the buffer is flushed between rounds, so one round must fit
   static_assert((uint32_t)IVF_THREADS * R <= IVF_BUF, "a round of postings must fit the candidate buffer");
+  constexpr uint32_t step = IVF_THREADS * R;
+  constexpr int MWW = MW > 0 && MODE != IVF_SQ8 ? MW : 1;
   extern __shared__ __align__(16) uint8_t smem[];
   uint64_t* keys = reinterpret_cast<uint64_t*>(smem);
   float* tab = reinterpret_cast<float*>(smem + (size_t)a.keys_pow2 * 8);
-  float* qs = tab + IvfSmem::table_floats(MODE, a.dim, a.m_pq, a.P);
-  __shared__ uint32_t s_q, s_cnt;
+  float* qs = tab + IvfSmem::table_floats(MODE, a.dim, a.m_pq, a.P, a.list_chunk);
+  float* qres = qs + (a.dim + 3) / 4 * 4;  // PQ only: q - centroid of the probed list
+  uint32_t* s_beg = reinterpret_cast<uint32_t*>(qres + (MODE == IVF_PQ ? a.dim : 0));
+  uint32_t* s_list = s_beg + a.list_chunk;     // top bit: s_beg indexes the admitted positions
+  uint32_t* s_cum = s_list + a.list_chunk;     // [chunk + 1] postings of the sequence before each list
+  __shared__ uint32_t s_q, s_cnt, s_long;
   __shared__ uint64_t s_tau;
+  __shared__ unsigned long long s_total;
+  __shared__ float s_red[MODE == IVF_RABITQ ? IVF_THREADS : 1];
 
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float* mins = tab;                     // SQ8 only
+  float* scales = tab + a.dim;
+  float* rq = tab;                       // RaBitQ only: rotated query, list codes
+  uint32_t* codes = reinterpret_cast<uint32_t*>(tab + a.P);
+  const uint32_t code_words = 4 * a.W + 4;
+  const bool cb4 = MODE == IVF_PQ && a.sub_dim == 4 && ((uintptr_t)a.codebooks % 16u) == 0;
   const bool vec16 = (a.code_bytes % 16u) == 0 && ((uintptr_t)a.codes % 16u) == 0;
-  float* mins = tab + a.dim;      // SQ8 only
-  float* scales = tab + 2 * a.dim;
-  float* qres = qs + a.dim;       // PQ only: q - centroid of the probed list
-  float* rq = tab;                // RaBitQ only: rotated query, rotated residual, bit-planes
-  float* rdiff = tab + a.P;
-  uint32_t* planes = reinterpret_cast<uint32_t*>(tab + 2 * a.P);
-  __shared__ float s_par[4];      // RaBitQ: min, delta, 15 / range, sum u of the list's query code
-  __shared__ float s_red[IVF_THREADS];
-  const bool cb4 = a.sub_dim == 4 && ((uintptr_t)a.codebooks % 16u) == 0;
+  const bool cent16 = a.dim % 4 == 0 && ((uintptr_t)a.centroids % 16u) == 0;
+  uint8_t* stage = smem + ((reinterpret_cast<uint8_t*>(s_cum + a.list_chunk + 1) - smem) + 15) / 16 * 16 +
+                   warp * SQ_WARP_BYTES;  // SQ8, MW = 1
 
   if (MODE == IVF_SQ8) {
     for (uint32_t d = tid; d < a.dim; d += IVF_THREADS) {
@@ -433,7 +597,6 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW, PIPE>())
     }
   }
 
-  __shared__ unsigned long long s_total;
   const uint32_t G = a.items_per_q;
   while (true) {
     __syncthreads();
@@ -441,7 +604,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW, PIPE>())
     __syncthreads();
     const uint32_t item = s_q;
     if (item >= a.nq * G) break;
-    const uint32_t q = item / G, g = item % G;
+    const uint32_t q = a.order ? __ldg(a.order + item / G) : item / G, g = item % G;
     uint32_t kq = a.q_topk ? __ldg(a.q_topk + q) : a.top_k;
     uint32_t npq = a.q_nprobe ? __ldg(a.q_nprobe + q) : a.nprobe;
     const uint32_t rrq = a.q_rerank ? __ldg(a.q_rerank + q) : a.rerank_k;
@@ -450,6 +613,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW, PIPE>())
     kq = min(kq, a.top_k);
     const bool do_rerank = rrq != 1u && a.vectors != nullptr;
     const QueryFilter qf = load_filter(a.filters, q);
+    const GpuSearchResult* probes = a.probes + (size_t)q * a.nprobe;
 
     const float* qv = a.queries + (size_t)q * a.dim;
     for (uint32_t d = tid; d < a.dim; d += IVF_THREADS) qs[d] = __ldg(qv + d);
@@ -457,20 +621,24 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW, PIPE>())
     if (tid == 0) {
       s_cnt = 0;
       s_tau = kSentinelKey;
+    }
+    if (G > 1 && warp == 0) {
+      // the query's probed postings, to cut this item's range out of
       unsigned long long total = 0;
-      if (G > 1)
-        for (uint32_t p = 0; p < npq; ++p) {
-          const uint32_t l = a.probes[(size_t)q * a.nprobe + p].id;
-          if (l < a.nlist) {
-            const ListSpan sp = list_span(a, l);
-            total += sp.end - sp.beg;
-          }
+      for (uint32_t p = lane; p < npq; p += 32) {
+        const uint32_t l = probes[p].id;
+        if (l < a.nlist) {
+          const ListSpan sp = list_span(a, l);
+          total += sp.end - sp.beg;
         }
-      s_total = total;
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+      if (lane == 0) s_total = total;
     }
     __syncthreads();
     float qn = 0.f;  // RaBitQ, inner product: ||q||^2
-    if (MODE == IVF_RABITQ) {
+    if constexpr (MODE == IVF_RABITQ) {
       if (a.metric == METRIC_INNER_PRODUCT) {
         // in the order of the reference's 256-thread block
         // (ivf_quant_lookup.cu:686-697): strided fmaf partials, pairwise fold
@@ -489,7 +657,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW, PIPE>())
     // this item's range of the query's probed postings (lists in probe order)
     const uint64_t lo = G > 1 ? s_total * g / G : 0ull;
     const uint64_t hi = G > 1 ? s_total * (g + 1) / G : ~0ull;
-    uint64_t cum = 0;
+    uint64_t cum = 0;  // postings of the lists before this chunk (warp 0)
 
     auto flush = [&]() {
       // keys[0, S) sorted shortlist, keys[S, S + cnt) new candidates
@@ -505,195 +673,340 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW, PIPE>())
       }
       __syncthreads();
     };
+    // one posting per lane into the buffer (warp-collective): `at` is its id,
+    // or its list position when the id has not been needed so far
+    auto offer = [&](bool pass, float d, uint32_t at, bool is_pos, uint64_t tau) {
+      pass = pass && d < kSentinelDist && float_order(d) <= (uint32_t)(tau >> 32);
+      uint64_t key = 0;
+      if (pass) {
+        key = make_key(d, is_pos ? __ldg(a.vec_ids + at) : at);
+        pass = key < tau;
+      }
+      const uint32_t m = __ballot_sync(0xffffffffu, pass);
+      if (m == 0u) return;
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(&s_cnt, (uint32_t)__popc(m));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (pass) keys[S + base + __popc(m & ((1u << lane) - 1u))] = key;
+    };
+    // Posting i of a span: whether it exists and, where the mask's list-order
+    // bits cover it, is admitted (its code row is loaded then), whether it is
+    // to be scored (also the id-based mask and the query's filter), its list
+    // position, and its id where that was needed.
+    struct Post {
+      uint32_t pos, id;
+      bool in, ok, has_id;
+    };
+    auto fetch = [&](uint32_t i, bool in, bool compact) {
+      Post p;
+      bool bits = true;
+      p.pos = i;
+      if (compact) {  // i indexes the admitted positions: all pass the mask
+        p.pos = in ? __ldg(a.adm_pos + i) : 0u;
+      } else if (a.mask != nullptr) {
+        bits = a.list_allow != nullptr && i < a.list_n;
+        if (in && bits) in = (__ldg(a.list_allow + (i >> 5)) >> (i & 31u)) & 1u;
+      }
+      p.has_id = !a.list_major || qf.words != nullptr || !bits;
+      p.id = in && p.has_id ? __ldg(a.vec_ids + p.pos) : 0u;
+      p.in = p.ok = in;
+      if (p.has_id && in) p.ok = (bits || mask_allows(a.mask, p.id)) && filter_allows(qf, p.id);
+      return p;
+    };
 
-    for (uint32_t p = 0; p < npq; ++p) {
-      const uint32_t l = a.probes[(size_t)q * a.nprobe + p].id;
-      if (l >= a.nlist) continue;  // uniform over the block
-      const ListSpan sp = list_span(a, l);
-      const uint32_t lbeg = sp.beg, llen = sp.end - sp.beg;
-      const bool compact = sp.compact;  // uniform over the block
-      const uint64_t s0 = max(lo, cum), s1 = min(hi, cum + llen);
-      const uint64_t at = cum;
-      cum += llen;
-      if (s0 >= s1) continue;  // uniform: the list lies outside this item's range
-      const float* cent = a.centroids + (size_t)l * a.dim;
-      if (MODE == IVF_PQ) {
-        // LUT[m][c] = sum_sd ((q - centroid) - codeword)^2 with fmaf in
-        // sub-dimension order; q - centroid is rounded once per dimension, as
-        // the reference's expression rounds it (ivf_pq_lookup.cu:150-162)
-        for (uint32_t d = tid; d < a.dim; d += IVF_THREADS) qres[d] = qs[d] - __ldg(cent + d);
-        __syncthreads();
-        const uint32_t entries = a.m_pq * 256;
-        if (cb4) {
-          const float4* cbv = reinterpret_cast<const float4*>(a.codebooks);
-          auto entry = [&](uint32_t e, float4 w) {  // codeword (m, c) = row e of 4 floats
-            const float* r = qres + (e >> 8) * 4;
-            const float t0 = r[0] - w.x, t1 = r[1] - w.y, t2 = r[2] - w.z, t3 = r[3] - w.w;
-            tab[e] = fmaf(t3, t3, fmaf(t2, t2, fmaf(t1, t1, fmaf(t0, t0, 0.f))));
-          };
-          // B codeword loads in flight per thread before any is used (the
-          // codebooks, 16 KB per sub-space, stream from L2 for every list)
-          constexpr uint32_t B = MW >= 2 ? 8 : 4;  // fewer where the register budget is small
-          uint32_t e0 = tid;
-          for (; e0 + (B - 1) * IVF_THREADS < entries; e0 += B * IVF_THREADS) {
-            float4 w[B];
-#pragma unroll
-            for (uint32_t b = 0; b < B; ++b) w[b] = __ldg(cbv + e0 + b * IVF_THREADS);
-#pragma unroll
-            for (uint32_t b = 0; b < B; ++b) entry(e0 + b * IVF_THREADS, w[b]);
-          }
-          for (uint32_t e = e0; e < entries; e += IVF_THREADS) entry(e, __ldg(cbv + e));
-        } else {
-          for (uint32_t e = tid; e < entries; e += IVF_THREADS) {
-            const uint32_t m = e >> 8, c = e & 255u;
-            const float* cb = a.codebooks + ((size_t)m * 256 + c) * a.sub_dim;
-            float s = 0.f;
-            for (uint32_t sd = 0; sd < a.sub_dim; ++sd) {
-              const float t = qres[m * a.sub_dim + sd] - __ldg(cb + sd);
-              s = fmaf(t, t, s);
-            }
-            tab[e] = s;
+    for (uint32_t c0 = 0; c0 < npq; c0 += a.list_chunk) {
+      const uint32_t nl = min(a.list_chunk, npq - c0);
+      if (warp == 0) {
+        // this item's part of each list, one list per lane
+        uint32_t l = 0xFFFFFFFFu, beg = 0, len = 0;
+        bool compact = false;
+        if (lane < (int)nl) {
+          l = probes[c0 + lane].id;
+          if (l < a.nlist) {
+            const ListSpan sp = list_span(a, l);
+            beg = sp.beg;
+            len = sp.end - sp.beg;
+            compact = sp.compact;
           }
         }
-      } else if (MODE == IVF_SQ8) {
-        for (uint32_t d = tid; d < a.dim; d += IVF_THREADS) tab[d] = qs[d] - __ldg(cent + d);
-      } else {
-        rabitq_query_code(rq, rdiff, planes, a, l, s_par);
+        unsigned long long before = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned long long y = __shfl_up_sync(0xffffffffu, before, o);
+          if (lane >= o) before += y;
+        }
+        const unsigned long long all = __shfl_sync(0xffffffffu, before, 31);
+        before = cum + before - len;
+        const uint64_t s0 = max((uint64_t)before, lo), s1 = min((uint64_t)before + len, hi);
+        cum += all;
+        if (s0 < s1) {
+          beg += (uint32_t)(s0 - before);
+          len = (uint32_t)(s1 - s0);
+        } else {
+          len = 0;
+        }
+        // a PQ list that is worth its tables leaves the common sequence
+        const bool tables = MODE == IVF_PQ && len >= PQ_TABLE_MIN;
+        const uint32_t longs = __ballot_sync(0xffffffffu, tables);
+        uint32_t x = tables ? 0u : len;
+        const uint32_t own = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+          if (lane >= o) x += y;
+        }
+        if (lane < (int)nl) {
+          s_beg[lane] = beg;
+          s_list[lane] = (l & 0x7FFFFFFFu) | (compact ? 0x80000000u : 0u);
+          s_cum[lane] = tables ? len : x - own;  // (a tabled list's entry: its length, see below)
+        }
+        if (lane == 0) s_long = longs;
+        if (lane == (int)nl - 1) s_cum[nl] = x;
+      }
+      if constexpr (MODE == IVF_RABITQ) {
+        for (uint32_t p = warp; p < nl; p += IVF_THREADS / 32) {
+          const GpuSearchResult pr = probes[c0 + p];
+          if (pr.id < a.nlist) rabitq_query_code(rq, codes + p * code_words, a, pr.id, pr.distance);
+        }
       }
       __syncthreads();
-      // RaBitQ: the list's query code and the query-to-centroid distance
-      const float qc = MODE == IVF_RABITQ ? a.probes[(size_t)q * a.nprobe + p].distance : 0.f;
-      const float qmin = s_par[0], qdelta = s_par[1], sum_u = s_par[3], Pf = (float)a.P;
 
-      const uint32_t beg = lbeg + (uint32_t)(s0 - at), end = lbeg + (uint32_t)(s1 - at);
-      auto offer = [&](float d, uint32_t vid) {
-        if (d < kSentinelDist) {
-          const uint64_t key = make_key(d, vid);
-          if (key < s_tau) {
-            const uint32_t pos = atomicAdd(&s_cnt, 1u);
-            keys[S + pos] = key;
-          }
-        }
-      };
-      if (MODE != IVF_SQ8 && MW > 0) {
-        // R postings per thread per round: the ids of all of them, then their
-        // mask / filter words, then the code rows of the admitted ones only
-        // (a 10% mask leaves 9 of 10 rows unread), all before any is scored.
-        // PIPE: the next round's loads are issued before this round is
-        // scored, so global-load latency overlaps the LUT arithmetic.
-        constexpr int MWW = MW > 0 ? MW : 1;
-        constexpr uint32_t step = IVF_THREADS * R;
-        auto issue = [&](uint32_t b0, uint32_t (&v)[R], uint4 (&c)[R][MWW], float4 (&mt)[R], bool (&o)[R]) {
-          // in: the posting exists and, where the list-order bits cover it,
-          // the mask admits it -- known from the bit word alone, so the code
-          // rows (list-major: addressed by position) load alongside the ids
-          bool bits[R], in[R];
-          uint32_t pos[R];
+      if constexpr (MODE == IVF_PQ) {
+        uint32_t longs = s_long;  // uniform over the block
+        while (longs) {
+          const uint32_t p = __ffs(longs) - 1;
+          longs &= longs - 1;
+          const uint32_t l = s_list[p] & 0x7FFFFFFFu, beg = s_beg[p], end = beg + s_cum[p];
+          const bool compact = s_list[p] >> 31;
+          const float* cent = a.centroids + (size_t)l * a.dim;
+          // LUT[m][c] = sum_sd ((q - centroid) - codeword)^2 with fmaf in
+          // sub-dimension order; q - centroid is rounded once per dimension, as
+          // the reference's expression rounds it (ivf_pq_lookup.cu:150-162)
+          for (uint32_t d = tid; d < a.dim; d += IVF_THREADS) qres[d] = qs[d] - __ldg(cent + d);
+          __syncthreads();
+          const uint32_t entries = a.m_pq * 256;
+          if (cb4) {
+            const float4* cbv = reinterpret_cast<const float4*>(a.codebooks);
+            auto entry = [&](uint32_t e, float4 w) {  // codeword (m, c) = row e of 4 floats
+              const float* r = qres + (e >> 8) * 4;
+              const float t0 = r[0] - w.x, t1 = r[1] - w.y, t2 = r[2] - w.z, t3 = r[3] - w.w;
+              tab[e] = fmaf(t3, t3, fmaf(t2, t2, fmaf(t1, t1, fmaf(t0, t0, 0.f))));
+            };
+            // B codeword loads in flight per thread before any is used (the
+            // codebooks, 16 KB per sub-space, stream from L2 for every list)
+            constexpr uint32_t B = 8;
+            uint32_t e0 = tid;
+            for (; e0 + (B - 1) * IVF_THREADS < entries; e0 += B * IVF_THREADS) {
+              float4 w[B];
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const uint32_t i = b0 + r * IVF_THREADS + tid;
-            if (compact) {  // i indexes the admitted positions: all pass the mask
-              bits[r] = true;
-              in[r] = i < end;
-              pos[r] = in[r] ? __ldg(a.adm_pos + i) : 0u;
-            } else {
-              bits[r] = a.list_allow != nullptr && i < a.list_n;
-              in[r] = i < end && (!bits[r] || ((__ldg(a.list_allow + (i >> 5)) >> (i & 31u)) & 1u));
-              pos[r] = i;
+              for (uint32_t b = 0; b < B; ++b) w[b] = __ldg(cbv + e0 + b * IVF_THREADS);
+#pragma unroll
+              for (uint32_t b = 0; b < B; ++b) entry(e0 + b * IVF_THREADS, w[b]);
             }
-            v[r] = in[r] ? __ldg(a.vec_ids + pos[r]) : 0xFFFFFFFFu;
-          }
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const size_t row_i = a.list_major ? pos[r] : v[r];
-            const uint4* row = reinterpret_cast<const uint4*>(a.codes + row_i * (16u * MW));
-#pragma unroll
-            for (int j = 0; j < MWW; ++j) c[r][j] = in[r] ? __ldg(row + j) : make_uint4(0u, 0u, 0u, 0u);
-            if (MODE == IVF_RABITQ)
-              mt[r] = in[r] ? __ldg(reinterpret_cast<const float4*>(a.rq_meta) + row_i) : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-          // scored: also the id-based mask (positions the bits do not cover)
-          // and the query's filter
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-            o[r] = in[r] && (bits[r] || mask_allows(a.mask, v[r])) && filter_allows(qf, v[r]);
-        };
-        auto score = [&](const uint4 (&c)[MWW], const float4& mt) -> float {
-          if (MODE == IVF_RABITQ)
-            return rabitq_estimate(rabitq_sbu<MWW>(planes, c), mt, Pf, qmin, qdelta, sum_u, qc, qn, a.metric);
-          return adc_words<MWW>(tab, c);
-        };
-        uint32_t vid[R];
-        uint4 w[R][MWW];
-        float4 mt[R];
-        bool ok[R];
-        if (PIPE && beg < end) issue(beg, vid, w, mt, ok);
-        for (uint32_t base = beg; base < end; base += step) {
-          if (PIPE) {
-            uint32_t vn[R];
-            uint4 wn[R][MWW];
-            float4 mn[R];
-            bool okn[R];
-            const bool more = base + step < end;  // uniform over the block
-            if (more) issue(base + step, vn, wn, mn, okn);
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-              if (ok[r]) offer(score(w[r], mt[r]), vid[r]);
-            if (more) {
-#pragma unroll
-              for (int r = 0; r < R; ++r) {
-                vid[r] = vn[r];
-                ok[r] = okn[r];
-                mt[r] = mn[r];
-#pragma unroll
-                for (int j = 0; j < MWW; ++j) w[r][j] = wn[r][j];
-              }
-            }
+            for (uint32_t e = e0; e < entries; e += IVF_THREADS) entry(e, __ldg(cbv + e));
           } else {
-            issue(base, vid, w, mt, ok);
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-              if (ok[r]) offer(score(w[r], mt[r]), vid[r]);
-          }
-          __syncthreads();
-          if (s_cnt > IVF_BUF - step) flush();
-        }
-      } else {
-        for (uint32_t base = beg; base < end; base += IVF_THREADS) {
-          const uint32_t j = base + tid;
-          const bool bits = compact || (a.list_allow != nullptr && j < a.list_n);
-          const uint32_t i = compact ? (j < end ? __ldg(a.adm_pos + j) : 0u) : j;
-          if (j < end && (compact || !bits || ((__ldg(a.list_allow + (i >> 5)) >> (i & 31u)) & 1u))) {
-            const uint32_t vid = __ldg(a.vec_ids + i);
-            if ((bits || mask_allows(a.mask, vid)) && filter_allows(qf, vid)) {
-              const size_t row_i = a.list_major ? i : vid;
-              const uint8_t* row = a.codes + row_i * a.code_bytes;
-              if (MODE == IVF_RABITQ) {
-                const float* mp = a.rq_meta + row_i * 4;
-                const float4 mt = make_float4(__ldg(mp), __ldg(mp + 1), __ldg(mp + 2), __ldg(mp + 3));
-                const uint32_t sbu = rabitq_sbu_any(planes, reinterpret_cast<const uint32_t*>(row), a.W);
-                offer(rabitq_estimate(sbu, mt, Pf, qmin, qdelta, sum_u, qc, qn, a.metric), vid);
-              } else {
-                offer(MODE == IVF_PQ ? adc_row(tab, row, a.m_pq, vec16)
-                                     : sq8_row(tab, mins, scales, row, a.dim, vec16),
-                      vid);
+            for (uint32_t e = tid; e < entries; e += IVF_THREADS) {
+              const uint32_t m = e >> 8, c = e & 255u;
+              const float* cb = a.codebooks + ((size_t)m * 256 + c) * a.sub_dim;
+              float s = 0.f;
+              for (uint32_t sd = 0; sd < a.sub_dim; ++sd) {
+                const float t = qres[m * a.sub_dim + sd] - __ldg(cb + sd);
+                s = fmaf(t, t, s);
               }
+              tab[e] = s;
             }
           }
           __syncthreads();
-          if (s_cnt > IVF_BUF - IVF_THREADS) flush();
+          for (uint32_t base = beg; base < end; base += step) {
+            Post post[R];
+            uint4 w[R][MWW];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const uint32_t i = base + r * IVF_THREADS + tid;
+              post[r] = fetch(i, i < end, compact);
+              if constexpr (MW > 0) {
+                const uint4* row = reinterpret_cast<const uint4*>(
+                    a.codes + (size_t)(a.list_major ? post[r].pos : post[r].id) * (16u * MW));
+#pragma unroll
+                for (int j = 0; j < MWW; ++j) w[r][j] = post[r].in ? __ldg(row + j) : make_uint4(0u, 0u, 0u, 0u);
+              }
+            }
+            const uint64_t tau = s_tau;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              float d = 0.f;
+              if (post[r].ok) {
+                if constexpr (MW > 0)
+                  d = adc_words<MWW>(tab, w[r]);
+                else
+                  d = adc_row(tab, a.codes + (size_t)(a.list_major ? post[r].pos : post[r].id) * a.code_bytes, a.m_pq,
+                              vec16);
+              }
+              offer(post[r].ok, d, post[r].has_id ? post[r].id : post[r].pos, !post[r].has_id, tau);
+            }
+            __syncthreads();
+            if (s_cnt > IVF_BUF - step) flush();
+          }
+        }
+        if (s_long) {
+          // the tabled lists drop out of the sequence: their prefix entry is
+          // the next list's
+          __syncthreads();
+          if (tid == 0)
+            for (int p = (int)nl - 1; p >= 0; --p)
+              if ((s_long >> p) & 1u) s_cum[p] = s_cum[p + 1];
+          __syncthreads();
         }
       }
-      __syncthreads();  // the table is rebuilt for the next list
+
+      // the sequence of the chunk's (other) postings
+      const uint32_t total = s_cum[nl];
+      for (uint32_t base = 0; base < total; base += step) {
+        uint32_t lp[R];
+        Post post[R];
+        uint4 w[R][MWW];
+        float4 mt[MODE == IVF_RABITQ ? R : 1];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t t = base + r * IVF_THREADS + tid;
+          // the last list whose prefix is <= t (empty lists repeat a prefix)
+          uint32_t p = 0;
+#pragma unroll
+          for (uint32_t h = LIST_CHUNK / 2; h; h >>= 1)
+            if (p + h < nl && s_cum[p + h] <= t) p += h;
+          lp[r] = p;
+          post[r] = fetch(s_beg[p] + (t - s_cum[p]), t < total, s_list[p] >> 31);
+          const size_t row = a.list_major ? post[r].pos : post[r].id;
+          if constexpr (MODE != IVF_SQ8 && MW > 0) {
+            const uint4* rw = reinterpret_cast<const uint4*>(a.codes + row * (16u * MW));
+#pragma unroll
+            for (int j = 0; j < MWW; ++j) w[r][j] = post[r].in ? __ldg(rw + j) : make_uint4(0u, 0u, 0u, 0u);
+            if constexpr (MODE == IVF_RABITQ)
+              mt[r] = post[r].in ? __ldg(reinterpret_cast<const float4*>(a.rq_meta) + row)
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+        }
+        const uint64_t tau = s_tau;
+        [[maybe_unused]] float sq[2] = {0.f, 0.f};
+        if constexpr (MODE == IVF_SQ8 && MW > 0) {
+          static_assert(R == 2, "two rows a lane");
+          const uint8_t* rows[2];
+          const float* cents[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            rows[r] = post[r].ok ? a.codes + (size_t)(a.list_major ? post[r].pos : post[r].id) * a.code_bytes : nullptr;
+            // (an unused row is scored against list 0's centroid and dropped)
+            cents[r] = a.centroids + (post[r].ok ? (size_t)(s_list[lp[r]] & 0x7FFFFFFFu) * a.dim : 0);
+          }
+          if (__any_sync(0xffffffffu, post[0].ok || post[1].ok))
+            sq8_rows(qs, cents, mins, scales, rows, a.dim, vec16, cent16, stage, sq);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float d = 0.f;
+          if (MODE == IVF_SQ8 && MW > 0) {
+            d = sq[r & 1];
+          } else if (post[r].ok) {
+            const size_t row = a.list_major ? post[r].pos : post[r].id;
+            const uint32_t l = s_list[lp[r]] & 0x7FFFFFFFu;
+            if constexpr (MODE == IVF_RABITQ) {
+              const uint32_t* code = codes + lp[r] * code_words;
+              const float4 par = *reinterpret_cast<const float4*>(code + 4 * a.W);  // min, delta, sum u, distance
+              if constexpr (MW > 0) {
+                d = rabitq_estimate(rabitq_sbu<MWW>(code, w[r]), mt[r], (float)a.P, par.x, par.y, par.z, par.w, qn,
+                                    a.metric);
+              } else {
+                const float* mp = a.rq_meta + row * 4;
+                const float4 meta = make_float4(__ldg(mp), __ldg(mp + 1), __ldg(mp + 2), __ldg(mp + 3));
+                const uint32_t sbu =
+                    rabitq_sbu_any(code, reinterpret_cast<const uint32_t*>(a.codes + row * a.code_bytes), a.W);
+                d = rabitq_estimate(sbu, meta, (float)a.P, par.x, par.y, par.z, par.w, qn, a.metric);
+              }
+            } else if constexpr (MODE == IVF_PQ) {
+              const float* cent = a.centroids + (size_t)l * a.dim;
+              if constexpr (MW > 0) {
+                // (the code bytes again, from the cache: indexing the registers
+                // by sub-space would spill them)
+                const uint32_t* cw = reinterpret_cast<const uint32_t*>(a.codes + row * (16u * MW));
+                d = adc_direct(a, qs, cent, [&](uint32_t m) { return (__ldg(cw + (m >> 2)) >> (8 * (m & 3))) & 255u; },
+                               cb4 && cent16);
+              } else {
+                const uint8_t* cw = a.codes + row * a.code_bytes;
+                d = adc_direct(a, qs, cent, [&](uint32_t m) { return (uint32_t)__ldg(cw + m); }, cb4 && cent16);
+              }
+            } else {
+              d = sq8_row(qs, a.centroids + (size_t)l * a.dim, mins, scales, a.codes + row * a.code_bytes, a.dim);
+            }
+          }
+          offer(post[r].ok, d, post[r].has_id ? post[r].id : post[r].pos, !post[r].has_id, tau);
+        }
+        __syncthreads();
+        if (s_cnt > IVF_BUF - step) flush();
+      }
+      __syncthreads();  // the chunk's lists and codes are replaced
     }
     flush();
     if (G > 1) {
       // a range's shortlist goes to the merge kernel
-      uint64_t* dst = a.partial + (size_t)item * a.part_stride;
+      uint64_t* dst = a.partial + ((size_t)q * G + g) * a.part_stride;
       for (uint32_t i = tid; i < S; i += IVF_THREADS) dst[i] = keys[i];
       continue;
     }
-    ivf_finish_query(a, keys, q, S, kq, do_rerank, qv);
+    ivf_finish_query<2, 4>(a, keys, q, S, kq, do_rerank, qv);
+  }
+}
+
+// The order in which CTAs pull queries when there are more than run at once:
+// most probed postings first, by half octaves (a counting sort: one warp per
+// query counts and takes a place in its bucket, a second launch turns places
+// into positions). A query over a Zipf base's head list takes several times
+// the mean, and one pulled last had the GPU to itself: 2,000 RaBitQ queries
+// over 1M rows, list scan 1,004 us in the given order.
+constexpr uint32_t ORDER_BUCKETS = 62;  // next to the work counter in its 64 words
+
+__device__ __forceinline__ uint32_t order_bucket(unsigned long long postings) {
+  const uint32_t v = (uint32_t)min(postings, 0x7FFFFFFFull) | 1u;
+  const uint32_t top = 31u - __clz(v);
+  return min(2 * top + (top ? (v >> (top - 1)) & 1u : 0u), ORDER_BUCKETS - 1);
+}
+
+__global__ void __launch_bounds__(256) ivf_order_count_kernel(IvfArgs a, uint32_t* __restrict__ hist,
+                                                              uint32_t* __restrict__ place) {
+  const uint32_t q = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (q >= a.nq) return;
+  uint32_t kq = a.top_k, npq = a.q_nprobe ? __ldg(a.q_nprobe + q) : a.nprobe;
+  ivf_clamps(kq, npq, 1u, a.nlist);
+  npq = min(npq, a.nprobe);
+  unsigned long long total = 0;
+  for (uint32_t p = lane; p < npq; p += 32) {
+    const uint32_t l = a.probes[(size_t)q * a.nprobe + p].id;
+    if (l < a.nlist) {
+      const ListSpan sp = list_span(a, l);
+      total += sp.end - sp.beg;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  if (lane == 0) {
+    const uint32_t b = order_bucket(total);
+    place[q] = atomicAdd(hist + b, 1u) << 6 | b;
+  }
+}
+
+__global__ void __launch_bounds__(256) ivf_order_kernel(uint32_t nq, const uint32_t* __restrict__ hist,
+                                                        const uint32_t* __restrict__ place,
+                                                        uint32_t* __restrict__ order) {
+  __shared__ uint32_t first[ORDER_BUCKETS];
+  if (threadIdx.x < ORDER_BUCKETS) {
+    uint32_t n = 0;  // queries in larger buckets
+    for (uint32_t b = threadIdx.x + 1; b < ORDER_BUCKETS; ++b) n += __ldg(hist + b);
+    first[threadIdx.x] = n;
+  }
+  __syncthreads();
+  const uint32_t q = blockIdx.x * 256 + threadIdx.x;
+  if (q < nq) {
+    const uint32_t p = place[q];
+    order[first[p & 63u] + (p >> 6)] = q;
   }
 }
 
@@ -710,15 +1023,61 @@ __global__ void __launch_bounds__(IVF_THREADS) ivf_merge_kernel(IvfArgs a) {
   const uint32_t S = ivf_clamps(kq, npq, rrq, a.nlist);
   kq = min(kq, a.top_k);
   const bool do_rerank = rrq != 1u && a.vectors != nullptr;
-  const uint32_t total = G * S, p2 = next_pow2_dev(total);
-  for (uint32_t i = threadIdx.x; i < p2; i += IVF_THREADS) {
-    uint64_t v = kSentinelKey;
-    if (i < total) v = a.partial[((size_t)q * G + i / S) * a.part_stride + i % S];
-    keys[i] = v;
+  const uint32_t total = G * S;
+  const uint64_t* src = a.partial + (size_t)q * G * a.part_stride;
+  // The S smallest of the ranges' sorted shortlists. With each thread's keys
+  // in registers their S-th key is built bit by bit by counting (64 rounds of
+  // compares and a barrier), and only S keys are sorted: 64 ranges of 100 took
+  // 127 us as one sort of 8,192 keys.
+  constexpr int NV = 32;
+  if (total > 2 * S && total <= NV * IVF_THREADS) {
+    __shared__ uint32_t part[2][IVF_THREADS / 32];
+    __shared__ uint32_t n_kept;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint64_t kv[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const uint32_t e = (uint32_t)i * IVF_THREADS + threadIdx.x;
+      kv[i] = e < total ? __ldcg(src + (size_t)(e / S) * a.part_stride + e % S) : kSentinelKey;
+    }
+    if (threadIdx.x == 0) n_kept = 0;
+    uint64_t kth = 0;
+    const int used = (int)((total + IVF_THREADS - 1) / IVF_THREADS);
+    for (int bit = 63; bit >= 0; --bit) {
+      const uint64_t test = kth | ((1ull << bit) - 1ull);
+      uint32_t c = 0;
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+        if (i < used) c += kv[i] <= test;
+      c = __reduce_add_sync(0xffffffffu, c);
+      if (lane == 0) part[bit & 1][warp] = c;
+      __syncthreads();
+      uint32_t sum = 0;
+#pragma unroll
+      for (int w = 0; w < IVF_THREADS / 32; ++w) sum += part[bit & 1][w];
+      if (sum < S) kth |= 1ull << bit;
+    }
+    // (fewer than S keys: the S-th is the sentinel, and all keys are kept)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      if (kv[i] <= kth && kv[i] != kSentinelKey) {
+        const uint32_t at = atomicAdd(&n_kept, 1u);
+        if (at < S) keys[at] = kv[i];
+      }
+    }
+    __syncthreads();
+    const uint32_t p2 = next_pow2_dev(S);
+    for (uint32_t i = n_kept + threadIdx.x; i < p2; i += IVF_THREADS) keys[i] = kSentinelKey;
+    __syncthreads();
+    block_bitonic_sort(keys, p2);
+  } else {
+    const uint32_t p2 = next_pow2_dev(total);
+    for (uint32_t i = threadIdx.x; i < p2; i += IVF_THREADS)
+      keys[i] = i < total ? src[(size_t)(i / S) * a.part_stride + i % S] : kSentinelKey;
+    __syncthreads();
+    block_bitonic_sort(keys, p2);
   }
-  __syncthreads();
-  block_bitonic_sort(keys, p2);
-  ivf_finish_query(a, keys, q, S, kq, do_rerank, a.queries + (size_t)q * a.dim);
+  ivf_finish_query<4, 8>(a, keys, q, S, kq, do_rerank, a.queries + (size_t)q * a.dim);
 }
 
 // The mask in list order (one word per 32 list positions), for one call.
@@ -885,7 +1244,25 @@ __global__ void __launch_bounds__(128) coarse_prep_kernel(const float* __restric
 // probe's arithmetic (flat_f32_scan_kernel, FUSED)
 __device__ __forceinline__ float coarse_exact(const float* qv, const float* __restrict__ c, uint32_t dim) {
   float acc = 0.f;
-  for (uint32_t d = 0; d < dim; ++d) {
+  uint32_t d = 0;
+  if (dim % 4 == 0 && (uintptr_t)c % 16 == 0) {
+    for (; d + 32 <= dim; d += 32) {  // eight 16-byte loads in flight
+      float4 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = __ldg(reinterpret_cast<const float4*>(c + d) + i);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 q = *reinterpret_cast<const float4*>(qv + d + 4 * i);
+        const float d0 = __fsub_rn(q.x, v[i].x), d1 = __fsub_rn(q.y, v[i].y);
+        const float d2 = __fsub_rn(q.z, v[i].z), d3 = __fsub_rn(q.w, v[i].w);
+        acc = fmaf(d0, d0, acc);
+        acc = fmaf(d1, d1, acc);
+        acc = fmaf(d2, d2, acc);
+        acc = fmaf(d3, d3, acc);
+      }
+    }
+  }
+  for (; d < dim; ++d) {
     const float diff = __fsub_rn(qv[d], __ldg(c + d));
     acc = fmaf(diff, diff, acc);
   }
@@ -893,8 +1270,12 @@ __device__ __forceinline__ float coarse_exact(const float* qv, const float* __re
 }
 
 // Per query: exact distances of the K candidates, the first nprobe, and the
-// exactness test. flags[q] = 1 sends the query to the exact fallback.
-__global__ void __launch_bounds__(CO_THREADS) coarse_finish_kernel(const float* __restrict__ queries,
+// exactness test. flags[q] = 1 sends the query to the exact fallback. NT
+// threads (>= K, and at least 64): one candidate each; blocks of 256 for 48
+// candidates left most threads idle and two thirds of the queries waiting
+// (2,000 queries: 61 us).
+template <int NT>
+__global__ void __launch_bounds__(NT) coarse_finish_kernel(const float* __restrict__ queries,
                                                                    const float* __restrict__ cent, uint32_t nlist,
                                                                    uint32_t dim, const GpuSearchResult* __restrict__ cand,
                                                                    uint32_t K, uint32_t nprobe,
@@ -903,13 +1284,13 @@ __global__ void __launch_bounds__(CO_THREADS) coarse_finish_kernel(const float* 
                                                                    uint32_t force_exact, uint32_t* __restrict__ flags,
                                                                    GpuSearchResult* __restrict__ probes) {
   extern __shared__ __align__(16) uint8_t co_smem[];
-  uint64_t* keys = reinterpret_cast<uint64_t*>(co_smem);          // [256]
-  float* qv = reinterpret_cast<float*>(co_smem + 256 * 8);        // [dim]
-  __shared__ float s_red[CO_THREADS / 32];
+  uint64_t* keys = reinterpret_cast<uint64_t*>(co_smem);          // [NT]
+  float* qv = reinterpret_cast<float*>(co_smem + NT * 8);         // [dim]
+  __shared__ float s_red[NT / 32];
   const uint32_t q = blockIdx.x;
   const int tid = threadIdx.x;
   float part = 0.f;
-  for (uint32_t d = tid; d < dim; d += CO_THREADS) {
+  for (uint32_t d = tid; d < dim; d += NT) {
     qv[d] = __ldg(queries + (size_t)q * dim + d);
     const float c = __ldg(qc + (size_t)q * dim + d);
     part = fmaf(c, c, part);
@@ -922,15 +1303,15 @@ __global__ void __launch_bounds__(CO_THREADS) coarse_finish_kernel(const float* 
   if (tid < (int)K) {
     const uint32_t id = cq[tid].id;
     keys[tid] = id < nlist ? make_key(coarse_exact(qv, cent + (size_t)id * dim, dim), id) : kSentinelKey;
-  } else if (tid < 256) {
+  } else {
     keys[tid] = kSentinelKey;
   }
   __syncthreads();
-  block_bitonic_sort(keys, 256);
-  for (uint32_t j = tid; j < nprobe; j += CO_THREADS) probes[(size_t)q * nprobe + j] = key_to_result(keys[j], nullptr);
+  block_bitonic_sort(keys, NT);
+  for (uint32_t j = tid; j < nprobe; j += NT) probes[(size_t)q * nprobe + j] = key_to_result(keys[j], nullptr);
   if (tid == 0 && K < nlist) {
     float qn2 = 0.f;
-    for (int w = 0; w < CO_THREADS / 32; ++w) qn2 += s_red[w];
+    for (int w = 0; w < NT / 32; ++w) qn2 += s_red[w];
     const float qn = sqrtf(qn2), cm = __uint_as_float(*cmax);
     const GpuSearchResult last = cq[K - 1];
     const float dnp = key_dist(keys[nprobe - 1]);
@@ -992,9 +1373,10 @@ size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // Committed autotuner results for the IVF scans (tuning/gb300.json
 // "ivf_entries", compiled in by build.py as tuning_ivf.inc): per shape range
-// the list-scan pipelining, the posting-range split and the coarse probe
-// that searched fastest (every choice gives the same answer). Knobs set
-// with fv_tune_set take precedence; "tc.table" = 0 ignores the table.
+// the posting-range split and the coarse probe that searched fastest (every
+// choice gives the same answer; the pipelining they also record belonged to
+// an earlier list scan). Knobs set with fv_tune_set take precedence;
+// "tc.table" = 0 ignores the table.
 struct IvfTuneEntry {
   int mode;
   uint32_t dim_lo, dim_hi;
@@ -1035,7 +1417,7 @@ struct IvfPlan {
   uint32_t P = 0, top_k = 0, nprobe = 0, shortlist = 0, G = 1, sms = 0, list_n = 0, nwords = 0, adm_blocks = 0;
   // tensor-core coarse probe: candidates per query and the byte offsets of
   // its buffers in the coarse part of the scratch
-  bool tcc = false, force_exact = false, pipeline = false;
+  bool tcc = false, force_exact = false;
   uint32_t K = 0;
   size_t co_mu = 0, co_c16 = 0, co_cnorm = 0, co_qc = 0, co_cand = 0, co_flags = 0, co_cmax = 0, co_tc = 0;
   FlatPlan cp;
@@ -1065,7 +1447,6 @@ IvfPlan plan_ivf_search(int mode, const IvfLaunch& L) {
   // them. "ivf.split": -1 automatic, 0 / 1 never, G > 1 force G.
   const uint32_t sms = (uint32_t)device_sm_count();
   const IvfTuneEntry* te = ivf_tune_lookup(mode, L.dim, L.num_vectors, L.nlist, L.nq, nprobe);
-  Q.pipeline = ivf_knob("ivf.pipeline", te ? te->pipeline : -1, 0) == 1;
   const int64_t split_knob = ivf_knob("ivf.split", te ? te->split : -1, -1);
   uint32_t G = 1;
   if (split_knob > 1)
@@ -1162,14 +1543,16 @@ static int launch_coarse_tc(const IvfPlan& Q, const IvfLaunch& L, uint8_t* scrat
   int rc = launch_tc_scan_ext(ct, qc, L.nq, Q.K, METRIC_L2, nullptr, cand, copt, stream, nullptr, scratch + Q.co_tc,
                               flags);
   if (rc != 0) return rc;
-  const size_t fsmem = 256 * 8 + (size_t)L.dim * 4;
+  const uint32_t fthreads = Q.K <= 64 ? 64u : 256u;
+  const size_t fsmem = fthreads * 8 + (size_t)L.dim * 4;
+  auto finish = fthreads == 64 ? coarse_finish_kernel<64> : coarse_finish_kernel<256>;
   const size_t xsmem = 4096 * 8 + (size_t)L.dim * 4;
-  e = cudaFuncSetAttribute(coarse_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
+  e = cudaFuncSetAttribute(finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(coarse_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xsmem);
   if (e != cudaSuccess) return (int)e;
-  coarse_finish_kernel<<<L.nq, CO_THREADS, fsmem, stream>>>(L.queries, L.centroids, L.nlist, L.dim, cand, Q.K, Q.nprobe,
-                                                           qc, cmax, Q.force_exact ? 1u : 0u, flags, probes);
+  finish<<<L.nq, fthreads, fsmem, stream>>>(L.queries, L.centroids, L.nlist, L.dim, cand, Q.K, Q.nprobe, qc, cmax,
+                                            Q.force_exact ? 1u : 0u, flags, probes);
   coarse_exact_kernel<<<L.nq, CO_THREADS, xsmem, stream>>>(L.queries, L.centroids, L.nlist, L.dim, Q.nprobe, flags,
                                                           probes);
   note_launch(2);
@@ -1214,7 +1597,7 @@ int launch_ivf_search(int mode, const IvfLaunch& L, cudaStream_t stream) {
                                  nullptr, probes, true, cp.scratch_bytes ? scratch : nullptr, stream);
   }
   if (rc != 0) return rc;
-  cudaError_t e = cudaMemsetAsync(work, 0, sizeof(uint32_t), stream);
+  cudaError_t e = cudaMemsetAsync(work, 0, 256, stream);  // the counter and the order's buckets
   if (e != cudaSuccess) return (int)e;
   if (list_n) {
     ProfScope ps("ivf_list_mask", stream);
@@ -1283,36 +1666,51 @@ int launch_ivf_search(int mode, const IvfLaunch& L, cudaStream_t stream) {
   a.partial = partial;
   a.part_stride = shortlist;
 
-  const size_t smem = IvfSmem::bytes(mode, a.keys_pow2, L.dim, L.m_pq, P);
+  // (calls near the limit walk four lists at a time, in the shared memory that
+  // one list's tables take)
+  a.list_chunk = LIST_CHUNK;
+  size_t smem = IvfSmem::bytes(mode, a.keys_pow2, L.dim, L.m_pq, P, a.list_chunk);
+  if (smem > 224 * 1024) {
+    a.list_chunk = 4;
+    smem = IvfSmem::bytes(mode, a.keys_pow2, L.dim, L.m_pq, P, a.list_chunk);
+  }
   if (smem > 227 * 1024) return FV_ERR_ARG;
+  const size_t staged = mode == IVF_SQ8 ? IvfSmem::staged_bytes(a.keys_pow2, L.dim, a.list_chunk) : 0;
+  const bool stage_rows = staged > 0 && staged <= 227 * 1024;
+  if (stage_rows) smem = staged;
   const bool rows16 = mode == IVF_PQ && ((uintptr_t)L.codes % 16u) == 0;
-  // "ivf.pipeline": 1 software-pipelines the PQ list scan (2 postings per
-  // thread per round, next round's loads in flight while scoring). Off by
-  // default: its 78 registers allow 3 CTAs per SM where the plain loop
-  // (60 registers, 4 postings per round) runs 4, which measured 7% faster.
-  const bool pipe = Q.pipeline;
-  auto kern = ivf_scan_kernel<IVF_SQ8, 0>;
+  auto kern = stage_rows ? ivf_scan_kernel<IVF_SQ8, 1, 2> : ivf_scan_kernel<IVF_SQ8, 0, 1>;
   if (mode == IVF_RABITQ) {
     // bits rows of P/8 bytes as 16-byte words when they and the meta rows
     // are 16-byte aligned; R postings per thread per round as registers allow
     const bool al = ((uintptr_t)L.rq_bits % 16u) == 0 && ((uintptr_t)L.rq_meta % 16u) == 0;
-    kern = ivf_scan_kernel<IVF_RABITQ, 0>;
+    kern = ivf_scan_kernel<IVF_RABITQ, 0, 1>;
     if (al && P == 128) kern = ivf_scan_kernel<IVF_RABITQ, 1, 4>;
     if (al && P == 256) kern = ivf_scan_kernel<IVF_RABITQ, 2, 2>;
     if (al && P == 512) kern = ivf_scan_kernel<IVF_RABITQ, 4, 2>;
     if (al && P == 1024) kern = ivf_scan_kernel<IVF_RABITQ, 8, 1>;
   }
   if (mode == IVF_PQ) {
-    kern = ivf_scan_kernel<IVF_PQ, 0>;
-    if (rows16 && L.m_pq == 16) kern = pipe ? ivf_scan_kernel<IVF_PQ, 1, 2, true> : ivf_scan_kernel<IVF_PQ, 1>;
-    if (rows16 && L.m_pq == 32) kern = pipe ? ivf_scan_kernel<IVF_PQ, 2, 2, true> : ivf_scan_kernel<IVF_PQ, 2>;
-    if (rows16 && L.m_pq == 64) kern = pipe ? ivf_scan_kernel<IVF_PQ, 4, 2, true> : ivf_scan_kernel<IVF_PQ, 4>;
+    kern = ivf_scan_kernel<IVF_PQ, 0, 1>;
+    if (rows16 && L.m_pq == 16) kern = ivf_scan_kernel<IVF_PQ, 1, 4>;
+    if (rows16 && L.m_pq == 32) kern = ivf_scan_kernel<IVF_PQ, 2, 4>;
+    if (rows16 && L.m_pq == 64) kern = ivf_scan_kernel<IVF_PQ, 4, 2>;
   }
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, IVF_THREADS, smem);
-  const uint32_t grid = std::max(1u, std::min<uint32_t>(L.nq * G, (uint32_t)(std::max(1, per_sm) * sms)));
+  const uint32_t slots = (uint32_t)(std::max(1, per_sm) * sms);
+  const uint32_t grid = std::max(1u, (uint32_t)std::min<uint64_t>((uint64_t)L.nq * G, slots));
+  if ((uint64_t)L.nq * G > slots && coarse_bytes >= (size_t)L.nq * 8 && L.nq < (1u << 26)) {
+    // (the coarse probe's part of the scratch is free by now)
+    uint32_t* place = reinterpret_cast<uint32_t*>(scratch);
+    uint32_t* order = place + L.nq;
+    ivf_order_count_kernel<<<(L.nq + 7) / 8, 256, 0, stream>>>(a, work + 1, place);
+    ivf_order_kernel<<<(L.nq + 255) / 256, 256, 0, stream>>>(L.nq, work + 1, place, order);
+    note_launch(2);
+    a.order = order;
+  }
   {
     ProfScope ps(mode == IVF_PQ ? "ivf_pq_scan" : mode == IVF_SQ8 ? "ivf_sq8_scan" : "ivf_rabitq_scan", stream);
     kern<<<grid, IVF_THREADS, smem, stream>>>(a);

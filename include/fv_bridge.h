@@ -363,10 +363,8 @@ int fv_profile_summary(char* buf, size_t len);
  *   "tc.table"          1 (default): knobs left automatic and a zero
  *                       over-fetch take the committed autotuner results
  *                       for the call's shape (tuning/gb300.json); 0: ignore
- *   "ivf.pipeline"      -1 (default): the committed autotuner's choice for
- *                       the call's shape, else 0; 0: the IVF-PQ list scan
- *                       loads and scores 4 postings per thread per round;
- *                       1: 2 per round with the next round's loads in flight
+ *   "ivf.pipeline"      accepted, without effect: it chose between two loops
+ *                       of an earlier IVF-PQ list scan
  *   "ivf.split"         -1 (default): batches of fewer than 4 queries per
  *                       SM cut each query's probed postings into G equal
  *                       ranges scanned by separate CTAs and merged (same

@@ -162,3 +162,45 @@ def test_filtered_flat_scan_equals_plain(cuda, metric, data, n, dim, nq, k, mask
         got = scan.flat_scan(x, q, k, metric, mask=mask, vec_ids=ids)
     torch.cuda.synchronize()
     assert torch.equal(got, ref)
+
+
+def _ivf_case(oracle_mod, n, dim, nlist, m_pq, seed, skew):
+    rng = np.random.default_rng(seed)
+    cent = rng.uniform(-2, 2, (nlist, dim)).astype(np.float32)
+    w = np.arange(1, nlist + 1, dtype=np.float64) ** -skew
+    assign = rng.choice(nlist, n, p=w / w.sum()).astype(np.uint32)
+    x = (cent[assign] + np.float32(0.6) * rng.standard_normal((n, dim))).astype(np.float32)
+    q = (cent[rng.integers(0, nlist, 21)] + np.float32(0.6) * rng.standard_normal((21, dim))).astype(np.float32)
+    t = oracle_mod.build_ivf(x, nlist=nlist, m_pq=m_pq, iters=2, seed=seed)
+    return x, q, t
+
+
+@pytest.mark.parametrize("mode", ["pq", "sq8", "rabitq"])
+@pytest.mark.parametrize("n,dim,nlist,m_pq,nprobe,rerank,skew", [
+    (3000, 64, 200, 16, 200, 33, 1.2),   # several chunks of 32 lists, many empty or of a few postings
+    (6000, 48, 33, 12, 33, 300, 0.5),    # one list over a chunk; PQ codes without 16-byte rows
+    (9000, 128, 12, 32, 9, 1, 1.0),      # lists on both sides of the PQ table threshold, no rerank
+    (2500, 256, 40, 64, 17, 128, 0.8),
+    (700, 20, 7, 5, 7, 64, 0.0),         # ragged rows
+])
+@pytest.mark.parametrize("masked", [False, True])
+def test_ivf_list_sequences(cuda, oracle_mod, mode, n, dim, nlist, m_pq, nprobe, rerank, skew, masked):
+    """The walk over many lists as one sequence: empty lists, lists shorter than
+    a warp, chunk borders, both code layouts, one CTA per query and ranges."""
+    from fvgb300 import datasets, scan
+    from fvgb300.ivf import IvfTable
+
+    torch = cuda
+    x, q, t = _ivf_case(oracle_mod, n, dim, nlist, m_pq, n + dim, skew)
+    mask = datasets.bernoulli_mask_words(n, 0.3, 5) if masked else None
+    fn = {"pq": oracle_mod.ivf_pq_search, "sq8": oracle_mod.ivf_sq_search, "rabitq": oracle_mod.ivf_rabitq_search}[mode]
+    ref = fn(t, x, q, 12, nprobe, rerank, mask=mask)
+    md = None if mask is None else torch.from_numpy(mask.view(np.int32)).cuda()
+    for list_major in (False, True):
+        table = IvfTable(mode, t, vectors=x, list_major=list_major)
+        for split in (0, 3, -1):
+            with scan.tuned(ivf_split=split):
+                r = table.search(torch.from_numpy(q).cuda(), 12, nprobe, rerank, mask=md).cpu().numpy()
+            assert np.array_equal(r[..., 0].view(np.uint32), ref["id"])
+            assert np.array_equal(r[..., 1].view(np.uint32), ref["distance"].view(np.uint32))
+    assert scan.device_status() == 0
