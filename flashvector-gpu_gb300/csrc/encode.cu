@@ -23,6 +23,8 @@
 //    scale_mode): s_v = max|x_v| / 448, codes e4m3(x / s_v), no digits.
 #include <cuda_fp8.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -50,16 +52,15 @@ __device__ __forceinline__ uint16_t f32_to_f16_halfup(float x) {
 // Four values at once: magnitudes in [2^-14, 65504 + rounding) share one
 // exponent shift, and a mantissa that rounds over carries into the exponent
 // (up to infinity) by itself; anything else takes the general conversion.
+__device__ __forceinline__ uint32_t f32_to_f16_normal(uint32_t b, bool& normal) {
+  const uint32_t a = (b & 0x7fffffffu) - 0x38800000u;  // 113 << 23: the exponent of 2^-14
+  normal = normal && a < 0x0f000000u;                  // below 143 << 23: the exponent of 2^16
+  return ((a + 0x00801000u) >> 13) | ((b >> 16) & 0x8000u);
+}
 __device__ __forceinline__ uint2 f32_to_f16_halfup4(float4 v) {
-  const uint32_t b[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
-  uint32_t h[4];
   bool normal = true;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t a = (b[i] & 0x7fffffffu) - 0x38800000u;  // 113 << 23: the exponent of 2^-14
-    normal = normal && a < 0x0f000000u;                     // below 143 << 23: the exponent of 2^16
-    h[i] = ((a + 0x00801000u) >> 13) | ((b[i] >> 16) & 0x8000u);
-  }
+  uint32_t h[4] = {f32_to_f16_normal(__float_as_uint(v.x), normal), f32_to_f16_normal(__float_as_uint(v.y), normal),
+                   f32_to_f16_normal(__float_as_uint(v.z), normal), f32_to_f16_normal(__float_as_uint(v.w), normal)};
   if (!normal) {
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) {
@@ -73,85 +74,94 @@ __device__ __forceinline__ uint2 f32_to_f16_halfup4(float4 v) {
   }
   return make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
 }
+__device__ __forceinline__ uint16_t f32_to_f16_halfup_fast(float v) {
+  bool normal = true;
+  const uint32_t h = f32_to_f16_normal(__float_as_uint(v), normal);
+  return normal ? (uint16_t)h : f32_to_f16_halfup(v);
+}
 
-// A warp encodes 32 rows, 32 dimensions at a time: the chunk is read with
-// whole-row segments (128 bytes a row; 16-byte loads where VEC), converted
-// and stored, and its squares are transposed through shared memory so that
-// lane r adds row r's squares in dimension order. The next chunk's loads are
-// in flight meanwhile. ||x||^2 is a sequential fp32 sum, so the transposition
-// is what lets 32 rows advance together: with one lane per row reading its
-// row alone, 500,000 x 768 took 2,221 us (15% of the copy
-// bandwidth), now 420 us (81%); what is left is the stores' partial lines.
-constexpr int E16_WARPS = 8;
+// A warp encodes 8 rows, 128 dimensions at a time: the chunk is read with
+// whole-row segments (16-byte loads where VEC), converted and stored, and its
+// squares are transposed through shared memory so that lane r adds row r's
+// squares in dimension order. The next chunk's loads are in flight meanwhile.
+// ||x||^2 is a sequential fp32 sum, so the transposition is what lets rows
+// advance together: with one lane per row reading its row alone, 500,000 x 768
+// took 2,221 us. Eight rows a warp rather than 32 keep small tables in enough
+// warps (10,357 x 633: 37 us at the start, 172 us with 32 rows a warp).
+constexpr int E16_WARPS = 8, E16_ROWS = 8, E16_DIMS = 128;
 template <bool VEC>
 __global__ void __launch_bounds__(32 * E16_WARPS, 3) encode_fp16_kernel(const float* __restrict__ x, uint32_t n,
-                                                                     uint32_t dim, uint32_t pd,
-                                                                     uint16_t* __restrict__ out,
-                                                                     float* __restrict__ norms) {
-  __shared__ float sq[E16_WARPS][32][33];
+                                                                        uint32_t dim, uint32_t pd,
+                                                                        uint16_t* __restrict__ out,
+                                                                        float* __restrict__ norms) {
+  // (a stride of 132 floats: 16-byte stores, and the eight summing lanes on
+  // different banks)
+  __shared__ __align__(16) float sq[E16_WARPS][E16_ROWS][E16_DIMS + 4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t row0 = ((uint64_t)blockIdx.x * E16_WARPS + warp) * 32;
+  const uint64_t row0 = ((uint64_t)blockIdx.x * E16_WARPS + warp) * E16_ROWS;
   if (row0 >= n) return;
-  const uint32_t rows = (uint32_t)min((uint64_t)32, n - row0);
-  float(*t)[33] = sq[warp];
+  const int rows = (int)min((uint64_t)E16_ROWS, n - row0);
+  float(*t)[E16_DIMS + 4] = sq[warp];
+  const float* src = x + row0 * dim;
+  uint16_t* dst = out + row0 * pd;
   float sum = 0.f;
-  if constexpr (VEC) {
-    const uint32_t r4 = lane >> 3, c4 = (lane & 7) * 4;  // load i: row 4 i + r4, columns c4..c4+3 of the chunk
-    float4 cur[8];
-    auto load = [&](uint32_t d0, float4 (&v)[8]) {
+  constexpr int NV = VEC ? 1 : 4;  // loads per row of a chunk: a float4, or four floats 32 apart
+  using V = typename std::conditional<VEC, float4, float>::type;
+  V cur[E16_ROWS][NV];
+  auto load = [&](uint32_t d0) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t r = 4 * i + r4;
-        v[i] = (r < rows && d0 + c4 < dim)
-                   ? __ldg(reinterpret_cast<const float4*>(x + (row0 + r) * dim + d0 + c4))
-                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = 0; r < E16_ROWS; ++r) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const uint32_t d = d0 + (VEC ? 4 * lane : lane + 32 * i);
+        if constexpr (VEC)
+          cur[r][i] = r < rows && d < dim ? __ldg(reinterpret_cast<const float4*>(src + (size_t)r * dim + d))
+                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+        else
+          cur[r][i] = r < rows && d < dim ? __ldg(src + (size_t)r * dim + d) : 0.f;
       }
-    };
-    load(0, cur);
-    for (uint32_t d0 = 0; d0 < pd; d0 += 32) {
-      float4 v[8];
+    }
+  };
+  load(0);
+  for (uint32_t d0 = 0; d0 < pd; d0 += E16_DIMS) {
+    __syncwarp();  // the previous chunk is summed
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = cur[i];
-      if (d0 + 32 < dim) load(d0 + 32, cur);
-      __syncwarp();
+    for (int r = 0; r < E16_ROWS; ++r) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t r = 4 * i + r4;
-        t[r][c4] = __fmul_rn(v[i].x, v[i].x);
-        t[r][c4 + 1] = __fmul_rn(v[i].y, v[i].y);
-        t[r][c4 + 2] = __fmul_rn(v[i].z, v[i].z);
-        t[r][c4 + 3] = __fmul_rn(v[i].w, v[i].w);
-        if (r < rows && d0 + c4 < pd) {
+      for (int i = 0; i < NV; ++i) {
+        const uint32_t c = VEC ? 4 * lane : lane + 32 * i;
+        const V v = cur[r][i];
+        if constexpr (VEC) {
+          *reinterpret_cast<float4*>(&t[r][c]) =
+              make_float4(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y), __fmul_rn(v.z, v.z), __fmul_rn(v.w, v.w));
           // dim is a multiple of 4: four columns in or out together
-          *reinterpret_cast<uint2*>(out + (row0 + r) * pd + d0 + c4) =
-              d0 + c4 < dim ? f32_to_f16_halfup4(v[i]) : make_uint2(0u, 0u);
+          if (r < rows && d0 + c < pd)
+            *reinterpret_cast<uint2*>(dst + (size_t)r * pd + d0 + c) =
+                d0 + c < dim ? f32_to_f16_halfup4(v) : make_uint2(0u, 0u);
+        } else {
+          t[r][c] = __fmul_rn(v, v);
+          if (r < rows && d0 + c < pd)
+            dst[(size_t)r * pd + d0 + c] = d0 + c < dim ? f32_to_f16_halfup_fast(v) : (uint16_t)0;
         }
       }
-      __syncwarp();
-      const int m = d0 < dim ? (int)min(32u, dim - d0) : 0;
-      if (m == 32) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) sum = __fadd_rn(sum, t[lane][j]);
-      } else {
-        for (int j = 0; j < m; ++j) sum = __fadd_rn(sum, t[lane][j]);
-      }
     }
-  } else {
-    for (uint32_t d0 = 0; d0 < pd; d0 += 32) {
-      const uint32_t d = d0 + lane;
-      __syncwarp();
-#pragma unroll 8
-      for (uint32_t r = 0; r < rows; ++r) {
-        const float v = d < dim ? __ldg(x + (row0 + r) * dim + d) : 0.f;
-        t[r][lane] = __fmul_rn(v, v);
-        if (d < pd) out[(row0 + r) * pd + d] = d < dim ? f32_to_f16_halfup(v) : (uint16_t)0;
+    if (d0 + E16_DIMS < dim) load(d0 + E16_DIMS);
+    __syncwarp();
+    if (lane < E16_ROWS) {
+      const int m = d0 < dim ? (int)min((uint32_t)E16_DIMS, dim - d0) : 0;
+      int j = 0;
+      for (; j + 16 <= m; j += 16) {
+        float4 w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(&t[lane][j + 4 * i]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, w[i].x), w[i].y), w[i].z), w[i].w);
       }
-      __syncwarp();
-      const int m = d0 < dim ? (int)min(32u, dim - d0) : 0;
-      for (int j = 0; j < m; ++j) sum = __fadd_rn(sum, t[lane][j]);
+      for (; j < m; ++j) sum = __fadd_rn(sum, t[lane][j]);
     }
   }
-  if (norms && lane < (int)rows) norms[row0 + lane] = sum;
+  if (norms && lane < rows) norms[row0 + lane] = sum;
 }
 
 // Neumaier accumulation of one term.
@@ -281,7 +291,7 @@ __global__ void __launch_bounds__(256) encode_fp8_per_vector_kernel(const float*
 int launch_encode_fp16(const float* x, uint32_t n, uint32_t dim, uint32_t pd, uint16_t* out, float* norms,
                        cudaStream_t stream) {
   if (n == 0) return 0;
-  const uint64_t blocks = ((uint64_t)n + 32 * E16_WARPS - 1) / (32 * E16_WARPS);
+  const uint64_t blocks = ((uint64_t)n + E16_ROWS * E16_WARPS - 1) / (E16_ROWS * E16_WARPS);
   // 16-byte loads and 8-byte stores where every row starts on such a boundary
   const bool vec = dim % 4 == 0 && pd % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)out % 8 == 0;
   if (vec)
