@@ -72,17 +72,18 @@ struct TcScanArgs {
 };
 
 // PAIR: a CTA of a cta_group::2 pair holds half of each 256-row base tile.
-// COLS: the epilogue stages per-column norms / scales (not the fused fp8
-// forms, whose accumulator is the ranking value). A_STAGES: query-tile
-// buffers (1 where the query tile is always resident).
-template <int KL, int STAGES, int G, bool PAIR = false, bool COLS = true, int A_STAGES = STAGES>
+// NCOL: per-column arrays that the epilogue stages (norms, scales, cosine's
+// factors; none in the fused fp8 forms, whose accumulator is the ranking
+// value). A_STAGES: query-tile buffers (1 where the query tile is always
+// resident).
+template <int KL, int STAGES, int G, bool PAIR = false, int NCOL = 2, int A_STAGES = STAGES>
 struct ScanSmem {
   static constexpr size_t b_stage = PAIR ? B_STAGE / 2 : B_STAGE;
   static constexpr size_t a_off = 0;
   static constexpr size_t b_off = a_off + (size_t)A_STAGES * A_STAGE;
   static constexpr size_t heap_off = b_off + (size_t)STAGES * b_stage;
-  static constexpr size_t col_off = heap_off + (size_t)G * KL * TC_M * 8;  // [4G warps][2][TC_N] floats
-  static constexpr size_t cmask_off = col_off + (COLS ? 4 * G * 2 * TC_N * 4 : 0);  // [4G warps][8] words
+  static constexpr size_t col_off = heap_off + (size_t)G * KL * TC_M * 8;  // [4G warps][NCOL][TC_N] floats
+  static constexpr size_t cmask_off = col_off + (size_t)4 * G * NCOL * TC_N * 4;  // [4G warps][8] words
   static constexpr size_t bar_off = cmask_off + 4 * G * 8 * 4;          // barriers
   static constexpr size_t nbars = 2 * STAGES + 5;
   static constexpr size_t misc_off = bar_off + nbars * 8;
@@ -97,7 +98,8 @@ constexpr bool kFusedScan = FP8 && TS && METRIC != METRIC_COSINE;
 // G = 4 runs only the fused fp8 forms with one K block per tile, whose query
 // tile is resident: one query-tile buffer.
 template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR, bool TS>
-using ScanLayout = ScanSmem<KL, STAGES, G, PAIR, !kFusedScan<FP8, METRIC, TS>, G == 4 ? 1 : STAGES>;
+using ScanLayout = ScanSmem<KL, STAGES, G, PAIR, kFusedScan<FP8, METRIC, TS> ? 0 : FP8 && METRIC == METRIC_COSINE ? 3 : 2,
+                            G == 4 ? 1 : STAGES>;
 
 // Sift `key` down from position i of a max-heap of kl keys stored with
 // stride TC_M (one heap per query row of the block).
@@ -418,10 +420,24 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     // by a relative slack, so thr errs on the admitting side; exact tests
     // follow). Fused fp8 tests the accumulator instead: v <= thr <=> acc >=
     // thr / sc (sc < 0, a power of two), padded the same way against underflow.
-    float thr = 0.f;
+    //
+    // Cosine: a division and a square root per value bounded the pass (64,931
+    // x 859, 16 queries: 159 us). Where sqrt(|q|^2 |x|^2) >= 0.01 for a tile's
+    // columns, v = -dot / |x| from a factor staged per column ranks within
+    // kCosPad of the distance 1 + v / |q| (the factors' few ulps, and 1e-8
+    // against 0.01), so v <= cthr, raised by it, admits every candidate and
+    // the exact distance is evaluated for those alone.
+    constexpr float kCosPad = 4e-6f;
+    const float q_over = METRIC == METRIC_COSINE ? sqrtf(qn) / (FP8 ? qs : 1.f) : 1.f;
+    const float q_inv = METRIC == METRIC_COSINE ? __fdiv_rn(1.f, q_over) : 1.f;
+    float thr = 0.f, cthr = 0.f;
     auto refresh = [&]() {
       const float w = fminf(worst, bound);
       thr = METRIC == METRIC_L2 ? (w - qn) + 1e-6f * (fabsf(w) + fabsf(qn)) + 1e-30f : w;
+      if (METRIC == METRIC_COSINE) {
+        cthr = (w - 1.0f + kCosPad) * q_over;
+        cthr += 1e-6f * fabsf(cthr);
+      }
       if (fused) {
         thr *= inv_sc;
         thr -= 1e-6f * fabsf(thr) + 1e-37f;
@@ -432,7 +448,9 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     // mask words): staged by the warp itself, so the epilogue warps never
     // wait on one another. The global loads for tile i + 1 are issued into
     // registers while tile i is processed (lane l holds columns l + 32 r).
-    float* cb = colbuf + (warp - 2) * 2 * TC_N;
+    constexpr int kCols = kFusedScan<FP8, METRIC, TS> ? 0 : FP8 && METRIC == METRIC_COSINE ? 3 : 2;
+    float* cb = colbuf + (warp - 2) * kCols * TC_N;
+    float* cf = cb + (kCols - 1) * TC_N;  // cosine: -1 / |x| (times the row's scale)
     uint32_t* cm = colmask + (warp - 2) * 8;
     // this group's columns [c_lo, c_hi) of each tile; only its own columns'
     // data is staged
@@ -466,11 +484,22 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
       const uint32_t buf = i & 1, use = i >> 1;
       const uint32_t v0 = (t_begin + i) * tstride * TC_N;
       __syncwarp();
+      [[maybe_unused]] float least = INFINITY;  // cosine: the smallest norm of the tile's rows
 #pragma unroll
       for (int r = 0; r < TC_N / 32; ++r) {
         if (32 * r < c_lo || 32 * r >= c_hi) continue;
         if (METRIC != METRIC_INNER_PRODUCT && !fused) cb[lane + 32 * r] = pre_n[r];
         if (FP8 && !fused) cb[TC_N + lane + 32 * r] = pre_s[r];
+        if (METRIC == METRIC_COSINE) {
+          cf[lane + 32 * r] = -rsqrtf(pre_n[r]) * (FP8 ? pre_s[r] : 1.f);
+          if (v0 + lane + 32 * r < a.n) least = fminf(least, pre_n[r]);
+        }
+      }
+      [[maybe_unused]] bool by_factor = false;
+      if (METRIC == METRIC_COSINE) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+        by_factor = __all_sync(0xffffffffu, !qvalid || (qn * least >= 1e-4f && qn < 1e30f));
       }
       if (lane < 8) cm[lane] = pre_m;
       __syncwarp();
@@ -554,8 +583,9 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
           if (!MINP && mw == 0ull) continue;
           // the chunk's admission test and insertions; FU: the accumulator is
           // the ranking value (fp8 table-scale tables)
-          auto chunk = [&](auto fu_tag) {
-            constexpr bool FU = decltype(fu_tag)::value;
+          // AP: cosine by the staged factors
+          auto chunk = [&](auto fu_tag, auto ap_tag) {
+            constexpr bool FU = decltype(fu_tag)::value, AP = decltype(ap_tag)::value;
             // per-column values v, v[0..32) columns c0.., v[32..64) columns
             // c0+32..; the distance is D(v): L2  D(v) = max(floor, ||q||^2 + v) with
             // v = ||x||^2 - 2 <q, x> (the query's norm is added after the
@@ -565,6 +595,18 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
             if constexpr (FU) {
 #pragma unroll
               for (int j = 0; j < 64; ++j) v[j] = __uint_as_float(j < 32 ? ra[j] : rb[j - 32]);
+            } else if constexpr (AP) {
+              const float4* fb = reinterpret_cast<const float4*>(cf + c0);
+#pragma unroll
+              for (int j4 = 0; j4 < 16; ++j4) {
+                const float4 f4 = fb[j4];
+                const float fv[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const int j = 4 * j4 + e;
+                  v[j] = __uint_as_float(j < 32 ? ra[j] : rb[j - 32]) * fv[e];
+                }
+              }
             } else if (METRIC == METRIC_COSINE) {
 #pragma unroll
               for (int j = 0; j < 64; ++j) {
@@ -592,14 +634,16 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
                 }
               }
             }
-            // D: distance from v (fused fp8: from the accumulator, v = sc * acc)
+            // D: distance from v (fused fp8: from the accumulator, v = sc * acc;
+            // cosine by factors: an upper bound)
             auto D = [&](float x) {
+              if (AP) return fmaf(x, q_inv, 1.0f + kCosPad);
               if (FU) x *= sc;
               return METRIC == METRIC_L2 ? fmaxf(a.floor, qn + x) : x;
             };
             // better(x, y): the smaller v, i.e. the larger accumulator when fused
             auto better = [](float x, float y) { return FU ? fmaxf(x, y) : fminf(x, y); };
-            auto may = [&](float x) { return FU ? x >= thr : x <= thr; };
+            auto may = [&](float x) { return FU ? x >= thr : x <= (AP ? cthr : thr); };
             // a tree of three-input bests: a 64-column batch whose best cannot
             // enter is skipped whole (the common case once warm); the pairwise
             // bests (j, j + 32) are formed only for a batch that passes
@@ -673,8 +717,22 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
             while (pass) {
               const int j = __ffs(pass) - 1;
               pass &= pass - 1;
-              const float dlo = D(select32(v, j));
-              const float dhi = D(select32(v + 32, j));
+              float dlo, dhi;
+              if constexpr (AP) {
+                auto exact = [&](const uint32_t (&rr)[32], int c) {
+                  float f[32];
+#pragma unroll
+                  for (int t = 0; t < 32; ++t) f[t] = __uint_as_float(rr[t]);
+                  float dot = select32(f, j);
+                  if (FP8) dot = dot * (qs * cb[TC_N + c]);
+                  return 1.0f - dot / (sqrtf(qn * cb[c]) + 1e-8f);
+                };
+                dlo = exact(ra, c0 + j);
+                dhi = exact(rb, c0 + j + 32);
+              } else {
+                dlo = D(select32(v, j));
+                dhi = D(select32(v + 32, j));
+              }
               if (((mw >> j) & 1ull) && dlo < worst && dlo <= bound) {
                 keep(dlo, v0 + c0 + j);
                 refresh();
@@ -686,7 +744,14 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
             }
             }
           };
-          chunk(std::integral_constant<bool, fused>{});
+          if constexpr (METRIC == METRIC_COSINE) {
+            if (by_factor)
+              chunk(std::false_type{}, std::true_type{});
+            else
+              chunk(std::false_type{}, std::false_type{});
+          } else {
+            chunk(std::integral_constant<bool, fused>{}, std::false_type{});
+          }
         }
       }
       tc::tc_fence_before();
