@@ -717,7 +717,7 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
     p.pmin = reinterpret_cast<float*>(partial);
     p.pm_stride = P.pcount;
     p.gran = P.pgran;
-    e = scan(p, 0, P.psplits, fp8 ? "tc_prepass_fp8" : "tc_prepass_fp16", pair, groups > 2 ? 2 : groups);
+    e = scan(p, kMinima, P.psplits, fp8 ? "tc_prepass_fp8" : "tc_prepass_fp16", pair, groups > 2 ? 2 : groups);
     if (e != cudaSuccess) return (int)e;
     {
       ProfScope ps("tc_tau", stream);
@@ -731,7 +731,7 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
   a.kl = kl;
   a.share = (kl == shortlist && !prepass) ? 1u : 0u;
   a.qbound = tau;
-  e = scan(a, (int)kl_tmpl, splits, fp8 ? "tc_scan_fp8" : "tc_scan_fp16", pair, groups);
+  e = scan(a, prepass ? kLists : (int)kl_tmpl, splits, fp8 ? "tc_scan_fp8" : "tc_scan_fp16", pair, groups);
   if (e != cudaSuccess) return (int)e;
 
   // The keys that a block sorts: all of them without a bound; with one, about
@@ -833,7 +833,7 @@ int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream) {
   p.pmin = reinterpret_cast<float*>(c.partial);
   p.pm_stride = P.pcount;
   p.gran = P.pgran;
-  cudaError_t e = scan(p, 0, P.psplits, "tc_prepass_fp16");
+  cudaError_t e = scan(p, kMinima, P.psplits, "tc_prepass_fp16");
   if (e != cudaSuccess) return (int)e;
   {
     ProfScope ps("tc_tau", stream);
@@ -847,7 +847,7 @@ int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream) {
   a.partial = c.partial;
   a.kl = P.kl;
   a.qbound = c.bound;
-  return (int)scan(a, (int)P.kl_tmpl, P.splits, "tc_scan_fp16");
+  return (int)scan(a, kLists, P.splits, "tc_scan_fp16");
 }
 
 }  // namespace fv

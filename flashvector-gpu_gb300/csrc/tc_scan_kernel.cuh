@@ -71,6 +71,10 @@ struct TcScanArgs {
   uint32_t pm_stride, gran;
 };
 
+enum { PASS_HEAP = 0, PASS_MIN = 1, PASS_LIST = 2 };
+// heap capacities that select the passes without shared-memory heaps
+constexpr int kMinima = 0, kLists = -1;
+
 // PAIR: a CTA of a cta_group::2 pair holds half of each 256-row base tile.
 // NCOL: per-column arrays that the epilogue stages (norms, scales, cosine's
 // factors; none in the fused fp8 forms, whose accumulator is the ranking
@@ -101,47 +105,31 @@ template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR, bool TS>
 using ScanLayout = ScanSmem<KL, STAGES, G, PAIR, kFusedScan<FP8, METRIC, TS> ? 0 : FP8 && METRIC == METRIC_COSINE ? 3 : 2,
                             G == 4 ? 1 : STAGES>;
 
-// Sift `key` down from position i of a max-heap of kl keys stored with
-// stride TC_M (one heap per query row of the block).
+// Sift `key` down from position i of a max-heap of kl keys stored with stride
+// HS (TC_M in shared memory, one heap per query row of the block; 1 in global
+// memory).
+template <int HS>
 static __device__ __forceinline__ void heap_down(uint64_t* h, int kl, int i, uint64_t key) {
   while (true) {
     int l = 2 * i + 1;
     if (l >= kl) break;
-    uint64_t cv = h[l * TC_M];
+    uint64_t cv = h[l * HS];
     int c = l;
     if (l + 1 < kl) {
-      uint64_t rv = h[(l + 1) * TC_M];
+      uint64_t rv = h[(l + 1) * HS];
       if (rv > cv) { cv = rv; c = l + 1; }
     }
     if (cv <= key) break;
-    h[i * TC_M] = cv;
+    h[i * HS] = cv;
     i = c;
   }
-  h[i * TC_M] = key;
+  h[i * HS] = key;
 }
 
 // Turns kl unordered keys into a max-heap (bottom-up).
+template <int HS>
 static __device__ __forceinline__ void heap_build(uint64_t* h, int kl) {
-  for (int i = kl / 2 - 1; i >= 0; --i) heap_down(h, kl, i, h[i * TC_M]);
-}
-
-static __device__ __forceinline__ void heap_sift(uint64_t* h, int kl, uint64_t key) {
-  // replace the root of a max-heap stored with stride TC_M
-  int i = 0;
-  while (true) {
-    int l = 2 * i + 1;
-    if (l >= kl) break;
-    uint64_t cv = h[l * TC_M];
-    int c = l;
-    if (l + 1 < kl) {
-      uint64_t rv = h[(l + 1) * TC_M];
-      if (rv > cv) { cv = rv; c = l + 1; }
-    }
-    if (cv <= key) break;
-    h[i * TC_M] = cv;
-    i = c;
-  }
-  h[i * TC_M] = key;
+  for (int i = kl / 2 - 1; i >= 0; --i) heap_down<HS>(h, kl, i, h[i * HS]);
 }
 
 // v[j] for a lane-varying j without local memory: a 5-level select tree.
@@ -178,7 +166,14 @@ static __device__ __forceinline__ float select32(const float* v, int j) {
 // are multicast to both CTAs' barriers; the odd CTA's epilogue arrives on
 // the even CTA's accumulator barriers.
 //
-// MINP: the pass that finds every query's admission bound. No heaps: the
+// PASS_HEAP: the heaps live in shared memory (a scan without a bound, where
+// every range keeps replacing its worst key).
+// PASS_LIST: a bounded scan, whose ranges hold a few keys and seldom fill: a
+// range's keys are appended to its list in the output itself, which becomes a
+// heap only when it fills. The 64 to 128 KB of shared memory that four groups'
+// heaps took hold base tiles instead: with two stages the ring could not
+// cover the latency of a tile.
+// PASS_MIN: the pass that finds every query's admission bound. No heaps: the
 // epilogue reduces each tile's accumulators to the smallest distance of every
 // `gran` columns and stores those, so its cost per tile is the minimum tree
 // alone and the freed shared memory holds a deeper ring. The r-th smallest
@@ -186,9 +181,11 @@ static __device__ __forceinline__ float select32(const float* v, int j) {
 // disjoint columns are distances of distinct rows), so it bounds from above.
 // Keeping the sample's best r keys in heaps instead spent the pass filling
 // them: 123 us for 1/32 of a 1M x 768 scan of 1,024 queries.
-template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR, bool TS, bool MINP>
+template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR, bool TS, int PASS>
 __global__ void __launch_bounds__(scan_threads(G), 1)
     tc_scan_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TcScanArgs a) {
+  constexpr bool MINP = PASS == PASS_MIN;
+  constexpr int HS = PASS == PASS_LIST ? 1 : TC_M;  // stride of a range's keys
   using L = ScanLayout<FP8, KL, STAGES, METRIC, G, PAIR, TS>;
   constexpr uint32_t b_stage = (uint32_t)L::b_stage;
   constexpr int SCAN_THREADS = scan_threads(G);
@@ -376,9 +373,11 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     const int row = quad * 32 + lane;             // query row in the block
     const uint32_t q = qb * TC_M + row;
     const bool qvalid = q < a.nq && (a.active == nullptr || a.active[q] != 0u);
-    uint64_t* h = heap + (size_t)grp * KL * TC_M + row;
     const int kl = MINP ? 0 : (int)a.kl;
-    for (int i = 0; i < kl; ++i) h[i * TC_M] = kSentinelKey;
+    uint64_t* const list = a.partial + (((size_t)q * a.splits + split) * G + grp) * kl;  // this range's output
+    uint64_t* h = PASS == PASS_LIST ? list : heap + (size_t)grp * KL * TC_M + row;
+    if (PASS == PASS_HEAP)
+      for (int i = 0; i < kl; ++i) h[i * HS] = kSentinelKey;
     const float qn = qvalid ? __ldg(a.qnorm + q) : 0.f;
     const QueryFilter qf = (a.filters && qvalid) ? load_filter(a.filters, q) : QueryFilter{nullptr, 0u, 0u};
     const float qs = (FP8 && qvalid) ? __ldg(a.qscale + q) : 1.f;
@@ -403,13 +402,13 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     auto keep = [&](float dist, uint32_t slot) {
       const uint64_t key = make_key(dist, slot);
       if (fill < kl) {
-        h[fill * TC_M] = key;
+        h[fill * HS] = key;
         if (++fill == kl) {
-          heap_build(h, kl);
+          heap_build<HS>(h, kl);
           worst = key_dist(h[0]);
         }
       } else {
-        heap_sift(h, kl, key);
+        heap_down<HS>(h, kl, 0, key);  // replaces the root
         worst = key_dist(h[0]);
       }
       if (slots) atomicMin(slots + __umulhi(slot * 2654435761u, (uint32_t)kl), float_order(dist));
@@ -422,7 +421,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     // thr / sc (sc < 0, a power of two), padded the same way against underflow.
     //
     // Cosine: a division and a square root per value bounded the pass (64,931
-    // x 859, 16 queries: 159 us). Where sqrt(|q|^2 |x|^2) >= 0.01 for a tile's
+    // x 859, 16 queries: 159 us a call, now 76). Where sqrt(|q|^2 |x|^2) >= 0.01 for a tile's
     // columns, v = -dot / |x| from a factor staged per column ranks within
     // kCosPad of the distance 1 + v / |q| (the factors' few ulps, and 1e-8
     // against 0.01), so v <= cthr, raised by it, admits every candidate and
@@ -770,11 +769,15 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
       // it for overflow): a full heap has it there already; a list that never
       // filled gets one of its sentinels moved there
       if (fill > 0 && fill < kl) {
-        h[fill * TC_M] = h[0];
+        h[fill * HS] = h[0];
         h[0] = kSentinelKey;
+        ++fill;
       }
-      uint64_t* dst = a.partial + (((size_t)q * a.splits + split) * G + grp) * kl;
-      for (int i = 0; i < kl; ++i) dst[i] = h[i * TC_M];
+      if (PASS == PASS_LIST) {
+        for (int i = fill; i < kl; ++i) h[i] = kSentinelKey;
+      } else {
+        for (int i = 0; i < kl; ++i) list[i] = h[i * HS];
+      }
     }
   }
 
@@ -797,12 +800,12 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
 }
 
 
-template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR = false, bool TS = true, bool MINP = false>
+template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR = false, bool TS = true, int PASS = PASS_HEAP>
 cudaError_t launch_scan_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const TcScanArgs& a, uint32_t grid,
                                cudaStream_t stream) {
   using L = ScanLayout<FP8, KL, STAGES, METRIC, G, PAIR, TS>;
   static_assert(L::bytes <= 227 * 1024, "scan shared memory above the 227 KB per-CTA limit");
-  auto kern = tc_scan_kernel<FP8, KL, STAGES, METRIC, G, PAIR, TS, MINP>;
+  auto kern = tc_scan_kernel<FP8, KL, STAGES, METRIC, G, PAIR, TS, PASS>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::bytes);
   if (e != cudaSuccess) return e;
   if constexpr (PAIR) {
@@ -836,11 +839,18 @@ cudaError_t launch_scan_kernel(const CUtensorMap& ta, const CUtensorMap& tb, con
 template <bool FP8, int METRIC, bool TS>
 cudaError_t dispatch_scan_kl(int kl, int groups, const CUtensorMap& ta, const CUtensorMap& tb, const TcScanArgs& a,
                              uint32_t grid, cudaStream_t stream) {
-  if (kl == 0) {
-    // the minima pass: no heaps, so the ring takes their shared memory
-    if (groups == -1) return launch_scan_kernel<FP8, 0, 6, METRIC, 1, true, TS, true>(ta, tb, a, grid, stream);
-    if (groups == 1) return launch_scan_kernel<FP8, 0, 4, METRIC, 1, false, TS, true>(ta, tb, a, grid, stream);
-    return launch_scan_kernel<FP8, 0, 4, METRIC, 2, false, TS, true>(ta, tb, a, grid, stream);
+  if (kl == kMinima) {
+    if (groups == -1) return launch_scan_kernel<FP8, 0, 6, METRIC, 1, true, TS, PASS_MIN>(ta, tb, a, grid, stream);
+    if (groups == 1) return launch_scan_kernel<FP8, 0, 4, METRIC, 1, false, TS, PASS_MIN>(ta, tb, a, grid, stream);
+    return launch_scan_kernel<FP8, 0, 4, METRIC, 2, false, TS, PASS_MIN>(ta, tb, a, grid, stream);
+  }
+  if (kl == kLists) {
+    if (groups == -1) return launch_scan_kernel<FP8, 0, 6, METRIC, 1, true, TS, PASS_LIST>(ta, tb, a, grid, stream);
+    if (groups == 1) return launch_scan_kernel<FP8, 0, 4, METRIC, 1, false, TS, PASS_LIST>(ta, tb, a, grid, stream);
+    if (groups == 2) return launch_scan_kernel<FP8, 0, 4, METRIC, 2, false, TS, PASS_LIST>(ta, tb, a, grid, stream);
+    if constexpr (kFusedScan<FP8, METRIC, TS>)
+      return launch_scan_kernel<FP8, 0, 6, METRIC, 4, false, TS, PASS_LIST>(ta, tb, a, grid, stream);
+    return cudaErrorInvalidValue;
   }
   if (groups == -1) {
     // cta_group::2 pairs (one epilogue group): 16 KB of base per stage frees
