@@ -132,6 +132,17 @@ static __device__ __forceinline__ void heap_build(uint64_t* h, int kl) {
   for (int i = kl / 2 - 1; i >= 0; --i) heap_down<HS>(h, kl, i, h[i * HS]);
 }
 
+// A range's list that has just filled (or is full): its heap, the rare part
+// of a bounded scan, out of the way of the common one. Returns the distance of
+// the worst key kept.
+static __device__ __noinline__ float list_full(uint64_t* list, int kl, uint64_t key, bool build) {
+  if (build)
+    heap_build<1>(list, kl);
+  else
+    heap_down<1>(list, kl, 0, key);  // replaces the root
+  return key_dist(list[0]);
+}
+
 // v[j] for a lane-varying j without local memory: a 5-level select tree.
 static __device__ __forceinline__ float select32(const float* v, int j) {
   float t[16];
@@ -401,6 +412,17 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     int fill = 0;
     auto keep = [&](float dist, uint32_t slot) {
       const uint64_t key = make_key(dist, slot);
+      if constexpr (PASS == PASS_LIST) {
+        // (worst stays at 1e30, and the threshold where it is, until it fills)
+        if (fill < kl) {
+          h[fill] = key;
+          if (++fill < kl) return;
+          worst = list_full(h, kl, key, true);
+        } else {
+          worst = list_full(h, kl, key, false);
+        }
+        return;
+      }
       if (fill < kl) {
         h[fill * HS] = key;
         if (++fill == kl) {
@@ -554,10 +576,11 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
           const float top = fmaxf(max3(max3(t1[0], t1[1], t1[2]), max3(t1[3], t1[4], t1[5]), max3(t1[6], t1[7], t1[8])),
                                   fmaxf(t1[9], t1[10]));
           if (!(top >= thr)) return;
-          uint32_t pass = 0;
+          // (four chains of eight: one chain of 32 was most of the mask's latency)
+          uint32_t p4[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-          for (int j = 0; j < 32; ++j) pass |= (uint32_t)(v[j] >= thr) << j;
-          pass &= m32;
+          for (int j = 0; j < 32; ++j) p4[j >> 3] |= (uint32_t)(v[j] >= thr) << j;
+          uint32_t pass = ((p4[0] | p4[1]) | (p4[2] | p4[3])) & m32;
           while (pass) {
             const int j = __ffs(pass) - 1;
             pass &= pass - 1;
@@ -565,7 +588,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
             const float d = METRIC == METRIC_L2 ? fmaxf(0.f, qn + x) : x;
             if (d < worst && d <= bound) {
               keep(d, v0 + col + (uint32_t)j);
-              refresh();
+              if (PASS != PASS_LIST) refresh();
             }
           }
         };
