@@ -40,7 +40,7 @@
 // codebook, 128 KB at m = 32) and evaluates the few table entries that a short
 // list needs in place, in the same operations. A running shortlist is kept in
 // shared memory: rows whose key cannot beat its worst key are dropped, the
-// rest are appended to a buffer that is sorted into it when it fills.
+// rest are appended to a buffer; when it fills, the best of both are kept.
 #include <cuda_fp16.h>
 
 #include "../../include/fv_bridge.h"
@@ -55,6 +55,11 @@ namespace {
 constexpr int IVF_THREADS = 256;
 constexpr uint32_t IVF_BUF = 1536;         // candidate buffer entries (>= 1.5 rounds of 1,024 postings)
 constexpr uint32_t MAX_SHORTLIST = 10240;  // reference clamp (ivf_rerank.cuh:12)
+// Keys of which a flush selects the shortlist from registers. Up to 512 a sort
+// is the quicker (5 queries, 20,000 x 128: 57 us sorting, 67 selecting), from
+// 1,024 the selection (2,000 RaBitQ queries over 1M rows: list scan 788 us
+// sorting, 646 selecting); past 2,048 the registers do not hold them.
+constexpr uint32_t KEEP_MIN = 512, KEEP_MAX = 2048;
 
 enum IvfMode { IVF_PQ = IVF_MODE_PQ, IVF_SQ8 = IVF_MODE_SQ8, IVF_RABITQ = IVF_MODE_RABITQ };
 
@@ -96,8 +101,9 @@ struct IvfArgs {
   uint32_t* status;
   uint32_t keys_pow2;             // pow2(largest shortlist + IVF_BUF)
   uint32_t list_chunk;            // probed lists walked as one sequence (<= 32)
+  uint32_t keep_at;               // byte offset of the flush's selection scratch (0: flushes sort)
   uint32_t items_per_q;           // G: a query's probed postings are cut into G ranges
-  uint64_t* partial;              // G > 1: [nq * G][part_stride] sorted shortlists of the ranges
+  uint64_t* partial;              // G > 1: [nq * G][part_stride] shortlists of the ranges
   uint32_t part_stride;           // >= every query's shortlist
   // RaBitQ
   const float* rot_centroids;     // [nlist][P]
@@ -130,20 +136,20 @@ __device__ __forceinline__ ListSpan list_span(const IvfArgs& a, uint32_t l) {
   return ListSpan{lbeg, lend, false};
 }
 
-// Rerank of a query's shortlist keys[0, S) (sorted, sentinels last) with the
-// reference's warp-order fp32 distance, sort, and the query's top k into
+// Rerank of a query's shortlist keys[0, S) (in any order, sentinels last) with
+// the reference's warp-order fp32 distance, sort, and the query's top k into
 // out[q][0, top_k) (sentinels past k). Block-collective.
-template <uint32_t R, int B>
+template <int NT, uint32_t R, int B>
 __device__ void ivf_finish_query(const IvfArgs& a, uint64_t* keys, uint32_t q, uint32_t S, uint32_t kq,
-                                 bool do_rerank, const float* qv) {
+                                 bool do_rerank, const float* qv, KeepScratch* keep) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (do_rerank) {
     // R candidates per warp pass (c, c + NW, .., all owned by warp c % NW as
     // with one at a time), so R rows' gathers, B loads ahead each, are in
     // flight per warp.
-    constexpr uint32_t NW = IVF_THREADS / 32;
+    constexpr uint32_t NW = NT / 32;
     for (uint32_t c0 = warp; c0 < S; c0 += R * NW) {
-      if (keys[c0] == kSentinelKey) break;  // sorted: the rest are sentinels too
+      if (keys[c0] == kSentinelKey) break;  // the rest are sentinels too
       const float* rows[R];
       uint32_t slot[R];
       bool any = false;
@@ -167,12 +173,18 @@ __device__ void ivf_finish_query(const IvfArgs& a, uint64_t* keys, uint32_t q, u
           if (slot[r] != kInvalidId) keys[c0 + r * NW] = make_key(d[r], slot[r]);
       }
     }
-    const uint32_t p2 = next_pow2_dev(S);
-    for (uint32_t i = S + tid; i < p2; i += IVF_THREADS) keys[i] = kSentinelKey;
     __syncthreads();
-    block_bitonic_sort(keys, p2);
   }
-  for (uint32_t r = tid; r < a.top_k; r += IVF_THREADS)
+  uint32_t sorted = S;
+  if (keep && S > 2 * kq && S > KEEP_MIN && S <= KEEP_MAX) {
+    block_keep_smallest<NT, KEEP_MAX / NT>(keys, S, kq, *keep);
+    sorted = kq;
+  }
+  const uint32_t p2 = next_pow2_dev(sorted);
+  for (uint32_t i = sorted + tid; i < p2; i += NT) keys[i] = kSentinelKey;
+  __syncthreads();
+  block_bitonic_sort(keys, p2);
+  for (uint32_t r = tid; r < a.top_k; r += NT)
     a.out[(size_t)q * a.top_k + r] = key_to_result(r < S && r < kq ? keys[r] : kSentinelKey, nullptr);
 }
 
@@ -578,6 +590,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
   __shared__ unsigned long long s_total;
   __shared__ float s_red[MODE == IVF_RABITQ ? IVF_THREADS : 1];
 
+  KeepScratch* keep = a.keep_at ? reinterpret_cast<KeepScratch*>(smem + a.keep_at) : nullptr;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* mins = tab;                     // SQ8 only
   float* scales = tab + a.dim;
@@ -660,16 +673,22 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
     uint64_t cum = 0;  // postings of the lists before this chunk (warp 0)
 
     auto flush = [&]() {
-      // keys[0, S) sorted shortlist, keys[S, S + cnt) new candidates
+      // keys[0, S) the shortlist, keys[S, S + cnt) new candidates
       const uint32_t cnt = s_cnt;  // block-uniform (read after a barrier)
       if (cnt == 0) return;
-      const uint32_t p2 = next_pow2_dev(S + cnt);  // sort only the occupied prefix
-      for (uint32_t i = S + cnt + tid; i < p2; i += IVF_THREADS) keys[i] = kSentinelKey;
-      __syncthreads();
-      block_bitonic_sort(keys, p2);
+      uint64_t tau;
+      if (keep && S + cnt > KEEP_MIN && S + cnt <= KEEP_MAX) {
+        tau = block_keep_smallest<IVF_THREADS, KEEP_MAX / IVF_THREADS>(keys, S + cnt, S, *keep);
+      } else {
+        const uint32_t p2 = next_pow2_dev(S + cnt);  // sort only the occupied prefix
+        for (uint32_t i = S + cnt + tid; i < p2; i += IVF_THREADS) keys[i] = kSentinelKey;
+        __syncthreads();
+        block_bitonic_sort(keys, p2);
+        tau = keys[S - 1];
+      }
       if (tid == 0) {
         s_cnt = 0;
-        s_tau = keys[S - 1];
+        s_tau = tau;
       }
       __syncthreads();
     };
@@ -680,7 +699,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
       uint64_t key = 0;
       if (pass) {
         key = make_key(d, is_pos ? __ldg(a.vec_ids + at) : at);
-        pass = key < tau;
+        pass = key <= tau;
       }
       const uint32_t m = __ballot_sync(0xffffffffu, pass);
       if (m == 0u) return;
@@ -861,6 +880,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
 
       // the sequence of the chunk's (other) postings
       const uint32_t total = s_cum[nl];
+      uint32_t at_list = 0;  // the list of this thread's last posting (they only move on)
       for (uint32_t base = 0; base < total; base += step) {
         uint32_t lp[R];
         Post post[R];
@@ -870,11 +890,14 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
         for (int r = 0; r < R; ++r) {
           const uint32_t t = base + r * IVF_THREADS + tid;
           // the last list whose prefix is <= t (empty lists repeat a prefix)
-          uint32_t p = 0;
+          uint32_t p = at_list;
+          if (p + 1 < nl && s_cum[p + 1] <= t) {
+            p = 0;
 #pragma unroll
-          for (uint32_t h = LIST_CHUNK / 2; h; h >>= 1)
-            if (p + h < nl && s_cum[p + h] <= t) p += h;
-          lp[r] = p;
+            for (uint32_t h = LIST_CHUNK / 2; h; h >>= 1)
+              if (p + h < nl && s_cum[p + h] <= t) p += h;
+          }
+          lp[r] = at_list = p;
           post[r] = fetch(s_beg[p] + (t - s_cum[p]), t < total, s_list[p] >> 31);
           const size_t row = a.list_major ? post[r].pos : post[r].id;
           if constexpr (MODE != IVF_SQ8 && MW > 0) {
@@ -952,7 +975,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
       for (uint32_t i = tid; i < S; i += IVF_THREADS) dst[i] = keys[i];
       continue;
     }
-    ivf_finish_query<2, 4>(a, keys, q, S, kq, do_rerank, qv);
+    ivf_finish_query<IVF_THREADS, 2, 4>(a, keys, q, S, kq, do_rerank, qv, keep);
   }
 }
 
@@ -1013,7 +1036,10 @@ __global__ void __launch_bounds__(256) ivf_order_kernel(uint32_t nq, const uint3
 // G > 1: one CTA per query merges the G range shortlists (top S of their
 // union, by key), reranks and writes the top k -- the same answer as one
 // range holding every posting.
-__global__ void __launch_bounds__(IVF_THREADS) ivf_merge_kernel(IvfArgs a) {
+// NT: 256, or 1,024 where the queries leave SMs idle (more rows of the rerank
+// are then in flight: 8 queries, 100 rows of 768: 57 us with 256).
+template <int NT>
+__global__ void __launch_bounds__(NT) ivf_merge_kernel(IvfArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   uint64_t* keys = reinterpret_cast<uint64_t*>(smem);
   const uint32_t q = blockIdx.x, G = a.items_per_q;
@@ -1023,61 +1049,25 @@ __global__ void __launch_bounds__(IVF_THREADS) ivf_merge_kernel(IvfArgs a) {
   const uint32_t S = ivf_clamps(kq, npq, rrq, a.nlist);
   kq = min(kq, a.top_k);
   const bool do_rerank = rrq != 1u && a.vectors != nullptr;
+  __shared__ KeepScratch keep;
   const uint32_t total = G * S;
   const uint64_t* src = a.partial + (size_t)q * G * a.part_stride;
-  // The S smallest of the ranges' sorted shortlists. With each thread's keys
-  // in registers their S-th key is built bit by bit by counting (64 rounds of
-  // compares and a barrier), and only S keys are sorted: 64 ranges of 100 took
-  // 127 us as one sort of 8,192 keys.
-  constexpr int NV = 32;
-  if (total > 2 * S && total <= NV * IVF_THREADS) {
-    __shared__ uint32_t part[2][IVF_THREADS / 32];
-    __shared__ uint32_t n_kept;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint64_t kv[NV];
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const uint32_t e = (uint32_t)i * IVF_THREADS + threadIdx.x;
-      kv[i] = e < total ? __ldcg(src + (size_t)(e / S) * a.part_stride + e % S) : kSentinelKey;
-    }
-    if (threadIdx.x == 0) n_kept = 0;
-    uint64_t kth = 0;
-    const int used = (int)((total + IVF_THREADS - 1) / IVF_THREADS);
-    for (int bit = 63; bit >= 0; --bit) {
-      const uint64_t test = kth | ((1ull << bit) - 1ull);
-      uint32_t c = 0;
-#pragma unroll
-      for (int i = 0; i < NV; ++i)
-        if (i < used) c += kv[i] <= test;
-      c = __reduce_add_sync(0xffffffffu, c);
-      if (lane == 0) part[bit & 1][warp] = c;
-      __syncthreads();
-      uint32_t sum = 0;
-#pragma unroll
-      for (int w = 0; w < IVF_THREADS / 32; ++w) sum += part[bit & 1][w];
-      if (sum < S) kth |= 1ull << bit;
-    }
-    // (fewer than S keys: the S-th is the sentinel, and all keys are kept)
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      if (kv[i] <= kth && kv[i] != kSentinelKey) {
-        const uint32_t at = atomicAdd(&n_kept, 1u);
-        if (at < S) keys[at] = kv[i];
-      }
-    }
-    __syncthreads();
-    const uint32_t p2 = next_pow2_dev(S);
-    for (uint32_t i = n_kept + threadIdx.x; i < p2; i += IVF_THREADS) keys[i] = kSentinelKey;
-    __syncthreads();
-    block_bitonic_sort(keys, p2);
+  for (uint32_t i = threadIdx.x; i < total; i += NT) keys[i] = __ldcg(src + (size_t)(i / S) * a.part_stride + i % S);
+  // The S smallest of the ranges' shortlists: selected from registers (64
+  // ranges of 100 took 127 us as one sort of 8,192 keys), or sorted where
+  // that is the quicker, or the registers do not hold them.
+  __syncthreads();
+  if (total > KEEP_MIN && total <= 2048) {
+    block_keep_smallest<NT, 2048 / NT>(keys, total, S, keep);
+  } else if (total > KEEP_MIN && total <= 8192) {
+    block_keep_smallest<NT, 8192 / NT>(keys, total, S, keep);
   } else {
     const uint32_t p2 = next_pow2_dev(total);
-    for (uint32_t i = threadIdx.x; i < p2; i += IVF_THREADS)
-      keys[i] = i < total ? src[(size_t)(i / S) * a.part_stride + i % S] : kSentinelKey;
+    for (uint32_t i = total + threadIdx.x; i < p2; i += NT) keys[i] = kSentinelKey;
     __syncthreads();
     block_bitonic_sort(keys, p2);
   }
-  ivf_finish_query<4, 8>(a, keys, q, S, kq, do_rerank, a.queries + (size_t)q * a.dim);
+  ivf_finish_query<NT, NT == 256 ? 4 : 2, 8>(a, keys, q, S, kq, do_rerank, a.queries + (size_t)q * a.dim, &keep);
 }
 
 // The mask in list order (one word per 32 list positions), for one call.
@@ -1451,8 +1441,13 @@ IvfPlan plan_ivf_search(int mode, const IvfLaunch& L) {
   uint32_t G = 1;
   if (split_knob > 1)
     G = (uint32_t)split_knob;
-  else if (split_knob < 0 && L.nq < 4 * sms)
-    G = (4 * sms + L.nq - 1) / L.nq;
+  else if (split_knob < 0 && L.nq < 4 * sms) {
+    // A few queries are cut into as many ranges as run at once (equal ones: a
+    // range too many is a second wave); more queries into somewhat more, whose
+    // unequal lists the CTAs even out by pulling.
+    const uint32_t slots = (mode == IVF_RABITQ ? 4u : 3u) * sms;
+    G = 8 * L.nq <= slots ? slots / L.nq : (4 * sms + L.nq - 1) / L.nq;
+  }
   G = std::max(1u, std::min<uint32_t>(std::min(G, 64u), 16384u / next_pow2(shortlist)));
 
   // coarse probe: exact fp32 scan, or the tensor-core candidates + exact
@@ -1678,6 +1673,13 @@ int launch_ivf_search(int mode, const IvfLaunch& L, cudaStream_t stream) {
   const size_t staged = mode == IVF_SQ8 ? IvfSmem::staged_bytes(a.keys_pow2, L.dim, a.list_chunk) : 0;
   const bool stage_rows = staged > 0 && staged <= 227 * 1024;
   if (stage_rows) smem = staged;
+  // scratch of the flushes' selection, where shortlist and buffer fit its
+  // registers (and the block has room: else they sort)
+  const size_t keep_at = (smem + 15) / 16 * 16;
+  if (shortlist + IVF_BUF <= KEEP_MAX && keep_at + sizeof(KeepScratch) <= 224 * 1024) {
+    a.keep_at = (uint32_t)keep_at;
+    smem = keep_at + sizeof(KeepScratch);
+  }
   const bool rows16 = mode == IVF_PQ && ((uintptr_t)L.codes % 16u) == 0;
   auto kern = stage_rows ? ivf_scan_kernel<IVF_SQ8, 1, 2> : ivf_scan_kernel<IVF_SQ8, 0, 1>;
   if (mode == IVF_RABITQ) {
@@ -1718,10 +1720,11 @@ int launch_ivf_search(int mode, const IvfLaunch& L, cudaStream_t stream) {
   }
   if (G > 1) {
     const size_t msmem = (size_t)next_pow2(G * shortlist) * 8;
-    e = cudaFuncSetAttribute(ivf_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem);
+    auto merge = L.nq <= 2 * sms ? ivf_merge_kernel<1024> : ivf_merge_kernel<256>;
+    e = cudaFuncSetAttribute(merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem);
     if (e != cudaSuccess) return (int)e;
     ProfScope ps("ivf_merge", stream);
-    ivf_merge_kernel<<<L.nq, IVF_THREADS, msmem, stream>>>(a);
+    merge<<<L.nq, L.nq <= 2 * sms ? 1024 : 256, msmem, stream>>>(a);
     note_launch();
   }
   return (int)cudaGetLastError();

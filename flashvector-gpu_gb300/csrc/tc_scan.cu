@@ -169,13 +169,15 @@ struct SelectArgs {
   uint32_t* incomplete_q;    // per-query flag set when a range heap may have dropped keys (or null)
 };
 
-constexpr int SEL_THREADS = 256;
 constexpr int BAND_MAX = 64;
 
 // One CTA per query: merge the per-range heaps, keep the best `shortlist`
 // keys, rescore them in fp32 (the reference's warp-order distance), sort,
 // re-rank the band |d - d_k| <= eps * scale in fp64, write the top k.
-__global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
+// NT: 256 threads, or 1,024 where the queries leave SMs idle (1 query of 1M x
+// 768: 22 us with 256, most of it the rows' latency).
+template <int NT>
+__global__ void __launch_bounds__(NT) tc_select_kernel(SelectArgs s) {
   extern __shared__ __align__(16) uint64_t keys[];
   __shared__ double band_d[BAND_MAX];
   __shared__ int band_lo, band_hi;
@@ -198,14 +200,14 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
     live = block_compact_keys(src, total, keys, &n_live, s.cap, limit);
   }
   const uint32_t sp2 = next_pow2_dev(max(max(live, kp), 2u));
-  for (uint32_t i = live + threadIdx.x; i < sp2; i += SEL_THREADS) keys[i] = kSentinelKey;
+  for (uint32_t i = live + threadIdx.x; i < sp2; i += NT) keys[i] = kSentinelKey;
   __syncthreads();
   block_bitonic_sort(keys, sp2);
   if (s.kl < kp) {
     // a range whose heap stayed full and whose worst kept key still beats the
     // kp-th merged key may have dropped keys that belong in the shortlist
     const uint64_t cut = keys[kp - 1];
-    for (uint32_t l = threadIdx.x; l < s.lists; l += SEL_THREADS) {
+    for (uint32_t l = threadIdx.x; l < s.lists; l += NT) {
       const uint64_t root = src[(size_t)l * s.kl];
       if (root != kSentinelKey && root < cut) incomplete = 1;
     }
@@ -221,8 +223,9 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
 
   const float* qv = s.queries + (size_t)q * s.dim;
   if (s.vectors) {
-    // four candidates per warp pass, so that four rows' gathers are in flight
-    constexpr uint32_t NW = SEL_THREADS / 32, R = 4;
+    // four candidates per warp pass (two of 32 warps), so that as many rows'
+    // gathers are in flight
+    constexpr uint32_t NW = NT / 32, R = NT == 256 ? 4 : 2;
     for (uint32_t c0 = warp; c0 < kp; c0 += R * NW) {
       if (keys[c0] == kSentinelKey) break;  // sorted: the rest are sentinels too
       const float* rows[R];
@@ -236,7 +239,7 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
         rows[r] = s.vectors + (size_t)slot[r] * s.dim;
       }
       float d[R];
-      warp_metric_distances<R, 4>(qv, rows, s.dim, lane, (MetricType)s.metric, d);
+      warp_metric_distances<R, NT == 256 ? 4 : 8>(qv, rows, s.dim, lane, (MetricType)s.metric, d);
       __syncwarp();
       if (lane == 0) {
 #pragma unroll
@@ -247,7 +250,7 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
       }
     }
     const uint32_t p2 = next_pow2_dev(kp);
-    for (uint32_t i = kp + threadIdx.x; i < p2; i += SEL_THREADS) keys[i] = kSentinelKey;
+    for (uint32_t i = kp + threadIdx.x; i < p2; i += NT) keys[i] = kSentinelKey;
     __syncthreads();
     block_bitonic_sort(keys, p2);
 
@@ -272,7 +275,7 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
       }
       __syncthreads();
       const int lo = band_lo, hi = band_hi;
-      for (int c = lo + warp; c < hi; c += SEL_THREADS / 32) {
+      for (int c = lo + warp; c < hi; c += NT / 32) {
         const double d = warp_distance_f64(qv, s.vectors + (size_t)key_slot(keys[c]) * s.dim, s.dim, lane, s.metric);
         if (lane == 0) band_d[c - lo] = d;
       }
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(SEL_THREADS) tc_select_kernel(SelectArgs s) {
       __syncthreads();
     }
   }
-  for (uint32_t r = threadIdx.x; r < s.k; r += SEL_THREADS)
+  for (uint32_t r = threadIdx.x; r < s.k; r += NT)
     s.out[(size_t)q * s.k + r] = key_to_result(r < kp ? keys[r] : kSentinelKey, nullptr);
 }
 
@@ -747,11 +750,13 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
                opt.boundary_fp64 ? 1u : 0u, 0.f, out, status_word(), tau, redo, nullptr, incomplete_q};
   s.eps = opt.boundary_eps > 0.f ? opt.boundary_eps : (float)((t.dim + 31) / 32 + 5) * 2.0f * 5.960464477539063e-08f;
   size_t sel_smem = (size_t)sel_keys * 8;
-  e = cudaFuncSetAttribute(tc_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem);
+  const int sel_threads = nq <= 2u * (uint32_t)device_sm_count() ? 1024 : 256;
+  auto select = sel_threads == 1024 ? tc_select_kernel<1024> : tc_select_kernel<256>;
+  e = cudaFuncSetAttribute(select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem);
   if (e != cudaSuccess) return (int)e;
   {
     ProfScope ps("tc_select_rescore", stream);
-    tc_select_kernel<<<nq, SEL_THREADS, sel_smem, stream>>>(s);
+    select<<<nq, sel_threads, sel_smem, stream>>>(s);
     note_launch();
   }
   if (prepass && P.pstride > 1) {
@@ -766,13 +771,13 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
     SelectArgs r = s;
     r.cap = std::max(sel_keys, all_keys);
     sel_smem = (size_t)r.cap * 8;
-    e = cudaFuncSetAttribute(tc_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem);
+    e = cudaFuncSetAttribute(select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem);
     if (e != cudaSuccess) return (int)e;
     r.tau = nullptr;
     r.redo = nullptr;
     r.only = redo;
     ProfScope ps("tc_select_rescore", stream);
-    tc_select_kernel<<<nq, SEL_THREADS, sel_smem, stream>>>(r);
+    select<<<nq, sel_threads, sel_smem, stream>>>(r);
     note_launch();
   }
   return (int)cudaGetLastError();
