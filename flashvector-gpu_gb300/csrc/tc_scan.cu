@@ -306,45 +306,63 @@ __global__ void __launch_bounds__(NT) tc_select_kernel(SelectArgs s) {
 
 // The admission bound of each query: the r-th smallest of its `cnt` minima
 // (no bound, 1e30, when fewer than r of them are distances), raised by a few
-// ulps so that the scan admits every row behind it. One block per
-// query, NV values per thread in registers (the rest re-read from L2), the
-// answer built bit by bit from the top of the ordered representation by
-// counting values: 32 rounds of NV compares and one barrier. Also clears the
-// query's re-scan flag. A scan whose distances carry an error raises the
-// bound b to b + m.rel |b| + m.per_norm qnorm[q] + m.abs.
+// ulps so that the scan admits every row behind it. NV values per thread in
+// registers (the rest re-read from L2), the answer built bit by bit from the
+// top of the ordered representation by counting values. Also clears the
+// query's re-scan flag. A scan whose distances carry an error raises the bound
+// b to b + m.rel |b| + m.per_norm qnorm[q] + m.abs.
 struct TauMargin {
   float rel = 1e-6f, per_norm = 0.f, abs = 0.f;
   const float* qnorm = nullptr;
 };
+//
+// Up to 2,048 minima a query is one warp's, without barriers (2,000 queries of
+// 512: 12 us with a block each); more take a block of 128 threads.
 constexpr int TAU_THREADS = 128;
-template <int NV>
-__global__ void __launch_bounds__(TAU_THREADS) tc_tau_kernel(const float* __restrict__ pmin, uint32_t cnt,
+template <int NV, bool WARP>
+__global__ void __launch_bounds__(TAU_THREADS) tc_tau_kernel(const float* __restrict__ pmin, uint32_t nq, uint32_t cnt,
                                                              uint32_t stride, uint32_t r, TauMargin m,
                                                              float* __restrict__ tau, uint32_t* __restrict__ redo) {
+  constexpr int LANES = WARP ? 32 : TAU_THREADS;  // threads of a query
   __shared__ uint32_t part[2][TAU_THREADS / 32];
-  const uint32_t q = blockIdx.x, tid = threadIdx.x;
+  const uint32_t q = WARP ? blockIdx.x * (TAU_THREADS / 32) + (threadIdx.x >> 5) : blockIdx.x;
+  const uint32_t tid = WARP ? threadIdx.x & 31u : threadIdx.x;
+  if (q >= nq) return;  // (whole warps)
   const float* src = pmin + (size_t)q * stride;
-  uint32_t u[NV];
+  uint32_t u[NV], lo = 0xFFFFFFFFu, hi = 0;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const uint32_t at = (uint32_t)i * TAU_THREADS + tid;
+    const uint32_t at = (uint32_t)i * LANES + tid;
     u[i] = at < cnt ? float_order(__ldcg(src + at)) : 0xFFFFFFFFu;
+    lo = min(lo, u[i]);
+    if (at < cnt) hi = max(hi, u[i]);
   }
+  // bits above the highest in which two values differ are common to all
+  int top = 31;
   uint32_t ans = 0;
+  if (WARP) {
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    top = 31 - __clz(lo ^ hi);
+    ans = top < 0 ? lo : lo & ~((2u << top) - 1u);
+  }
 #pragma unroll 1
-  for (int bit = 31; bit >= 0; --bit) {
+  for (int bit = top; bit >= 0; --bit) {
     const uint32_t test = ans | ((1u << bit) - 1u);
     uint32_t c = 0;
 #pragma unroll
     for (int i = 0; i < NV; ++i) c += u[i] <= test;
-    for (uint32_t at = NV * TAU_THREADS + tid; at < cnt; at += TAU_THREADS) c += float_order(__ldcg(src + at)) <= test;
+    if (!WARP)
+      for (uint32_t at = NV * LANES + tid; at < cnt; at += LANES) c += float_order(__ldcg(src + at)) <= test;
     c = __reduce_add_sync(0xffffffffu, c);
-    if ((tid & 31) == 0) part[bit & 1][tid >> 5] = c;
-    __syncthreads();
-    uint32_t total = 0;
+    if (!WARP) {
+      if ((tid & 31) == 0) part[bit & 1][tid >> 5] = c;
+      __syncthreads();
+      c = 0;
 #pragma unroll
-    for (int w = 0; w < TAU_THREADS / 32; ++w) total += part[bit & 1][w];
-    if (total < r) ans |= 1u << bit;
+      for (int w = 0; w < TAU_THREADS / 32; ++w) c += part[bit & 1][w];
+    }
+    if (c < r) ans |= 1u << bit;
   }
   if (tid == 0) {
     const float t = order_float(ans);
@@ -356,15 +374,20 @@ __global__ void __launch_bounds__(TAU_THREADS) tc_tau_kernel(const float* __rest
 
 void launch_tau(const float* pmin, uint32_t nq, uint32_t cnt, uint32_t stride, uint32_t r, const TauMargin& m,
                 float* tau, uint32_t* redo, cudaStream_t stream) {
-  auto go = [&](auto kern) { kern<<<nq, TAU_THREADS, 0, stream>>>(pmin, cnt, stride, r, m, tau, redo); };
-  if (cnt <= 4 * TAU_THREADS)
-    go(tc_tau_kernel<4>);
-  else if (cnt <= 8 * TAU_THREADS)
-    go(tc_tau_kernel<8>);
-  else if (cnt <= 16 * TAU_THREADS)
-    go(tc_tau_kernel<16>);
+  auto go = [&](auto kern, uint32_t per_block) {
+    kern<<<(nq + per_block - 1) / per_block, TAU_THREADS, 0, stream>>>(pmin, nq, cnt, stride, r, m, tau, redo);
+  };
+  constexpr uint32_t W = TAU_THREADS / 32;
+  if (cnt <= 256)
+    go(tc_tau_kernel<8, true>, W);
+  else if (cnt <= 512)
+    go(tc_tau_kernel<16, true>, W);
+  else if (cnt <= 1024)
+    go(tc_tau_kernel<32, true>, W);
+  else if (cnt <= 2048)
+    go(tc_tau_kernel<64, true>, W);
   else
-    go(tc_tau_kernel<32>);
+    go(tc_tau_kernel<32, false>, 1);
 }
 
 // cuTensorMapEncodeTiled resolved through the runtime, so the library does
