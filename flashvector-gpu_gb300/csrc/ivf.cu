@@ -206,12 +206,12 @@ struct IvfSmem {
   // [keys_pow2] u64 keys | table | query (dim f32) | PQ: query residual to the
   // probed centroid (dim f32) | the lists of a chunk: first posting, list,
   // postings before it (3 LC + 1 u32)
-  // table: PQ LUT (m*256 f32); SQ8 mins+scales (2*dim f32); RaBitQ rotated
+  // table: PQ LUT (m*256 f32); SQ8 mins+scales+residual (3*dim f32); RaBitQ rotated
   //        query (P f32) + per list of a chunk its query code (4*W u32
   //        bit-planes, min, delta, sum u, centroid distance)
   __host__ __device__ static size_t table_floats(int mode, uint32_t dim, uint32_t m_pq, uint32_t P, uint32_t lc) {
     return mode == IVF_PQ ? (size_t)m_pq * 256
-                          : mode == IVF_SQ8 ? ((size_t)2 * dim + 3) / 4 * 4 : (size_t)P + (size_t)lc * (P / 8 + 4);
+                          : mode == IVF_SQ8 ? (size_t)3 * dim : (size_t)P + (size_t)lc * (P / 8 + 4);
   }
   static size_t bytes(int mode, uint32_t keys_pow2, uint32_t dim, uint32_t m_pq, uint32_t P, uint32_t lc) {
     size_t b = (size_t)keys_pow2 * 8;
@@ -321,19 +321,39 @@ __device__ __forceinline__ float rabitq_estimate(uint32_t s_bu, float4 m, float 
   return est;
 }
 
-// s_bu of a row of MW 16-byte words of bits held in registers
+// s_bu of a row of MW 16-byte words of bits held in registers. The masked
+// words of the four planes are added bitwise before they are counted: a full
+// adder turns three words of one weight into a sum and a carry of twice the
+// weight (two logic instructions), so nine population counts (a quarter-rate
+// unit) replace sixteen per 128 bits.
+__device__ __forceinline__ void full_add(uint32_t a, uint32_t b, uint32_t c, uint32_t& sum, uint32_t& carry) {
+  sum = a ^ b ^ c;
+  carry = (a & b) | (c & (a | b));
+}
 template <int MW>
 __device__ __forceinline__ uint32_t rabitq_sbu(const uint32_t* planes, const uint4 (&b)[MW]) {
   uint32_t acc = 0;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    uint32_t c = 0;
+  for (int w = 0; w < MW; ++w) {
+    uint32_t x[4][4];
 #pragma unroll
-    for (int w = 0; w < MW; ++w) {
+    for (int j = 0; j < 4; ++j) {
       const uint4 p = *reinterpret_cast<const uint4*>(planes + j * 4 * MW + 4 * w);
-      c += __popc(b[w].x & p.x) + __popc(b[w].y & p.y) + __popc(b[w].z & p.z) + __popc(b[w].w & p.w);
+      x[j][0] = b[w].x & p.x;
+      x[j][1] = b[w].y & p.y;
+      x[j][2] = b[w].z & p.z;
+      x[j][3] = b[w].w & p.w;
     }
-    acc += c << j;
+    uint32_t s1, c2, s2, t2, c4a, c4b, s4, t4, c8a, c8b, s8, t8, c16a, c16b;
+    full_add(x[0][0], x[0][1], x[0][2], s1, c2);      // weight 1: s1, x[0][3]
+    full_add(x[1][0], x[1][1], x[1][2], t2, c4a);
+    full_add(t2, x[1][3], c2, s2, c4b);               // weight 2: s2
+    full_add(x[2][0], x[2][1], x[2][2], s4, c8a);
+    full_add(x[2][3], c4a, c4b, t4, c8b);             // weight 4: s4, t4
+    full_add(x[3][0], x[3][1], x[3][2], s8, c16a);
+    full_add(x[3][3], c8a, c8b, t8, c16b);            // weight 8: s8, t8
+    acc += (__popc(s1) + __popc(x[0][3])) + (__popc(s2) << 1) + ((__popc(s4) + __popc(t4)) << 2) +
+           ((__popc(s8) + __popc(t8)) << 3) + ((__popc(c16a) + __popc(c16b)) << 4);
   }
   return acc;
 }
@@ -450,13 +470,15 @@ __device__ __forceinline__ float sq8_row(const float* qs, const float* __restric
 // at a time. The rows' codes come in through shared memory by whole segments
 // (a lane reading its own row touches one line per 16 bytes: 32 L1 wavefronts
 // where the segment takes 8), and one read of the query, centroid and decoding
-// parameters serves both rows. Rows may start at any byte: words are loaded
+// parameters serves both rows. RES: qs already holds the residual to the
+// centroid that all rows share. Rows may start at any byte: words are loaded
 // aligned and shifted into place. A byte becomes a float by taking the
 // mantissa's place in 2^23. row[i]: the lane's rows (null: none).
 // Warp-collective.
 constexpr uint32_t SQ_CHUNK = 64;   // dimensions per staged chunk
 constexpr uint32_t SQ_STRIDE = 80;  // bytes per staged row: 17 words, 16-byte steps off the same bank
 constexpr uint32_t SQ_WARP_BYTES = 2 * 32 * SQ_STRIDE;
+template <bool RES>
 __device__ __forceinline__ void sq8_rows(const float* qs, const float* const (&cent)[2], const float* mins,
                                          const float* scales, const uint8_t* const (&row)[2], uint32_t dim,
                                          bool aligned, bool cent16, uint8_t* stage, float (&out)[2]) {
@@ -509,7 +531,7 @@ __device__ __forceinline__ void sq8_rows(const float* qs, const float* const (&c
     const uint8_t* st1 = st0 + 32 * SQ_STRIDE;
     auto term = [&](float& s, uint32_t w, int b, float qd, float cd, float m, float k) {
       const float code = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + b)) - 8388608.0f;  // exact
-      const float t = __fsub_rn(__fsub_rn(qd, cd), fmaf(code, k, m));
+      const float t = __fsub_rn(RES ? qd : __fsub_rn(qd, cd), fmaf(code, k, m));
       s = fmaf(t, t, s);
     };
     if (aligned && cent16) {
@@ -522,8 +544,11 @@ __device__ __forceinline__ void sq8_rows(const float* qs, const float* const (&c
           const float4 q = *reinterpret_cast<const float4*>(qs + at);
           const float4 mn = *reinterpret_cast<const float4*>(mins + at);
           const float4 sc = *reinterpret_cast<const float4*>(scales + at);
-          const float4 ca = __ldg(reinterpret_cast<const float4*>(cent[0] + at));
-          const float4 cb = cent[1] == cent[0] ? ca : __ldg(reinterpret_cast<const float4*>(cent[1] + at));
+          float4 ca = q, cb = q;
+          if (!RES) {
+            ca = __ldg(reinterpret_cast<const float4*>(cent[0] + at));
+            cb = cent[1] == cent[0] ? ca : __ldg(reinterpret_cast<const float4*>(cent[1] + at));
+          }
           term(out[0], a4[j], 0, q.x, ca.x, mn.x, sc.x);
           term(out[1], b4[j], 0, q.x, cb.x, mn.x, sc.x);
           term(out[0], a4[j], 1, q.y, ca.y, mn.y, sc.y);
@@ -544,7 +569,11 @@ __device__ __forceinline__ void sq8_rows(const float* qs, const float* const (&c
           const uint32_t at = d0 + d + b;
           if (at >= dim) break;
           const float q = qs[at], mn = mins[at], sc = scales[at];
-          const float ca = __ldg(cent[0] + at), cb = cent[1] == cent[0] ? ca : __ldg(cent[1] + at);
+          float ca = q, cb = q;
+          if (!RES) {
+            ca = __ldg(cent[0] + at);
+            cb = cent[1] == cent[0] ? ca : __ldg(cent[1] + at);
+          }
           term(out[0], wa, b, q, ca, mn, sc);
           term(out[1], wb, b, q, cb, mn, sc);
         }
@@ -557,6 +586,10 @@ __device__ __forceinline__ void sq8_rows(const float* qs, const float* const (&c
 // reads the whole codebook and costs about as much as evaluating 128 rows in
 // place (32 of the 8,192 entries each).
 constexpr uint32_t PQ_TABLE_MIN = 128;
+// A longer list of the other modes is walked by itself too: one list's query
+// code (RaBitQ) or residual (SQ8) serves every posting without a search for
+// its list. Below, a round of the CTA would be part empty.
+constexpr uint32_t LIST_ALONE_MIN = 1024;
 
 // Resident CTAs per SM each variant is compiled for (its register budget:
 // 4 -> 64, 3 -> 85, 2 -> 128 registers per thread): the list scans are
@@ -764,8 +797,8 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
         } else {
           len = 0;
         }
-        // a PQ list that is worth its tables leaves the common sequence
-        const bool tables = MODE == IVF_PQ && len >= PQ_TABLE_MIN;
+        // a list that is worth a walk of its own leaves the common sequence
+        const bool tables = MODE == IVF_PQ ? len >= PQ_TABLE_MIN : MW > 0 && len >= LIST_ALONE_MIN;
         const uint32_t longs = __ballot_sync(0xffffffffu, tables);
         uint32_t x = tables ? 0u : len;
         const uint32_t own = x;
@@ -777,7 +810,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
         if (lane < (int)nl) {
           s_beg[lane] = beg;
           s_list[lane] = (l & 0x7FFFFFFFu) | (compact ? 0x80000000u : 0u);
-          s_cum[lane] = tables ? len : x - own;  // (a tabled list's entry: its length, see below)
+          s_cum[lane] = tables ? len : x - own;  // (such a list's entry: its length, see below)
         }
         if (lane == 0) s_long = longs;
         if (lane == (int)nl - 1) s_cum[nl] = x;
@@ -790,7 +823,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
       }
       __syncthreads();
 
-      if constexpr (MODE == IVF_PQ) {
+      if constexpr (MODE == IVF_PQ || MW > 0) {
         uint32_t longs = s_long;  // uniform over the block
         while (longs) {
           const uint32_t p = __ffs(longs) - 1;
@@ -798,52 +831,65 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
           const uint32_t l = s_list[p] & 0x7FFFFFFFu, beg = s_beg[p], end = beg + s_cum[p];
           const bool compact = s_list[p] >> 31;
           const float* cent = a.centroids + (size_t)l * a.dim;
-          // LUT[m][c] = sum_sd ((q - centroid) - codeword)^2 with fmaf in
-          // sub-dimension order; q - centroid is rounded once per dimension, as
-          // the reference's expression rounds it (ivf_pq_lookup.cu:150-162)
-          for (uint32_t d = tid; d < a.dim; d += IVF_THREADS) qres[d] = qs[d] - __ldg(cent + d);
-          __syncthreads();
-          const uint32_t entries = a.m_pq * 256;
-          if (cb4) {
-            const float4* cbv = reinterpret_cast<const float4*>(a.codebooks);
-            auto entry = [&](uint32_t e, float4 w) {  // codeword (m, c) = row e of 4 floats
-              const float* r = qres + (e >> 8) * 4;
-              const float t0 = r[0] - w.x, t1 = r[1] - w.y, t2 = r[2] - w.z, t3 = r[3] - w.w;
-              tab[e] = fmaf(t3, t3, fmaf(t2, t2, fmaf(t1, t1, fmaf(t0, t0, 0.f))));
-            };
-            // B codeword loads in flight per thread before any is used (the
-            // codebooks, 16 KB per sub-space, stream from L2 for every list)
-            constexpr uint32_t B = 8;
-            uint32_t e0 = tid;
-            for (; e0 + (B - 1) * IVF_THREADS < entries; e0 += B * IVF_THREADS) {
-              float4 w[B];
+          if constexpr (MODE == IVF_PQ) {
+            // LUT[m][c] = sum_sd ((q - centroid) - codeword)^2 with fmaf in
+            // sub-dimension order; q - centroid is rounded once per dimension, as
+            // the reference's expression rounds it (ivf_pq_lookup.cu:150-162)
+            for (uint32_t d = tid; d < a.dim; d += IVF_THREADS) qres[d] = qs[d] - __ldg(cent + d);
+            __syncthreads();
+            const uint32_t entries = a.m_pq * 256;
+            if (cb4) {
+              const float4* cbv = reinterpret_cast<const float4*>(a.codebooks);
+              auto entry = [&](uint32_t e, float4 w) {  // codeword (m, c) = row e of 4 floats
+                const float* r = qres + (e >> 8) * 4;
+                const float t0 = r[0] - w.x, t1 = r[1] - w.y, t2 = r[2] - w.z, t3 = r[3] - w.w;
+                tab[e] = fmaf(t3, t3, fmaf(t2, t2, fmaf(t1, t1, fmaf(t0, t0, 0.f))));
+              };
+              // B codeword loads in flight per thread before any is used (the
+              // codebooks, 16 KB per sub-space, stream from L2 for every list)
+              constexpr uint32_t B = 8;
+              uint32_t e0 = tid;
+              for (; e0 + (B - 1) * IVF_THREADS < entries; e0 += B * IVF_THREADS) {
+                float4 w[B];
 #pragma unroll
-              for (uint32_t b = 0; b < B; ++b) w[b] = __ldg(cbv + e0 + b * IVF_THREADS);
+                for (uint32_t b = 0; b < B; ++b) w[b] = __ldg(cbv + e0 + b * IVF_THREADS);
 #pragma unroll
-              for (uint32_t b = 0; b < B; ++b) entry(e0 + b * IVF_THREADS, w[b]);
-            }
-            for (uint32_t e = e0; e < entries; e += IVF_THREADS) entry(e, __ldg(cbv + e));
-          } else {
-            for (uint32_t e = tid; e < entries; e += IVF_THREADS) {
-              const uint32_t m = e >> 8, c = e & 255u;
-              const float* cb = a.codebooks + ((size_t)m * 256 + c) * a.sub_dim;
-              float s = 0.f;
-              for (uint32_t sd = 0; sd < a.sub_dim; ++sd) {
-                const float t = qres[m * a.sub_dim + sd] - __ldg(cb + sd);
-                s = fmaf(t, t, s);
+                for (uint32_t b = 0; b < B; ++b) entry(e0 + b * IVF_THREADS, w[b]);
               }
-              tab[e] = s;
+              for (uint32_t e = e0; e < entries; e += IVF_THREADS) entry(e, __ldg(cbv + e));
+            } else {
+              for (uint32_t e = tid; e < entries; e += IVF_THREADS) {
+                const uint32_t m = e >> 8, c = e & 255u;
+                const float* cb = a.codebooks + ((size_t)m * 256 + c) * a.sub_dim;
+                float s = 0.f;
+                for (uint32_t sd = 0; sd < a.sub_dim; ++sd) {
+                  const float t = qres[m * a.sub_dim + sd] - __ldg(cb + sd);
+                  s = fmaf(t, t, s);
+                }
+                tab[e] = s;
+              }
             }
+          } else if constexpr (MODE == IVF_SQ8) {
+            float* res = tab + 2 * a.dim;
+            for (uint32_t d = tid; d < a.dim; d += IVF_THREADS) res[d] = __fsub_rn(qs[d], __ldg(cent + d));
           }
+          [[maybe_unused]] const uint32_t* code = codes + p * code_words;
+          [[maybe_unused]] float4 par = make_float4(0.f, 0.f, 0.f, 0.f);
+          if constexpr (MODE == IVF_RABITQ) par = *reinterpret_cast<const float4*>(code + 4 * a.W);
           __syncthreads();
           for (uint32_t base = beg; base < end; base += step) {
             Post post[R];
             uint4 w[R][MWW];
+            float4 mt[MODE == IVF_RABITQ ? R : 1];
 #pragma unroll
             for (int r = 0; r < R; ++r) {
               const uint32_t i = base + r * IVF_THREADS + tid;
               post[r] = fetch(i, i < end, compact);
-              if constexpr (MW > 0) {
+              if constexpr (MODE == IVF_RABITQ)
+                mt[r] = post[r].in ? __ldg(reinterpret_cast<const float4*>(a.rq_meta) +
+                                           (a.list_major ? post[r].pos : post[r].id))
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+              if constexpr (MW > 0 && MODE != IVF_SQ8) {
                 const uint4* row = reinterpret_cast<const uint4*>(
                     a.codes + (size_t)(a.list_major ? post[r].pos : post[r].id) * (16u * MW));
 #pragma unroll
@@ -851,11 +897,26 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
               }
             }
             const uint64_t tau = s_tau;
+            [[maybe_unused]] float sq[2] = {0.f, 0.f};
+            if constexpr (MODE == IVF_SQ8) {
+              const uint8_t* rows[2];
+#pragma unroll
+              for (int r = 0; r < 2; ++r)
+                rows[r] = post[r].ok ? a.codes + (size_t)(a.list_major ? post[r].pos : post[r].id) * a.code_bytes : nullptr;
+              const float* const none[2] = {nullptr, nullptr};
+              if (__any_sync(0xffffffffu, post[0].ok || post[1].ok))
+                sq8_rows<true>(tab + 2 * a.dim, none, mins, scales, rows, a.dim, vec16, a.dim % 4 == 0, stage, sq);
+            }
 #pragma unroll
             for (int r = 0; r < R; ++r) {
               float d = 0.f;
-              if (post[r].ok) {
-                if constexpr (MW > 0)
+              if constexpr (MODE == IVF_SQ8) {
+                d = sq[r & 1];
+              } else if (post[r].ok) {
+                if constexpr (MODE == IVF_RABITQ)
+                  d = rabitq_estimate(rabitq_sbu<MWW>(code, w[r]), mt[r], (float)a.P, par.x, par.y, par.z, par.w, qn,
+                                      a.metric);
+                else if constexpr (MW > 0)
                   d = adc_words<MWW>(tab, w[r]);
                 else
                   d = adc_row(tab, a.codes + (size_t)(a.list_major ? post[r].pos : post[r].id) * a.code_bytes, a.m_pq,
@@ -868,8 +929,8 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
           }
         }
         if (s_long) {
-          // the tabled lists drop out of the sequence: their prefix entry is
-          // the next list's
+          // the lists walked alone drop out of the sequence: their prefix entry
+          // is the next list's
           __syncthreads();
           if (tid == 0)
             for (int p = (int)nl - 1; p >= 0; --p)
@@ -922,7 +983,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
             cents[r] = a.centroids + (post[r].ok ? (size_t)(s_list[lp[r]] & 0x7FFFFFFFu) * a.dim : 0);
           }
           if (__any_sync(0xffffffffu, post[0].ok || post[1].ok))
-            sq8_rows(qs, cents, mins, scales, rows, a.dim, vec16, cent16, stage, sq);
+            sq8_rows<false>(qs, cents, mins, scales, rows, a.dim, vec16, cent16, stage, sq);
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
