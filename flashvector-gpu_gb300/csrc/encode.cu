@@ -183,31 +183,82 @@ __device__ __forceinline__ int fp8_table_exponent(float mx) {
   return b;
 }
 
+// One step of the butterfly over the lanes' compensated sums, for rows r and
+// r + H at once: the lower half of each 2o lanes goes on with row r, the upper
+// half with row r + H. A row's left operand is the lower lane's, as in a
+// butterfly of one row read at lane 0.
+template <int H>
+__device__ __forceinline__ void neumaier_halve(float* sum, float* comp, int o, int lane) {
+  const bool up = (lane & o) != 0;
+#pragma unroll
+  for (int r = 0; r < H; ++r) {
+    const float os = __shfl_xor_sync(0xffffffffu, up ? sum[r] : sum[r + H], o);
+    const float oc = __shfl_xor_sync(0xffffffffu, up ? comp[r] : comp[r + H], o);
+    float a = up ? os : sum[r], c = up ? oc : comp[r];
+    neumaier_add(a, c, up ? sum[r + H] : os);
+    c += up ? comp[r + H] : oc;
+    sum[r] = a;
+    comp[r] = c;
+  }
+}
+
 // ||x||^2 of each row (compensated), and the largest of them as ordered
 // bits in *max_bits (norms are >= 0, so the bit patterns order like the values).
+// Bound by the read of the table: a warp takes eight rows at a time (eight
+// loads in flight, and three of the five steps across the lanes shared by all
+// eight) and raises the maximum once for all its rows: 47 us for 328,756 x 157.
+// With a row and an atomic on one word per warp the whole encoder took 307 us
+// there and takes 120 (500,000 x 768: 972 and 612 us; two reads and the write
+// at the measured copy rate: 510).
+constexpr int F8_ROWS = 8;
 __global__ void __launch_bounds__(256) fp8_norms_kernel(const float* __restrict__ x, uint32_t n, uint32_t dim,
                                                         float* __restrict__ norms, uint32_t* __restrict__ max_bits) {
-  const uint64_t row = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  const float* src = x + row * dim;
-  float sum = 0.f, comp = 0.f;
-  for (uint32_t d = lane; d < dim; d += 32) {
-    const float v = __ldg(src + d);
-    neumaier_add(sum, comp, __fmul_rn(v, v));
-  }
+  uint32_t top = 0;
+  for (uint64_t row0 = (uint64_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * F8_ROWS; row0 < n;
+       row0 += (uint64_t)warps * F8_ROWS) {
+    float sum[F8_ROWS], comp[F8_ROWS];
+    const float* src[F8_ROWS];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float os = __shfl_xor_sync(0xffffffffu, sum, o);
-    const float oc = __shfl_xor_sync(0xffffffffu, comp, o);
-    neumaier_add(sum, comp, os);
-    comp += oc;
+    for (int r = 0; r < F8_ROWS; ++r) {
+      sum[r] = comp[r] = 0.f;
+      src[r] = x + min(row0 + r, (uint64_t)n - 1) * dim;
+    }
+    // (the next 32 dimensions of every row are in flight while these are added)
+    float v[F8_ROWS];
+#pragma unroll
+    for (int r = 0; r < F8_ROWS; ++r) v[r] = (uint32_t)lane < dim ? __ldg(src[r] + lane) : 0.f;
+    for (uint32_t d = lane; d < dim; d += 32) {
+      float w[F8_ROWS];
+#pragma unroll
+      for (int r = 0; r < F8_ROWS; ++r) w[r] = d + 32 < dim ? __ldg(src[r] + d + 32) : 0.f;
+#pragma unroll
+      for (int r = 0; r < F8_ROWS; ++r) neumaier_add(sum[r], comp[r], __fmul_rn(v[r], v[r]));
+#pragma unroll
+      for (int r = 0; r < F8_ROWS; ++r) v[r] = w[r];
+    }
+    __syncwarp();
+    neumaier_halve<4>(sum, comp, 16, lane);
+    neumaier_halve<2>(sum, comp, 8, lane);
+    neumaier_halve<1>(sum, comp, 4, lane);
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1) {
+      const float os = __shfl_xor_sync(0xffffffffu, sum[0], o);
+      const float oc = __shfl_xor_sync(0xffffffffu, comp[0], o);
+      neumaier_add(sum[0], comp[0], os);
+      comp[0] += oc;
+    }
+    // row r's sum is lane 4 r's
+    const uint64_t row = row0 + (lane >> 2);
+    if ((lane & 3) == 0 && row < n) {
+      const float nrm = sum[0] + comp[0];
+      norms[row] = nrm;
+      if (nrm > 0.f) top = max(top, __float_as_uint(nrm));
+    }
   }
-  if (lane == 0) {
-    const float nrm = sum + comp;
-    norms[row] = nrm;
-    if (nrm > 0.f) atomicMax(max_bits, __float_as_uint(nrm));
-  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0 && top) atomicMax(max_bits, top);
 }
 
 // The table's scale exponent b from the largest norm (written over the
@@ -227,29 +278,80 @@ __device__ __forceinline__ float e4m3_value(uint8_t c) {
   return (c & 0x80u) ? -mag : mag;
 }
 
+// A warp encodes eight rows as one run of 4-byte words (rows are stored one
+// after the other), so that no lane is idle at any width; each of the first
+// eight lanes makes one row's norm digits. Bound by the read of the rows: the
+// grid goes from the last row to the first, as the norms' pass has just left
+// the last ones in L2 (66 us for 328,756 x 157).
+template <bool VEC>
 __global__ void __launch_bounds__(256) encode_fp8_kernel(const float* __restrict__ x, uint32_t n, uint32_t dim,
                                                          uint32_t pd, uint8_t* __restrict__ out,
                                                          float* __restrict__ scales,
                                                          const float* __restrict__ norms) {
-  const uint64_t row = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t groups = ((uint64_t)n + F8_ROWS - 1) / F8_ROWS;
+  const uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (row >= n) return;
+  if (g >= groups) return;
+  const uint64_t row0 = (groups - 1 - g) * F8_ROWS;
+  const uint32_t rows = (uint32_t)min((uint64_t)F8_ROWS, n - row0);
   // scales[0] holds the table scale (row 0 rewrites it with the same value)
   const float s = scales[0];
   const int b = ilogbf(s);
-  const float* src = x + row * dim;
-  uint8_t* dst = out + row * pd;
-  for (uint32_t d = lane; d < dim; d += 32) dst[d] = e4m3_code(ldexpf(__ldg(src + d), -b));
-  if (lane == 0) {
-    float r = ldexpf(norms[row], -1 - 2 * b);
+  const float inv = ldexpf(1.0f, -b);  // (b in [-62, 62]: the product is what ldexpf gives)
+  uint32_t digits = 0;                 // lane r: row r's
+  if (lane < (int)rows) {
+    float r = ldexpf(norms[row0 + lane], -1 - 2 * b);
     for (int i = 0; i < 3; ++i) {
       const uint8_t c = e4m3_code(r);
-      dst[dim + i] = c;
+      digits |= (uint32_t)c << (8 * i);
       r -= e4m3_value(c);
     }
+    scales[row0 + lane] = s;
   }
-  for (uint32_t d = dim + 3 + lane; d < pd; d += 32) dst[d] = 0;
-  if (lane == 0) scales[row] = s;
+  const uint32_t wpr = pd / 4, total = rows * wpr;
+  const float* src = x + row0 * dim;
+  uint8_t* dst = out + row0 * pd;
+  const bool words = (uintptr_t)out % 4 == 0;
+  constexpr uint32_t U = 4;
+  for (uint32_t e0 = 0; e0 < total; e0 += 32 * U) {
+    float v[U][4];
+    uint32_t r[U], d[U];
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      const uint32_t e = min(e0 + 32 * u + lane, total - 1);
+      r[u] = e / wpr;
+      d[u] = (e - r[u] * wpr) * 4;
+      const float* p = src + (size_t)r[u] * dim + d[u];
+      if constexpr (VEC) {
+        // dim is a multiple of 4: four columns in or out together
+        const float4 w = d[u] < dim ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[u][0] = w.x, v[u][1] = w.y, v[u][2] = w.z, v[u][3] = w.w;
+      } else {
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) v[u][i] = d[u] + i < dim ? __ldg(p + i) : 0.f;
+      }
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      const uint32_t dg = __shfl_sync(0xffffffffu, digits, r[u]);
+      uint32_t w = 0;
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i) {
+        // (a column past the row's digits: 0, as a shift by 24 leaves it)
+        const uint32_t col = d[u] + i, dgt = (dg >> min(8 * (col - dim), 24u)) & 255u;
+        w |= (col < dim ? (uint32_t)e4m3_code(__fmul_rn(v[u][i], inv)) : dgt) << (8 * i);
+      }
+      if (e0 + 32 * u + lane < total) {
+        uint8_t* o = dst + (size_t)r[u] * pd + d[u];
+        if (words) {
+          *reinterpret_cast<uint32_t*>(o) = w;
+        } else {
+#pragma unroll
+          for (uint32_t i = 0; i < 4; ++i) o[i] = (uint8_t)(w >> (8 * i));
+        }
+      }
+    }
+  }
 }
 
 // Per-row-scale table (the other fp8 layout): s_v = max|x_v| / 448 (1 for a
@@ -305,13 +407,18 @@ int launch_encode_fp16(const float* x, uint32_t n, uint32_t dim, uint32_t pd, ui
 int launch_encode_fp8(const float* x, uint32_t n, uint32_t dim, uint32_t pd, uint8_t* out, float* scales,
                       float* norms, cudaStream_t stream) {
   if (n == 0) return 0;
-  const uint64_t blocks = ((uint64_t)n * 32 + 255) / 256;
+  // eight warps of eight rows a block; the norms' blocks stay and go on to further rows
+  const uint64_t blocks = ((uint64_t)n + 8 * F8_ROWS - 1) / (8 * F8_ROWS);
   uint32_t* word = reinterpret_cast<uint32_t*>(scales);
   cudaError_t e = cudaMemsetAsync(word, 0, sizeof(uint32_t), stream);
   if (e != cudaSuccess) return (int)e;
-  fp8_norms_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, n, dim, norms, word);
+  const uint64_t stay = (uint64_t)device_sm_count() * 8;
+  fp8_norms_kernel<<<(unsigned)(blocks < stay ? blocks : stay), 256, 0, stream>>>(x, n, dim, norms, word);
   fp8_table_scale_kernel<<<1, 1, 0, stream>>>(word);
-  encode_fp8_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, n, dim, pd, out, scales, norms);
+  if (dim % 4 == 0 && (uintptr_t)x % 16 == 0)
+    encode_fp8_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(x, n, dim, pd, out, scales, norms);
+  else
+    encode_fp8_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(x, n, dim, pd, out, scales, norms);
   note_launch(3);
   return (int)cudaGetLastError();
 }

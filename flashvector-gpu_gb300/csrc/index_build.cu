@@ -23,6 +23,7 @@
 //     scale), sign bits by warp ballot, |r|^2, |x|^2 and sum |rot r| summed
 //     sequentially by single lanes in the reference's order
 //     (quant.rs:156-234), so the tables equal the host encoder's bit for bit.
+#include <type_traits>
 #include <algorithm>
 #include <cmath>
 
@@ -242,7 +243,8 @@ constexpr int RQ_WARPS = 4;
 
 // RaBitQ encoder. bits == nullptr: rot_out row = rotation of x row (the
 // rotated centroids). Otherwise the residual of x row to centroid
-// assign[row] is rotated and its sign bits and meta written.
+// assign[row] is rotated and its sign bits and meta written. For rows of more
+// than 32 x 32 dimensions, which do not fit a warp's registers.
 __global__ void __launch_bounds__(RQ_WARPS * 32)
     rabitq_encode_kernel(const float* __restrict__ x, uint32_t n, uint32_t dim, const float* __restrict__ centroids,
                          uint32_t nlist, const GpuSearchResult* __restrict__ assign, const float* __restrict__ signs,
@@ -311,6 +313,135 @@ __global__ void __launch_bounds__(RQ_WARPS * 32)
       m[0] = res_sq;
       m[1] = (rn > 1e-12f && abs_sum > 1e-12f) ? __fdiv_rn(__fmul_rn(rn, rn), abs_sum) : 0.f;
       m[2] = (float)pop;
+      m[3] = vec_sq;
+    }
+    __syncwarp();
+  }
+}
+
+// The same with the row in registers (dimension 32 e + lane in x[e], which is
+// also the layout that the ballots of the sign bits want): rotation steps
+// below 32 are shuffles, the others register pairs. What bounded the kernel
+// above were its three sums, each sequential over the row and so one lane's
+// work while the warp waited: here a warp keeps R rows' terms in shared memory
+// and 3 R lanes add them up together. The next row is loaded while one is
+// rotated. Now bound by the shuffles; whole calls, with some 100 us of host
+// work: 518,826 x 212 2,750 -> 585 us, 100,000 x 768 2,380 -> 620 us.
+template <int E>
+__host__ __device__ constexpr int rq_rows() {
+  return E <= 4 ? 8 : E == 8 ? 4 : E == 16 ? 2 : 1;
+}
+template <int E>
+constexpr size_t rq_smem_bytes() {
+  return (size_t)RQ_WARPS * 3 * rq_rows<E>() * (32 * E + 4) * 4;
+}
+template <int E>
+__global__ void __launch_bounds__(RQ_WARPS * 32, 4)
+    rabitq_encode_reg_kernel(const float* __restrict__ x, uint32_t n, uint32_t dim, const float* __restrict__ centroids,
+                             uint32_t nlist, const GpuSearchResult* __restrict__ assign,
+                             const float* __restrict__ signs, float scale, float* __restrict__ rot_out,
+                             uint32_t* __restrict__ bits, float* __restrict__ meta) {
+  constexpr int R = rq_rows<E>(), P = 32 * E, STRIDE = P + 4;
+  extern __shared__ __align__(16) float rq_terms[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* terms = rq_terms + (size_t)warp * 3 * R * STRIDE;  // [residual^2 | x^2 | |rotated|][row][STRIDE]
+  float sgn[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) sgn[i] = (lane >> i) & 1 ? -1.f : 1.f;
+  for (uint64_t row0 = ((uint64_t)blockIdx.x * RQ_WARPS + warp) * R; row0 < n;
+       row0 += (uint64_t)gridDim.x * RQ_WARPS * R) {
+    const int rows = (int)min((uint64_t)R, n - row0);
+    uint32_t cid = 0xffffffffu;  // lane r: row r's centroid
+    if (bits && lane < rows) cid = assign[row0 + lane].id;
+    float nv[E], nc[E];
+    auto load = [&](int r) {
+      const float* v = x + (row0 + r) * dim;
+      const uint32_t c = __shfl_sync(0xffffffffu, cid, r);
+      const float* ce = bits && c < nlist ? centroids + (size_t)c * dim : nullptr;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const uint32_t d = 32 * e + lane;
+        nv[e] = d < dim ? __ldg(v + d) : 0.f;
+        nc[e] = ce && d < dim ? __ldg(ce + d) : 0.f;  // (x - 0 is x)
+      }
+    };
+    load(0);
+    uint32_t pops = 0;  // lane r: row r's sign bits
+    for (int r = 0; r < rows; ++r) {
+      float f[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        f[e] = __fsub_rn(nv[e], nc[e]);
+        if (bits) {
+          terms[r * STRIDE + 32 * e + lane] = __fmul_rn(f[e], f[e]);
+          terms[(R + r) * STRIDE + 32 * e + lane] = __fmul_rn(nv[e], nv[e]);
+        }
+      }
+      if (r + 1 < rows) load(r + 1);
+      for (int st = 0; st < 3; ++st) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) f[e] = __fmul_rn(f[e], __ldg(signs + st * P + 32 * e + lane));
+        // (a lane with the step's bit set holds b of (a + b, a - b): a - b is
+        // b (-1) + a, rounded once either way)
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+#pragma unroll
+          for (int e = 0; e < E; ++e) f[e] = fmaf(f[e], sgn[i], __shfl_xor_sync(0xffffffffu, f[e], 1 << i));
+#pragma unroll
+        for (int h = 1; h < E; h <<= 1)
+#pragma unroll
+          for (int e = 0; e < E; ++e)
+            if (!(e & h)) {
+              const float a = f[e], b = f[e + h];
+              f[e] = __fadd_rn(a, b);
+              f[e + h] = __fsub_rn(a, b);
+            }
+#pragma unroll
+        for (int e = 0; e < E; ++e) f[e] = __fmul_rn(f[e], scale);
+      }
+      if (!bits) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) rot_out[(row0 + r) * P + 32 * e + lane] = f[e];
+        continue;
+      }
+      uint32_t word = 0, pop = 0;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const uint32_t b = __ballot_sync(0xffffffffu, f[e] >= 0.f);
+        if (lane == e) word = b;
+        pop += __popc(b);
+        terms[(2 * R + r) * STRIDE + 32 * e + lane] = fabsf(f[e]);
+      }
+      if (lane < E) bits[(row0 + r) * E + lane] = word;
+      if (lane == r) pops = pop;
+    }
+    if (!bits) continue;
+    __syncwarp();
+    // res_norm_sq += r * r, vec_norm_sq += x * x, abs_sum += |rotated|, each in
+    // dimension order: lane t R + r adds row r's terms of kind t
+    float sum = 0.f;
+    if (lane < 3 * R && lane % R < rows) {
+      const float* t = terms + lane * STRIDE;
+      const int m = lane < 2 * R ? (int)dim : P;
+      int j = 0;
+      for (; j + 16 <= m; j += 16) {
+        float4 w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(t + j + 4 * i);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, w[i].x), w[i].y), w[i].z), w[i].w);
+      }
+      for (; j < m; ++j) sum = __fadd_rn(sum, t[j]);
+    }
+    const float vec_sq = __shfl_down_sync(0xffffffffu, sum, R);
+    const float abs_sum = __shfl_down_sync(0xffffffffu, sum, 2 * R);
+    if (lane < rows) {
+      const float rn = __fsqrt_rn(sum);
+      float* m = meta + (row0 + lane) * 4;
+      m[0] = sum;
+      m[1] = (rn > 1e-12f && abs_sum > 1e-12f) ? __fdiv_rn(__fmul_rn(rn, rn), abs_sum) : 0.f;
+      m[2] = (float)pops;
       m[3] = vec_sq;
     }
     __syncwarp();
@@ -443,29 +574,59 @@ void rabitq_rot_signs(uint32_t padded_dim, uint64_t seed, float* out) {
   }
 }
 
+namespace {
+
+// One launch over n rows: a row of up to 1,024 dimensions in registers, longer
+// ones in shared memory.
+int rabitq_encode_rows(const float* x, uint32_t n, uint32_t dim, const float* centroids, uint32_t nlist,
+                       const GpuSearchResult* assign, const float* signs, uint32_t P, float* rot_out, uint32_t* bits,
+                       float* meta, cudaStream_t stream) {
+  const float scale = rabitq_inv_sqrt(P);
+  const uint64_t cap = (uint64_t)device_sm_count() * 16;
+  auto blocks_of = [&](uint64_t rows) { return (unsigned)std::max<uint64_t>(1, std::min(cap, (n + rows - 1) / rows)); };
+  auto in_registers = [&](auto e) -> cudaError_t {
+    constexpr int E = decltype(e)::value;
+    constexpr size_t smem = rq_smem_bytes<E>();
+    const cudaError_t rc = cudaFuncSetAttribute(rabitq_encode_reg_kernel<E>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (rc != cudaSuccess) return rc;
+    rabitq_encode_reg_kernel<E><<<blocks_of(RQ_WARPS * rq_rows<E>()), RQ_WARPS * 32, smem, stream>>>(
+        x, n, dim, centroids, nlist, assign, signs, scale, rot_out, bits, meta);
+    return cudaSuccess;
+  };
+  cudaError_t e = cudaSuccess;
+  switch (P / 32) {
+    case 1: e = in_registers(std::integral_constant<int, 1>{}); break;
+    case 2: e = in_registers(std::integral_constant<int, 2>{}); break;
+    case 4: e = in_registers(std::integral_constant<int, 4>{}); break;
+    case 8: e = in_registers(std::integral_constant<int, 8>{}); break;
+    case 16: e = in_registers(std::integral_constant<int, 16>{}); break;
+    case 32: e = in_registers(std::integral_constant<int, 32>{}); break;
+    default: {
+      const size_t smem = (size_t)RQ_WARPS * P * 4;
+      e = cudaFuncSetAttribute(rabitq_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) break;
+      rabitq_encode_kernel<<<blocks_of(RQ_WARPS), RQ_WARPS * 32, smem, stream>>>(
+          x, n, dim, centroids, nlist, assign, signs, P, scale, rot_out, bits, meta);
+    }
+  }
+  if (e != cudaSuccess) return (int)e;
+  note_launch();
+  return (int)cudaGetLastError();
+}
+
+}  // namespace
+
 int launch_rabitq_encode(const float* x, uint32_t n, uint32_t dim, const float* centroids, uint32_t nlist,
                          const GpuSearchResult* assign, const float* signs, uint32_t padded_dim, float* rot_centroids,
                          uint32_t* bits, float* meta, cudaStream_t stream) {
   const uint32_t P = padded_dim;
   if (P < 32 || P > 4096 || (P & (P - 1)) || P < dim) return FV_ERR_ARG;
-  const size_t smem = (size_t)RQ_WARPS * P * 4;
-  cudaError_t e = cudaFuncSetAttribute(rabitq_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
-  const float scale = rabitq_inv_sqrt(P);
-  const uint32_t cap = (uint32_t)device_sm_count() * 16;
-  if (nlist) {
-    const uint32_t blocks = std::max(1u, std::min(cap, (nlist + RQ_WARPS - 1) / RQ_WARPS));
-    rabitq_encode_kernel<<<blocks, RQ_WARPS * 32, smem, stream>>>(centroids, nlist, dim, nullptr, 0, nullptr, signs, P,
-                                                                   scale, rot_centroids, nullptr, nullptr);
-    note_launch();
-  }
-  if (n) {
-    const uint32_t blocks = std::max(1u, std::min(cap, (n + RQ_WARPS - 1) / RQ_WARPS));
-    rabitq_encode_kernel<<<blocks, RQ_WARPS * 32, smem, stream>>>(x, n, dim, centroids, nlist, assign, signs, P, scale,
-                                                                   nullptr, bits, meta);
-    note_launch();
-  }
-  return (int)cudaGetLastError();
+  int rc = 0;
+  if (nlist)
+    rc = rabitq_encode_rows(centroids, nlist, dim, nullptr, 0, nullptr, signs, P, rot_centroids, nullptr, nullptr, stream);
+  if (!rc && n) rc = rabitq_encode_rows(x, n, dim, centroids, nlist, assign, signs, P, nullptr, bits, meta, stream);
+  return rc;
 }
 
 int launch_fill_f32(float* p, size_t n, float v, cudaStream_t stream) {

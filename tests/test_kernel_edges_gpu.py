@@ -204,3 +204,63 @@ def test_ivf_list_sequences(cuda, oracle_mod, mode, n, dim, nlist, m_pq, nprobe,
             assert np.array_equal(r[..., 0].view(np.uint32), ref["id"])
             assert np.array_equal(r[..., 1].view(np.uint32), ref["distance"].view(np.uint32))
     assert scan.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 65, 1000])
+@pytest.mark.parametrize("dim,pad,offset", [(1, 0, 0), (4, 0, 0), (13, 0, 0), (14, 16, 0), (96, 0, 0), (96, 0, 1),
+                                            (157, 0, 0), (260, 32, 0)])
+def test_encode_fp8_row_and_column_remainders(cuda, n, dim, pad, offset):
+    """Groups of eight rows, rows that end inside a word, a row's last digit at
+    its last column (13), wider padding, and rows off a 16-byte boundary
+    (offset floats): codes, digits and scales as from the definition, and the
+    norms to the last bit of a compensated sum (2^-23 of relative error)."""
+    from fvgb300 import scan
+
+    torch = cuda
+    rng = np.random.default_rng(n * 131 + dim)
+    x = (rng.standard_normal((n, dim)) * np.exp(rng.uniform(-3, 3, (n, 1)))).astype(np.float32)
+    x[n // 2] = 0.0
+    buf = torch.empty(n * dim + offset, device="cuda")
+    xd = buf[offset:].view(n, dim)
+    xd.copy_(torch.from_numpy(x))
+    pd = scan.fp8_padded_dim(dim) + pad
+    codes, scales, norms = scan.encode_fp8(xd, pd)
+    nrm = norms.cpu().numpy()
+    exact = (x.astype(np.float64) ** 2).sum(1)
+    # each square and the final sum rounded once
+    assert np.all(np.abs(nrm - exact) <= exact * 2.0 ** -23)
+    s = scales.cpu().numpy()
+    assert np.all(s == s[0])
+    b = int(np.log2(s[0]))
+    if nrm.max() > 0:
+        assert np.ldexp(np.float32(896.0), 2 * b - 2) < nrm.max() <= np.ldexp(np.float32(896.0), 2 * b)
+    to_e4m3 = lambda v: torch.from_numpy(np.ascontiguousarray(v, dtype=np.float32)).cuda().to(torch.float8_e4m3fn)
+    want = np.zeros((n, pd), dtype=np.uint8)
+    want[:, :dim] = to_e4m3(np.ldexp(x, -b)).view(torch.uint8).cpu().numpy()
+    r = np.ldexp(nrm, -1 - 2 * b).astype(np.float32)
+    for i in range(3):
+        c = to_e4m3(r)
+        want[:, dim + i] = c.view(torch.uint8).cpu().numpy()
+        r = (r - c.float().cpu().numpy()).astype(np.float32)
+    assert np.array_equal(codes.cpu().numpy().view(np.uint8), want)
+
+
+@pytest.mark.parametrize("n", [1, 3, 9, 500])
+@pytest.mark.parametrize("dim", [5, 32, 33, 64, 100, 129, 256, 500, 777, 1024, 1100])
+def test_rabitq_encoder_row_lengths(cuda, oracle_mod, n, dim):
+    """Every padded length held in registers, the first that is not, batches of
+    rows that are not full, and a residual of zero."""
+    from fvgb300.ivf import build_rabitq
+
+    torch = cuda
+    rng = np.random.default_rng(dim * 7 + n)
+    x = rng.standard_normal((n, dim)).astype(np.float32)
+    cent = rng.standard_normal((6, dim)).astype(np.float32)
+    x[0] = cent[2]  # a zero residual
+    assign = rng.integers(0, 6, n).astype(np.int32)
+    assign[0] = 2
+    ref = oracle_mod.rabitq_encode(x, cent, assign)
+    got = build_rabitq(torch.from_numpy(x).cuda(), torch.from_numpy(cent).cuda(), torch.from_numpy(assign).cuda())
+    torch.cuda.synchronize()
+    for key in ("rot_centroids", "rabitq_bits", "rabitq_meta"):
+        assert np.array_equal(got[key].cpu().numpy().view(np.uint32), ref[key].view(np.uint32)), key
