@@ -41,6 +41,8 @@
 // list needs in place, in the same operations. A running shortlist is kept in
 // shared memory: rows whose key cannot beat its worst key are dropped, the
 // rest are appended to a buffer; when it fills, the best of both are kept.
+#include <type_traits>
+
 #include <cuda_fp16.h>
 
 #include "../../include/fv_bridge.h"
@@ -202,6 +204,13 @@ __host__ __device__ __forceinline__ uint32_t ivf_clamps(uint32_t& top_k, uint32_
 
 constexpr uint32_t LIST_CHUNK = 32;
 
+// staging of SQ8 rows, see sq8_rows
+constexpr uint32_t SQ_STRIDE = 80;                  // bytes per row of a 64-dimension chunk: 16-byte steps off the same bank
+constexpr uint32_t SQ_WORDS = 32 / 4 + 1;           // words per row of a 32-dimension chunk that starts at any byte
+constexpr uint32_t SQ_BUF_BYTES = 64 * SQ_WORDS * 4;  // of two chunks of 32 dimensions each
+constexpr uint32_t SQ_WARP_BYTES = 64 * SQ_STRIDE;
+static_assert(2 * SQ_BUF_BYTES <= SQ_WARP_BYTES, "both forms in one area");
+
 struct IvfSmem {
   // [keys_pow2] u64 keys | table | query (dim f32) | PQ: query residual to the
   // probed centroid (dim f32) | the lists of a chunk: first posting, list,
@@ -222,7 +231,7 @@ struct IvfSmem {
   }
   // SQ8 with staged rows: the warps' staging areas follow, 16-byte aligned
   static size_t staged_bytes(uint32_t keys_pow2, uint32_t dim, uint32_t lc) {
-    return (bytes(IVF_SQ8, keys_pow2, dim, 0, 0, lc) + 15) / 16 * 16 + (size_t)(IVF_THREADS / 32) * (2 * 32 * 80);
+    return (bytes(IVF_SQ8, keys_pow2, dim, 0, 0, lc) + 15) / 16 * 16 + (size_t)(IVF_THREADS / 32) * SQ_WARP_BYTES;
   }
 };
 
@@ -466,119 +475,170 @@ __device__ __forceinline__ float sq8_row(const float* qs, const float* __restric
   return s;
 }
 
-// SQ8, staged: a warp scores 2 x 32 rows, each lane two of them, 64 dimensions
-// at a time. The rows' codes come in through shared memory by whole segments
-// (a lane reading its own row touches one line per 16 bytes: 32 L1 wavefronts
-// where the segment takes 8), and one read of the query, centroid and decoding
-// parameters serves both rows. RES: qs already holds the residual to the
-// centroid that all rows share. Rows may start at any byte: words are loaded
-// aligned and shifted into place. A byte becomes a float by taking the
+// SQ8, staged: a warp scores 2 x 32 rows, each lane two of them (one where no
+// lane has a second). The rows' codes come in through shared memory by whole
+// segments (a lane reading its own row touches one line per 16 bytes: 32 L1
+// wavefronts where the segment takes 8), and one read of the query, centroid
+// and decoding parameters serves both rows. RES: qs already holds the residual
+// to the centroid that all rows share. A byte becomes a float by taking the
 // mantissa's place in 2^23. row[i]: the lane's rows (null: none).
 // Warp-collective.
-constexpr uint32_t SQ_CHUNK = 64;   // dimensions per staged chunk
-constexpr uint32_t SQ_STRIDE = 80;  // bytes per staged row: 17 words, 16-byte steps off the same bank
-constexpr uint32_t SQ_WARP_BYTES = 2 * 32 * SQ_STRIDE;
-template <bool RES>
+//   PIPE: 32 dimensions at a time, the next ones copied while these are scored,
+// which is what a call of few warps waits for (8 queries x 64 lists of 768
+// dimensions 268 -> 232 us). Rows may start at any byte: words are copied
+// aligned and shifted into place (397 dimensions, 300 queries: 2,588 -> 2,239).
+//   Otherwise 16-byte-aligned rows, 64 dimensions at a time: fewer steps, for
+// calls whose warps cover each other's loads (2,000 queries, 128 dimensions:
+// 2,721 us, and 3,081 with PIPE).
+__device__ __forceinline__ void cp_async16(void* dst, uint64_t src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, uint64_t src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+template <bool RES, bool PIPE>
 __device__ __forceinline__ void sq8_rows(const float* qs, const float* const (&cent)[2], const float* mins,
                                          const float* scales, const uint8_t* const (&row)[2], uint32_t dim,
                                          bool aligned, bool cent16, uint8_t* stage, float (&out)[2]) {
   const uint32_t lane = threadIdx.x & 31u;
+  const int rows = __any_sync(0xffffffffu, row[1] != nullptr) ? 2 : 1;
+  constexpr uint32_t CHUNK = PIPE ? 32 : 64;
   out[0] = out[1] = 0.f;
-  for (uint32_t d0 = 0; d0 < dim; d0 += SQ_CHUNK) {
-    const uint32_t nd = min(SQ_CHUNK, dim - d0);
-    __syncwarp();  // the previous chunk is consumed
-    if (aligned) {
-      // four lanes a row, 16 bytes each
+  // dimensions [d0, d0 + CHUNK) of the rows into buffer buf
+  auto copy = [&](uint32_t d0, uint8_t* buf) {
+    const uint32_t nd = min(CHUNK, dim - d0);
+    for (int i = 0; i < rows; ++i) {
+      const uint64_t mine = (uint64_t)(uintptr_t)(i ? row[1] : row[0]);
+      if (aligned) {
+        // two lanes a row, 16 bytes each; a row's halves change places every
+        // four rows, which puts eight lanes' halves on different banks
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        uint4 w[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t r = 8 * j + (lane >> 2), c = (lane & 3u) * 16;
-          const uint64_t p = __shfl_sync(0xffffffffu, (uint64_t)(uintptr_t)row[i], r);
-          w[j] = p && c < nd ? __ldg(reinterpret_cast<const uint4*>(p + d0 + c)) : make_uint4(0u, 0u, 0u, 0u);
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t r = 16 * j + (lane >> 1), c = (lane & 1u) * 16;
+          const uint64_t p = __shfl_sync(0xffffffffu, mine, r);
+          if (p && c < nd) cp_async16(buf + (i * 32 + r) * 32 + (c ^ ((r & 4u) * 4)), p + d0 + c);
         }
+      } else {
+        // eight lanes a row, one aligned word each, and a ninth word where the
+        // row's chunk reaches into it
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t r = 8 * j + (lane >> 2), c = (lane & 3u) * 16;
-          *reinterpret_cast<uint4*>(stage + (i * 32 + r) * SQ_STRIDE + c) = w[j];
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t r = 4 * j + (lane >> 3), w = lane & 7u;
+          const uint64_t p = __shfl_sync(0xffffffffu, mine, r);
+          const uint64_t at = ((p + d0) & ~(uint64_t)3) + 4 * w;
+          if (p && at < p + d0 + nd) cp_async4(buf + ((i * 32 + r) * SQ_WORDS + w) * 4, at);
         }
-      }
-    } else {
-      // a half-warp a row, one aligned word each, and a 17th word where the
-      // row's chunk reaches into it
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-#pragma unroll 4
-        for (int j = 0; j < 16; ++j) {
-          const uint32_t r = 2 * j + (lane >> 4), c = (lane & 15u) * 4;
-          const uint64_t p = __shfl_sync(0xffffffffu, (uint64_t)(uintptr_t)row[i], r);
-          const uint64_t at = (p + d0) & ~(uint64_t)3, end = p + d0 + nd;
-          if (p && at + c < end)
-            *reinterpret_cast<uint32_t*>(stage + (i * 32 + r) * SQ_STRIDE + c) =
-                __ldg(reinterpret_cast<const uint32_t*>(at + c));
-        }
-        const uint64_t p = (uint64_t)(uintptr_t)row[i];
-        const uint64_t at = ((p + d0) & ~(uint64_t)3) + 64;
-        if (p && at < p + d0 + nd)
-          *reinterpret_cast<uint32_t*>(stage + (i * 32 + lane) * SQ_STRIDE + 64) =
-              __ldg(reinterpret_cast<const uint32_t*>(at));
+        const uint64_t at = ((mine + d0) & ~(uint64_t)3) + CHUNK;
+        if (mine && at < mine + d0 + nd) cp_async4(buf + ((i * 32 + lane) * SQ_WORDS + SQ_WORDS - 1) * 4, at);
       }
     }
+  };
+  auto copy64 = [&](uint32_t d0) {
+    const uint32_t nd = min(CHUNK, dim - d0);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (i == rows) break;
+      // four lanes a row, 16 bytes each
+      uint4 w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t r = 8 * j + (lane >> 2), c = (lane & 3u) * 16;
+        const uint64_t p = __shfl_sync(0xffffffffu, (uint64_t)(uintptr_t)row[i], r);
+        w[j] = p && c < nd ? __ldg(reinterpret_cast<const uint4*>(p + d0 + c)) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t r = 8 * j + (lane >> 2), c = (lane & 3u) * 16;
+        *reinterpret_cast<uint4*>(stage + (i * 32 + r) * SQ_STRIDE + c) = w[j];
+      }
+    }
+  };
+  __syncwarp();  // the buffers are free
+  if constexpr (PIPE) {
+    copy(0, stage);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  uint32_t which = 0;
+  for (uint32_t d0 = 0; d0 < dim; d0 += CHUNK, which ^= 1u) {
+    const uint32_t nd = min(CHUNK, dim - d0);
+    if constexpr (PIPE) {
+      if (d0 + CHUNK < dim) copy(d0 + CHUNK, stage + (which ^ 1u) * SQ_BUF_BYTES);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      copy64(d0);
+    }
     __syncwarp();
+    const uint8_t* buf = PIPE ? stage + which * SQ_BUF_BYTES : stage;
+    const uint32_t stride = !PIPE ? SQ_STRIDE : aligned ? 32u : SQ_WORDS * 4;
     const uint32_t sh0 = 8 * ((uint32_t)((uintptr_t)row[0] + d0) & 3u), sh1 = 8 * ((uint32_t)((uintptr_t)row[1] + d0) & 3u);
-    const uint8_t* st0 = stage + lane * SQ_STRIDE;
-    const uint8_t* st1 = st0 + 32 * SQ_STRIDE;
+    const uint8_t* st0 = buf + lane * stride;
+    const uint8_t* st1 = st0 + 32 * stride;
+    const uint32_t swap = PIPE ? (lane & 4u) * 4 : 0u;
     auto term = [&](float& s, uint32_t w, int b, float qd, float cd, float m, float k) {
       const float code = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + b)) - 8388608.0f;  // exact
       const float t = __fsub_rn(RES ? qd : __fsub_rn(qd, cd), fmaf(code, k, m));
       s = fmaf(t, t, s);
     };
-    if (aligned && cent16) {
-      for (uint32_t d = 0; d < nd; d += 16) {
-        const uint4 wa = *reinterpret_cast<const uint4*>(st0 + d), wb = *reinterpret_cast<const uint4*>(st1 + d);
-        const uint32_t a4[4] = {wa.x, wa.y, wa.z, wa.w}, b4[4] = {wb.x, wb.y, wb.z, wb.w};
+    auto score = [&](auto two) {
+      constexpr bool TWO = decltype(two)::value;
+      if ((!PIPE || aligned) && cent16) {
+        for (uint32_t d = 0; d < nd; d += 16) {
+          const uint4 wa = *reinterpret_cast<const uint4*>(st0 + (d ^ swap));
+          const uint4 wb = TWO ? *reinterpret_cast<const uint4*>(st1 + (d ^ swap)) : wa;
+          const uint32_t a4[4] = {wa.x, wa.y, wa.z, wa.w}, b4[4] = {wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t at = d0 + d + 4 * j;
-          const float4 q = *reinterpret_cast<const float4*>(qs + at);
-          const float4 mn = *reinterpret_cast<const float4*>(mins + at);
-          const float4 sc = *reinterpret_cast<const float4*>(scales + at);
-          float4 ca = q, cb = q;
-          if (!RES) {
-            ca = __ldg(reinterpret_cast<const float4*>(cent[0] + at));
-            cb = cent[1] == cent[0] ? ca : __ldg(reinterpret_cast<const float4*>(cent[1] + at));
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t at = d0 + d + 4 * j;
+            const float4 q = *reinterpret_cast<const float4*>(qs + at);
+            const float4 mn = *reinterpret_cast<const float4*>(mins + at);
+            const float4 sc = *reinterpret_cast<const float4*>(scales + at);
+            float4 ca = q, cb = q;
+            if (!RES) {
+              ca = __ldg(reinterpret_cast<const float4*>(cent[0] + at));
+              if (TWO) cb = cent[1] == cent[0] ? ca : __ldg(reinterpret_cast<const float4*>(cent[1] + at));
+            }
+            term(out[0], a4[j], 0, q.x, ca.x, mn.x, sc.x);
+            if (TWO) term(out[1], b4[j], 0, q.x, cb.x, mn.x, sc.x);
+            term(out[0], a4[j], 1, q.y, ca.y, mn.y, sc.y);
+            if (TWO) term(out[1], b4[j], 1, q.y, cb.y, mn.y, sc.y);
+            term(out[0], a4[j], 2, q.z, ca.z, mn.z, sc.z);
+            if (TWO) term(out[1], b4[j], 2, q.z, cb.z, mn.z, sc.z);
+            term(out[0], a4[j], 3, q.w, ca.w, mn.w, sc.w);
+            if (TWO) term(out[1], b4[j], 3, q.w, cb.w, mn.w, sc.w);
           }
-          term(out[0], a4[j], 0, q.x, ca.x, mn.x, sc.x);
-          term(out[1], b4[j], 0, q.x, cb.x, mn.x, sc.x);
-          term(out[0], a4[j], 1, q.y, ca.y, mn.y, sc.y);
-          term(out[1], b4[j], 1, q.y, cb.y, mn.y, sc.y);
-          term(out[0], a4[j], 2, q.z, ca.z, mn.z, sc.z);
-          term(out[1], b4[j], 2, q.z, cb.z, mn.z, sc.z);
-          term(out[0], a4[j], 3, q.w, ca.w, mn.w, sc.w);
-          term(out[1], b4[j], 3, q.w, cb.w, mn.w, sc.w);
+        }
+      } else {
+        for (uint32_t d = 0; d < nd; d += 4) {
+          // (aligned rows, whose halves may have changed places: shifted by 0)
+          const uint32_t at4 = !PIPE || aligned ? d ^ swap : d;
+          const uint32_t* pa = reinterpret_cast<const uint32_t*>(st0 + at4);
+          const uint32_t* pb = reinterpret_cast<const uint32_t*>(st1 + at4);
+          const uint32_t wa = __funnelshift_r(pa[0], pa[1], sh0);
+          const uint32_t wb = TWO ? __funnelshift_r(pb[0], pb[1], sh1) : 0u;
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const uint32_t at = d0 + d + b;
+            if (at >= dim) break;
+            const float q = qs[at], mn = mins[at], sc = scales[at];
+            float ca = q, cb = q;
+            if (!RES) {
+              ca = __ldg(cent[0] + at);
+              if (TWO) cb = cent[1] == cent[0] ? ca : __ldg(cent[1] + at);
+            }
+            term(out[0], wa, b, q, ca, mn, sc);
+            if (TWO) term(out[1], wb, b, q, cb, mn, sc);
+          }
         }
       }
-    } else {
-      for (uint32_t d = 0; d < nd; d += 4) {
-        const uint32_t* pa = reinterpret_cast<const uint32_t*>(st0 + d);
-        const uint32_t* pb = reinterpret_cast<const uint32_t*>(st1 + d);
-        const uint32_t wa = __funnelshift_r(pa[0], pa[1], sh0), wb = __funnelshift_r(pb[0], pb[1], sh1);
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const uint32_t at = d0 + d + b;
-          if (at >= dim) break;
-          const float q = qs[at], mn = mins[at], sc = scales[at];
-          float ca = q, cb = q;
-          if (!RES) {
-            ca = __ldg(cent[0] + at);
-            cb = cent[1] == cent[0] ? ca : __ldg(cent[1] + at);
-          }
-          term(out[0], wa, b, q, ca, mn, sc);
-          term(out[1], wb, b, q, cb, mn, sc);
-        }
-      }
-    }
+    };
+    if (rows == 2)
+      score(std::true_type{});
+    else
+      score(std::false_type{});
+    __syncwarp();  // this buffer is consumed
   }
 }
 
@@ -596,12 +656,13 @@ constexpr uint32_t LIST_ALONE_MIN = 1024;
 // load-latency bound, so occupancy is worth more than registers.
 template <int MODE, int MW>
 constexpr int ivf_min_blocks() {
-  return MODE == IVF_PQ ? (MW == 4 ? 2 : 3) : MODE == IVF_RABITQ && MW >= 4 ? 3 : 4;
+  return MODE == IVF_PQ ? (MW == 4 ? 2 : 3) : MODE == IVF_SQ8 || (MODE == IVF_RABITQ && MW >= 4) ? 3 : 4;
 }
 
 // MODE: PQ, SQ8 or RaBitQ. MW > 0: code rows of 16 * MW bytes at 16-byte-
 // aligned rows (PQ m_pq = 16, 32, 64; RaBitQ P = 128 MW with 16-byte-aligned
-// meta rows; SQ8 with staged rows, MW = 1, R = 2), R postings per thread per
+// meta rows; SQ8 with staged rows, R = 2: MW = 1 the rows in turn, MW = 2 the next
+// ones copied meanwhile), R postings per thread per
 // round, all their loads before any is scored.
 template <int MODE, int MW, int R>
 __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_scan_kernel(IvfArgs a) {
@@ -634,7 +695,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
   const bool vec16 = (a.code_bytes % 16u) == 0 && ((uintptr_t)a.codes % 16u) == 0;
   const bool cent16 = a.dim % 4 == 0 && ((uintptr_t)a.centroids % 16u) == 0;
   uint8_t* stage = smem + ((reinterpret_cast<uint8_t*>(s_cum + a.list_chunk + 1) - smem) + 15) / 16 * 16 +
-                   warp * SQ_WARP_BYTES;  // SQ8, MW = 1
+                   warp * SQ_WARP_BYTES;  // SQ8, MW > 0
 
   if (MODE == IVF_SQ8) {
     for (uint32_t d = tid; d < a.dim; d += IVF_THREADS) {
@@ -910,7 +971,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
                 rows[r] = post[r].ok ? a.codes + (size_t)(a.list_major ? post[r].pos : post[r].id) * a.code_bytes : nullptr;
               const float* const none[2] = {nullptr, nullptr};
               if (__any_sync(0xffffffffu, post[0].ok || post[1].ok))
-                sq8_rows<true>(tab + 2 * a.dim, none, mins, scales, rows, a.dim, vec16, a.dim % 4 == 0, stage, sq);
+                sq8_rows<true, MW == 2>(tab + 2 * a.dim, none, mins, scales, rows, a.dim, vec16, a.dim % 4 == 0, stage, sq);
             }
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -987,7 +1048,7 @@ __global__ void __launch_bounds__(IVF_THREADS, ivf_min_blocks<MODE, MW>()) ivf_s
             cents[r] = a.centroids + (post[r].ok ? (size_t)(s_list[lp[r]] & 0x7FFFFFFFu) * a.dim : 0);
           }
           if (__any_sync(0xffffffffu, post[0].ok || post[1].ok))
-            sq8_rows<false>(qs, cents, mins, scales, rows, a.dim, vec16, cent16, stage, sq);
+            sq8_rows<false, MW == 2>(qs, cents, mins, scales, rows, a.dim, vec16, cent16, stage, sq);
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -1747,7 +1808,12 @@ int launch_ivf_search(int mode, const IvfLaunch& L, cudaStream_t stream) {
     smem = keep_at + sizeof(KeepScratch);
   }
   const bool rows16 = mode == IVF_PQ && ((uintptr_t)L.codes % 16u) == 0;
-  auto kern = stage_rows ? ivf_scan_kernel<IVF_SQ8, 1, 2> : ivf_scan_kernel<IVF_SQ8, 0, 1>;
+  // SQ8: rows copied ahead where they may start at any byte, or where all
+  // ranges run at once and their warps are too few to cover the loads
+  const bool sq_rows16 = a.code_bytes % 16 == 0 && (uintptr_t)L.codes % 16 == 0;
+  auto kern = !stage_rows                                          ? ivf_scan_kernel<IVF_SQ8, 0, 1>
+              : sq_rows16 && (uint64_t)L.nq * G > 3ull * sms ? ivf_scan_kernel<IVF_SQ8, 1, 2>
+                                                             : ivf_scan_kernel<IVF_SQ8, 2, 2>;
   if (mode == IVF_RABITQ) {
     // bits rows of P/8 bytes as 16-byte words when they and the meta rows
     // are 16-byte aligned; R postings per thread per round as registers allow

@@ -264,3 +264,29 @@ def test_rabitq_encoder_row_lengths(cuda, oracle_mod, n, dim):
     torch.cuda.synchronize()
     for key in ("rot_centroids", "rabitq_bits", "rabitq_meta"):
         assert np.array_equal(got[key].cpu().numpy().view(np.uint32), ref[key].view(np.uint32)), key
+
+
+@pytest.mark.parametrize("dim,offset", [(16, 0), (48, 0), (64, 0), (100, 0), (37, 0), (128, 4), (130, 0)])
+@pytest.mark.parametrize("nq,nlist", [(3, 11), (520, 40)])
+def test_ivf_sq8_row_staging(cuda, oracle_mod, dim, offset, nq, nlist):
+    """Rows copied ahead (few queries, or rows off a 16-byte boundary by their
+    length or the table's start) and rows staged in turn: last chunks of every
+    width, lists shorter than a warp, lanes without a second row."""
+    from fvgb300.ivf import IvfTable
+
+    torch = cuda
+    x, q, t = _ivf_case(oracle_mod, 2200, dim, nlist, max(d for d in (1, 2, 4) if dim % d == 0), dim + nq, 1.0)
+    q = np.resize(q, (nq, dim)).astype(np.float32)
+    ref = oracle_mod.ivf_sq_search(t, x, q, 10, 9, 40)
+    for list_major in (False, True):
+        table = IvfTable("sq8", t, vectors=x, list_major=list_major)
+        if offset:
+            name = "codes_lm" if list_major else "codes"
+            codes = getattr(table, name)
+            buf = torch.empty(codes.numel() + offset, dtype=torch.uint8, device="cuda")
+            buf[offset:].copy_(codes.reshape(-1).view(torch.uint8))
+            setattr(table, name, buf[offset:].view(codes.shape))
+            table._build_structs()
+        r = table.search(torch.from_numpy(q).cuda(), 10, 9, 40).cpu().numpy()
+        assert np.array_equal(r[..., 0].view(np.uint32), ref["id"])
+        assert np.array_equal(r[..., 1].view(np.uint32), ref["distance"].view(np.uint32))
