@@ -777,6 +777,16 @@ def run_workload(a, world, rank, local):
                 "note": "the exact form spends 3 FP32 ops (sub, mul, add) per element for bit-identical sums",
                 # 3 separately rounded ops per 2 algorithmic flops: the issue bound is a third of the FMA rate
                 "issue_bound": fp32_peak / 3.0, "issue_bound_frac": flops / (kms / 1e3) / 1e12 / (fp32_peak / 3.0)}
+        if "flat_tc_prep" in prof:
+            # batches of this size choose the rows worth an exact distance with
+            # a tensor-core pass (the plain scan only answers flagged queries):
+            # the call as a whole against the tensor rate
+            kms = sum(v["ms"] for v in prof.values()) / a.steps
+            roof = {"bound": "tensor", "achieved": flops / (kms / 1e3) / 1e12, "peak": peaks["bf16_tflops"],
+                    "unit": "TFLOP/s", "frac": flops / (kms / 1e3) / 1e12 / peaks["bf16_tflops"], "traffic": None,
+                    "kernel": "all kernels of one call", "kernel_ms": kms,
+                    "peak_source": f"{peak_kind} bf16 burst rate",
+                    "note": "short rows: the filter pass is bound by its epilogue, not by the MMA"}
         cpu = None
         if not a.no_cpu_baseline:
             sys.path.insert(0, str(ROOT / "oracle"))

@@ -18,10 +18,12 @@
 //   warps 2.. epilogue, 4 warps per group: thread r of a group owns query r
 //             of the block (TMEM lane r),
 //             turns dot products into distances, applies the slot mask and
-//             keeps that query's best KL (distance, slot) keys in a shared-
-//             memory max-heap. No distance matrix ever reaches HBM.
-// A CTA scans a contiguous range of base tiles; the per-(query, range)
-// heaps are merged by tc_select_kernel, which also rescores them in fp32.
+//             keeps that query's best (distance, slot) keys. No distance
+//             matrix ever reaches HBM.
+// A call first finds a bound per query from column minima (of a sample of the
+// base, or of all of it) and then scans with it: a range's few keys under the
+// bound are appended to its list. A CTA scans a contiguous range of base tiles;
+// the lists are merged by tc_select_kernel, which also rescores them in fp32.
 #include <cmath>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>

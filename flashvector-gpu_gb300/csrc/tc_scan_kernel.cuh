@@ -12,10 +12,11 @@
 //   warps 2.. epilogue, 4 warps per group: thread r of a group owns query r
 //             of the block (TMEM lane r),
 //             turns dot products into distances, applies the slot mask and
-//             keeps that query's best kl (distance, slot) keys in a shared-
-//             memory max-heap. No distance matrix ever reaches HBM.
+//             keeps that query's best kl (distance, slot) keys: appended to a
+//             list where an admission bound is known, else in a shared-memory
+//             max-heap. No distance matrix ever reaches HBM.
 //
-// Shared bound. Every query owns kl global "slots"; a CTA that keeps a key
+// Shared bound (scans without an admission bound). Every query owns kl global "slots"; a CTA that keeps a key
 // also lowers slot hash(row) of its query to the key's distance (red.min).
 // Each slot then holds a distance of a distinct real row, so the maximum
 // over the kl slots is >= the query's global kl-th best distance: a row

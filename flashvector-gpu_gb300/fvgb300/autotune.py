@@ -5,7 +5,8 @@ them for calls of a matching shape.
 
 For each benchmark shape it sweeps
   * tc.pair          one-SM CTAs or cta_group::2 pairs (long rows only),
-  * tc.prepass       sampled pre-pass bound on / off, and its stride,
+  * tc.prepass       bound from a pass over (a sample of) the base on / off,
+                     and its stride,
   * over-fetch       the fp32-rescored shortlist = over-fetch x k,
 times each configuration (CUDA events around the whole search call, median
 of several runs, after warm-up) and measures recall@10 and recall@k against
@@ -17,7 +18,6 @@ this), the over-fetch can.
 For each IVF benchmark shape (the 10M-row IVF-PQ / IVF-RaBitQ list scans over
 Zipf-skewed lists at nprobe 8 / 32 / 128, the serving configuration's
 IVF-SQ8 at nprobe 16 / 64) it sweeps
-  * ivf.pipeline     the PQ list scan's plain or software-pipelined loop,
   * ivf.split        the work items of the persistent list scan: each
                      query's probed postings as one item (0), cut into 2 or
                      4 equal (query, posting-range) items merged per query
@@ -133,7 +133,7 @@ def tune_ivf_shape(name, spec, runs=3, nsub=100, log=print):
                   C.c_void_p(out.data_ptr()), C.c_void_p(stream.cuda_stream))
 
     results, answer = [], None
-    for pipeline in ((0, 1) if mode == "pq" else (0,)):
+    for pipeline in (0,):  # ivf.pipeline has no effect (one loop)
         for split in (-1, 0, 2, 4):
             for tcc in (0, 1):
                 with scan.tuned(tc_table=0, ivf_pipeline=pipeline, ivf_split=split, ivf_tc_coarse=tcc):

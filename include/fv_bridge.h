@@ -346,8 +346,8 @@ int fv_profile_summary(char* buf, size_t len);
  *   "tc.groups"         -1 (default): fp8 scans of a table-scale table (L2,
  *                       inner product) with one K block per tile and a
  *                       shortlist above 48 keys drain each tile with four
- *                       epilogue groups (16 warps, heaps of <= 32 keys),
- *                       other short-row scans with two (heaps of <= 48);
+ *                       epilogue groups (16 warps, ranges of <= 32 keys),
+ *                       other short-row scans with two (of <= 48);
  *                       2 or 4: that many wherever the four-group form
  *                       applies. Same answers
  *   "flat.tc"           -1 (default): large exact scans find the rows worth
