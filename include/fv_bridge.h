@@ -335,7 +335,9 @@ int fv_profile_summary(char* buf, size_t len);
  *                       base (all of it where it is small); bases too small
  *                       to bound are scanned without
  *   "tc.prepass_stride" sample stride in 256-row tiles (0 automatic: the
- *                       tuned value, else 1 to 32 growing with the base)
+ *                       tuned value, else 1 to 32 growing with the base);
+ *                       raised where the sample's minima would not fit the
+ *                       scan's scratch
  *   "tc.prepass_margin" 0 (default): the sampled rank r is the smallest
  *                       with P(Poisson(shortlist / stride) >= r) < 1e-7;
  *                       m > 0: r = ceil(m * shortlist / stride)

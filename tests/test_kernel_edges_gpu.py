@@ -290,3 +290,23 @@ def test_ivf_sq8_row_staging(cuda, oracle_mod, dim, offset, nq, nlist):
         r = table.search(torch.from_numpy(q).cuda(), 10, 9, 40).cpu().numpy()
         assert np.array_equal(r[..., 0].view(np.uint32), ref["id"])
         assert np.array_equal(r[..., 1].view(np.uint32), ref["distance"].view(np.uint32))
+
+
+@pytest.mark.parametrize("stride", [2, 3, 16])
+def test_sample_stride_that_does_not_fit(cuda, stride):
+    """A stride whose minima would not fit the scan's scratch (many queries, few
+    ranges) is raised until they do; the answer stays the unbounded scan's."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(stride)
+    x = torch.randn((300_000, 32), generator=g, device="cuda")
+    q = torch.randn((2500, 32), generator=g, device="cuda")
+    t = scan.Fp16Table(x)
+    with scan.tuned(tc_prepass=0):
+        ref = scan.fp16_search(t, q, 5, "l2")
+    with scan.tuned(tc_prepass_stride=stride):
+        got = scan.fp16_search(t, q, 5, "l2")
+    torch.cuda.synchronize()
+    assert scan.device_status() == 0
+    assert torch.equal(got, ref)
