@@ -476,7 +476,12 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     uint32_t* cm = colmask + (warp - 2) * 8;
     // this group's columns [c_lo, c_hi) of each tile; only its own columns'
     // data is staged
-    const int c_lo = col_split ? grp * (TC_N / G) : 0, c_hi = col_split ? c_lo + TC_N / G : TC_N;
+    // (per-row scales: c_hi is no constant step from c_lo for the compiler, which
+    // otherwise schedules the two steps of the column loop worse: 4M x 96,
+    // 4,000 queries, L2: 7.42 ms, 6.59 like this)
+    const int c_lo = col_split ? grp * (TC_N / G) : 0;
+    const bool whole = FP8 && !TS && a.tile_stride > 1u << 30;  // (never)
+    const int c_hi = col_split && !whole ? c_lo + TC_N / G : TC_N;
     float pre_n[TC_N / 32], pre_s[TC_N / 32];
     uint32_t pre_m = 0;
     auto prefetch = [&](uint32_t tile) {
