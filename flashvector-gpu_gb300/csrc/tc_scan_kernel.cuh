@@ -720,29 +720,33 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
                 m[b] = best3(best3(w[0], w[1], w[2]), best3(w[3], w[4], w[5]), better(w[6], w[7]));
               }
               if (!qvalid) return;
+              // The minimum of columns that are all NaN (an fp16 row that overflowed
+              // times a zero, a NaN row) is NaN, whose D would be L2's floor: such
+              // columns hold no distance.
+              auto M = [&](float x) { return x == x ? D(x) : INFINITY; };
               float* dst = a.pmin + (size_t)q * a.pm_stride;
               const uint32_t at = (t_begin + i) * TC_N + (uint32_t)c0;  // scanned column
               if (a.gran == 8) {
                 float4* o = reinterpret_cast<float4*>(dst + at / 8);
-                o[0] = make_float4(D(m[0]), D(m[1]), D(m[2]), D(m[3]));
-                o[1] = make_float4(D(m[4]), D(m[5]), D(m[6]), D(m[7]));
+                o[0] = make_float4(M(m[0]), M(m[1]), M(m[2]), M(m[3]));
+                o[1] = make_float4(M(m[4]), M(m[5]), M(m[6]), M(m[7]));
                 return;
               }
               const float p0 = better(m[0], m[1]), p1 = better(m[2], m[3]), p2 = better(m[4], m[5]),
                           p3 = better(m[6], m[7]);
               if (a.gran == 16) {
-                *reinterpret_cast<float4*>(dst + at / 16) = make_float4(D(p0), D(p1), D(p2), D(p3));
+                *reinterpret_cast<float4*>(dst + at / 16) = make_float4(M(p0), M(p1), M(p2), M(p3));
                 return;
               }
               const float h0 = better(p0, p1), h1 = better(p2, p3), all = better(h0, h1);
               if (a.gran == 32) {
-                *reinterpret_cast<float2*>(dst + at / 32) = make_float2(D(h0), D(h1));
+                *reinterpret_cast<float2*>(dst + at / 32) = make_float2(M(h0), M(h1));
               } else if (a.gran == 64) {
-                dst[at / 64] = D(all);
+                dst[at / 64] = M(all);
               } else if ((c0 & 64) == 0) {
                 best128 = all;
               } else {
-                dst[at / 128] = D(better(best128, all));
+                dst[at / 128] = M(better(best128, all));
               }
               return;
             } else {

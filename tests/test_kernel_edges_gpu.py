@@ -310,3 +310,34 @@ def test_sample_stride_that_does_not_fit(cuda, stride):
     torch.cuda.synchronize()
     assert scan.device_status() == 0
     assert torch.equal(got, ref)
+
+
+def _fp_table(scan, precision, x):
+    return scan.Fp16Table(x) if precision == "fp16" else scan.Fp8Table(x, per_vector=precision == "fp8_rows")
+
+
+@pytest.mark.parametrize("precision,broken", [("fp16", "nan"), ("fp16", "overflow"), ("fp8", "nan"), ("fp8_rows", "nan")])
+@pytest.mark.parametrize("k", [1, 10])
+def test_bound_ignores_columns_without_a_distance(cuda, precision, broken, k):
+    """Whole groups of columns whose distance is NaN (NaN rows; finite rows
+    beyond fp16's range against queries with zeros) are no rows near the query:
+    the bounded scan still returns what the scan without a bound returns."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn((10_000, 128), generator=g, device="cuda")
+    q = torch.randn((70, 128), generator=g, device="cuda")
+    if broken == "nan":
+        x[1024:4096] = float("nan")
+    else:
+        x[1024:4096] = 1e6
+        q[:, ::3] = 0.0
+    t = _fp_table(scan, precision, x)
+    search = scan.fp16_search if precision == "fp16" else scan.fp8_search
+    with scan.tuned(tc_prepass=0):
+        ref = search(t, q, k, "l2")
+    got = search(t, q, k, "l2")
+    torch.cuda.synchronize()
+    assert (ref[..., 0] != -1).all()
+    assert torch.equal(got, ref)
