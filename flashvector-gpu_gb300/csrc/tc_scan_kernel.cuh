@@ -448,7 +448,8 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     // columns, v = -dot / |x| from a factor staged per column ranks within
     // kCosPad of the distance 1 + v / |q| (the factors' few ulps, and 1e-8
     // against 0.01), so v <= cthr, raised by it, admits every candidate and
-    // the exact distance is evaluated for those alone.
+    // the exact distance is evaluated for those alone. Nor does |q|^2 |x|^2
+    // overflow for any of them: the distance would then be 1 at every angle.
     constexpr float kCosPad = 4e-6f;
     const float q_over = METRIC == METRIC_COSINE ? sqrtf(qn) / (FP8 ? qs : 1.f) : 1.f;
     const float q_inv = METRIC == METRIC_COSINE ? __fdiv_rn(1.f, q_over) : 1.f;
@@ -511,7 +512,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
       const uint32_t buf = i & 1, use = i >> 1;
       const uint32_t v0 = (t_begin + i) * tstride * TC_N;
       __syncwarp();
-      [[maybe_unused]] float least = INFINITY;  // cosine: the smallest norm of the tile's rows
+      [[maybe_unused]] float least = INFINITY, most = 0.f;  // cosine: the squared norms of the tile's rows
 #pragma unroll
       for (int r = 0; r < TC_N / 32; ++r) {
         if (32 * r < c_lo || 32 * r >= c_hi) continue;
@@ -519,14 +520,20 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
         if (FP8 && !fused) cb[TC_N + lane + 32 * r] = pre_s[r];
         if (METRIC == METRIC_COSINE) {
           cf[lane + 32 * r] = -rsqrtf(pre_n[r]) * (FP8 ? pre_s[r] : 1.f);
-          if (v0 + lane + 32 * r < a.n) least = fminf(least, pre_n[r]);
+          if (v0 + lane + 32 * r < a.n) {
+            least = fminf(least, pre_n[r]);
+            most = fmaxf(most, pre_n[r]);
+          }
         }
       }
       [[maybe_unused]] bool by_factor = false;
       if (METRIC == METRIC_COSINE) {
 #pragma unroll
-        for (int o = 16; o; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
-        by_factor = __all_sync(0xffffffffu, !qvalid || (qn * least >= 1e-4f && qn < 1e30f));
+        for (int o = 16; o; o >>= 1) {
+          least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+          most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+        }
+        by_factor = __all_sync(0xffffffffu, !qvalid || (qn * least >= 1e-4f && qn * most < 1e38f));
       }
       if (lane < 8) cm[lane] = pre_m;
       __syncwarp();

@@ -341,3 +341,27 @@ def test_bound_ignores_columns_without_a_distance(cuda, precision, broken, k):
     torch.cuda.synchronize()
     assert (ref[..., 0] != -1).all()
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("precision", ["fp8", "fp8_rows"])
+@pytest.mark.parametrize("rows", ["all", "some"])
+def test_cosine_bound_with_norms_that_overflow(cuda, precision, rows):
+    """Cosine rows and queries whose product of squared norms overflows fp32
+    have the distance 1, whatever their angle: the bounded scan ranks them so too."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn((10_000, 64), generator=g, device="cuda")
+    q = torch.randn((70, 64), generator=g, device="cuda") * 1e10
+    if rows == "all":
+        x *= 1e10
+    else:
+        x[1000:3000] *= 1e10
+    t = _fp_table(scan, precision, x)
+    with scan.tuned(tc_prepass=0):
+        ref = scan.fp8_search(t, q, 10, "cosine")
+    got = scan.fp8_search(t, q, 10, "cosine")
+    torch.cuda.synchronize()
+    assert (ref[..., 0] != -1).all()
+    assert torch.equal(got, ref)
