@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(TAU_THREADS) tc_tau_kernel(const float* __rest
   if (tid == 0) {
     const float t = order_float(ans);
     const float up = m.rel * fabsf(t) + m.abs + (m.qnorm ? m.per_norm * fabsf(m.qnorm[q]) : 0.f);
-    tau[q] = t < kSentinelDist ? t + up : kSentinelDist;
+    tau[q] = t < kSentinelDist ? (t > -INFINITY ? t + up : t) : kSentinelDist;  // (-inf + inf is NaN)
     redo[q] = 0u;
   }
 }

@@ -453,12 +453,15 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     constexpr float kCosPad = 4e-6f;
     const float q_over = METRIC == METRIC_COSINE ? sqrtf(qn) / (FP8 ? qs : 1.f) : 1.f;
     const float q_inv = METRIC == METRIC_COSINE ? __fdiv_rn(1.f, q_over) : 1.f;
+    // (A bound of -inf, where products overflowed, admits the rows at -inf: the
+    // thresholds stay finite, or their slack would make them NaN.)
+    constexpr float kLowest = -3.402823466e38f;
     float thr = 0.f, cthr = 0.f;
     auto refresh = [&]() {
-      const float w = fminf(worst, bound);
+      const float w = fmaxf(fminf(worst, bound), kLowest);
       thr = METRIC == METRIC_L2 ? (w - qn) + 1e-6f * (fabsf(w) + fabsf(qn)) + 1e-30f : w;
       if (METRIC == METRIC_COSINE) {
-        cthr = (w - 1.0f + kCosPad) * q_over;
+        cthr = fmaxf((w - 1.0f + kCosPad) * q_over, kLowest);
         cthr += 1e-6f * fabsf(cthr);
       }
       if (fused) {

@@ -365,3 +365,25 @@ def test_cosine_bound_with_norms_that_overflow(cuda, precision, rows):
     torch.cuda.synchronize()
     assert (ref[..., 0] != -1).all()
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("metric", ["ip", "cosine", "l2"])
+@pytest.mark.parametrize("k", [1, 10, 100])
+def test_bound_of_products_that_overflow(cuda, metric, k):
+    """One coordinate beyond fp16's range makes a product infinite, and the row
+    nearer than any other: a bound that is itself infinite admits those rows."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn((20_000, 96), generator=g, device="cuda")
+    q = torch.randn((70, 96), generator=g, device="cuda")
+    x[::5, 3] = 1e6
+    q[::2, 3] = q[::2, 3].abs() + 0.1
+    t = scan.Fp16Table(x)
+    with scan.tuned(tc_prepass=0):
+        ref = scan.fp16_search(t, q, k, metric)
+    scan.device_status()
+    got = scan.fp16_search(t, q, k, metric)
+    torch.cuda.synchronize()
+    assert torch.equal(got, ref)
