@@ -25,7 +25,8 @@
 //     the largest key of any list that filled up), hence A >= B: when the
 //     k-th exact distance among the collected rows is below B the collected
 //     rows hold the answer. A query that fails this test, or whose values
-//     leave fp16's range, is flagged, and the plain scan answers it.
+//     leave fp16's range, is flagged, and the plain scan answers it; so are
+//     all of a call one of whose passes gave up a wait.
 //
 // Measured: 100,000 x 128 x 1,000, k 10: 1,592 -> 160 us (encoding 37, minima
 // pass 37, scan 50, finish 15); 200,000 x 512 x 100: 1,131 -> 263 us. Bounded
@@ -54,7 +55,7 @@ constexpr float kMaxNorm = 3.0e4f;   // of a scaled row or query: no fp16 value 
 constexpr float kUnit = 256.f;       // norm of a scaled unit vector (cosine)
 
 // words of the call's shared state
-enum { W_MAX_NORM = 0, W_MIN_NORM = 1, W_COUNT = 2 };
+enum { W_MAX_NORM = 0, W_MIN_NORM = 1, W_STATUS = 2, W_COUNT = 3 };  // W_STATUS: status bits of the scans
 
 struct QueryInfo {
   float to_a;    // A = to_a * distance (cosine: to_a * (distance - 1))
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(32 * CEN_GROUPS) flat_tc_center_kernel(const f
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     words[W_MAX_NORM] = 0u;
     words[W_MIN_NORM] = 0x7f800000u;  // +inf
+    words[W_STATUS] = 0u;
   }
   auto total = [&](float v) {  // over the row groups, to every thread of the dimension
     part[g][lane] = v;
@@ -395,7 +397,8 @@ __global__ void __launch_bounds__(FIN_THREADS) flat_tc_finish_kernel(FinishArgs 
   if (tid == 0) {
     const QueryInfo inf = a.info[q];
     const float low = order_float(s_low);
-    bool ok = __uint_as_float(a.words[W_MAX_NORM]) < kMaxNorm && inf.scaled < kMaxNorm;
+    // (a pass that gave up a wait has not seen every row)
+    bool ok = a.words[W_STATUS] == 0u && __uint_as_float(a.words[W_MAX_NORM]) < kMaxNorm && inf.scaled < kMaxNorm;
     if (METRIC == METRIC_COSINE) ok = ok && inf.norm * __uint_as_float(a.words[W_MIN_NORM]) > 8.2e-5f;
     if (ok && low < kSentinelDist) {  // else every admissible row was collected
       const uint64_t kth = keys[a.k - 1];
@@ -552,6 +555,7 @@ int launch_flat_tc(const float* vectors, const uint32_t* vec_ids, uint32_t n, ui
   c.q16 = p.q16;
   c.qnorm = p.qnorm;
   c.mask = mask;
+  c.status = words + W_STATUS;
   int rc = launch_tc_collect(c, base + P.collect, stream);
   if (rc) return rc;
   const float slack = metric == METRIC_L2 ? (float)std::ldexp((double)dim + 2, -23) : 1e-6f;

@@ -146,6 +146,7 @@ struct TcCollect {
   const float* qnorm;      // [nq]
   float floor, margin_rel, margin_norm, margin_abs;
   const uint32_t* mask;
+  uint32_t* status;        // gets the passes' status bits (zeroed by the caller): the lists are then not complete
   // set by launch_tc_collect, inside its scratch
   uint64_t* partial;       // [nq][lists][kl]
   uint32_t lists, kl;

@@ -854,7 +854,7 @@ int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream) {
   a.qnorm = c.qnorm;
   a.mask = c.mask;
   a.floor = c.floor;
-  a.status = status_word();
+  a.status = c.status;
   const int64_t wl = tune_value("tc.wait_limit_ns", 0);
   a.wait_ns = wl > 0 ? (uint64_t)wl : 2000000000ull;
   auto scan = [&](const TcScanArgs& args, int kl_t, uint32_t splits_n, const char* name) -> cudaError_t {

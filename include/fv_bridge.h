@@ -361,7 +361,9 @@ int fv_profile_summary(char* buf, size_t len);
  *                       out ends the scan early (its answer is not valid)
  *                       and sets the timeout bit that fv_read_device_status
  *                       reports; the context stays usable (a short limit
- *                       exercises that path)
+ *                       exercises that path). An exact scan's tensor-core
+ *                       pass that ends so is answered by the plain scan and
+ *                       sets no bit
  *   "tc.table"          1 (default): knobs left automatic and a zero
  *                       over-fetch take the committed autotuner results
  *                       for the call's shape (tuning/gb300.json); 0: ignore

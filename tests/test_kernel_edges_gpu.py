@@ -387,3 +387,23 @@ def test_bound_of_products_that_overflow(cuda, metric, k):
     got = scan.fp16_search(t, q, k, metric)
     torch.cuda.synchronize()
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("metric", ["l2", "ip", "cosine"])
+def test_filtered_flat_scan_survives_a_wait_that_runs_out(cuda, metric):
+    """A tensor-core pass that gives up a wait (a 1 ns limit) has not seen every
+    row: the plain scan answers the call, which is exact and reports nothing."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.randn((20_000, 64), generator=g, device="cuda")
+    q = torch.randn((200, 64), generator=g, device="cuda")
+    with scan.tuned(flat_tc=0):
+        ref = scan.flat_scan(x, q, 10, metric)
+    scan.device_status()
+    with scan.tuned(flat_tc=1, tc_wait_limit_ns=1):
+        got = scan.flat_scan(x, q, 10, metric)
+        torch.cuda.synchronize()
+    assert scan.device_status() == 0
+    assert torch.equal(got, ref)
