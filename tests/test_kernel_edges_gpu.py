@@ -407,3 +407,36 @@ def test_filtered_flat_scan_survives_a_wait_that_runs_out(cuda, metric):
         torch.cuda.synchronize()
     assert scan.device_status() == 0
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("offset", [0, 8, 16])
+def test_filtered_flat_scan_in_a_callers_arena(cuda, offset):
+    """A caller's arena that starts on an 8-byte boundary serves the plain scan,
+    one on a 16-byte boundary the filtered one: the same answer."""
+    import ctypes as C
+
+    from fvgb300 import _lib, scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn((20_000, 64), generator=g, device="cuda")
+    q = torch.randn((200, 64), generator=g, device="cuda")
+    with scan.tuned(flat_tc=0):
+        ref = scan.flat_scan(x, q, 10, "l2")
+    arena = torch.empty(64 << 20, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    handle = C.c_void_p(stream.cuda_stream)
+    _lib.call("fv_set_stream_scratch", handle, C.c_void_p(arena.data_ptr() + offset), arena.numel() - offset)
+    try:
+        with scan.tuned(flat_tc=1):
+            scan.profile_enable(True)
+            scan.profile_summary()
+            got = scan.flat_scan(x, q, 10, "l2", stream=stream)
+            stream.synchronize()
+            ran = scan.profile_summary()
+    finally:
+        scan.profile_enable(False)
+        _lib.call("fv_release_stream_scratch", handle)
+    assert ("flat_tc_prep" in ran) == (offset % 16 == 0)
+    assert torch.equal(got, ref)
