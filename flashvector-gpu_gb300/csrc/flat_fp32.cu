@@ -520,11 +520,11 @@ int launch_flat_f32(const float* vectors, const uint32_t* vec_ids, uint32_t n, u
                     uint32_t forced_splits, cudaStream_t stream, const QueryFilter* filters) {
   void* scratch = nullptr;
   if (!filters && !forced_splits) {
-    const size_t bytes = flat_tc_bytes(n, dim, nq, k, metric);
+    const FlatTcPlan t = plan_flat_tc(n, dim, nq, k, metric);
     // (a caller's arena that only fits the plain scan keeps it, as does one that
     // is not 16-byte aligned, which the filter's TMA and vector accesses need)
-    if (bytes && (scratch = scratch_get(stream, bytes)) != nullptr && (uintptr_t)scratch % 16 == 0)
-      return launch_flat_tc(vectors, vec_ids, n, dim, queries, nq, k, metric, mask, out, scratch, stream);
+    if (t.bytes && (scratch = scratch_get(stream, t.bytes)) != nullptr && (uintptr_t)scratch % 16 == 0)
+      return launch_flat_tc(t, vectors, vec_ids, n, dim, queries, nq, k, metric, mask, out, scratch, stream);
   }
   const FlatPlan p = plan_flat_f32(n, nq, k, forced_splits);
   if (p.scratch_bytes) {

@@ -427,17 +427,13 @@ constexpr uint64_t kFlatTcWork = 120000000ull;
 // The copies and lists live in the stream's scratch arena, which keeps them.
 constexpr size_t kMaxScratch = (size_t)1 << 30;
 
-struct FlatTcPlan {
-  size_t bytes = 0;  // 0: use the plain scan
-  uint32_t pd = 0, query_rows = 0;
-  TcCollect c{};
-  FlatPlan f;
-  size_t x16 = 0, xnorm = 0, q16 = 0, qnorm = 0, info = 0, mu = 0, var = 0, words = 0, collect = 0, plain = 0;
-};
+}  // namespace
 
-FlatTcPlan plan_flat_tc(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, MetricType metric, bool forced) {
+FlatTcPlan plan_flat_tc(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, MetricType metric) {
   FlatTcPlan P;
-  if (nq < 32 || n < 2048 || dim < 8 || dim > 4096) return P;
+  const int64_t knob = tune_value("flat.tc", -1);
+  const bool forced = knob == 1;
+  if (knob == 0 || nq < 32 || n < 2048 || dim < 8 || dim > 4096) return P;
   if (!forced && (uint64_t)nq * n * dim < kFlatTcWork) return P;
   P.pd = (dim + 15) / 16 * 16;
   const size_t table = (size_t)n * P.pd * 2;
@@ -466,8 +462,7 @@ FlatTcPlan plan_flat_tc(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, Metri
     c.margin_norm = metric == METRIC_COSINE ? 0.f : 3.f;  // qnorm holds -e |Q|^2
     c.margin_abs = metric == METRIC_COSINE ? 5.f * e * kUnit * kUnit : 2.f * e * 524288.f;
   }
-  const size_t cb = tc_collect_bytes(c, &P.query_rows);
-  if (!cb) return P;
+  if (!plan_tc_collect(c)) return P;
   size_t at = 0;
   auto take = [&](size_t bytes) {
     const size_t o = at;
@@ -476,29 +471,21 @@ FlatTcPlan plan_flat_tc(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, Metri
   };
   P.x16 = take(table);
   P.xnorm = take((size_t)n * 4);
-  P.q16 = take((size_t)P.query_rows * P.pd * 2);
+  P.q16 = take((size_t)c.query_rows * P.pd * 2);
   P.qnorm = take((size_t)nq * 4);
   P.info = take((size_t)nq * sizeof(QueryInfo));
   P.mu = take((size_t)dim * 4);
   P.var = take((size_t)dim * 4);
   P.words = take(W_COUNT * 4);
-  P.collect = take(cb);
+  P.collect = take(c.bytes);
   P.plain = take(P.f.scratch_bytes);
   if (at <= kMaxScratch) P.bytes = at;
   return P;
 }
 
-}  // namespace
-
-size_t flat_tc_bytes(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, MetricType metric) {
-  const int64_t knob = tune_value("flat.tc", -1);
-  return knob == 0 ? 0 : plan_flat_tc(n, dim, nq, k, metric, knob == 1).bytes;
-}
-
-int launch_flat_tc(const float* vectors, const uint32_t* vec_ids, uint32_t n, uint32_t dim, const float* queries,
-                   uint32_t nq, uint32_t k, MetricType metric, const uint32_t* mask, GpuSearchResult* out,
-                   void* scratch, cudaStream_t stream) {
-  FlatTcPlan P = plan_flat_tc(n, dim, nq, k, metric, true);
+int launch_flat_tc(const FlatTcPlan& P, const float* vectors, const uint32_t* vec_ids, uint32_t n, uint32_t dim,
+                   const float* queries, uint32_t nq, uint32_t k, MetricType metric, const uint32_t* mask,
+                   GpuSearchResult* out, void* scratch, cudaStream_t stream) {
   uint8_t* base = static_cast<uint8_t*>(scratch);
   const bool vec = dim % 4 == 0 && (uintptr_t)vectors % 16 == 0 && (uintptr_t)queries % 16 == 0;
   float* mu = reinterpret_cast<float*>(base + P.mu);
@@ -509,7 +496,7 @@ int launch_flat_tc(const float* vectors, const uint32_t* vec_ids, uint32_t n, ui
   p.q = queries;
   p.n = n;
   p.nq = nq;
-  p.nq_rows = P.query_rows;
+  p.nq_rows = P.c.query_rows;
   p.dim = dim;
   p.pd = P.pd;
   p.metric = (int)metric;
@@ -527,7 +514,7 @@ int launch_flat_tc(const float* vectors, const uint32_t* vec_ids, uint32_t n, ui
     ProfScope ps("flat_tc_prep", stream);
     flat_tc_center_kernel<<<(dim + 31) / 32, 32 * CEN_GROUPS, 0, stream>>>(vectors, n, dim, (int)metric, mu, var,
                                                                            words);
-    const uint64_t rows = (uint64_t)n + P.query_rows;
+    const uint64_t rows = (uint64_t)n + P.c.query_rows;
     auto prep = [&](auto kern, uint32_t lanes) {
       const uint64_t per_block = (uint64_t)PREP_WARPS * PREP_ROWS * (32 / lanes);
       const uint32_t blocks = (uint32_t)std::min<uint64_t>((rows + per_block - 1) / per_block, 8ull * device_sm_count());
@@ -549,7 +536,7 @@ int launch_flat_tc(const float* vectors, const uint32_t* vec_ids, uint32_t n, ui
     }
     note_launch(2);
   }
-  TcCollect& c = P.c;
+  TcCollect c = P.c;
   c.rows16 = p.x16;
   c.row_norms = p.xnorm;
   c.q16 = p.q16;

@@ -131,6 +131,21 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
 // same arguments (same plan, same tuning knobs).
 size_t tc_scan_scratch_bytes(const TcTables& t, uint32_t nq, uint32_t k, MetricType metric, const FvScanOptions& opt);
 
+// Every launch parameter of one tensor-core scan call and the scratch it
+// takes, computed once: launch_tc_scan launches from it and the serving
+// loop admits a batch by its scratch_bytes (tc_scan_scratch_bytes).
+struct TcPlan {
+  bool fp8 = false, pair = false, prepass = false;
+  uint32_t elem = 0, kblocks = 0, shortlist = 0, kl = 0, kl_tmpl = 0;
+  int groups = 1;  // epilogue groups of the main scan (the minima pass runs at most 2)
+  uint32_t nqb = 0, nqb_grid = 0, splits = 0, tps = 0;
+  uint32_t pstride = 0, pr = 0, psplits = 0, ptps = 0;  // minima pass: tile stride, rank of the bound, splits
+  uint32_t pgran = 0, pcount = 0;                        // columns per minimum, minima per query
+  uint32_t nq_rows = 0, slot_stride = 0;
+  size_t q_bytes = 0, qn_bytes = 0, part_bytes = 0, slot_bytes = 0, tau_bytes = 0;
+  size_t scratch_bytes = 0;
+};
+
 // The collecting pass behind the exact flat scan's tensor-core filter
 // (tc_scan.cu): every row whose ranking value max(floor, qnorm + row_norm -
 // 2 <q16, row16>) is at most the query's bound, which is a bound on the
@@ -147,23 +162,34 @@ struct TcCollect {
   float floor, margin_rel, margin_norm, margin_abs;
   const uint32_t* mask;
   uint32_t* status;        // gets the passes' status bits (zeroed by the caller): the lists are then not complete
+  // set by plan_tc_collect
+  TcPlan plan;
+  uint32_t query_rows;     // rows of q16
+  size_t bytes;            // scratch
   // set by launch_tc_collect, inside its scratch
   uint64_t* partial;       // [nq][lists][kl]
   uint32_t lists, kl;
   float* bound;            // [nq]
   uint32_t* flags;         // [nq], zero
 };
-// scratch of the pass and the rows its query table must have; 0: no bound can
-// be found for this shape
-size_t tc_collect_bytes(const TcCollect& c, uint32_t* query_rows);
+// Plans the pass from the sizes in c, once: the tuning knobs it reads may be set
+// by another thread before the launch. False: no bound can be found for them.
+bool plan_tc_collect(TcCollect& c);
 int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream);
 
-// exact flat scan behind a tensor-core filter (flat_tc.cu): the scratch it
-// takes, 0 where the plain scan is the better (or only) way
-size_t flat_tc_bytes(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, MetricType metric);
-int launch_flat_tc(const float* vectors, const uint32_t* vec_ids, uint32_t n, uint32_t dim, const float* queries,
-                   uint32_t nq, uint32_t k, MetricType metric, const uint32_t* mask, GpuSearchResult* out,
-                   void* scratch, cudaStream_t stream);
+// exact flat scan behind a tensor-core filter (flat_tc.cu)
+struct FlatTcPlan {
+  size_t bytes = 0;  // scratch; 0: the plain scan is the better (or only) way
+  uint32_t pd = 0;
+  TcCollect c{};
+  FlatPlan f;        // the plain scan of the flagged queries
+  // byte offsets in the scratch
+  size_t x16 = 0, xnorm = 0, q16 = 0, qnorm = 0, info = 0, mu = 0, var = 0, words = 0, collect = 0, plain = 0;
+};
+FlatTcPlan plan_flat_tc(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, MetricType metric);
+int launch_flat_tc(const FlatTcPlan& plan, const float* vectors, const uint32_t* vec_ids, uint32_t n, uint32_t dim,
+                   const float* queries, uint32_t nq, uint32_t k, MetricType metric, const uint32_t* mask,
+                   GpuSearchResult* out, void* scratch, cudaStream_t stream);
 
 // IVF-PQ / IVF-SQ8 search (ivf.cu)
 struct IvfLaunch {

@@ -496,21 +496,6 @@ uint32_t fill_waves(uint32_t s_min, uint32_t nqb, uint32_t ntiles, uint32_t sms,
 
 }  // namespace
 
-// Every launch parameter of one tensor-core scan call and the scratch it
-// takes, computed once: launch_tc_scan launches from it and the serving
-// loop admits a batch by its scratch_bytes (tc_scan_scratch_bytes).
-struct TcPlan {
-  bool fp8 = false, pair = false, prepass = false;
-  uint32_t elem = 0, kblocks = 0, shortlist = 0, kl = 0, kl_tmpl = 0;
-  int groups = 1;  // epilogue groups of the main scan (the minima pass runs at most 2)
-  uint32_t nqb = 0, nqb_grid = 0, splits = 0, tps = 0;
-  uint32_t pstride = 0, pr = 0, psplits = 0, ptps = 0;  // minima pass: tile stride, rank of the bound, splits
-  uint32_t pgran = 0, pcount = 0;                        // columns per minimum, minima per query
-  uint32_t nq_rows = 0, slot_stride = 0;
-  size_t q_bytes = 0, qn_bytes = 0, part_bytes = 0, slot_bytes = 0, tau_bytes = 0;
-  size_t scratch_bytes = 0;
-};
-
 // rank > 0: a collecting pass (launch_tc_collect): the bound is for the rank
 // best rows, and the heaps have room for k.
 TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metric, const FvScanOptions& opt,
@@ -819,21 +804,16 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
 // prepared fp16 rows and queries, ranking by max(floor, qnorm + norm -
 // 2 dot). Leaves the range lists and the bounds for the caller to finish.
 // ---------------------------------------------------------------------------
-static TcPlan plan_collect(const TcCollect& c) {
+bool plan_tc_collect(TcCollect& c) {
   const TcTables t{false, c.rows16, c.row_norms, nullptr, nullptr, c.n, c.dim, c.padded_dim};
-  return plan_tc_scan(t, c.nq, c.room, METRIC_L2, FvScanOptions{0, 0, 0.f, 0}, c.rank);
-}
-
-size_t tc_collect_bytes(const TcCollect& c, uint32_t* query_rows) {
-  const TcPlan P = plan_collect(c);
-  if (!P.prepass) return 0;
-  *query_rows = P.nq_rows;
-  return P.part_bytes + P.tau_bytes;
+  c.plan = plan_tc_scan(t, c.nq, c.room, METRIC_L2, FvScanOptions{0, 0, 0.f, 0}, c.rank);
+  c.query_rows = c.plan.nq_rows;
+  c.bytes = c.plan.part_bytes + c.plan.tau_bytes;
+  return c.plan.prepass;
 }
 
 int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream) {
-  const TcPlan P = plan_collect(c);
-  if (!P.prepass) return FV_ERR_ARG;
+  const TcPlan& P = c.plan;
   c.partial = static_cast<uint64_t*>(scratch);
   c.bound = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + P.part_bytes);
   c.flags = reinterpret_cast<uint32_t*>(c.bound + c.nq);

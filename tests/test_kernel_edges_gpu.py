@@ -440,3 +440,38 @@ def test_filtered_flat_scan_in_a_callers_arena(cuda, offset):
         _lib.call("fv_release_stream_scratch", handle)
     assert ("flat_tc_prep" in ran) == (offset % 16 == 0)
     assert torch.equal(got, ref)
+
+
+def test_filtered_flat_scan_while_knobs_change(cuda):
+    """Another thread sets the knobs that the filter's passes are planned by: each
+    call keeps the plan that its scratch was taken for."""
+    import threading
+
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(8)
+    x = torch.randn((20_000, 200), generator=g, device="cuda")
+    q = torch.randn((150, 200), generator=g, device="cuda")
+    with scan.tuned(flat_tc=0):
+        ref = scan.flat_scan(x, q, 10, "l2")
+    stop = threading.Event()
+
+    def turn():
+        i = 0
+        while not stop.is_set():
+            scan.tune_set("tc.pair", (-1, 0)[i % 2])
+            scan.tune_set("tc.prepass_stride", (0, 2, 7)[i % 3])
+            scan.tune_set("tc.prepass", (-1, 0)[i % 5 == 0])
+            i += 1
+
+    with scan.tuned(flat_tc=1, tc_pair=-1, tc_prepass_stride=0, tc_prepass=-1):
+        thread = threading.Thread(target=turn)
+        thread.start()
+        try:
+            got = [scan.flat_scan(x, q, 10, "l2") for _ in range(300)]
+        finally:
+            stop.set()
+            thread.join()
+    torch.cuda.synchronize()
+    assert all(torch.equal(r, ref) for r in got)
