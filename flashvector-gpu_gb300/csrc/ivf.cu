@@ -1537,6 +1537,7 @@ struct IvfPlan {
   bool tcc = false, force_exact = false;
   uint32_t K = 0;
   size_t co_mu = 0, co_c16 = 0, co_cnorm = 0, co_qc = 0, co_cand = 0, co_flags = 0, co_cmax = 0, co_tc = 0;
+  TcPlan tc;
   FlatPlan cp;
   size_t coarse_bytes = 0, probe_bytes = 0, part_bytes = 0, allow_bytes = 0, scratch_bytes = 0;
 };
@@ -1600,7 +1601,8 @@ IvfPlan plan_ivf_search(int mode, const IvfLaunch& L) {
     Q.co_flags = align256(Q.co_cand + (size_t)L.nq * K * 8);
     Q.co_cmax = align256(Q.co_flags + (size_t)L.nq * 4);
     Q.co_tc = (Q.co_cmax + 256 + 1023) / 1024 * 1024;
-    tc_bytes = Q.co_tc + tc_scan_scratch_bytes(ct, L.nq, K, METRIC_L2, copt);
+    Q.tc = plan_tc_scan(ct, L.nq, K, METRIC_L2, copt);
+    tc_bytes = Q.co_tc + Q.tc.scratch_bytes;
   }
   Q.tcc = tcc;
   Q.K = K;
@@ -1662,8 +1664,8 @@ static int launch_coarse_tc(const IvfPlan& Q, const IvfLaunch& L, uint8_t* scrat
   note_launch(2);
   const TcTables ct{false, c16, cnorm, nullptr, nullptr, L.nlist, L.dim, pd16};
   const FvScanOptions copt{0, 0, 0.f, 0};
-  int rc = launch_tc_scan_ext(ct, qc, L.nq, Q.K, METRIC_L2, nullptr, cand, copt, stream, nullptr, scratch + Q.co_tc,
-                              flags);
+  int rc = launch_tc_scan_planned(Q.tc, ct, qc, L.nq, Q.K, METRIC_L2, nullptr, cand, copt, stream, nullptr,
+                                  scratch + Q.co_tc, flags);
   if (rc != 0) return rc;
   const uint32_t fthreads = Q.K <= 64 ? 64u : 256u;
   const size_t fsmem = fthreads * 8 + (size_t)L.dim * 4;

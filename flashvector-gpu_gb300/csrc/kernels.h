@@ -120,13 +120,6 @@ cudaError_t dispatch_tc_scan_fp8(int kl, int groups, int metric, bool table_scal
 int launch_tc_scan(const TcTables& t, const float* queries, uint32_t nq, uint32_t k, MetricType metric,
                    const uint32_t* mask, GpuSearchResult* out, const FvScanOptions& opt, cudaStream_t stream,
                    const QueryFilter* filters = nullptr);
-// launch_tc_scan with the scratch given by the caller (ext_scratch: at
-// least tc_scan_scratch_bytes, 1 KB aligned; null: the stream's arena) and
-// an optional per-query flag array set for a query whose merged shortlist
-// may have lost keys to a full range heap (the caller zeroes it).
-int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uint32_t k, MetricType metric,
-                       const uint32_t* mask, GpuSearchResult* out, const FvScanOptions& opt, cudaStream_t stream,
-                       const QueryFilter* filters, void* ext_scratch, uint32_t* incomplete_q);
 // The scratch bytes launch_tc_scan takes from the stream's arena for the
 // same arguments (same plan, same tuning knobs).
 size_t tc_scan_scratch_bytes(const TcTables& t, uint32_t nq, uint32_t k, MetricType metric, const FvScanOptions& opt);
@@ -145,6 +138,18 @@ struct TcPlan {
   size_t q_bytes = 0, qn_bytes = 0, part_bytes = 0, slot_bytes = 0, tau_bytes = 0;
   size_t scratch_bytes = 0;
 };
+
+// The plan of launch_tc_scan for the same arguments, and the launch from one, with
+// scratch of its scratch_bytes (1 KB aligned) given by the caller and an
+// optional per-query flag array set for a query whose merged shortlist may have
+// lost keys to a full range heap (the caller zeroes it). The plan that the
+// scratch was taken for is the one to launch: the tuning knobs it reads may be
+// set by another thread in between.
+TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metric, const FvScanOptions& opt,
+                    uint32_t rank = 0);
+int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* queries, uint32_t nq, uint32_t k,
+                           MetricType metric, const uint32_t* mask, GpuSearchResult* out, const FvScanOptions& opt,
+                           cudaStream_t stream, const QueryFilter* filters, void* scratch, uint32_t* incomplete_q);
 
 // The collecting pass behind the exact flat scan's tensor-core filter
 // (tc_scan.cu): every row whose ranking value max(floor, qnorm + row_norm -

@@ -499,7 +499,7 @@ uint32_t fill_waves(uint32_t s_min, uint32_t nqb, uint32_t ntiles, uint32_t sms,
 // rank > 0: a collecting pass (launch_tc_collect): the bound is for the rank
 // best rows, and the heaps have room for k.
 TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metric, const FvScanOptions& opt,
-                    uint32_t rank = 0) {
+                    uint32_t rank) {
   TcPlan P{};
   const bool fp8 = t.fp8;
   const uint32_t elem = fp8 ? 1 : 2;
@@ -650,13 +650,16 @@ size_t tc_scan_scratch_bytes(const TcTables& t, uint32_t nq, uint32_t k, MetricT
 int launch_tc_scan(const TcTables& t, const float* queries, uint32_t nq, uint32_t k, MetricType metric,
                    const uint32_t* mask, GpuSearchResult* out, const FvScanOptions& opt, cudaStream_t stream,
                    const QueryFilter* filters) {
-  return launch_tc_scan_ext(t, queries, nq, k, metric, mask, out, opt, stream, filters, nullptr, nullptr);
+  const TcPlan P = plan_tc_scan(t, nq, k, metric, opt);
+  void* scratch = scratch_get(stream, P.scratch_bytes);
+  if (!scratch) return (int)cudaErrorMemoryAllocation;
+  return launch_tc_scan_planned(P, t, queries, nq, k, metric, mask, out, opt, stream, filters, scratch, nullptr);
 }
 
-int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uint32_t k, MetricType metric,
-                       const uint32_t* mask, GpuSearchResult* out, const FvScanOptions& opt, cudaStream_t stream,
-                       const QueryFilter* filters, void* ext_scratch, uint32_t* incomplete_q) {
-  const TcPlan P = plan_tc_scan(t, nq, k, metric, opt);
+int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* queries, uint32_t nq, uint32_t k,
+                           MetricType metric, const uint32_t* mask, GpuSearchResult* out, const FvScanOptions& opt,
+                           cudaStream_t stream, const QueryFilter* filters, void* scratch_at,
+                           uint32_t* incomplete_q) {
   const bool fp8 = P.fp8;
   const uint32_t elem = P.elem, kblocks = P.kblocks, shortlist = P.shortlist, kl = P.kl, kl_tmpl = P.kl_tmpl;
   const int groups = P.groups;
@@ -664,8 +667,7 @@ int launch_tc_scan_ext(const TcTables& t, const float* queries, uint32_t nq, uin
   const bool pair = P.pair, prepass = P.prepass;
   const uint32_t nq_rows = P.nq_rows, slot_stride = P.slot_stride;
   const size_t q_bytes = P.q_bytes, qn_bytes = P.qn_bytes, part_bytes = P.part_bytes;
-  uint8_t* scratch = static_cast<uint8_t*>(ext_scratch ? ext_scratch : scratch_get(stream, P.scratch_bytes));
-  if (!scratch) return (int)cudaErrorMemoryAllocation;
+  uint8_t* scratch = static_cast<uint8_t*>(scratch_at);
   void* qprep = scratch;
   float* qnorm = reinterpret_cast<float*>(scratch + q_bytes);
   float* qscale = reinterpret_cast<float*>(scratch + q_bytes + qn_bytes);

@@ -442,19 +442,29 @@ def test_filtered_flat_scan_in_a_callers_arena(cuda, offset):
     assert torch.equal(got, ref)
 
 
-def test_filtered_flat_scan_while_knobs_change(cuda):
-    """Another thread sets the knobs that the filter's passes are planned by: each
-    call keeps the plan that its scratch was taken for."""
+@pytest.mark.parametrize("path", ["flat", "ivf"])
+def test_scans_while_knobs_change(cuda, oracle_mod, path):
+    """Another thread sets the knobs that the tensor-core passes of an exact scan
+    or a coarse probe are planned by: each call keeps the plan that its scratch
+    was taken for."""
     import threading
 
     from fvgb300 import scan
+    from fvgb300.ivf import IvfTable
 
     torch = cuda
-    g = torch.Generator(device="cuda").manual_seed(8)
-    x = torch.randn((20_000, 200), generator=g, device="cuda")
-    q = torch.randn((150, 200), generator=g, device="cuda")
-    with scan.tuned(flat_tc=0):
-        ref = scan.flat_scan(x, q, 10, "l2")
+    if path == "flat":
+        g = torch.Generator(device="cuda").manual_seed(8)
+        x = torch.randn((20_000, 200), generator=g, device="cuda")
+        q = torch.randn((150, 200), generator=g, device="cuda")
+        search = lambda: scan.flat_scan(x, q, 10, "l2")
+    else:
+        x, q, t = _ivf_case(oracle_mod, 6000, 200, 400, 8, 3, 0.5)
+        table = IvfTable("sq8", t, vectors=x)
+        q = torch.from_numpy(np.resize(q, (150, 200)).astype(np.float32)).cuda()
+        search = lambda: table.search(q, 10, 9, 40)
+    with scan.tuned(flat_tc=0, ivf_tc_coarse=0):
+        ref = search()
     stop = threading.Event()
 
     def turn():
@@ -465,11 +475,11 @@ def test_filtered_flat_scan_while_knobs_change(cuda):
             scan.tune_set("tc.prepass", (-1, 0)[i % 5 == 0])
             i += 1
 
-    with scan.tuned(flat_tc=1, tc_pair=-1, tc_prepass_stride=0, tc_prepass=-1):
+    with scan.tuned(flat_tc=1, ivf_tc_coarse=1, tc_pair=-1, tc_prepass_stride=0, tc_prepass=-1):
         thread = threading.Thread(target=turn)
         thread.start()
         try:
-            got = [scan.flat_scan(x, q, 10, "l2") for _ in range(300)]
+            got = [search() for _ in range(300)]
         finally:
             stop.set()
             thread.join()
