@@ -71,11 +71,30 @@ struct Arena {
 std::mutex g_arena_mu;
 // keyed by (device, stream)
 std::unordered_map<uint64_t, Arena> g_arenas;
+// scratch_try's memory, apart from the arena: a captured graph keeps the arena's
+// address, which a call must not free that never needed a larger one. What a
+// capture was given of it stays (retired) until the stream's scratch is released.
+struct LargeArena {
+  void* ptr = nullptr;
+  size_t bytes = 0;
+  bool captured = false;
+  std::vector<void*> retired;
+};
+std::unordered_map<uint64_t, LargeArena> g_large;
 
 uint64_t arena_key(cudaStream_t s) {
   int dev = 0;
   cudaGetDevice(&dev);
   return (uint64_t)(uintptr_t)s * 64u + (uint64_t)dev;
+}
+
+// (g_arena_mu held)
+void free_large(uint64_t key, cudaStream_t stream) {
+  auto it = g_large.find(key);
+  if (it == g_large.end()) return;
+  if (it->second.ptr) cudaFreeAsync(it->second.ptr, stream);
+  for (void* p : it->second.retired) cudaFreeAsync(p, stream);
+  g_large.erase(it);
 }
 
 std::mutex g_dev_mu;
@@ -162,6 +181,36 @@ void* scratch_get(cudaStream_t stream, size_t bytes) {
   return a.ptr;
 }
 
+void* scratch_try(cudaStream_t stream, size_t bytes) {
+  bytes = (bytes + 255) & ~(size_t)255;
+  std::lock_guard<std::mutex> lk(g_arena_mu);
+  const uint64_t key = arena_key(stream);
+  const Arena& a = g_arenas[key];
+  if (a.bytes >= bytes) return a.ptr;
+  if (!a.owned) return nullptr;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  const bool capturing = cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+  if (capturing) cudaGetLastError();
+  LargeArena& l = g_large[key];
+  if (l.bytes < bytes) {
+    void* p = nullptr;
+    const size_t grow = bytes + bytes / 4;
+    if (capturing || cudaMallocAsync(&p, grow, stream) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    if (l.ptr && l.captured)
+      l.retired.push_back(l.ptr);
+    else if (l.ptr)
+      cudaFreeAsync(l.ptr, stream);
+    l.ptr = p;
+    l.bytes = grow;
+    l.captured = false;
+  }
+  l.captured = l.captured || capturing;
+  return l.ptr;
+}
+
 }  // namespace fv
 
 using fv::note_launch;
@@ -221,6 +270,7 @@ int cuda_destroy_stream(void* stream) {
   if (!stream) return 0;
   {
     std::lock_guard<std::mutex> lk(fv::g_arena_mu);
+    fv::free_large(fv::arena_key((cudaStream_t)stream), (cudaStream_t)stream);
     auto it = fv::g_arenas.find(fv::arena_key((cudaStream_t)stream));
     if (it != fv::g_arenas.end()) {
       if (it->second.owned && it->second.ptr) cudaFreeAsync(it->second.ptr, (cudaStream_t)stream);
@@ -628,6 +678,7 @@ int fv_profile_summary(char* buf, size_t len) {
 
 int fv_set_stream_scratch(void* stream, void* d_ptr, size_t bytes) {
   std::lock_guard<std::mutex> lk(fv::g_arena_mu);
+  fv::free_large(fv::arena_key((cudaStream_t)stream), (cudaStream_t)stream);
   fv::Arena& a = fv::g_arenas[fv::arena_key((cudaStream_t)stream)];
   if (a.owned && a.ptr) cudaFreeAsync(a.ptr, (cudaStream_t)stream);
   if (d_ptr) {

@@ -522,8 +522,9 @@ int launch_flat_f32(const float* vectors, const uint32_t* vec_ids, uint32_t n, u
   if (!filters && !forced_splits) {
     const FlatTcPlan t = plan_flat_tc(n, dim, nq, k, metric);
     // (a caller's arena that only fits the plain scan keeps it, as does one that
-    // is not 16-byte aligned, which the filter's TMA and vector accesses need)
-    if (t.bytes && (scratch = scratch_get(stream, t.bytes)) != nullptr && (uintptr_t)scratch % 16 == 0)
+    // is not 16-byte aligned, which the filter's TMA and vector accesses need, and
+    // a capture or a full device, where the arena cannot grow for the filter)
+    if (t.bytes && (scratch = scratch_try(stream, t.bytes)) != nullptr && (uintptr_t)scratch % 16 == 0)
       return launch_flat_tc(t, vectors, vec_ids, n, dim, queries, nq, k, metric, mask, out, scratch, stream);
   }
   const FlatPlan p = plan_flat_f32(n, nq, k, forced_splits);

@@ -424,7 +424,8 @@ float error_bound(uint32_t dim, MetricType metric) {
 // launches and the encoding outweigh the arithmetic that it saves (50,000 x 64
 // x 32: 70 against 54 us; 20,000 x 64 x 100, 1.3e8: 68 against 88).
 constexpr uint64_t kFlatTcWork = 120000000ull;
-// The copies and lists live in the stream's scratch arena, which keeps them.
+// The copies and lists live in the stream's scratch (scratch_try), which keeps
+// up to a quarter more until it is released.
 constexpr size_t kMaxScratch = (size_t)1 << 30;
 
 }  // namespace

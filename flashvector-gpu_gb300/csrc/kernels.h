@@ -80,6 +80,11 @@ struct ProfScope {
 // allocation; returns nullptr on failure. A caller-provided arena installed
 // with fv_set_stream_scratch() takes precedence.
 void* scratch_get(cudaStream_t stream, size_t bytes);
+// Scratch for a caller that can do with less: the arena where it is large enough,
+// else memory of its own, with the same lifetime, and nullptr where that cannot
+// grow (no memory; a capture, whose graph would own the new memory; a
+// caller-provided arena). The arena stays as it is.
+void* scratch_try(cudaStream_t stream, size_t bytes);
 
 // Writes `count` {0xFFFFFFFF, 1e30} results (fixtures.cu).
 int launch_fill_sentinel(GpuSearchResult* out, size_t count, cudaStream_t stream);

@@ -408,9 +408,15 @@ int fv_tune_lookup(int fp8, MetricType metric, uint32_t dim, uint64_t num_vector
  * needing more than `bytes` fails with cudaErrorMemoryAllocation).
  * d_ptr == NULL removes the caller buffer and returns to library-managed
  * stream-ordered allocation. Replaces the reference's per-call
- * cudaMallocAsync in ivf_pq_lookup.cu:397-401. */
+ * cudaMallocAsync in ivf_pq_lookup.cu:397-401. d_ptr should be 256-byte
+ * aligned (the tensor-core paths need 16; an exact scan with less than that,
+ * or with less room than its tensor-core filter takes, runs without it).
+ * Library-managed, a stream whose exact scans use the filter holds up to
+ * 1.25 GiB for it, apart from the arena of the other calls; a filter whose
+ * memory cannot be had (a full device, inside a capture) is left out. */
 int fv_set_stream_scratch(void* stream, void* d_ptr, size_t bytes);
-/* Frees the library-managed scratch arena of `stream`. */
+/* Frees the library-managed scratch of `stream`; graphs captured on it may not
+ * be launched afterwards. */
 int fv_release_stream_scratch(void* stream);
 
 #ifdef __cplusplus

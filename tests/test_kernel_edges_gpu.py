@@ -485,3 +485,52 @@ def test_scans_while_knobs_change(cuda, oracle_mod, path):
             thread.join()
     torch.cuda.synchronize()
     assert all(torch.equal(r, ref) for r in got)
+
+
+def test_filtered_flat_scan_and_captured_graphs(cuda):
+    """A capture that finds no memory for the filter takes the plain scan; a graph
+    that holds the filter's memory keeps it when a larger call asks for more; and
+    a filtered call leaves the arena that another graph holds alone."""
+    import ctypes as C
+
+    from fvgb300 import _lib, scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x = torch.randn((20_000, 64), generator=g, device="cuda")
+    q = torch.randn((200, 64), generator=g, device="cuda")
+    x2 = torch.randn((60_000, 128), generator=g, device="cuda")
+    q2 = torch.randn((500, 128), generator=g, device="cuda")
+    table, q16 = scan.Fp16Table(x[:2000].clone()), q[:10].clone()
+    with scan.tuned(flat_tc=0):
+        ref, ref2 = scan.flat_scan(x, q, 10, "l2"), scan.flat_scan(x2, q2, 10, "l2")
+    ref16 = scan.fp16_search(table, q16, 10, "l2")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    outs = [torch.zeros_like(r) for r in (ref, ref, ref16)]
+    flat = lambda out: scan.flat_scan(x, q, 10, "l2", out=out, stream=stream)
+    fp16 = lambda: scan.fp16_search(table, q16, 10, "l2", out=outs[2], stream=stream)
+    try:
+        with scan.tuned(flat_tc=0):
+            flat(outs[0])  # the arena fits the plain scan (and the tensor-core scan)
+        fp16()
+        with scan.tuned(flat_tc=1):
+            plain = scan.Graph.capture(lambda: flat(outs[0]), stream)
+            fp16_graph = scan.Graph.capture(fp16, stream)
+            flat(outs[1])
+            filtered = scan.Graph.capture(lambda: flat(outs[1]), stream)
+            assert filtered.kernels > plain.kernels
+            got2 = scan.flat_scan(x2, q2, 10, "l2", stream=stream)  # grows the filter's memory
+            noise = torch.full((1 << 26,), 7, dtype=torch.int32, device="cuda")
+            for o in outs:
+                o.zero_()
+            torch.cuda.synchronize()
+            for graph in (plain, fp16_graph, filtered):
+                graph.launch(stream)
+            stream.synchronize()
+        del noise
+        assert torch.equal(got2, ref2)
+        assert torch.equal(outs[0], ref) and torch.equal(outs[1], ref) and torch.equal(outs[2], ref16)
+    finally:
+        stream.synchronize()
+        _lib.call("fv_release_stream_scratch", C.c_void_p(stream.cuda_stream))
