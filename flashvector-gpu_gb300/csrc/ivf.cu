@@ -1800,7 +1800,8 @@ int launch_ivf_search(int mode, const IvfLaunch& L, cudaStream_t stream) {
   }
   if (smem > 227 * 1024) return FV_ERR_ARG;
   const size_t staged = mode == IVF_SQ8 ? IvfSmem::staged_bytes(a.keys_pow2, L.dim, a.list_chunk) : 0;
-  const bool stage_rows = staged > 0 && staged <= 227 * 1024;
+  // (1 KB short of the limit, which the kernel's static shared memory counts against)
+  const bool stage_rows = staged > 0 && staged <= 226 * 1024;
   if (stage_rows) smem = staged;
   // scratch of the flushes' selection, where shortlist and buffer fit its
   // registers (and the block has room: else they sort)

@@ -534,3 +534,17 @@ def test_filtered_flat_scan_and_captured_graphs(cuda):
     finally:
         stream.synchronize()
         _lib.call("fv_release_stream_scratch", C.c_void_p(stream.cuda_stream))
+
+
+@pytest.mark.parametrize("dim,rerank", [(3750, 7000), (3751, 7000), (3752, 7000), (10_918, 100), (10_919, 100)])
+def test_ivf_sq8_staging_at_the_shared_memory_limit(cuda, oracle_mod, dim, rerank):
+    """Rows and shortlists with which the staging takes the last bytes of a
+    block's shared memory: the call runs (unstaged where it must)."""
+    from fvgb300.ivf import IvfTable
+
+    torch = cuda
+    x, q, t = _ivf_case(oracle_mod, 600, dim, 4, 1, dim, 0.5)
+    ref = oracle_mod.ivf_sq_search(t, x, q[:3], 10, 4, rerank)
+    r = IvfTable("sq8", t, vectors=x).search(torch.from_numpy(q[:3]).cuda(), 10, 4, rerank).cpu().numpy()
+    assert np.array_equal(r[..., 0].view(np.uint32), ref["id"])
+    assert np.array_equal(r[..., 1].view(np.uint32), ref["distance"].view(np.uint32))
