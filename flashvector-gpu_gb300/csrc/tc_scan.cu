@@ -552,8 +552,10 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   // is unlucky (probability < 1e-7 per query); with s = 1 it always is, at
   // r = shortlist (the same accumulators, hence the same distances, are
   // behind the bound and the scan). The scan then admits only rows within it.
-  // After a sample (s > 1), queries whose bounded scan comes up short are
-  // scanned again without the bound (device-side, no host round trip).
+  // Queries whose bounded scan comes up short are scanned again without the
+  // bound (device-side, no host round trip): after a sample (s > 1), and where a
+  // range's list holds less than the shortlist (rows stored in an order that
+  // keeps a query's best together fill one range and leave the others empty).
   //
   // Automatic stride. Long rows are bound by the MMA, whose pass costs 1 / s
   // of the scan again: 64 sampled tiles. Short rows (at most two K blocks)
@@ -777,9 +779,10 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
     select<<<nq, sel_threads, sel_smem, stream>>>(s);
     note_launch();
   }
-  if (prepass && P.pstride > 1) {
-    // queries whose bound was too tight: scanned again without it (blocks
-    // holding none of them exit at once), then selected again
+  if (prepass && (P.pstride > 1 || kl < shortlist)) {
+    // queries whose bound was too tight, or whose range it admits overflowed:
+    // scanned again without it (blocks holding none of them exit at once), then
+    // selected again
     TcScanArgs f = a;
     f.qbound = nullptr;
     f.active = redo;

@@ -548,3 +548,31 @@ def test_ivf_sq8_staging_at_the_shared_memory_limit(cuda, oracle_mod, dim, reran
     r = IvfTable("sq8", t, vectors=x).search(torch.from_numpy(q[:3]).cuda(), 10, 4, rerank).cpu().numpy()
     assert np.array_equal(r[..., 0].view(np.uint32), ref["id"])
     assert np.array_equal(r[..., 1].view(np.uint32), ref["distance"].view(np.uint32))
+
+
+@pytest.mark.parametrize("precision", ["fp16", "fp8", "fp8_rows"])
+@pytest.mark.parametrize("n,dim,nq,k,overfetch,splits", [(20_000, 96, 300, 100, 0, 0), (33_000, 64, 2500, 256, 0, 0),
+                                                         (131_000, 64, 300, 100, 1, 6), (4000, 300, 70, 150, 1, 4)])
+def test_certain_bound_over_rows_in_order(cuda, precision, n, dim, nq, k, overfetch, splits):
+    """All rows near a query in one range, whose list holds fewer than the
+    answer: the query is scanned again without its bound, and the slots are
+    filled (and the overflow reported) as the scan without a bound does."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    x = torch.randn((n, dim), generator=g, device="cuda")
+    q = torch.randn((nq, dim), generator=g, device="cuda") * 0.05
+    x = x[torch.argsort(x.square().sum(1))]
+    t = _fp_table(scan, precision, x)
+    opts = scan.options(overfetch=overfetch, splits=splits)
+    search = lambda: (scan.fp16_search if precision == "fp16" else scan.fp8_search)(t, q, k, "l2", opts=opts)
+    scan.device_status()
+    with scan.tuned(tc_prepass=0):
+        ref = search()
+    status = scan.device_status()
+    got = search()
+    torch.cuda.synchronize()
+    assert scan.device_status() == status
+    assert (ref[..., 0] != -1).all()
+    assert torch.equal(got, ref)
