@@ -136,9 +136,9 @@ struct TcPlan {
   bool fp8 = false, pair = false, prepass = false;
   uint32_t elem = 0, kblocks = 0, shortlist = 0, kl = 0, kl_tmpl = 0;
   int groups = 1;  // epilogue groups of the main scan (the minima pass runs at most 2)
-  uint32_t nqb = 0, nqb_grid = 0, splits = 0, tps = 0;
-  uint32_t pstride = 0, pr = 0, psplits = 0, ptps = 0;  // minima pass: tile stride, rank of the bound, splits
-  uint32_t pgran = 0, pcount = 0;                        // columns per minimum, minima per query
+  uint32_t nqb = 0, nqb_grid = 0, splits = 0;
+  uint32_t pstride = 0, pr = 0, psplits = 0;  // minima pass: stride of its runs, rank of the bound, splits
+  uint32_t pgran = 0, pcount = 0, ptiles = 0;            // columns per minimum, minima per query, tiles
   uint32_t nq_rows = 0, slot_stride = 0;
   size_t q_bytes = 0, qn_bytes = 0, part_bytes = 0, slot_bytes = 0, tau_bytes = 0;
   size_t scratch_bytes = 0;

@@ -166,9 +166,10 @@ struct SelectArgs {
   GpuSearchResult* out;
   uint32_t* status;
   const float* tau;          // per-query admission bound of the scan (null: none)
-  uint32_t* redo;            // set for a bounded query whose shortlist came up short
+  uint32_t* redo;            // set for a bounded query with fewer than redo_below keys
   const uint32_t* only;      // process only the flagged queries (null: all)
   uint32_t* incomplete_q;    // per-query flag set when a range heap may have dropped keys (or null)
+  uint32_t redo_below;       // (<= shortlist)
 };
 
 constexpr int BAND_MAX = 64;
@@ -219,9 +220,10 @@ __global__ void __launch_bounds__(NT) tc_select_kernel(SelectArgs s) {
     set_status(s.status, kStatusOverflow);
     if (s.incomplete_q) s.incomplete_q[q] = 1u;
   }
-  // a bounded scan admitted fewer than kp rows: the bound from the sample was
-  // below the query's kp-th distance, so the query is scanned again unbounded
-  if (s.redo && threadIdx.x == 0 && keys[kp - 1] == kSentinelKey && s.tau[q] < kSentinelDist) s.redo[q] = 1u;
+  // a bounded scan kept too few rows (see plan_tc_scan): the query is scanned
+  // again unbounded
+  if (s.redo && threadIdx.x == 0 && keys[min(kp, s.redo_below) - 1] == kSentinelKey && s.tau[q] < kSentinelDist)
+    s.redo[q] = 1u;
 
   const float* qv = s.queries + (size_t)q * s.dim;
   if (s.vectors) {
@@ -421,6 +423,23 @@ bool encode_tmap(CUtensorMap* m, const void* ptr, bool fp8, uint64_t inner_elems
   return r == CUDA_SUCCESS;
 }
 
+// The base as the minima pass reads it: tile t of `tiles` holds the runs of RUN
+// rows t, t + tiles, t + 2 tiles, .. of every stride-th one (box_runs of the RUNS
+// a box); every coordinate inside the table, as RUNS RUN stride tiles <= n.
+bool encode_runs(CUtensorMap* m, const void* ptr, bool fp8, uint64_t inner_elems, uint64_t row_bytes, uint32_t stride,
+                 uint32_t tiles, uint32_t box_runs) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = tmap_encoder();
+  if (!enc) return false;
+  const cuuint64_t run_bytes = (cuuint64_t)RUN * stride * row_bytes;
+  cuuint64_t dims[4] = {inner_elems, RUN, tiles, RUNS};
+  cuuint64_t strides[3] = {row_bytes, run_bytes, run_bytes * tiles};
+  cuuint32_t box[4] = {(cuuint32_t)(fp8 ? 128 : 64), RUN, 1, box_runs};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return enc(m, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(ptr), dims,
+             strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // ---------------------------------------------------------------------------
@@ -540,7 +559,7 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   if (!opt.splits) splits = fill_waves(splits, nqb_grid, ntiles, (uint32_t)sms, groups * kl);
   // the select kernel sorts lists*kl keys in shared memory: <= 16384
   while (splits > 1 && next_pow2(splits * groups * kl) > 16384u) --splits;
-  uint32_t tps = (ntiles + splits - 1) / splits;
+  const uint32_t tps = (ntiles + splits - 1) / splits;
   splits = (ntiles + tps - 1) / tps;
 
   // Pre-pass: each query's admission bound for the scan, from the minima pass
@@ -553,9 +572,11 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   // r = shortlist (the same accumulators, hence the same distances, are
   // behind the bound and the scan). The scan then admits only rows within it.
   // Queries whose bounded scan comes up short are scanned again without the
-  // bound (device-side, no host round trip): after a sample (s > 1), and where a
-  // range's list holds less than the shortlist (rows stored in an order that
-  // keeps a query's best together fill one range and leave the others empty).
+  // bound (device-side, no host round trip). After a sample (s > 1) that is
+  // fewer keys than the shortlist, as its bound may be too tight. With s = 1
+  // keys are missing only where a range's list, which then holds less than the
+  // shortlist, filled up (rows that the base's order puts into one tile; the
+  // scan without a bound loses the same rows): fewer than k.
   //
   // Automatic stride. Long rows are bound by the MMA, whose pass costs 1 / s
   // of the scan again: 64 sampled tiles. Short rows (at most two K blocks)
@@ -575,20 +596,28 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   const uint32_t ranked = rank ? rank : shortlist;  // rows that the bound is for
   const size_t part_bytes = align_up((size_t)nq * splits * groups * kl * 8, 256);
   // The coarsest minima (fewest to store and to select from) that still number
-  // 8 r, so that two of a query's r best rows seldom share one. They live in
-  // the space of the range heaps, which are written after the bound is
-  // known: a call takes no more scratch than its unbounded scan. Where a
-  // stride's minima do not fit there, the sample is thinned until they do
-  // (4M x 96 fp8 rows, 4,000 queries, a stride of 8 asked for: 14.2 ms without
-  // a bound, 7.4 with one).
+  // 8 r, so that two of a query's r best rows seldom share one: with c minima the
+  // bound admits about -c ln(1 - r / c) rows, 1.07 r for 8 r and 1.4 r for 2 r.
+  // They live in the space of the range heaps, which are written after the bound
+  // is known: a call takes no more scratch than its unbounded scan. Where 8 r do
+  // not fit there, the most that fit down to 2 r; where those do not either, the
+  // sample is thinned until they do (4M x 96 fp8 rows, 4,000 queries, a stride of
+  // 8 asked for: 14.2 ms without a bound, 7.4 with one).
   uint32_t pgran = 0, pcount = 0, psampled = 0, pr = 0;
   while (true) {
-    psampled = (ntiles + pstride - 1) / pstride;
+    psampled = t.n / (TC_N * pstride);
     pr = std::max<uint32_t>(1u, pmargin > 0 ? (uint32_t)((pmargin * ranked + pstride - 1) / pstride)
                                             : (pstride == 1 ? ranked : poisson_rank((double)ranked / pstride, 1e-7)));
     for (uint32_t g = 128; g >= 8 && !pgran; g >>= 1) {
       const uint32_t c = psampled * (TC_N / g);
       if ((c >= 8 * pr || g == 8) && (size_t)nq * c * 4 <= part_bytes) {
+        pgran = g;
+        pcount = c;
+      }
+    }
+    for (uint32_t g = 16; g <= 128 && !pgran; g <<= 1) {
+      const uint32_t c = psampled * (TC_N / g);
+      if (c >= 2 * pr && (size_t)nq * c * 4 <= part_bytes) {
         pgran = g;
         pcount = c;
       }
@@ -599,6 +628,7 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   // off where the base is so small that the minima cannot bound (the heaps
   // then hold about every row anyway); the knob turns it off anywhere
   const bool prepass = pp_knob != 0 && pgran && pcount >= 2 * pr;
+  psampled = std::max(1u, psampled);
   uint32_t psplits = std::max<uint32_t>(1u, std::min<uint32_t>((uint32_t)sms / nqb_grid, psampled));
   psplits = fill_waves(psplits, nqb_grid, psampled, (uint32_t)sms, 0);
   const uint32_t ptps = (psampled + psplits - 1) / psplits;
@@ -625,14 +655,13 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   P.pair = pair;
   P.nqb_grid = nqb_grid;
   P.splits = splits;
-  P.tps = tps;
   P.prepass = prepass;
   P.pstride = pstride;
   P.pr = pr;
+  P.ptiles = psampled;
   P.pgran = pgran;
   P.pcount = pcount;
   P.psplits = psplits;
-  P.ptps = ptps;
   P.nq_rows = nq_rows;
   P.q_bytes = q_bytes;
   P.qn_bytes = qn_bytes;
@@ -665,7 +694,7 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
   const bool fp8 = P.fp8;
   const uint32_t elem = P.elem, kblocks = P.kblocks, shortlist = P.shortlist, kl = P.kl, kl_tmpl = P.kl_tmpl;
   const int groups = P.groups;
-  const uint32_t nqb = P.nqb, nqb_grid = P.nqb_grid, splits = P.splits, tps = P.tps;
+  const uint32_t nqb = P.nqb, nqb_grid = P.nqb_grid, splits = P.splits;
   const bool pair = P.pair, prepass = P.prepass;
   const uint32_t nq_rows = P.nq_rows, slot_stride = P.slot_stride;
   const size_t q_bytes = P.q_bytes, qn_bytes = P.qn_bytes, part_bytes = P.part_bytes;
@@ -695,10 +724,13 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
     note_launch();
   }
 
-  CUtensorMap ta, tb, tb_half;
-  if (!encode_tmap(&ta, qprep, fp8, t.padded_dim, nq_rows, (uint64_t)t.padded_dim * elem, TC_M) ||
-      !encode_tmap(&tb, t.base, fp8, t.padded_dim, t.n, (uint64_t)t.padded_dim * elem, TC_N) ||
-      (pair && !encode_tmap(&tb_half, t.base, fp8, t.padded_dim, t.n, (uint64_t)t.padded_dim * elem, TC_N / 2)))
+  const uint64_t row_bytes = (uint64_t)t.padded_dim * elem;
+  CUtensorMap ta, tb, tb_half, tb_runs;
+  if (!encode_tmap(&ta, qprep, fp8, t.padded_dim, nq_rows, row_bytes, TC_M) ||
+      !encode_tmap(&tb, t.base, fp8, t.padded_dim, t.n, row_bytes, TC_N) ||
+      (pair && !encode_tmap(&tb_half, t.base, fp8, t.padded_dim, t.n, row_bytes, TC_N / 2)) ||
+      (prepass && !encode_runs(&tb_runs, t.base, fp8, t.padded_dim, row_bytes, P.pstride, P.ptiles,
+                               pair ? RUNS / 2 : RUNS)))
     return FV_ERR_ARG;
 
   TcScanArgs a{};
@@ -715,7 +747,6 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
   a.tslot_stride = slot_stride;
   a.status = status_word();
   a.filters = filters;
-  a.tile_stride = 1;
   // "tc.wait_limit_ns" (0: 2 s) bounds the pipeline's waits; a wait that runs
   // out ends the scan early and is reported through the status word
   const int64_t wl = tune_value("tc.wait_limit_ns", 0);
@@ -727,7 +758,7 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
     ProfScope ps(name, stream);
     const int g = use_pair ? -1 : groups_n;
     const uint32_t grid = (use_pair ? nqb_grid : nqb) * splits_n;
-    const CUtensorMap& b = use_pair ? tb_half : tb;
+    const CUtensorMap& b = kl_t == kMinima ? tb_runs : use_pair ? tb_half : tb;
     return fp8 ? dispatch_tc_scan_fp8(kl_t, g, (int)metric, t.fp8_table_scale, ta, b, args, grid, stream)
                : dispatch_tc_scan_fp16(kl_t, g, (int)metric, true, ta, b, args, grid, stream);
   };
@@ -735,8 +766,7 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
   if (prepass) {
     TcScanArgs p = a;
     p.splits = P.psplits;
-    p.tiles_per_split = P.ptps;
-    p.tile_stride = P.pstride;
+    p.run_stride = P.pstride;
     p.pmin = reinterpret_cast<float*>(partial);
     p.pm_stride = P.pcount;
     p.gran = P.pgran;
@@ -749,7 +779,6 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
     }
   }
   a.splits = splits;
-  a.tiles_per_split = tps;
   a.partial = partial;
   a.kl = kl;
   a.share = (kl == shortlist && !prepass) ? 1u : 0u;
@@ -768,6 +797,7 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
   SelectArgs s{partial, splits * groups, kl, sel_keys, shortlist, k, queries, t.vectors, t.dim,
                (int)metric,
                opt.boundary_fp64 ? 1u : 0u, 0.f, out, status_word(), tau, redo, nullptr, incomplete_q};
+  s.redo_below = P.pstride > 1 ? shortlist : k;
   s.eps = opt.boundary_eps > 0.f ? opt.boundary_eps : (float)((t.dim + 31) / 32 + 5) * 2.0f * 5.960464477539063e-08f;
   size_t sel_smem = (size_t)sel_keys * 8;
   const int sel_threads = nq <= 2u * (uint32_t)device_sm_count() ? 1024 : 256;
@@ -825,10 +855,11 @@ int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream) {
   c.lists = P.splits * P.groups;
   c.kl = P.kl;
   const uint64_t row_bytes = (uint64_t)c.padded_dim * 2;
-  CUtensorMap ta, tb, tb_half;
+  CUtensorMap ta, tb, tb_half, tb_runs;
   if (!encode_tmap(&ta, c.q16, false, c.padded_dim, P.nq_rows, row_bytes, TC_M) ||
       !encode_tmap(&tb, c.rows16, false, c.padded_dim, c.n, row_bytes, TC_N) ||
-      (P.pair && !encode_tmap(&tb_half, c.rows16, false, c.padded_dim, c.n, row_bytes, TC_N / 2)))
+      (P.pair && !encode_tmap(&tb_half, c.rows16, false, c.padded_dim, c.n, row_bytes, TC_N / 2)) ||
+      !encode_runs(&tb_runs, c.rows16, false, c.padded_dim, row_bytes, P.pstride, P.ptiles, P.pair ? RUNS / 2 : RUNS))
     return FV_ERR_ARG;
   TcScanArgs a{};
   a.n = c.n;
@@ -844,13 +875,13 @@ int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream) {
   a.wait_ns = wl > 0 ? (uint64_t)wl : 2000000000ull;
   auto scan = [&](const TcScanArgs& args, int kl_t, uint32_t splits_n, const char* name) -> cudaError_t {
     ProfScope ps(name, stream);
-    return dispatch_tc_scan_fp16(kl_t, P.pair ? -1 : P.groups, METRIC_L2, true, ta, P.pair ? tb_half : tb, args,
+    return dispatch_tc_scan_fp16(kl_t, P.pair ? -1 : P.groups, METRIC_L2, true, ta,
+                                 kl_t == kMinima ? tb_runs : P.pair ? tb_half : tb, args,
                                  (P.pair ? P.nqb_grid : P.nqb) * splits_n, stream);
   };
   TcScanArgs p = a;
   p.splits = P.psplits;
-  p.tiles_per_split = P.ptps;
-  p.tile_stride = P.pstride;
+  p.run_stride = P.pstride;
   p.pmin = reinterpret_cast<float*>(c.partial);
   p.pm_stride = P.pcount;
   p.gran = P.pgran;
@@ -863,8 +894,6 @@ int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream) {
     note_launch();
   }
   a.splits = P.splits;
-  a.tiles_per_split = P.tps;
-  a.tile_stride = 1;
   a.partial = c.partial;
   a.kl = P.kl;
   a.qbound = c.bound;

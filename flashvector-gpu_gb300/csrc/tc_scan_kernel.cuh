@@ -39,6 +39,8 @@ namespace fv {
 
 constexpr int TC_M = 128;                  // queries per CTA (TMEM lanes)
 constexpr int TC_N = 256;                  // base rows per tile (MMA N)
+constexpr int RUN = 8;                     // consecutive rows of a minima-pass tile
+constexpr int RUNS = TC_N / RUN;           // runs of a minima-pass tile
 constexpr int KB_BYTES = 128;              // K bytes per stage row (one 128B swizzle atom)
 constexpr int A_STAGE = TC_M * KB_BYTES;   // 16 KB
 constexpr int B_STAGE = TC_N * KB_BYTES;   // 32 KB
@@ -48,7 +50,7 @@ constexpr int B_STAGE = TC_N * KB_BYTES;   // 32 KB
 __host__ __device__ constexpr int scan_threads(int G) { return 64 + 128 * G; }
 
 struct TcScanArgs {
-  uint32_t n, nq, kblocks, nqb, splits, tiles_per_split;
+  uint32_t n, nq, kblocks, nqb, splits;
   const float* xnorm;    // [n] ||x||^2 of the fp32 rows (L2, cosine)
   const float* xscale;   // [n] per-row fp8 scale (FP8 only)
   const float* qnorm;    // [nq] ||q||^2
@@ -64,10 +66,11 @@ struct TcScanArgs {
   const float* qbound;         // per-query admission bound (distance), or null
   const uint32_t* active;      // per-query flags: only flagged queries are scanned (null: all)
   float floor;                 // L2: lower limit of a distance (0, or -inf for a ranking value that may be negative)
-  uint32_t tile_stride;        // scan every tile_stride-th 256-row tile (a sample when > 1)
   uint64_t wait_ns;            // limit of the pipeline's waits (the drains keep their own)
-  // minima pass only: the smallest distance of every `gran` consecutive
-  // scanned columns (8, 16, 32, 64 or 128), [nq][pm_stride], column order
+  // minima pass only (PASS_MIN): scans every run_stride-th run of RUN rows (a
+  // sample when > 1), 256 / RUN runs to a tile; the smallest distance of `gran`
+  // columns (8, 16, 32, 64 or 128), [nq][pm_stride], in tile order
+  uint32_t run_stride;
   float* pmin;
   uint32_t pm_stride, gran;
 };
@@ -190,7 +193,14 @@ static __device__ __forceinline__ float select32(const float* v, int j) {
 // `gran` columns and stores those, so its cost per tile is the minimum tree
 // alone and the freed shared memory holds a deeper ring. The r-th smallest
 // of a query's minima is >= the r-th smallest distance scanned (minima of
-// disjoint columns are distances of distinct rows), so it bounds from above.
+// disjoint columns are distances of distinct rows), so it bounds from above. It
+// is a tight bound while the r best rows lie in nearly as many minima, and bases
+// are often stored in an order that keeps a query's best rows together. So a
+// tile is 32 runs of 8 rows, spread evenly over the base (whole sectors of norms
+// and bytes of masks still), and a minimum of 8 or 16 columns takes one row of
+// each run. (Tiles of 256 consecutive rows and minima of consecutive columns:
+// 1,000,000 x 96 fp16 stored by cluster, 500 queries, L2, k 10: 1,235 us a call,
+// 523 with the runs.)
 // Keeping the sample's best r keys in heaps instead spent the pass filling
 // them: 123 us for 1/32 of a 1M x 768 scan of 1,024 queries.
 template <bool FP8, int KL, int STAGES, int METRIC, int G, bool PAIR, bool TS, int PASS>
@@ -237,12 +247,14 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     }
     if (!__syncthreads_or(any)) return;
   }
-  const uint32_t tstride = a.tile_stride ? a.tile_stride : 1u;
   constexpr bool col_split = G >= 2;
-  const uint32_t ntiles = ((a.n + TC_N - 1) / TC_N + tstride - 1) / tstride;
-  const uint32_t t_begin = split * a.tiles_per_split;
-  const uint32_t t_end = min(t_begin + a.tiles_per_split, ntiles);
-  const uint32_t my_tiles = t_end > t_begin ? t_end - t_begin : 0;
+  const uint32_t ntiles = MINP ? a.n / (TC_N * a.run_stride) : (a.n + TC_N - 1) / TC_N;
+  // A range is every splits-th tile, so that rows which a base's order keeps
+  // together are shared out over the ranges, their lists and their threads. (1M x
+  // 96 as above: 523 us a call with ranges of consecutive tiles, 274 like this;
+  // 200,000 x 768 by cluster, 512 queries, k 100: 2,204, and three quarters of
+  // the best 100 found, to 802 and all of them.)
+  const uint32_t my_tiles = split < ntiles ? (ntiles - split - 1) / a.splits + 1 : 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -290,7 +302,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
       for (int s = 0; s < STAGES; ++s) issued_parity[s] = -1;
       bool ok = true;
       for (uint32_t i = 0; ok && i < my_tiles; ++i) {
-        const int32_t row_b = (int32_t)((t_begin + i) * tstride * TC_N);
+        const int32_t tile_b = (int32_t)(split + i * a.splits), row_b = tile_b * TC_N;
         for (uint32_t kb = 0; kb < a.kblocks; ++kb) {
           if (!tc::mbar_wait(&empty[stage], phase ^ 1, abort_flag, a.status, a.wait_ns)) {
             ok = false;
@@ -301,15 +313,22 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
             if (rank == 0) tc::mbar_arrive_expect_tx(&full[stage], 2 * (A_STAGE + b_stage));
             tc::tma_load_2d_pair(sA + stage * A_STAGE, &tmA, fb, (int32_t)(kb * kb_elems), (int32_t)(qb * TC_M),
                                  pol_a);
-            tc::tma_load_2d_pair(sB + stage * b_stage, &tmB, fb, (int32_t)(kb * kb_elems),
-                                 row_b + (int32_t)(rank * (TC_N / 2)), pol_b);
+            if constexpr (MINP)
+              tc::tma_load_4d_pair(sB + stage * b_stage, &tmB, fb, (int32_t)(kb * kb_elems), 0, tile_b,
+                                   (int32_t)(rank * (RUNS / 2)), pol_b);
+            else
+              tc::tma_load_2d_pair(sB + stage * b_stage, &tmB, fb, (int32_t)(kb * kb_elems),
+                                   row_b + (int32_t)(rank * (TC_N / 2)), pol_b);
           } else {
             const bool load_a = !a_resident || i == 0;
             tc::mbar_arrive_expect_tx(&full[stage], (load_a ? A_STAGE : 0) + B_STAGE);
             if (load_a)
               tc::tma_load_2d(sA + (a_resident ? kb : stage) * A_STAGE, &tmA, &full[stage], (int32_t)(kb * kb_elems),
                               (int32_t)(qb * TC_M), pol_a);
-            tc::tma_load_2d(sB + stage * B_STAGE, &tmB, &full[stage], (int32_t)(kb * kb_elems), row_b, pol_b);
+            if constexpr (MINP)
+              tc::tma_load_4d(sB + stage * B_STAGE, &tmB, &full[stage], (int32_t)(kb * kb_elems), 0, tile_b, 0, pol_b);
+            else
+              tc::tma_load_2d(sB + stage * B_STAGE, &tmB, &full[stage], (int32_t)(kb * kb_elems), row_b, pol_b);
           }
           issued_parity[stage] = (int32_t)phase;
           if (++stage == STAGES) {
@@ -484,15 +503,17 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     // otherwise schedules the two steps of the column loop worse: 4M x 96,
     // 4,000 queries, L2: 7.42 ms, 6.59 like this)
     const int c_lo = col_split ? grp * (TC_N / G) : 0;
-    const bool whole = FP8 && !TS && a.tile_stride > 1u << 30;  // (never)
+    const bool whole = FP8 && !TS && a.nqb > 1u << 30;  // (never)
     const int c_hi = col_split && !whole ? c_lo + TC_N / G : TC_N;
     float pre_n[TC_N / 32], pre_s[TC_N / 32];
     uint32_t pre_m = 0;
+    // minima pass: the first row of run r of a tile
+    auto run_row = [&](uint32_t tile, uint32_t r) { return RUN * a.run_stride * (tile + r * ntiles); };
     auto prefetch = [&](uint32_t tile) {
-      const uint32_t v0n = (t_begin + tile) * tstride * TC_N;
+      const uint32_t v0n = tile * TC_N;
 #pragma unroll
       for (int r = 0; r < TC_N / 32; ++r) {
-        const uint32_t slot = v0n + lane + 32 * r;
+        const uint32_t slot = MINP ? run_row(tile, (lane + 32 * r) / RUN) + lane % RUN : v0n + lane + 32 * r;
         const bool in = slot < a.n && 32 * r >= c_lo && 32 * r < c_hi;
         pre_n[r] = (METRIC != METRIC_INNER_PRODUCT && !fused && in) ? __ldg(a.xnorm + slot) : 0.f;
         // per-column factor of the scaled dot: -2 xs (L2), -xs (IP), xs
@@ -501,7 +522,17 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
         pre_s[r] = METRIC == METRIC_L2 ? -2.0f * xs : (METRIC == METRIC_INNER_PRODUCT ? -xs : xs);
       }
       pre_m = 0;
-      if (lane < 8) {
+      if (MINP && lane < 8) {
+        pre_m = 0xFFFFFFFFu;
+        if (a.mask) {
+          pre_m = 0;
+#pragma unroll
+          for (int b = 0; b < 32 / RUN; ++b) {
+            const uint32_t row = run_row(tile, 32 / RUN * lane + b);
+            pre_m |= ((__ldg(a.mask + (row >> 5)) >> (row & 31u)) & 0xFFu) << (RUN * b);
+          }
+        }
+      } else if (lane < 8) {
         const uint32_t c0 = v0n + lane * 32;
         if (c0 < a.n) {
           const uint32_t cnt = min(32u, a.n - c0);
@@ -510,10 +541,11 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
         }
       }
     };
-    if (my_tiles) prefetch(0);
-    for (uint32_t i = 0; i < my_tiles; ++i) {
+    if (my_tiles) prefetch(split);
+    uint32_t tile = split;
+    for (uint32_t i = 0; i < my_tiles; ++i, tile += a.splits) {
       const uint32_t buf = i & 1, use = i >> 1;
-      const uint32_t v0 = (t_begin + i) * tstride * TC_N;
+      const uint32_t v0 = tile * TC_N;
       __syncwarp();
       [[maybe_unused]] float least = INFINITY, most = 0.f;  // cosine: the squared norms of the tile's rows
 #pragma unroll
@@ -523,7 +555,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
         if (FP8 && !fused) cb[TC_N + lane + 32 * r] = pre_s[r];
         if (METRIC == METRIC_COSINE) {
           cf[lane + 32 * r] = -rsqrtf(pre_n[r]) * (FP8 ? pre_s[r] : 1.f);
-          if (v0 + lane + 32 * r < a.n) {
+          if (MINP || v0 + lane + 32 * r < a.n) {
             least = fminf(least, pre_n[r]);
             most = fmaxf(most, pre_n[r]);
           }
@@ -540,7 +572,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
       }
       if (lane < 8) cm[lane] = pre_m;
       __syncwarp();
-      if (i + 1 < my_tiles) prefetch(i + 1);
+      if (i + 1 < my_tiles) prefetch(tile + a.splits);
       // the shared bound, loaded before the accumulator wait hides its latency
       uint32_t smax = 0;
       if (slots)
@@ -624,7 +656,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
         chunk32(ra, col, ma);
         chunk32(rb, 128u + col, mb);
       } else {
-        [[maybe_unused]] float best128 = 0.f;
+        [[maybe_unused]] float m[8];  // minima pass: of 128 columns (64 where gran is 8)
 #pragma unroll 1
         for (int c0 = c_lo; c0 < c_hi; c0 += 64) {
           uint32_t ra[32], rb[32];
@@ -633,8 +665,18 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
           tc::tmem_ld32_async(t_row + c0 + 32, rb);
           uint64_t mw = qvalid ? ((uint64_t)cm[(c0 >> 5) + 1] << 32 | cm[c0 >> 5]) : 0ull;
           if (qf.words) {
-            const uint32_t w0 = (v0 + (uint32_t)c0) >> 5;
-            mw &= ((uint64_t)filter_word(qf, w0 + 1) << 32) | filter_word(qf, w0);
+            uint64_t fw = 0;
+            if constexpr (MINP) {
+#pragma unroll
+              for (int b = 0; b < 64 / RUN; ++b) {
+                const uint32_t row = run_row(tile, c0 / RUN + b);
+                fw |= (uint64_t)((filter_word(qf, row >> 5) >> (row & 31u)) & 0xFFu) << (RUN * b);
+              }
+            } else {
+              const uint32_t w0 = (v0 + (uint32_t)c0) >> 5;
+              fw = ((uint64_t)filter_word(qf, w0 + 1) << 32) | filter_word(qf, w0);
+            }
+            mw &= fw;
           }
           tc::tmem_wait_ld(ra);
           tc::reg_fence(rb);
@@ -716,48 +758,40 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
               return d;
             };
             if constexpr (MINP) {
-              // the smallest distance of every 8 columns (none where the mask
-              // admits none), then of every `gran`
+              // the smallest distance of 8 columns, one of each run (none where the
+              // mask admits none), then of `gran`: with the other 64 columns' runs
+              // first, then of neighbours in a run. Columns whose product is NaN (an
+              // fp16 row that overflowed times a zero, a NaN row) drop out of a
+              // minimum: what starts it is no distance, not L2's floor.
               const float none = FU ? -INFINITY : INFINITY;
               if (mw != ~0ull) {
 #pragma unroll
                 for (int j = 0; j < 64; ++j) v[j] = ((mw >> j) & 1ull) ? v[j] : none;
               }
-              float m[8];
+              if (a.gran == 8 || (c0 & 64) == 0) {
 #pragma unroll
-              for (int b = 0; b < 8; ++b) {
-                const float* w = v + 8 * b;
-                m[b] = best3(best3(w[0], w[1], w[2]), best3(w[3], w[4], w[5]), better(w[6], w[7]));
+                for (int j = 0; j < 8; ++j) m[j] = none;
               }
-              if (!qvalid) return;
-              // The minimum of columns that are all NaN (an fp16 row that overflowed
-              // times a zero, a NaN row) is NaN, whose D would be L2's floor: such
-              // columns hold no distance.
-              auto M = [&](float x) { return x == x ? D(x) : INFINITY; };
-              float* dst = a.pmin + (size_t)q * a.pm_stride;
-              const uint32_t at = (t_begin + i) * TC_N + (uint32_t)c0;  // scanned column
-              if (a.gran == 8) {
-                float4* o = reinterpret_cast<float4*>(dst + at / 8);
-                o[0] = make_float4(M(m[0]), M(m[1]), M(m[2]), M(m[3]));
-                o[1] = make_float4(M(m[4]), M(m[5]), M(m[6]), M(m[7]));
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                m[j] = best3(best3(v[j], v[j + 8], v[j + 16]), best3(v[j + 24], v[j + 32], v[j + 40]),
+                             best3(v[j + 48], v[j + 56], m[j]));
+              if (!qvalid || (a.gran != 8 && (c0 & 64) == 0)) return;
+              const uint32_t at = tile * TC_N + (uint32_t)c0;  // scanned column
+              float* o = a.pmin + (size_t)q * a.pm_stride + (a.gran == 8 ? at : at & ~127u) / a.gran;
+              if (a.gran <= 16) {
+                reinterpret_cast<float4*>(o)[0] = make_float4(D(m[0]), D(m[1]), D(m[2]), D(m[3]));
+                reinterpret_cast<float4*>(o)[1] = make_float4(D(m[4]), D(m[5]), D(m[6]), D(m[7]));
                 return;
               }
-              const float p0 = better(m[0], m[1]), p1 = better(m[2], m[3]), p2 = better(m[4], m[5]),
-                          p3 = better(m[6], m[7]);
-              if (a.gran == 16) {
-                *reinterpret_cast<float4*>(dst + at / 16) = make_float4(M(p0), M(p1), M(p2), M(p3));
-                return;
-              }
-              const float h0 = better(p0, p1), h1 = better(p2, p3), all = better(h0, h1);
-              if (a.gran == 32) {
-                *reinterpret_cast<float2*>(dst + at / 32) = make_float2(M(h0), M(h1));
-              } else if (a.gran == 64) {
-                dst[at / 64] = M(all);
-              } else if ((c0 & 64) == 0) {
-                best128 = all;
-              } else {
-                dst[at / 128] = M(better(best128, all));
-              }
+              const float p0 = better(m[0], m[4]), p1 = better(m[1], m[5]), p2 = better(m[2], m[6]),
+                          p3 = better(m[3], m[7]);
+              if (a.gran == 32)
+                *reinterpret_cast<float4*>(o) = make_float4(D(p0), D(p1), D(p2), D(p3));
+              else if (a.gran == 64)
+                *reinterpret_cast<float2*>(o) = make_float2(D(better(p0, p2)), D(better(p1, p3)));
+              else
+                *o = D(better(better(p0, p2), better(p1, p3)));
               return;
             } else {
             float r[22], s8[8];

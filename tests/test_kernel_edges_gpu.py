@@ -576,3 +576,54 @@ def test_certain_bound_over_rows_in_order(cuda, precision, n, dim, nq, k, overfe
     assert scan.device_status() == status
     assert (ref[..., 0] != -1).all()
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("metric", ["l2", "ip", "cosine"])
+@pytest.mark.parametrize("n,dim,nq,k,clusters", [(255, 64, 9, 1, 3), (257, 64, 9, 1, 3), (2047, 32, 140, 3, 11),
+                                                 (20_001, 96, 64, 10, 50), (70_003, 300, 130, 10, 90),
+                                                 (400_010, 40, 200, 12, 200)])
+@pytest.mark.parametrize("precision,masked", [("fp16", False), ("fp16", True), ("fp8", True), ("fp8_rows", True)])
+def test_bounded_scan_of_rows_in_clusters(cuda, metric, n, dim, nq, k, clusters, precision, masked):
+    """Rows stored by cluster: the bound's sample (runs of 8 rows spread over the
+    base, partial last tiles, bases of less than one tile) and the ranges (every
+    so many tiles) give the answer of the scan without a bound."""
+    from fvgb300 import datasets, scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(n + dim)
+    c = torch.randn((clusters, dim), generator=g, device="cuda")
+    own = torch.randint(0, clusters, (n,), generator=g, device="cuda").sort().values
+    x = torch.randn((n, dim), generator=g, device="cuda") * 0.3 + c[own]
+    q = torch.randn((nq, dim), generator=g, device="cuda") * 0.3 + c[torch.arange(nq, device="cuda") % clusters]
+    t = _fp_table(scan, precision, x)
+    search = scan.fp16_search if precision == "fp16" else scan.fp8_search
+    mask = torch.from_numpy(datasets.bernoulli_mask_words(n, 0.3, 7).view(np.int32)).cuda() if masked else None
+    scan.device_status()
+    with scan.tuned(tc_prepass=0):
+        ref = search(t, q, k, metric, mask=mask)
+    got = search(t, q, k, metric, mask=mask)
+    torch.cuda.synchronize()
+    assert scan.device_status() == 0
+    assert torch.equal(got, ref)
+
+
+def test_select_with_more_keys_than_foreseen_by_runs(cuda):
+    """The sampled runs (every 32nd run of 8 rows) hold only far rows, so the
+    bound admits nearly every row: full range lists, and a selection that falls
+    back to their k-th key, same answer."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(3)
+    n = 64 * 32 * 256 + 77
+    x = torch.randn((n, 32), generator=g, device="cuda")
+    x[(torch.arange(n, device="cuda") // 8) % 32 == 0] *= 100.0
+    q = torch.randn((130, 32), generator=g, device="cuda")
+    t = scan.Fp16Table(x)
+    with scan.tuned(tc_prepass=0):
+        ref = scan.fp16_search(t, q, 10, "l2")
+    with scan.tuned(tc_prepass_stride=32):
+        got = scan.fp16_search(t, q, 10, "l2")
+    torch.cuda.synchronize()
+    assert scan.device_status() == 0
+    assert torch.equal(got, ref)
