@@ -472,6 +472,15 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     constexpr float kCosPad = 4e-6f;
     const float q_over = METRIC == METRIC_COSINE ? sqrtf(qn) / (FP8 ? qs : 1.f) : 1.f;
     const float q_inv = METRIC == METRIC_COSINE ? __fdiv_rn(1.f, q_over) : 1.f;
+    // the range of the warp's squared query norms
+    [[maybe_unused]] float q_least = qvalid ? qn : INFINITY, q_most = qvalid ? qn : 0.f;
+    if (METRIC == METRIC_COSINE) {
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        q_least = fminf(q_least, __shfl_xor_sync(0xffffffffu, q_least, o));
+        q_most = fmaxf(q_most, __shfl_xor_sync(0xffffffffu, q_most, o));
+      }
+    }
     // (A bound of -inf, where products overflowed, admits the rows at -inf: the
     // thresholds stay finite, or their slack would make them NaN.)
     constexpr float kLowest = -3.402823466e38f;
@@ -547,7 +556,7 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
       const uint32_t buf = i & 1, use = i >> 1;
       const uint32_t v0 = tile * TC_N;
       __syncwarp();
-      [[maybe_unused]] float least = INFINITY, most = 0.f;  // cosine: the squared norms of the tile's rows
+      [[maybe_unused]] bool by_factor = true;  // cosine: all norms of the tile allow it
 #pragma unroll
       for (int r = 0; r < TC_N / 32; ++r) {
         if (32 * r < c_lo || 32 * r >= c_hi) continue;
@@ -555,21 +564,12 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
         if (FP8 && !fused) cb[TC_N + lane + 32 * r] = pre_s[r];
         if (METRIC == METRIC_COSINE) {
           cf[lane + 32 * r] = -rsqrtf(pre_n[r]) * (FP8 ? pre_s[r] : 1.f);
-          if (MINP || v0 + lane + 32 * r < a.n) {
-            least = fminf(least, pre_n[r]);
-            most = fmaxf(most, pre_n[r]);
-          }
+          // (a NaN passes: it has no distance either way)
+          if (MINP || v0 + lane + 32 * r < a.n)
+            by_factor = by_factor && !(pre_n[r] * q_least < 1e-4f) && !(pre_n[r] * q_most >= 1e38f);
         }
       }
-      [[maybe_unused]] bool by_factor = false;
-      if (METRIC == METRIC_COSINE) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-          least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
-          most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
-        }
-        by_factor = __all_sync(0xffffffffu, !qvalid || (qn * least >= 1e-4f && qn * most < 1e38f));
-      }
+      if (METRIC == METRIC_COSINE) by_factor = __all_sync(0xffffffffu, by_factor);
       if (lane < 8) cm[lane] = pre_m;
       __syncwarp();
       if (i + 1 < my_tiles) prefetch(tile + a.splits);
