@@ -26,7 +26,11 @@
 //     k-th exact distance among the collected rows is below B the collected
 //     rows hold the answer. A query that fails this test, or whose values
 //     leave fp16's range, is flagged, and the plain scan answers it; so are
-//     all of a call one of whose passes gave up a wait.
+//     all of a call one of whose passes gave up a wait;
+//   * a row that leaves fp16's range, or is not finite, has no such bound: it
+//     gets zero codes, no part in the minima and a = -inf in the scan, so that
+//     every query collects it. (One such row in 100,000 x 128 x 1,000 used to
+//     flag every query: 1,698 us, plain scan 1,612; now 173.)
 //
 // Measured: 100,000 x 128 x 1,000, k 10: 1,592 -> 160 us (encoding 37, minima
 // pass 37, scan 50, finish 15); 200,000 x 512 x 100: 1,131 -> 263 us. Bounded
@@ -55,7 +59,7 @@ constexpr float kMaxNorm = 3.0e4f;   // of a scaled row or query: no fp16 value 
 constexpr float kUnit = 256.f;       // norm of a scaled unit vector (cosine)
 
 // words of the call's shared state
-enum { W_MAX_NORM = 0, W_MIN_NORM = 1, W_STATUS = 2, W_COUNT = 3 };  // W_STATUS: status bits of the scans
+enum { W_MIN_NORM = 0, W_STATUS = 1, W_COUNT = 2 };  // smallest row norm (cosine), status bits of the scans
 
 struct QueryInfo {
   float to_a;    // A = to_a * distance (cosine: to_a * (distance - 1))
@@ -65,7 +69,8 @@ struct QueryInfo {
 };
 
 // mu[d] and the variance about it (inner product, cosine: 0 and the mean
-// square), over up to 256 evenly spaced rows. A block owns 32 dimensions.
+// square), over up to 256 evenly spaced rows (values that are not finite left
+// out: any centre and scale will do). A block owns 32 dimensions.
 __global__ void __launch_bounds__(32 * CEN_GROUPS) flat_tc_center_kernel(const float* __restrict__ x, uint32_t n,
                                                                          uint32_t dim, int metric,
                                                                          float* __restrict__ mu,
@@ -76,7 +81,6 @@ __global__ void __launch_bounds__(32 * CEN_GROUPS) flat_tc_center_kernel(const f
   const uint32_t d = blockIdx.x * 32 + lane;
   const uint32_t s = min(n, SAMPLE);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    words[W_MAX_NORM] = 0u;
     words[W_MIN_NORM] = 0x7f800000u;  // +inf
     words[W_STATUS] = 0u;
   }
@@ -93,7 +97,10 @@ __global__ void __launch_bounds__(32 * CEN_GROUPS) flat_tc_center_kernel(const f
   if (metric == METRIC_L2) {
     if (d < dim) {
 #pragma unroll 8
-      for (uint32_t i = g; i < s; i += CEN_GROUPS) acc += __ldg(x + (size_t)((uint64_t)i * n / s) * dim + d);
+      for (uint32_t i = g; i < s; i += CEN_GROUPS) {
+        const float v = __ldg(x + (size_t)((uint64_t)i * n / s) * dim + d);
+        acc += fabsf(v) < INFINITY ? v : 0.f;
+      }
     }
     m = total(acc) / (float)s;
   }
@@ -102,7 +109,7 @@ __global__ void __launch_bounds__(32 * CEN_GROUPS) flat_tc_center_kernel(const f
 #pragma unroll 8
     for (uint32_t i = g; i < s; i += CEN_GROUPS) {
       const float v = __ldg(x + (size_t)((uint64_t)i * n / s) * dim + d) - m;
-      acc = fmaf(v, v, acc);
+      acc = fabsf(v) < INFINITY ? fmaf(v, v, acc) : acc;
     }
   }
   acc = total(acc) / (float)s;
@@ -128,9 +135,11 @@ struct PrepArgs {
   const float* var;
   __half* x16;
   __half* q16;
-  float* xnorm;
+  float* xnorm;       // of the scan: -inf for a row out of range
+  float* xnorm_min;   // of the minima pass: inf there
   float* qnorm;
   QueryInfo* info;
+  const uint32_t* mask;
   uint32_t* words;
 };
 
@@ -157,10 +166,9 @@ __global__ void __launch_bounds__(32 * PREP_WARPS) flat_tc_prep_kernel(PrepArgs 
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     s = scale_for(sqrtf(v));
   }
-  // largest scaled norm and smallest row norm (cosine) of the warp's rows: one
-  // atomic a warp, and only where it moves the word (an atomic per row on two
-  // words took 80 us for 100,000 rows)
-  uint32_t w_max = 0u, w_min = 0x7f800000u;
+  // smallest row norm (cosine) of the warp's rows: one atomic a warp, and only
+  // where it moves the word (an atomic per row took 40 us for 100,000 rows)
+  uint32_t w_min = 0x7f800000u;
   constexpr uint64_t WARP_ROWS = (uint64_t)R * (32 / LPR);
   for (uint64_t wb = ((uint64_t)blockIdx.x * PREP_WARPS + (threadIdx.x >> 5)) * WARP_ROWS; wb < rows;
        wb += (uint64_t)gridDim.x * PREP_WARPS * WARP_ROWS) {
@@ -263,10 +271,11 @@ __global__ void __launch_bounds__(32 * PREP_WARPS) flat_tc_prep_kernel(PrepArgs 
 #pragma unroll
     for (uint32_t i = 0; i < R; ++i) {
       const float nn = group_sum(n2[i]);
-      if (sub || !src[i]) continue;
+      if (!src[i]) continue;
       const uint64_t w = w0 + i;
       const float low = a.metric == METRIC_L2 ? nn - a.e * nn : -a.e * nn;
       if (w >= a.n) {
+        if (sub) continue;
         const uint64_t r = w - a.n;
         a.qnorm[r] = low;
         QueryInfo inf;
@@ -276,20 +285,25 @@ __global__ void __launch_bounds__(32 * PREP_WARPS) flat_tc_prep_kernel(PrepArgs 
         inf.scaled = odd[i] ? INFINITY : sqrtf(nn);
         inf.pad = 0.f;
         a.info[r] = inf;
-      } else {
-        a.xnorm[w] = low - a.e_abs;
-        // (NaN orders above every number)
-        w_max = max(w_max, odd[i] ? 0x7f800000u : __float_as_uint(sqrtf(nn)) & 0x7fffffffu);
-        if (a.metric == METRIC_COSINE && norm[i] > 0.f) w_min = min(w_min, __float_as_uint(norm[i]));
+        continue;
       }
+      const bool out = odd[i] || !(sqrtf(nn) < kMaxNorm);
+      if (out) {
+        // (each lane over what it wrote)
+        for (uint32_t d = E * sub; d < a.pd; d += E * LPR) {
+#pragma unroll
+          for (int e = 0; e < E; ++e) a.x16[w * a.pd + d + e] = __float2half_rn(0.f);
+        }
+      }
+      if (sub) continue;
+      a.xnorm[w] = out ? -INFINITY : low - a.e_abs;
+      a.xnorm_min[w] = out ? INFINITY : low - a.e_abs;
+      if (a.metric == METRIC_COSINE && !out && norm[i] > 0.f && mask_allows(a.mask, (uint32_t)w))
+        w_min = min(w_min, __float_as_uint(norm[i]));
     }
   }
-  w_max = __reduce_max_sync(0xffffffffu, w_max);
   w_min = __reduce_min_sync(0xffffffffu, w_min);
-  if (lane == 0) {
-    if (w_max > __ldcg(a.words + W_MAX_NORM)) atomicMax(a.words + W_MAX_NORM, w_max);
-    if (w_min < __ldcg(a.words + W_MIN_NORM)) atomicMin(a.words + W_MIN_NORM, w_min);
-  }
+  if (lane == 0 && w_min < __ldcg(a.words + W_MIN_NORM)) atomicMin(a.words + W_MIN_NORM, w_min);
 }
 
 // The plain scan's distance of one row (flat_f32_scan_kernel): separately
@@ -398,7 +412,7 @@ __global__ void __launch_bounds__(FIN_THREADS) flat_tc_finish_kernel(FinishArgs 
     const QueryInfo inf = a.info[q];
     const float low = order_float(s_low);
     // (a pass that gave up a wait has not seen every row)
-    bool ok = a.words[W_STATUS] == 0u && __uint_as_float(a.words[W_MAX_NORM]) < kMaxNorm && inf.scaled < kMaxNorm;
+    bool ok = a.words[W_STATUS] == 0u && inf.scaled < kMaxNorm;
     if (METRIC == METRIC_COSINE) ok = ok && inf.norm * __uint_as_float(a.words[W_MIN_NORM]) > 8.2e-5f;
     if (ok && low < kSentinelDist) {  // else every admissible row was collected
       const uint64_t kth = keys[a.k - 1];
@@ -411,8 +425,6 @@ __global__ void __launch_bounds__(FIN_THREADS) flat_tc_finish_kernel(FinishArgs 
   }
 }
 
-size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
-
 // e of the file comment.
 float error_bound(uint32_t dim, MetricType metric) {
   const double d = dim, sub = std::ldexp(std::sqrt(d), -24);
@@ -420,7 +432,7 @@ float error_bound(uint32_t dim, MetricType metric) {
   return (float)(std::ldexp(1.0, -10) + 1.25 * std::ldexp(d, -22) + std::ldexp(1.0, -20) + sub);
 }
 
-// Pairs x dimensions from which the filter is the faster way: below, its nine
+// Pairs x dimensions from which the filter is the faster way: below, its eight
 // launches and the encoding outweigh the arithmetic that it saves (50,000 x 64
 // x 32: 70 against 54 us; 20,000 x 64 x 100, 1.3e8: 68 against 88).
 constexpr uint64_t kFlatTcWork = 120000000ull;
@@ -472,6 +484,7 @@ FlatTcPlan plan_flat_tc(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, Metri
   };
   P.x16 = take(table);
   P.xnorm = take((size_t)n * 4);
+  P.xnorm_min = take((size_t)n * 4);
   P.q16 = take((size_t)c.query_rows * P.pd * 2);
   P.qnorm = take((size_t)nq * 4);
   P.info = take((size_t)nq * sizeof(QueryInfo));
@@ -508,6 +521,8 @@ int launch_flat_tc(const FlatTcPlan& P, const float* vectors, const uint32_t* ve
   p.x16 = reinterpret_cast<__half*>(base + P.x16);
   p.q16 = reinterpret_cast<__half*>(base + P.q16);
   p.xnorm = reinterpret_cast<float*>(base + P.xnorm);
+  p.xnorm_min = reinterpret_cast<float*>(base + P.xnorm_min);
+  p.mask = mask;
   p.qnorm = reinterpret_cast<float*>(base + P.qnorm);
   p.info = reinterpret_cast<QueryInfo*>(base + P.info);
   p.words = words;
@@ -540,6 +555,7 @@ int launch_flat_tc(const FlatTcPlan& P, const float* vectors, const uint32_t* ve
   TcCollect c = P.c;
   c.rows16 = p.x16;
   c.row_norms = p.xnorm;
+  c.row_norms_min = p.xnorm_min;
   c.q16 = p.q16;
   c.qnorm = p.qnorm;
   c.mask = mask;

@@ -164,7 +164,8 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
 // key of a full list (a list's entry 0, the sentinel when it is not full).
 struct TcCollect {
   const void* rows16;      // [n][padded_dim] fp16
-  const float* row_norms;  // [n]
+  const float* row_norms;  // [n] of the scan, and of the minima pass (a row may have part in one only)
+  const float* row_norms_min;
   uint32_t n, dim, padded_dim, nq;
   uint32_t rank, room;     // bound rank; rows per query that the lists should hold
   const void* q16;         // [query_rows][padded_dim] fp16, zero past nq
@@ -194,7 +195,7 @@ struct FlatTcPlan {
   TcCollect c{};
   FlatPlan f;        // the plain scan of the flagged queries
   // byte offsets in the scratch
-  size_t x16 = 0, xnorm = 0, q16 = 0, qnorm = 0, info = 0, mu = 0, var = 0, words = 0, collect = 0, plain = 0;
+  size_t x16 = 0, xnorm = 0, xnorm_min = 0, q16 = 0, qnorm = 0, info = 0, mu = 0, var = 0, words = 0, collect = 0, plain = 0;
 };
 FlatTcPlan plan_flat_tc(uint32_t n, uint32_t dim, uint32_t nq, uint32_t k, MetricType metric);
 int launch_flat_tc(const FlatTcPlan& plan, const float* vectors, const uint32_t* vec_ids, uint32_t n, uint32_t dim,

@@ -881,6 +881,7 @@ int launch_tc_collect(TcCollect& c, void* scratch, cudaStream_t stream) {
   };
   TcScanArgs p = a;
   p.splits = P.psplits;
+  p.xnorm = c.row_norms_min;
   p.run_stride = P.pstride;
   p.pmin = reinterpret_cast<float*>(c.partial);
   p.pm_stride = P.pcount;

@@ -627,3 +627,55 @@ def test_select_with_more_keys_than_foreseen_by_runs(cuda):
     torch.cuda.synchronize()
     assert scan.device_status() == 0
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("metric", ["l2", "ip", "cosine"])
+@pytest.mark.parametrize("data", ["normal", "integers", "sorted", "nan row", "inf rows", "far rows", "masked far row",
+                                  "zero row"])
+def test_filtered_flat_scan_answers_by_itself(cuda, metric, data):
+    """The filter proves nearly every query of a call, rows that are not finite or
+    far outside the others' scale among the base or not: the plain scan of the
+    flagged queries takes a small part of the plain scan's time (a twentieth as
+    a rule; the limit is a half)."""
+    from fvgb300 import scan
+
+    torch = cuda
+    n, dim, nq = 60_000, 128, 512
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn((n, dim), generator=g, device="cuda")
+    q = torch.randn((nq, dim), generator=g, device="cuda")
+    mask = None
+    if data == "integers":
+        x, q = (x * 20).round(), (q * 20).round()
+    elif data == "sorted":
+        x = x[torch.argsort((x - q[0]).square().sum(1))]
+    elif data == "nan row":
+        x[777, 3] = float("nan")
+    elif data == "inf rows":
+        x[777, 3], x[20_001] = float("inf"), -float("inf")
+    elif data == "far rows":
+        x[777] *= 1000.0
+        x[20_001:20_020] *= 3e6
+    elif data == "masked far row":
+        x[777] *= 1000.0
+        mask = torch.full(((n + 31) // 32,), -1, dtype=torch.int32, device="cuda")
+        mask[777 // 32] &= ~(1 << (777 % 32))
+    elif data == "zero row":
+        x[777] = 0.0
+    run = lambda: scan.flat_scan(x, q, 10, metric, mask=mask)
+    res = {}
+    for knob in (0, 1):
+        with scan.tuned(flat_tc=knob):
+            run()
+            torch.cuda.synchronize()
+            scan.profile_enable(True)
+            try:
+                scan.profile_summary()
+                out = run()
+                torch.cuda.synchronize()
+                res[knob] = out, scan.profile_summary()
+            finally:
+                scan.profile_enable(False)
+    assert torch.equal(res[1][0], res[0][0])
+    assert "flat_tc_prep" in res[1][1] and "flat_tc_prep" not in res[0][1]
+    assert res[1][1]["flat_f32_scan"]["ms"] < 0.5 * res[0][1]["flat_f32_scan"]["ms"]
