@@ -88,8 +88,8 @@ __device__ __forceinline__ uint16_t f32_to_f16_halfup_fast(float v) {
 // advance together: with one lane per row reading its row alone, 500,000 x 768
 // took 2,221 us. Eight rows a warp rather than 32 keep small tables in enough
 // warps (10,357 x 633: 37 us at the start, 172 us with 32 rows a warp).
-constexpr int E16_WARPS = 8, E16_ROWS = 8, E16_DIMS = 128;
-template <bool VEC>
+constexpr int E16_WARPS = 8, E16_DIMS = 128;
+template <bool VEC, int E16_ROWS>
 __global__ void __launch_bounds__(32 * E16_WARPS, 3) encode_fp16_kernel(const float* __restrict__ x, uint32_t n,
                                                                         uint32_t dim, uint32_t pd,
                                                                         uint16_t* __restrict__ out,
@@ -204,54 +204,72 @@ __device__ __forceinline__ void neumaier_halve(float* sum, float* comp, int o, i
 
 // ||x||^2 of each row (compensated), and the largest of them as ordered
 // bits in *max_bits (norms are >= 0, so the bit patterns order like the values).
-// Bound by the read of the table: a warp takes eight rows at a time (eight
+// Bound by the read of the table: a warp takes R = 8 rows at a time (eight
 // loads in flight, and three of the five steps across the lanes shared by all
 // eight) and raises the maximum once for all its rows: 47 us for 328,756 x 157.
 // With a row and an atomic on one word per warp the whole encoder took 307 us
 // there and takes 120 (500,000 x 768: 972 and 612 us; two reads and the write
-// at the measured copy rate: 510).
-constexpr int F8_ROWS = 8;
+// at the measured copy rate: 510). Tables of fewer and longer rows, whose warps
+// of eight rows would not fill the GPU, take two rows or one a warp and as many
+// loads in flight.
+template <int R>
 __global__ void __launch_bounds__(256) fp8_norms_kernel(const float* __restrict__ x, uint32_t n, uint32_t dim,
                                                         float* __restrict__ norms, uint32_t* __restrict__ max_bits) {
+  constexpr int B = 8 / R, LPR = 32 / R;  // loads of a row in flight; lanes that end with a row
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   const int lane = threadIdx.x & 31;
   uint32_t top = 0;
-  for (uint64_t row0 = (uint64_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * F8_ROWS; row0 < n;
-       row0 += (uint64_t)warps * F8_ROWS) {
-    float sum[F8_ROWS], comp[F8_ROWS];
-    const float* src[F8_ROWS];
+  for (uint64_t row0 = (uint64_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * R; row0 < n;
+       row0 += (uint64_t)warps * R) {
+    float sum[R], comp[R];
+    const float* src[R];
 #pragma unroll
-    for (int r = 0; r < F8_ROWS; ++r) {
+    for (int r = 0; r < R; ++r) {
       sum[r] = comp[r] = 0.f;
       src[r] = x + min(row0 + r, (uint64_t)n - 1) * dim;
     }
-    // (the next 32 dimensions of every row are in flight while these are added)
-    float v[F8_ROWS];
+    // (the next 32 B dimensions of every row are in flight while these are added)
+    auto load = [&](float (&v)[R][B], uint32_t d) {
 #pragma unroll
-    for (int r = 0; r < F8_ROWS; ++r) v[r] = (uint32_t)lane < dim ? __ldg(src[r] + lane) : 0.f;
-    for (uint32_t d = lane; d < dim; d += 32) {
-      float w[F8_ROWS];
+      for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int r = 0; r < F8_ROWS; ++r) w[r] = d + 32 < dim ? __ldg(src[r] + d + 32) : 0.f;
+        for (int b = 0; b < B; ++b) v[r][b] = d + 32 * b < dim ? __ldg(src[r] + d + 32 * b) : 0.f;
+    };
+    float v[R][B];
+    load(v, lane);
+    for (uint32_t d = lane; d < dim; d += 32 * B) {
+      float w[R][B];
+      load(w, d + 32 * B);
 #pragma unroll
-      for (int r = 0; r < F8_ROWS; ++r) neumaier_add(sum[r], comp[r], __fmul_rn(v[r], v[r]));
+      for (int b = 0; b < B; ++b) {
+        if (b && d + 32 * b >= dim) break;
 #pragma unroll
-      for (int r = 0; r < F8_ROWS; ++r) v[r] = w[r];
+        for (int r = 0; r < R; ++r) neumaier_add(sum[r], comp[r], __fmul_rn(v[r][b], v[r][b]));
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int b = 0; b < B; ++b) v[r][b] = w[r][b];
     }
     __syncwarp();
-    neumaier_halve<4>(sum, comp, 16, lane);
-    neumaier_halve<2>(sum, comp, 8, lane);
-    neumaier_halve<1>(sum, comp, 4, lane);
+    if constexpr (R == 8) {
+      neumaier_halve<4>(sum, comp, 16, lane);
+      neumaier_halve<2>(sum, comp, 8, lane);
+      neumaier_halve<1>(sum, comp, 4, lane);
+    } else {
+      static_assert(R <= 2, "eight rows, two or one");
+      if constexpr (R == 2) neumaier_halve<1>(sum, comp, 16, lane);
+    }
 #pragma unroll
-    for (int o = 2; o > 0; o >>= 1) {
+    for (int o = LPR / 2; o > 0; o >>= 1) {
       const float os = __shfl_xor_sync(0xffffffffu, sum[0], o);
       const float oc = __shfl_xor_sync(0xffffffffu, comp[0], o);
       neumaier_add(sum[0], comp[0], os);
       comp[0] += oc;
     }
-    // row r's sum is lane 4 r's
-    const uint64_t row = row0 + (lane >> 2);
-    if ((lane & 3) == 0 && row < n) {
+    // row r's sum is lane LPR r's
+    const uint64_t row = row0 + lane / LPR;
+    if (lane % LPR == 0 && row < n) {
       const float nrm = sum[0] + comp[0];
       norms[row] = nrm;
       if (nrm > 0.f) top = max(top, __float_as_uint(nrm));
@@ -278,12 +296,12 @@ __device__ __forceinline__ float e4m3_value(uint8_t c) {
   return (c & 0x80u) ? -mag : mag;
 }
 
-// A warp encodes eight rows as one run of 4-byte words (rows are stored one
-// after the other), so that no lane is idle at any width; each of the first
-// eight lanes makes one row's norm digits. Bound by the read of the rows: the
+// A warp encodes its rows (as many as in the norms' pass) as one run of 4-byte
+// words (rows are stored one after the other), so that no lane is idle at any
+// width; lane r makes row r's norm digits. Bound by the read of the rows: the
 // grid goes from the last row to the first, as the norms' pass has just left
 // the last ones in L2 (66 us for 328,756 x 157).
-template <bool VEC>
+template <bool VEC, int F8_ROWS>
 __global__ void __launch_bounds__(256) encode_fp8_kernel(const float* __restrict__ x, uint32_t n, uint32_t dim,
                                                          uint32_t pd, uint8_t* __restrict__ out,
                                                          float* __restrict__ scales,
@@ -393,13 +411,19 @@ __global__ void __launch_bounds__(256) encode_fp8_per_vector_kernel(const float*
 int launch_encode_fp16(const float* x, uint32_t n, uint32_t dim, uint32_t pd, uint16_t* out, float* norms,
                        cudaStream_t stream) {
   if (n == 0) return 0;
-  const uint64_t blocks = ((uint64_t)n + E16_ROWS * E16_WARPS - 1) / (E16_ROWS * E16_WARPS);
   // 16-byte loads and 8-byte stores where every row starts on such a boundary
   const bool vec = dim % 4 == 0 && pd % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)out % 8 == 0;
-  if (vec)
-    encode_fp16_kernel<true><<<(unsigned)blocks, 32 * E16_WARPS, 0, stream>>>(x, n, dim, pd, out, norms);
+  auto go = [&](auto kern, uint64_t rows) {
+    const uint64_t blocks = ((uint64_t)n + rows * E16_WARPS - 1) / (rows * E16_WARPS);
+    kern<<<(unsigned)blocks, 32 * E16_WARPS, 0, stream>>>(x, n, dim, pd, out, norms);
+  };
+  // two rows a warp for a few long ones, whose warps of eight would leave most of
+  // the GPU idle (1,000 x 4,096: 63 us with eight, 30 with two; 10,000 x 1,024: 26
+  // and 24; 20,000 x 1,536: 45 and 52)
+  if (dim >= 512 && n < 64 * (uint32_t)device_sm_count())
+    vec ? go(encode_fp16_kernel<true, 2>, 2) : go(encode_fp16_kernel<false, 2>, 2);
   else
-    encode_fp16_kernel<false><<<(unsigned)blocks, 32 * E16_WARPS, 0, stream>>>(x, n, dim, pd, out, norms);
+    vec ? go(encode_fp16_kernel<true, 8>, 8) : go(encode_fp16_kernel<false, 8>, 8);
   note_launch();
   return (int)cudaGetLastError();
 }
@@ -407,18 +431,29 @@ int launch_encode_fp16(const float* x, uint32_t n, uint32_t dim, uint32_t pd, ui
 int launch_encode_fp8(const float* x, uint32_t n, uint32_t dim, uint32_t pd, uint8_t* out, float* scales,
                       float* norms, cudaStream_t stream) {
   if (n == 0) return 0;
-  // eight warps of eight rows a block; the norms' blocks stay and go on to further rows
-  const uint64_t blocks = ((uint64_t)n + 8 * F8_ROWS - 1) / (8 * F8_ROWS);
   uint32_t* word = reinterpret_cast<uint32_t*>(scales);
   cudaError_t e = cudaMemsetAsync(word, 0, sizeof(uint32_t), stream);
   if (e != cudaSuccess) return (int)e;
-  const uint64_t stay = (uint64_t)device_sm_count() * 8;
-  fp8_norms_kernel<<<(unsigned)(blocks < stay ? blocks : stay), 256, 0, stream>>>(x, n, dim, norms, word);
-  fp8_table_scale_kernel<<<1, 1, 0, stream>>>(word);
-  if (dim % 4 == 0 && (uintptr_t)x % 16 == 0)
-    encode_fp8_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(x, n, dim, pd, out, scales, norms);
+  const bool vec = dim % 4 == 0 && (uintptr_t)x % 16 == 0;
+  const uint64_t sms = (uint64_t)device_sm_count();
+  auto go = [&](auto norms_kern, auto kern, uint64_t rows) {
+    // eight warps a block; the norms' blocks stay and go on to further rows
+    const uint64_t blocks = ((uint64_t)n + 8 * rows - 1) / (8 * rows);
+    norms_kern<<<(unsigned)(blocks < 8 * sms ? blocks : 8 * sms), 256, 0, stream>>>(x, n, dim, norms, word);
+    fp8_table_scale_kernel<<<1, 1, 0, stream>>>(word);
+    kern<<<(unsigned)blocks, 256, 0, stream>>>(x, n, dim, pd, out, scales, norms);
+  };
+  // Eight rows a warp for short rows, which have the fewest steps to share the
+  // sums over, and for tables that fill the GPU so (80,000 x 96: 35 us, 46 with
+  // two a warp; 160,000 x 384: 125 and 136). Else two (40,000 x 768: 85 and 72 us;
+  // 20,000 x 1,536: 91 and 68; 10,000 x 1,024: 44 and 36), and one for a few rows
+  // (1,000 x 4,096: 93 us with eight, 36 with two, 29 with one).
+  if (dim < 256 || n >= 640 * sms)
+    vec ? go(fp8_norms_kernel<8>, encode_fp8_kernel<true, 8>, 8) : go(fp8_norms_kernel<8>, encode_fp8_kernel<false, 8>, 8);
+  else if (n >= 32 * sms)
+    vec ? go(fp8_norms_kernel<2>, encode_fp8_kernel<true, 2>, 2) : go(fp8_norms_kernel<2>, encode_fp8_kernel<false, 2>, 2);
   else
-    encode_fp8_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(x, n, dim, pd, out, scales, norms);
+    vec ? go(fp8_norms_kernel<1>, encode_fp8_kernel<true, 1>, 1) : go(fp8_norms_kernel<1>, encode_fp8_kernel<false, 1>, 1);
   note_launch(3);
   return (int)cudaGetLastError();
 }

@@ -679,3 +679,42 @@ def test_filtered_flat_scan_answers_by_itself(cuda, metric, data):
     assert torch.equal(res[1][0], res[0][0])
     assert "flat_tc_prep" in res[1][1] and "flat_tc_prep" not in res[0][1]
     assert res[1][1]["flat_f32_scan"]["ms"] < 0.5 * res[0][1]["flat_f32_scan"]["ms"]
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 63, 65])
+@pytest.mark.parametrize("dim,pd", [(127, 128), (128, 144), (129, 144), (132, 144), (120, 272), (256, 256), (300, 304),
+                                    (511, 512), (512, 512), (768, 768), (1031, 1040)])
+def test_encode_fp16_chunks(cuda, oracle_mod, n, dim, pd):
+    """Rows of several 128-dimension chunks, full and partial, as 16-byte loads and
+    single values, two rows a warp (from 512 dimensions) and eight: the norms'
+    sums go on across chunks; padding that reaches a chunk past the row."""
+    from fvgb300 import scan
+
+    torch = cuda
+    rng = np.random.default_rng(n * 131 + dim)
+    x = (rng.standard_normal((n, dim)) * np.exp(rng.uniform(-8, 8, (n, 1)))).astype(np.float32)
+    codes, norms = scan.encode_fp16(torch.from_numpy(x).cuda(), pd)
+    ref_codes, ref_norms = oracle_mod.encode_fp16_padded(x)
+    got = codes.cpu().numpy().view(np.uint16)
+    assert np.array_equal(got[:, :dim], ref_codes[:, :dim])
+    assert not got[:, dim:].any()
+    assert np.array_equal(norms.cpu().numpy().view(np.uint32), ref_norms.view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [1, 3, 8, 200])
+@pytest.mark.parametrize("dim", [255, 256, 263, 768, 1000])
+def test_encode_fp8_rows_a_warp(cuda, n, dim):
+    """One row a warp gives the codes, scale and norms, bit for bit, that two
+    (the same rows at the head of a table of 20,000) and eight (of 100,000) give."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(n + dim)
+    x = torch.randn((n, dim), generator=g, device="cuda")
+    few = scan.encode_fp8(x)
+    for total in (20_000, 100_000):
+        big = torch.zeros((total, dim), device="cuda")
+        big[:n] = x
+        many = scan.encode_fp8(big)
+        for a, b in zip(few, many):
+            assert torch.equal(a, b[:n])
