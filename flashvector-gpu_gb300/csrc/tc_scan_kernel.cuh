@@ -468,7 +468,11 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
     // kCosPad of the distance 1 + v / |q| (the factors' few ulps, and 1e-8
     // against 0.01), so v <= cthr, raised by it, admits every candidate and
     // the exact distance is evaluated for those alone. Nor does |q|^2 |x|^2
-    // overflow for any of them: the distance would then be 1 at every angle.
+    // overflow for any of them: the distance would then be 1 at every angle. Rows
+    // of zeros, whose distance is 1 too, have the factor 0 (|x|^2 underflows below
+    // |x| = 1e-22: with |q| < 1e8 the dot is then nothing against the 1e-8). (600,000
+    // x 64 with a row of zeros in most tiles, 200 queries: 626 us without that,
+    // 225 with it.)
     constexpr float kCosPad = 4e-6f;
     const float q_over = METRIC == METRIC_COSINE ? sqrtf(qn) / (FP8 ? qs : 1.f) : 1.f;
     const float q_inv = METRIC == METRIC_COSINE ? __fdiv_rn(1.f, q_over) : 1.f;
@@ -559,10 +563,12 @@ __global__ void __launch_bounds__(scan_threads(G), 1)
         if (METRIC != METRIC_INNER_PRODUCT && !fused) cb[lane + 32 * r] = pre_n[r];
         if (FP8 && !fused) cb[TC_N + lane + 32 * r] = pre_s[r];
         if (METRIC == METRIC_COSINE) {
-          cf[lane + 32 * r] = -rsqrtf(pre_n[r]) * (FP8 ? pre_s[r] : 1.f);
-          // (a NaN passes: it has no distance either way)
+          // (a row of zeros has the distance 1, the factor 0; a NaN passes, as it has
+          // no distance either way)
+          const bool zero = pre_n[r] == 0.f;
+          cf[lane + 32 * r] = zero ? 0.f : -rsqrtf(pre_n[r]) * (FP8 ? pre_s[r] : 1.f);
           if (MINP || v0 + lane + 32 * r < a.n)
-            by_factor = by_factor && !(pre_n[r] * q_least < 1e-4f) && !(pre_n[r] * q_most >= 1e38f);
+            by_factor = by_factor && (zero ? q_most < 1e16f : !(pre_n[r] * q_least < 1e-4f) && !(pre_n[r] * q_most >= 1e38f));
         }
       }
       if (METRIC == METRIC_COSINE) by_factor = __all_sync(0xffffffffu, by_factor);

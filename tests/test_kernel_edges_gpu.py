@@ -718,3 +718,28 @@ def test_encode_fp8_rows_a_warp(cuda, n, dim):
         many = scan.encode_fp8(big)
         for a, b in zip(few, many):
             assert torch.equal(a, b[:n])
+
+
+@pytest.mark.parametrize("precision", ["fp16", "fp8", "fp8_rows"])
+@pytest.mark.parametrize("scale", [1.0, 1e-9, 1e9])
+def test_cosine_bound_with_rows_of_zeros(cuda, precision, scale):
+    """Zero rows (distance 1) among the base, queries of any scale and a zero
+    query: the bounded scan returns what the scan without a bound returns, also
+    where the zero rows are among the answer."""
+    from fvgb300 import scan
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(12)
+    x = torch.randn((9_000, 64), generator=g, device="cuda")
+    x[::7] = 0.0
+    q = torch.randn((150, 64), generator=g, device="cuda") * scale
+    q[::10] = -x[1].abs() * scale
+    x[1::2] = x[1::2].abs()
+    q[5] = 0.0
+    t = _fp_table(scan, precision, x)
+    search = scan.fp16_search if precision == "fp16" else scan.fp8_search
+    with scan.tuned(tc_prepass=0):
+        ref = search(t, q, 10, "cosine")
+    got = search(t, q, 10, "cosine")
+    torch.cuda.synchronize()
+    assert torch.equal(got, ref)
