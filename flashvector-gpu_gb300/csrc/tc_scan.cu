@@ -166,10 +166,9 @@ struct SelectArgs {
   GpuSearchResult* out;
   uint32_t* status;
   const float* tau;          // per-query admission bound of the scan (null: none)
-  uint32_t* redo;            // set for a bounded query with fewer than redo_below keys
+  uint32_t* redo;            // set for a bounded query that kept too few keys
   const uint32_t* only;      // process only the flagged queries (null: all)
   uint32_t* incomplete_q;    // per-query flag set when a range heap may have dropped keys (or null)
-  uint32_t redo_below;       // (<= shortlist)
 };
 
 constexpr int BAND_MAX = 64;
@@ -222,7 +221,8 @@ __global__ void __launch_bounds__(NT) tc_select_kernel(SelectArgs s) {
   }
   // a bounded scan kept too few rows (see plan_tc_scan): the query is scanned
   // again unbounded
-  if (s.redo && threadIdx.x == 0 && keys[min(kp, s.redo_below) - 1] == kSentinelKey && s.tau[q] < kSentinelDist)
+  if (s.redo && threadIdx.x == 0 && keys[kp - 1] == kSentinelKey && s.tau[q] < kSentinelDist &&
+      (!incomplete || keys[min(s.k, kp) - 1] == kSentinelKey))
     s.redo[q] = 1u;
 
   const float* qv = s.queries + (size_t)q * s.dim;
@@ -572,11 +572,11 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   // r = shortlist (the same accumulators, hence the same distances, are
   // behind the bound and the scan). The scan then admits only rows within it.
   // Queries whose bounded scan comes up short are scanned again without the
-  // bound (device-side, no host round trip). After a sample (s > 1) that is
-  // fewer keys than the shortlist, as its bound may be too tight. With s = 1
-  // keys are missing only where a range's list, which then holds less than the
-  // shortlist, filled up (rows that the base's order puts into one tile; the
-  // scan without a bound loses the same rows): fewer than k.
+  // bound (device-side, no host round trip): the bound was too tight (s > 1), or a
+  // range's list, which holds less than the shortlist where that is above 48 or
+  // 64, filled up (rows that the base's order puts into one tile). The scan without
+  // a bound loses the same rows to a full list, so that one is no reason while
+  // there are k keys.
   //
   // Automatic stride. Long rows are bound by the MMA, whose pass costs 1 / s
   // of the scan again: 64 sampled tiles. Short rows (at most two K blocks)
@@ -597,7 +597,11 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   const size_t part_bytes = align_up((size_t)nq * splits * groups * kl * 8, 256);
   // The coarsest minima (fewest to store and to select from) that still number
   // 8 r, so that two of a query's r best rows seldom share one: with c minima the
-  // bound admits about -c ln(1 - r / c) rows, 1.07 r for 8 r and 1.4 r for 2 r.
+  // bound admits about -c ln(1 - r / c) rows, 1.07 r for 8 r and 1.4 r for 2 r. Up
+  // to 512, which cost nothing to select from, 32 r: a minimum of 128 columns
+  // holds eight neighbours of a run, which a base in order of distance all has
+  // among the best (60,000 x 128 in order of norm, 200 queries, L2, k 10: 290 us a
+  // call with 8 r, 208 so).
   // They live in the space of the range heaps, which are written after the bound
   // is known: a call takes no more scratch than its unbounded scan. Where 8 r do
   // not fit there, the most that fit down to 2 r; where those do not either, the
@@ -610,7 +614,7 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
                                             : (pstride == 1 ? ranked : poisson_rank((double)ranked / pstride, 1e-7)));
     for (uint32_t g = 128; g >= 8 && !pgran; g >>= 1) {
       const uint32_t c = psampled * (TC_N / g);
-      if ((c >= 8 * pr || g == 8) && (size_t)nq * c * 4 <= part_bytes) {
+      if ((c >= std::max(8 * pr, std::min(32 * pr, 512u)) || g == 8) && (size_t)nq * c * 4 <= part_bytes) {
         pgran = g;
         pcount = c;
       }
@@ -797,7 +801,6 @@ int launch_tc_scan_planned(const TcPlan& P, const TcTables& t, const float* quer
   SelectArgs s{partial, splits * groups, kl, sel_keys, shortlist, k, queries, t.vectors, t.dim,
                (int)metric,
                opt.boundary_fp64 ? 1u : 0u, 0.f, out, status_word(), tau, redo, nullptr, incomplete_q};
-  s.redo_below = P.pstride > 1 ? shortlist : k;
   s.eps = opt.boundary_eps > 0.f ? opt.boundary_eps : (float)((t.dim + 31) / 32 + 5) * 2.0f * 5.960464477539063e-08f;
   size_t sel_smem = (size_t)sel_keys * 8;
   const int sel_threads = nq <= 2u * (uint32_t)device_sm_count() ? 1024 : 256;
