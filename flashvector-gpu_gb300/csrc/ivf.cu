@@ -419,7 +419,7 @@ __device__ __forceinline__ float adc_words(const float* __restrict__ lut, const 
 // PQ: ADC of one row without tables: the entry of each sub-space evaluated in
 // place with the table's operations (the residual to the list's centroid
 // rounded once per dimension, fmaf in sub-dimension order), added in sub-space
-// order. Eight sub-spaces' codewords are in flight at a time where rows of
+// order. Four sub-spaces' codewords are in flight at a time where rows of
 // four dimensions load as float4 (v4).
 template <typename CodeAt>
 __device__ __forceinline__ float adc_direct(const IvfArgs& a, const float* qs, const float* __restrict__ cent,
@@ -486,7 +486,12 @@ __device__ __forceinline__ float sq8_row(const float* qs, const float* __restric
 //   PIPE: 32 dimensions at a time, the next ones copied while these are scored,
 // which is what a call of few warps waits for (8 queries x 64 lists of 768
 // dimensions 268 -> 232 us). Rows may start at any byte: words are copied
-// aligned and shifted into place (397 dimensions, 300 queries: 2,588 -> 2,239).
+// aligned and shifted into place (397 dimensions, 300 queries: 2,588 -> 2,239). A
+// word that holds a row's first or last byte is copied whole, so that up to 3
+// bytes before and behind the table are read with it, and dropped; a word never
+// crosses into another page or allocation. (Copying only a row's bytes of each word, by
+// cp.async's source size, costs up to 15%: 100 dimensions, 3,000 queries: 2,167 us a
+// call, 2,544.)
 //   Otherwise 16-byte-aligned rows, 64 dimensions at a time: fewer steps, for
 // calls whose warps cover each other's loads (2,000 queries, 128 dimensions:
 // 2,721 us, and 3,081 with PIPE).

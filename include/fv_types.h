@@ -61,7 +61,9 @@ typedef struct {
     const float* d_centroids;      /* [nlist * dim]                              */
     const float* d_sq_mins;        /* [dim] per-dimension residual minimum       */
     const float* d_sq_scales;      /* [dim] per-dimension step (range / 255)     */
-    const uint8_t* d_sq_codes;     /* [num_vectors * dim] indexed by vector id   */
+    const uint8_t* d_sq_codes;     /* [num_vectors * dim] indexed by vector id; read
+                                      by whole 4-byte words: up to 3 bytes of the
+                                      words that hold its first and last byte     */
     const uint32_t* d_ivf_offsets; /* [nlist + 1]                                */
     const uint32_t* d_ivf_vec_ids; /* [num_vectors]                              */
     const float* d_vectors;        /* [num_vectors * dim] fp32 rows for rerank   */
