@@ -629,9 +629,19 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
     if (pgran || psampled < 64) break;
     pstride *= 2;
   }
-  // off where the base is so small that the minima cannot bound (the heaps
-  // then hold about every row anyway); the knob turns it off anywhere
-  const bool prepass = pp_knob != 0 && pgran && pcount >= 2 * pr;
+  // Off where the base is so small that the minima cannot bound (the heaps then
+  // hold about every row anyway), and where the heaps of a few keys, with the bound
+  // that ranges share, cost less than the pass (us a call with and without it):
+  // shortlists of 4 for one or two queries, which fill one lane (100,000 x 768: 78
+  // and 61; 300,000 x 64: 56 and 50), of 8 there over long rows of larger bases (78
+  // and 68), and of 4 for many queries over larger bases (866 of 300,000 x 156, half
+  // masked: 225 and 189; 1M x 64: 299 and 274; for 128 queries it is 61 and 111).
+  // The knob turns it off, or on, anywhere.
+  const bool long_rows = kblocks > 2, one_lane = nq <= 2, many = nqb >= 4;
+  const bool quick = !rank && ((shortlist <= 4 && ((one_lane && (long_rows || ntiles >= 1024)) ||
+                                                   (many && ntiles >= (long_rows ? 256u : 2048u)))) ||
+                               (shortlist <= 8 && one_lane && long_rows && ntiles >= 256));
+  const bool prepass = pp_knob != 0 && (pp_knob > 0 || !quick) && pgran && pcount >= 2 * pr;
   psampled = std::max(1u, psampled);
   uint32_t psplits = std::max<uint32_t>(1u, std::min<uint32_t>((uint32_t)sms / nqb_grid, psampled));
   psplits = fill_waves(psplits, nqb_grid, psampled, (uint32_t)sms, 0);
