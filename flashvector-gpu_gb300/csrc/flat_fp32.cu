@@ -638,9 +638,9 @@ cudaError_t noalloc_scratch_address(uint64_t** out) {
 }
 }  // namespace
 
-// Same work split and kernels as launch_flat_f32, with the per-split heaps
-// in the fixed array; refuses (FV_ERR_SCRATCH_LIMIT) a call whose heaps
-// would not fit instead of allocating.
+// Same work split and kernels as launch_flat_f32's plain scan (never the
+// tensor-core filter), with the per-split lists in the fixed array; refuses
+// (FV_ERR_SCRATCH_LIMIT) a call whose lists would not fit instead of allocating.
 int launch_flat_f32_noalloc(const float* vectors, const uint32_t* vec_ids, uint32_t n, uint32_t dim,
                             const float* queries, uint32_t nq, uint32_t k, MetricType metric, const uint32_t* mask,
                             GpuSearchResult* out, cudaStream_t stream) {

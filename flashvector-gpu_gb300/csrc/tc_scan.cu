@@ -22,7 +22,7 @@
 //             matrix ever reaches HBM.
 // A call first finds a bound per query from column minima (of a sample of the
 // base, or of all of it) and then scans with it: a range's few keys under the
-// bound are appended to its list. A CTA scans a contiguous range of base tiles;
+// bound are appended to its list. A CTA scans a range of base tiles, every so many;
 // the lists are merged by tc_select_kernel, which also rescores them in fp32.
 #include <cmath>
 #include <cuda_fp16.h>
@@ -471,7 +471,7 @@ const TuneEntry* tune_lookup(bool fp8, int metric, uint32_t dim, uint64_t n, uin
   return nullptr;
 }
 
-// Sampled rank for the pre-pass bound. A sample of every stride-th tile
+// Sampled rank for the pre-pass bound. A sample of every stride-th run of rows
 // holds each of a query's top (shortlist - 1) rows with probability
 // 1 / stride, so the number of them in the sample is about Poisson(lambda =
 // shortlist / stride); the sample's r-th best distance is below the query's
@@ -563,7 +563,7 @@ TcPlan plan_tc_scan(const TcTables& t, uint32_t nq, uint32_t k, MetricType metri
   splits = (ntiles + tps - 1) / tps;
 
   // Pre-pass: each query's admission bound for the scan, from the minima pass
-  // over every pstride-th tile. A sample of stride s holds each of the
+  // over every pstride-th run of 8 rows. A sample of stride s holds each of the
   // query's top (shortlist - 1) rows with probability 1 / s; the bound is the
   // r-th smallest minimum, r from the Poisson tail below (or ceil(margin *
   // shortlist / stride) when the margin knob is set), and the sampled r-th

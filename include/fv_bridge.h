@@ -333,8 +333,9 @@ int fv_profile_summary(char* buf, size_t len);
  *                       tensor-core scans first find a per-query admission
  *                       bound from the minima of a strided sample of the
  *                       base (all of it where it is small); bases too small
- *                       to bound are scanned without
- *   "tc.prepass_stride" sample stride in 256-row tiles (0 automatic: the
+ *                       to bound are scanned without, as are (automatic)
+ *                       a few keys for one or two queries or for many
+ *   "tc.prepass_stride" sample stride in runs of 8 rows (0 automatic: the
  *                       tuned value, else 1 to 32 growing with the base);
  *                       raised where the sample's minima would not fit the
  *                       scan's scratch
